@@ -78,9 +78,6 @@ struct csm_ctx {
   bool has_graph = false;
   DevGraph g{};
   std::vector<uint32_t> h_vlabel;  // folded vertex labels (kNone: no vertex), mirrored on the host
-  // edge table (DevGraph::ekeys): upper bounds of its live keys and deleted
-  // slots, from the updates submitted since it was last filled
-  uint64_t e_live = 0, e_tomb = 0;
   uint64_t num_edges = 0;
   // candidate index
   IndexState index{};
@@ -92,9 +89,9 @@ struct csm_ctx {
   UpdInfo* d_info = nullptr;
   uint64_t *d_ins = nullptr, *d_ins2 = nullptr, *d_del = nullptr, *d_del2 = nullptr;
   uint64_t *d_tk = nullptr, *d_tk2 = nullptr, *d_ts = nullptr, *d_ts2 = nullptr;
-  VRange *d_rins = nullptr, *d_rdel = nullptr, *d_rt = nullptr;
+  VRange *d_rins = nullptr, *d_rdel = nullptr;
   uint32_t* d_ins_dst = nullptr;
-  unsigned int* d_cnt = nullptr;  // [0] n_ins [1] n_del [2] n_t [3] n_rins [4] n_rdel [5] n_rt [6] n_tasks [7] task_next
+  unsigned int* d_cnt = nullptr;  // [0] n_ins [1] n_del [2] n_t [3] n_rins [4] n_rdel [6] n_tasks [7] task_next
   Task* d_tasks = nullptr;
   unsigned long long *d_count = nullptr, *d_hash = nullptr, *d_bytes = nullptr;
   unsigned int* d_stop = nullptr;
@@ -262,6 +259,7 @@ static int build_plan(csm_ctx* ctx) {
         if (nb_total >= kMaxQE || pp.nb >= kMaxBack) return set_err(CSM_EUNSUPPORTED, "query too dense");
         A.back_pos[nb_total] = (uint8_t)j;
         A.back_combo[nb_total] = (uint16_t)(ctx->qvl_f[o[d]] * n_el + l);
+        A.back_el[nb_total] = (uint8_t)l;
         nb_total++; pp.nb++;
       }
       if (pp.nb == 0) return set_err(CSM_EINVAL, "query graph is not connected");
@@ -299,7 +297,6 @@ static int ensure_batch_buffers(csm_ctx* ctx) {
   AL(ctx->d_tk, 8ull * L); AL(ctx->d_tk2, 8ull * L);
   AL(ctx->d_ts, 8ull * L); AL(ctx->d_ts2, 8ull * L);
   AL(ctx->d_rins, sizeof(VRange) * (size_t)L); AL(ctx->d_rdel, sizeof(VRange) * (size_t)L);
-  AL(ctx->d_rt, sizeof(VRange) * (size_t)L);
   AL(ctx->d_ins_dst, 4ull * L);
   AL(ctx->d_cnt, 64);
   AL(ctx->d_tasks, sizeof(Task) * (size_t)ctx->task_cap);
@@ -411,10 +408,8 @@ static int batch_mutate_insert(csm_ctx* ctx, const csm_update* ups, uint32_t B, 
   CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, ctx->d_tk, ctx->d_tk2, ctx->d_ts, ctx->d_ts2, (int)L, 0, end_bit, st));
   k_ranges<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_ins2, L, kb, ctx->d_rins, c + 3, g.dir, g.nc); CKL();
   k_ranges<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_del2, L, kb, ctx->d_rdel, c + 4, g.dir, g.nc); CKL();
-  k_ranges<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_tk2, L, kb, ctx->d_rt, c + 5, g.dir, g.nc); CKL();
   g.t_key = ctx->d_tk2;
   g.t_span = reinterpret_cast<int2*>(ctx->d_ts2);
-  k_temporal_set<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_rt, c + 5, g); CKL();
   // CSR -> union graph (relocating rows, and compacting the pools first if needed)
   k_reloc_need<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_rins, c + 3, g); CKL();
   k_compact_check<<<1, 1, 0, st>>>(g); CKL();
@@ -424,20 +419,42 @@ static int batch_mutate_insert(csm_ctx* ctx, const csm_update* ups, uint32_t B, 
   launch_mut_insert(ctx->d_rins, c + 3, ctx->d_ins2, ctx->d_ins_dst, g, mut_blocks, (uint32_t)ctx->sm_count * 2, st);
   CKL();
   ctx->launches++;
-  if (g.emask) { k_edge_list<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_ins2, L, g, 0u); CKL(); }
+  g.t_mask = temporal_slots(B) - 1;
+  CK(cudaMemsetAsync(g.t_tab, 0xff, sizeof(ulonglong2) * (size_t)(g.t_mask + 1), st));
+  k_temporal_set<<<blocks_for(L, 256), 256, 0, st>>>(L, g); CKL();
   return CSM_OK;
+}
+
+// Instantiation of the search a context's batches run (search_max_blocks).
+static int search_mode_of(const csm_ctx* q) {
+  return q->d_enum ? 1 : ((!q->cfg.want_hash && !q->cfg.tail_enumerate) ? 2 : 0);
+}
+
+static void set_search_shape(SearchParams& sp, const Plan& plan) {
+  const SearchShape s = search_shape_of(plan, search_mode(sp));
+  sp.levels = s.levels;
+  sp.warp_bytes = s.warp_bytes;
+}
+
+// The configured warps per block (8 by default; fewer where the levels of that
+// many walks do not fit in a block's shared memory) and blocks per SM (by
+// default as many as can be resident).
+static void search_fit(const csm_ctx* q, const SearchShape& shape, int mode, uint32_t& warps, uint32_t& bps) {
+  warps = q->cfg.warps_per_block ? q->cfg.warps_per_block : 8;
+  if (warps != 4 && warps != 8 && warps != 16) warps = 8;
+  uint32_t resident = search_max_blocks(shape, warps, mode);
+  while (resident == 0 && warps > 4) {
+    warps /= 2;
+    resident = search_max_blocks(shape, warps, mode);
+  }
+  bps = q->cfg.blocks_per_sm ? q->cfg.blocks_per_sm : std::max<uint32_t>(1, resident);
 }
 
 // Launch shape of the search: the configured (or autotuned) one, else 8
 // warps per block and as many blocks per SM as can be resident.
 static void search_shape(const csm_ctx* q, uint32_t& warps, uint32_t& bps) {
-  warps = q->cfg.warps_per_block ? q->cfg.warps_per_block : 8;
-  if (warps != 4 && warps != 8 && warps != 16) warps = 8;
-  bps = q->cfg.blocks_per_sm ? q->cfg.blocks_per_sm : 0;
-  if (!bps) {
-    const int mode = q->d_enum ? 1 : ((!q->cfg.want_hash && !q->cfg.tail_enumerate) ? 2 : 0);
-    bps = std::max<uint32_t>(1, search_max_blocks(q->nq, warps, mode));
-  }
+  const int mode = search_mode_of(q);
+  search_fit(q, search_shape_of(*q->h_plan, mode), mode, warps, bps);
 }
 
 static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out);
@@ -492,10 +509,11 @@ static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out
     sp.enum_base = (uint32_t)(out - q->d_results);  // this batch's first update within the submit
     sp.enum_stride = 1 + q->nq;
   }
+  set_search_shape(sp, *q->h_plan);
   uint32_t warps, bps;
   search_shape(q, warps, bps);
   if (o->capturing) {  // replays are not timed per search
-    launch_search(sp, q->nq, (uint32_t)q->sm_count * bps, warps, st); CKL();
+    launch_search(sp, (uint32_t)q->sm_count * bps, warps, st); CKL();
   } else {
     if (q->sev_used == q->sev.size()) {
       cudaEvent_t a, b;
@@ -504,7 +522,7 @@ static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out
       q->sev.emplace_back(a, b);
     }
     CK(cudaEventRecord(q->sev[q->sev_used].first, st));
-    launch_search(sp, q->nq, (uint32_t)q->sm_count * bps, warps, st); CKL();
+    launch_search(sp, (uint32_t)q->sm_count * bps, warps, st); CKL();
     CK(cudaEventRecord(q->sev[q->sev_used].second, st));
     q->sev_used++;
   }
@@ -552,7 +570,6 @@ static int run_edge_batch(csm_ctx* ctx, const csm_update* ups, uint32_t B, csm_r
   launch_mut_delete(ctx->d_rdel, c + 4, ctx->d_del2, ctx->d_ins_dst, g, mut_blocks, (uint32_t)ctx->sm_count * 2, st);
   CKL();
   ctx->launches++;
-  if (g.emask) { k_edge_list<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_del2, L, g, 1u); CKL(); }
   for (csm_ctx* a : ctx->attached) {
     rc = stream_after(a->st, st, ctx->ev_fork);
     if (!rc) rc = index_apply_edges(a->index, g, ctx->d_del2, L, a->st, &a->launches);
@@ -564,7 +581,7 @@ static int run_edge_batch(csm_ctx* ctx, const csm_update* ups, uint32_t B, csm_r
   }
   rc = index_apply_edges(ctx->index, g, ctx->d_del2, L, st, &ctx->launches);
   if (rc) return rc;
-  k_temporal_clear<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_rt, c + 5, g); CKL();
+  k_temporal_clear<<<blocks_for(L, 256), 256, 0, st>>>(L, g); CKL();
   ctx->batches++;
   for (csm_ctx* a : ctx->attached) a->batches++;
   return CSM_OK;
@@ -678,8 +695,6 @@ static int run_vertex_delete(csm_ctx* ctx, uint32_t v) {
                       st);
     CKL();
     ctx->launches++;
-    if (g.emask) { k_edge_list<<<blocks_for(K, 256), 256, 0, st>>>(keys2, K, g, 1u); CKL(); }
-    ctx->e_tomb += deg;
     for (csm_ctx* q : all) {
       if (q != ctx) { q->g = g; rc = stream_after(q->st, st, ctx->ev_fork); }
       if (!rc) rc = index_apply_edges(q->index, g, keys2, K, q->st, &q->launches);
@@ -803,46 +818,6 @@ static int run_edge_batch_graph(csm_ctx* ctx, const csm_update* ups, uint32_t B_
   return CSM_OK;
 }
 
-// Keeps the edge table's load below one half (live keys plus deleted slots)
-// before the updates `h` of a submit run: refills it from the CSR when the
-// deleted slots would push it over, in a table twice as large when the live
-// keys alone fill a third.  The counts are upper bounds (every insertion
-// record counts as a new edge, every deletion as a deleted slot).
-static int edge_table_maintain(csm_ctx* ctx, const csm_update* h, uint64_t n) {
-  DevGraph& g = ctx->g;
-  if (!g.emask) return CSM_OK;
-  uint64_t ins = 0, del = 0;
-  for (uint64_t i = 0; i < n; i++) {
-    if (h[i].type != 'e') continue;
-    if (h[i].is_add) ins++; else del++;
-  }
-  uint64_t slots = g.emask + 1;
-  if ((ctx->e_live + ctx->e_tomb + ins + del) * 2 > slots) {
-    cudaStream_t st = ctx->st;
-    uint64_t want = slots;
-    while ((ctx->e_live + ins) * 3 > want) want <<= 1;
-    if (want != slots) {
-      uint64_t* nk = nullptr;
-      CK(cudaStreamSynchronize(st));  // no kernel of an earlier submit still reads the old table
-      for (csm_ctx* a : ctx->attached) CK(cudaStreamSynchronize(a->st));
-      int rc = ctx->mem.alloc((void**)&nk, 8ull * want);
-      if (rc) return rc;
-      ctx->mem.release(g.ekeys, 8ull * slots);
-      g.ekeys = nk;
-      g.emask = want - 1;
-      slots = want;
-      ctx->graph_version++;  // captured launch sequences hold the old table
-    }
-    CK(cudaMemsetAsync(g.ekeys, 0xff, 8ull * slots, st));
-    k_edge_fill<<<ctx->sm_count * 8, 256, 0, st>>>(g);
-    CKL();
-    ctx->e_tomb = 0;
-  }
-  ctx->e_live += ins;
-  ctx->e_tomb += del;
-  return CSM_OK;
-}
-
 static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, const csm_update* h_ups) {
   if (ctx->owner) return set_err(CSM_ESTATE, "updates of an attached query are submitted to its owner");
   if (!ctx->has_graph || !ctx->has_plan) return set_err(CSM_ESTATE, "load the query, the graph and build the index first");
@@ -877,8 +852,6 @@ static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, cons
     CK(cudaStreamSynchronize(st));
     h = hv.data();
   }
-  rc = edge_table_maintain(ctx, h, n);
-  if (rc) return rc;
   uint64_t i = 0;
   while (i < n) {
     for (size_t k = 0; k < ctx->attached.size(); k++) out_q[k] = ctx->attached[k]->d_results + i;
@@ -1026,7 +999,7 @@ static int fetch_last(csm_ctx* ctx) {
 // at a time, so this sets how many subtrees share a block's shared memory)
 // and resident blocks per SM -- is chosen per query and graph by timing the
 // search on a sample of update edges for every shape the SM admits (shared
-// memory of the per-warp level buffers, 32 warps of 64 registers per SM).
+// memory of the per-warp level buffers, 16 warps of 128 registers per SM).
 // The sample is searched as insertions against the current graph, which is
 // not modified: each edge's seeds run the ordinary search with positions 0
 // and 1 fixed, whether or not the edge is present.
@@ -1069,8 +1042,9 @@ static int tune_run(csm_ctx* ctx, uint32_t B, uint32_t warps, uint32_t bps, floa
   sp.donate_every = donate_every;
   sp.split_deep = split_deep;
   sp.tail = (!ctx->cfg.want_hash && !ctx->d_enum && !ctx->cfg.tail_enumerate) ? 1u : 0u;  // as the batches run
+  set_search_shape(sp, *ctx->h_plan);
   CK(cudaEventRecord(ctx->ev_start, st));
-  launch_search(sp, ctx->nq, (uint32_t)ctx->sm_count * bps, warps, st); CKL();
+  launch_search(sp, (uint32_t)ctx->sm_count * bps, warps, st); CKL();
   CK(cudaEventRecord(ctx->ev_end, st));
   CK(cudaEventSynchronize(ctx->ev_end));
   CK(cudaEventElapsedTime(ms, ctx->ev_start, ctx->ev_end));
@@ -1090,16 +1064,17 @@ static int autotune(csm_ctx* ctx, uint32_t n, const csm_update* h_edges, uint32_
   // the default shape (8 warps, every resident block), then the others; a
   // shape replaces the default only when it is at least 5 % faster, since
   // capped updates make single timings vary by a few percent
-  const int kmode = ctx->d_enum ? 1 : ((!ctx->cfg.want_hash && !ctx->cfg.tail_enumerate) ? 2 : 0);  // as the batches run
-  uint32_t best_w = 8, best_b = std::max<uint32_t>(1, search_max_blocks(ctx->nq, 8, kmode));
+  const int kmode = search_mode_of(ctx);  // as the batches run
+  const SearchShape shape = search_shape_of(*ctx->h_plan, kmode);
+  uint32_t best_w = 8, best_b = std::max<uint32_t>(1, search_max_blocks(shape, 8, kmode));
   float best = 0;
   rc = tune_run(ctx, B, best_w, best_b, &best);
   if (rc) return rc;
   const float def_ms = best;
   for (uint32_t w : {4u, 8u, 16u}) {
-    const uint32_t bmax = search_max_blocks(ctx->nq, w, kmode);  // resident blocks per SM
+    const uint32_t bmax = search_max_blocks(shape, w, kmode);  // resident blocks per SM
     for (uint32_t b = std::max<uint32_t>(1, bmax > 3 ? bmax - 3 : 1); b <= bmax; b++) {
-      if (w == 8 && b == std::max<uint32_t>(1, search_max_blocks(ctx->nq, 8, kmode))) continue;
+      if (w == 8 && b == std::max<uint32_t>(1, search_max_blocks(shape, 8, kmode))) continue;
       rc = tune_run(ctx, B, w, b, &ms);
       if (rc) return rc;
       if (ms < best && ms < 0.95f * def_ms) { best = ms; best_w = w; best_b = b; }
@@ -1160,7 +1135,7 @@ __global__ void k_init_fill(DevGraph g, uint32_t combo, uint32_t label, const un
   const uint32_t x = lo;
   const uint32_t* pool = g.pools[g.ps->active];
   const uint32_t* d = g.dir + (size_t)x * (g.nc + 1) + combo;
-  const uint32_t y = pool[g.row_off[x] + d[0] + (e - off[x])];
+  const uint32_t y = pool[(uint64_t)g.row[x].x + d[0] + (e - off[x])];
   UpdInfo u;
   u.v1 = x; u.v2 = y; u.label = label; u.flags = UF_VALID | UF_ADD;
   info[i] = u;
@@ -1231,7 +1206,8 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
     sp.batch = B;
     sp.sstat = ctx->d_sstat;
     sp.tail = ctx->cfg.tail_enumerate ? 0u : 1u;
-    launch_search(sp, ctx->nq, (uint32_t)ctx->sm_count * bps, warps, st); CKL();
+    set_search_shape(sp, *ctx->h_plan);
+    launch_search(sp, (uint32_t)ctx->sm_count * bps, warps, st); CKL();
     ctx->search_launches++;
     k_init_sum<<<std::min<uint32_t>(blocks_for(B, 256), 1024), 256, 0, st>>>(B, ctx->d_count, total); CKL();
     ctx->launches += 3;
@@ -1486,10 +1462,9 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   int rc = 0;
 #define AL(p, sz) do { rc = m.alloc((void**)&(p), (sz)); if (rc) return rc; } while (0)
   AL(g.vlabel, 4ull * n_cap);
-  AL(g.row_off, 8ull * n_cap);
-  AL(g.row_cap, 4ull * n_cap);
+  AL(g.row, 8ull * n_cap);
   AL(g.dir, 4ull * n_cap * (nc + 1));
-  AL(g.t_start, 4ull * n_cap);
+  AL(g.t_tab, sizeof(ulonglong2) * (size_t)temporal_slots(ctx->bmax));
   AL(g.t_count, 4ull * n_cap);
   AL(g.ps, sizeof(PoolState));
   AL(ctx->d_qlab, 4ull * (ctx->qlab_v.size() + ctx->qlab_e.size()));
@@ -1506,14 +1481,13 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   for (uint32_t v = 0; v < n_v; v++)
     if (vlabels[v] != kNone) ctx->h_vlabel[v] = fold_host(ctx->qlab_v, vlabels[v]);
   if (n_v) { k_fold_vlabels<<<blocks_for(n_v, 256), 256, 0, st>>>(g.vlabel, n_v, g); CKL(); }
-  CK(cudaMemsetAsync(g.row_off, 0, 8ull * n_cap, st));
-  CK(cudaMemsetAsync(g.row_cap, 0, 4ull * n_cap, st));
   CK(cudaMemsetAsync(g.dir, 0, 4ull * n_cap * (nc + 1), st));
   CK(cudaMemsetAsync(g.t_count, 0, 4ull * n_cap, st));
   CK(cudaMemsetAsync(g.ps, 0, sizeof(PoolState), st));
   // temporaries
   uint32_t* d_e = nullptr; uint64_t *ukey = nullptr, *ukey2 = nullptr, *uidx = nullptr, *uidx2 = nullptr;
-  uint64_t *dkey = nullptr, *dkey2 = nullptr, *first = nullptr, *cap64 = nullptr;
+  uint64_t *dkey = nullptr, *dkey2 = nullptr, *first = nullptr, *cap64 = nullptr, *off64 = nullptr;
+  uint32_t* cap32 = nullptr;
   unsigned long long* d_small = nullptr;
   const uint64_t M = 2 * n_e;
   AL(d_e, 12ull * n_e);
@@ -1526,7 +1500,7 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, ukey, ukey2, uidx, uidx2, (int64_t)n_e, 0, 64, st));
   CK(cub::DeviceRadixSort::SortKeys(nullptr, tb2, dkey, dkey2, (int64_t)M, 0, (int)kb.total(), st));
   size_t tb3 = 0;
-  CK(cub::DeviceScan::ExclusiveSum(nullptr, tb3, cap64, g.row_off, (int64_t)n_cap, st));
+  CK(cub::DeviceScan::ExclusiveSum(nullptr, tb3, cap64, off64, (int64_t)n_cap, st));
   const size_t tbmax = std::max(tb, std::max(tb2, tb3));
   AL(tmp, tbmax);
   if (n_e) {
@@ -1548,54 +1522,52 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
     CK(cub::DeviceRadixSort::SortKeys(tmp, tb, dkey, dkey2, (int64_t)M, 0, (int)kb.total(), st));
   }
   m.release(dkey, 8ull * std::max<uint64_t>(M, 1));
-  AL(first, 8ull * n_cap); AL(cap64, 8ull * n_cap);
+  AL(first, 8ull * n_cap); AL(cap64, 8ull * n_cap); AL(off64, 8ull * n_cap); AL(cap32, 4ull * n_cap);
   if (M) { k_load_count<<<blocks_for(M, 256), 256, 0, st>>>(dkey2, M, kb, (uint32_t)nc, g.dir, first, d_small + 1); CKL(); }
   k_dir_scan<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc); CKL();
-  k_load_caps<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc, g.row_cap, cap64); CKL();
+  k_load_caps<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc, cap32, cap64); CKL();
   tb = tbmax;
-  CK(cub::DeviceScan::ExclusiveSum(tmp, tb, cap64, g.row_off, (int64_t)n_cap, st));
+  CK(cub::DeviceScan::ExclusiveSum(tmp, tb, cap64, off64, (int64_t)n_cap, st));
+  k_load_rows<<<blocks_for(n_cap, 256), 256, 0, st>>>(off64, cap32, n_cap, g.row); CKL();
   unsigned long long last_off = 0, last_cap = 0, n_valid = 0;
-  CK(cudaMemcpyAsync(&last_off, g.row_off + (n_cap - 1), 8, cudaMemcpyDeviceToHost, st));
+  CK(cudaMemcpyAsync(&last_off, off64 + (n_cap - 1), 8, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(&last_cap, cap64 + (n_cap - 1), 8, cudaMemcpyDeviceToHost, st));
   CK(cudaMemcpyAsync(&n_valid, d_small + 1, 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
   const uint64_t used = last_off + last_cap;
-  const uint64_t pool_cap = std::max<uint64_t>(2 * used + 16ull * ctx->bmax + (1ull << 20), 1ull << 20);
+  const uint64_t pool_cap = 2 * used + 16ull * ctx->bmax + (1ull << 20);  // a multiple of four, as every row's capacity
   if (pool_cap >= (1ull << 32)) return set_err(CSM_EUNSUPPORTED, "graph too large for 32-bit pool offsets");
   g.pool_cap = pool_cap;
   AL(g.pools[0], 4ull * pool_cap);
   AL(g.pools[1], 4ull * pool_cap);
-  if (M) { k_load_scatter<<<blocks_for(M, 256), 256, 0, st>>>(dkey2, M, kb, first, g.row_off, g.pools[0]); CKL(); }
+  // row tables: two slots per row slot.  Without room for them, or when an id
+  // and a folded edge label do not fit in 31 bits, the search joins by binary
+  // search in the rows instead
+  g.htab = nullptr;
+  g.htomb = nullptr;
+  g.hlb = ceil_log2(n_el);
+  if (((uint64_t)n_cap << g.hlb) < (kSlotTomb & ~kSlotTouched)) {
+    uint32_t *tab = nullptr, *tomb = nullptr;
+    if (m.alloc((void**)&tab, 8ull * pool_cap) == CSM_OK && m.alloc((void**)&tomb, 4ull * n_cap) == CSM_OK) {
+      g.htab = tab;
+      g.htomb = tomb;
+      CK(cudaMemsetAsync(g.htab, 0xff, 8ull * used, st));
+      CK(cudaMemsetAsync(g.htomb, 0, 4ull * n_cap, st));
+    } else {
+      m.release(tab, 8ull * pool_cap);
+      set_err(CSM_OK, "");  // the tables are optional
+    }
+  }
   PoolState ps{};
   ps.top[0] = used;
   CK(cudaMemcpyAsync(g.ps, &ps, sizeof(ps), cudaMemcpyHostToDevice, st));
+  if (M) { k_load_scatter<<<blocks_for(M, 256), 256, 0, st>>>(dkey2, M, first, g, g.pools[0]); CKL(); }
   CK(cudaStreamSynchronize(st));
   m.release(dkey2, 8ull * std::max<uint64_t>(M, 1)); m.release(first, 8ull * n_cap); m.release(cap64, 8ull * n_cap);
+  m.release(off64, 8ull * n_cap); m.release(cap32, 4ull * n_cap);
   m.release(tmp, tbmax); m.release(d_small, 64);
 #undef AL
   ctx->num_edges = n_valid / 2;
-  // edge table: four slots per edge (a power of two); without room for it,
-  // or for ids of 30 bits and more or over 16 folded edge labels, the
-  // search joins by binary search in the rows instead
-  g.ekeys = nullptr;
-  g.emask = 0;
-  if (n_cap < (1u << 30) && n_el <= 16) {
-    uint64_t slots = 1ull << 20;
-    while (slots < 4 * std::max<uint64_t>(ctx->num_edges, 1)) slots <<= 1;
-    uint64_t* ek = nullptr;
-    if (m.alloc((void**)&ek, 8ull * slots) == CSM_OK) {
-      g.ekeys = ek;
-      g.emask = slots - 1;
-      CK(cudaMemsetAsync(g.ekeys, 0xff, 8ull * slots, st));
-      k_edge_fill<<<ctx->sm_count * 8, 256, 0, st>>>(g);
-      CK(cudaGetLastError());
-      CK(cudaStreamSynchronize(st));
-      ctx->e_live = ctx->num_edges;
-      ctx->e_tomb = 0;
-    } else {
-      set_err(CSM_OK, "");  // the table is optional
-    }
-  }
   ctx->has_graph = true;
   return CSM_OK;
 }
@@ -1898,6 +1870,7 @@ struct CtxView {
   uint64_t cap;
   int homo, want_hash;
   uint32_t warps, bps;
+  SearchShape shape;
   uint32_t dup_zero;       // CaLiG: an insertion of a present edge counts 0
   cudaEvent_t owner_end;   // attached query: end of the owner's last submit (null otherwise)
 };
@@ -1923,12 +1896,8 @@ bool ctx_view(csm_ctx* ctx, CtxView* v) {
   v->want_hash = ctx->cfg.want_hash;
   // the launch shape of the submit path's enumerating search (the probe does
   // not count tails)
-  uint32_t warps = ctx->cfg.warps_per_block ? ctx->cfg.warps_per_block : 8;
-  if (warps != 4 && warps != 8 && warps != 16) warps = 8;
-  uint32_t bps = ctx->cfg.blocks_per_sm;
-  if (!bps) bps = std::max<uint32_t>(1, search_max_blocks(ctx->nq, warps, 0));
-  v->warps = warps;
-  v->bps = bps;
+  v->shape = search_shape_of(*ctx->h_plan, 0);
+  search_fit(ctx, v->shape, 0, v->warps, v->bps);
   return true;
 }
 

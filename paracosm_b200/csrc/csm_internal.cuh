@@ -1,11 +1,11 @@
 // Internal device-side layout shared by the engine's translation units.
 //
 // Data graph in HBM: a label-partitioned dynamic CSR.
-//   - Row v lives at pool[row_off[v] .. row_off[v] + row_cap[v]); its first
+//   - Row v lives at pool[row[v].x .. row[v].x + row[v].y); its first
 //     deg(v) slots hold neighbour ids, grouped by "combo" = (neighbour vertex
 //     label, edge label) and sorted by id inside each group, so the segment
 //     S(v, a, l) (neighbours of v with vertex label a over edges labelled l)
-//     is contiguous.  The remaining row_cap - deg slots are slack for
+//     is contiguous.  The remaining row[v].y - deg slots are slack for
 //     insertions; a row that outgrows its slack is moved to fresh pool space.
 //   - dir[v * (NC + 1) + c] is the offset of combo c's segment inside row v
 //     (dir[..NC] = deg(v)), so a segment is found with two 4-byte loads.
@@ -76,16 +76,16 @@ enum : uint32_t { kErrNone = 0, kErrPoolFull = 1, kErrListOverflow = 2, kErrTask
 // Device view of the dynamic CSR (pointers into device memory).
 struct DevGraph {
   uint32_t* vlabel;      // [n_cap]
-  uint64_t* row_off;     // [n_cap]  offset into the active pool
-  uint32_t* row_cap;     // [n_cap]
+  uint2* row;            // [n_cap]  x: offset into the active pool, y: capacity
   uint32_t* dir;         // [n_cap * (nc + 1)]
   uint32_t* pools[2];    // the two row pools
   PoolState* ps;
   // temporal entries of the current batch, sorted by packed key (x, combo, nbr)
-  uint32_t* t_start;     // [n_cap]
   uint32_t* t_count;     // [n_cap]  0 = vertex untouched in this batch
   uint64_t* t_key;       // packed keys
   int2* t_span;          // presence interval [start, end] in batch sequence numbers
+  ulonglong2* t_tab;     // hash table (key, value) over them: see touched_present
+  uint32_t t_mask;       // its slots - 1 for the current batch
   uint64_t pool_cap;     // entries per pool
   // label folding: sorted distinct query labels; label i of the list maps
   // to i, every other label to the inert label (n_qv / n_qe)
@@ -94,58 +94,103 @@ struct DevGraph {
   uint32_t n_qv, n_qe;
   uint32_t n, n_cap, n_vl, n_el, nc;  // n_vl = n_qv + 1, n_el = n_qe + 1
   KeyBits kb;
-  // Edge table: every (edge, label) of the graph -- the union graph during a
-  // batch -- as one key in an open-addressing hash set (linear probing), so
-  // that "is x a neighbour of v over label l" is one probe instead of a
-  // binary search in v's segment.  emask = slots - 1; 0: no table (ids of
-  // 30 bits or more, or more than 16 folded edge labels).
-  uint64_t* ekeys;
-  uint64_t emask;
+  // Row tables: the entries of row v -- the union graph's during a batch --
+  // as a hash set of cap / 4 buckets of 8 slots at htab[2 * off ..), so that
+  // "is x a neighbour of v over label l" is one 32-byte load instead of a
+  // binary search in v's segment.  An entry whose bucket is full goes to the
+  // next one (cyclically); a bucket with an empty slot was never full, which
+  // ends a search.  The region moves with the row and is at most half full of
+  // live entries; htomb[v] counts its deleted slots.
+  // null: no tables (an id and a label do not fit in 31 bits, or no memory).
+  uint32_t* htab;
+  uint32_t* htomb;       // [n_cap]
+  uint32_t hlb;          // bits of a folded edge label in a table entry
 };
 
-// Edge-table keys: the smaller endpoint (30 bits), the larger (30 bits), the
-// folded edge label (4 bits); two values no key takes mark empty and deleted
-// slots.
-constexpr uint64_t kEdgeEmpty = ~0ULL, kEdgeTomb = ~0ULL - 1;
-__host__ __device__ __forceinline__ uint64_t edge_key(uint32_t a, uint32_t b, uint32_t l) {
-  const uint32_t lo = a < b ? a : b, hi = a < b ? b : a;
-  return ((uint64_t)lo << 34) | ((uint64_t)hi << 4) | (uint64_t)l;
+// Row-table entries: neighbour id, then the folded edge label in the low hlb
+// bits, 31 bits together; the top bit marks an entry touched in this batch
+// (it has temporal entries).  Two values no entry takes, with or without that
+// bit, mark empty and deleted slots.
+constexpr uint32_t kSlotEmpty = 0xffffffffu, kSlotTomb = 0xfffffffeu, kSlotTouched = 0x80000000u;
+__host__ __device__ __forceinline__ uint32_t row_entry(uint32_t y, uint32_t l, uint32_t hlb) { return (y << hlb) | l; }
+// A row's slots come in multiples of four, so that its table starts on a bucket.
+__host__ __device__ __forceinline__ uint32_t row_round(uint32_t cap) { return (cap + 3u) & ~3u; }
+// Home bucket of an entry in a row table of `buckets` buckets.
+__device__ __forceinline__ uint32_t row_bucket(uint32_t entry, uint32_t buckets) {
+  uint32_t h = entry * 0x9E3779B1u;  // multiplicative hashing, folded once so that the low bits count too
+  h ^= h >> 15;
+  h *= 0x85EBCA77u;
+  return __umulhi(h, buckets);
 }
-__device__ __forceinline__ uint64_t edge_slot(uint64_t key, uint64_t mask) {
-  uint64_t x = key ^ (key >> 33);  // MurmurHash3 fmix64, as mix64
-  x *= 0xff51afd7ed558ccdULL; x ^= x >> 33;
-  x *= 0xc4ceb9fe1a85ec53ULL; x ^= x >> 33;
-  return x & mask;
+// A bucket in one 32-byte load, past L1: its lines are scattered over the
+// lanes, and no other load of the SM is likely to want them.
+struct RowBucket {
+  uint32_t k[8];
+};
+__device__ __forceinline__ RowBucket ld_bucket(const uint32_t* a) {
+  uint64_t w0, w1, w2, w3;
+  asm volatile("ld.global.L1::no_allocate.v4.b64 {%0,%1,%2,%3}, [%4];"
+               : "=l"(w0), "=l"(w1), "=l"(w2), "=l"(w3)
+               : "l"(a));
+  return RowBucket{{(uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32), (uint32_t)w2,
+                    (uint32_t)(w2 >> 32), (uint32_t)w3, (uint32_t)(w3 >> 32)}};
 }
-// Loads of data read once per use at random places (edge-table slots, filter
-// words, driver segments): they may fill L1 but go first when L1 needs room,
+// Loads of driver segments, read once per use: they may fill L1 but go first when L1 needs room,
 // so they do not push out the lines that are reused -- the search's register
 // spills and the plan.
-__device__ __forceinline__ uint64_t ld_stream(const uint64_t* a) {
-  uint64_t v;
-  asm("ld.global.L1::evict_first.u64 %0, [%1];" : "=l"(v) : "l"(a));
-  return v;
-}
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t* a) {
   uint32_t v;
   asm("ld.global.L1::evict_first.u32 %0, [%1];" : "=r"(v) : "l"(a));
   return v;
 }
 
-// Probe sequence from a slot already loaded (first = ekeys[slot]).
-__device__ __forceinline__ bool edge_probe_rest(const DevGraph& g, uint64_t key, uint64_t slot, uint64_t first) {
-  uint64_t k = first;
-  for (uint64_t n = 0; n <= g.emask; n++) {
-    if (k == key) return true;
-    if (k == kEdgeEmpty) return false;
-    slot = (slot + 1) & g.emask;
-    k = ld_stream(g.ekeys + slot);
+// Loads scattered over the lanes, whose lines no other load of the SM is likely
+// to want: past L1 altogether.
+__device__ __forceinline__ uint64_t ld_gather(const uint64_t* a) {
+  uint64_t v;
+  asm("ld.global.L1::no_allocate.u64 %0, [%1];" : "=l"(v) : "l"(a));
+  return v;
+}
+__device__ __forceinline__ uint32_t ld_gather(const uint32_t* a) {
+  uint32_t v;
+  asm("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(a));
+  return v;
+}
+
+// The word of `entry` in the row table of row r (with its touched bit), or
+// kSlotEmpty when it is not there.  One load settles nearly every search: at
+// the tables' load of 0.4 a bucket of 8 overflows for one row entry in 200,
+// where linear probing over single slots made a warp wait for the longest of
+// its 32 chains (about 8 dependent loads).
+// The word of `entry` in the row table of row r (with its touched bit), or
+// kSlotEmpty when it is not there.  One load settles nearly every search: at
+// the tables' load of 0.4 a bucket of 8 overflows for one row entry in 200,
+// where linear probing over single slots made a warp wait for the longest of
+// its 32 chains (about 8 dependent loads; the hash-enumerating search of 3,001
+// updates 9.7 -> 5.9 ms).
+__device__ __forceinline__ uint32_t row_find(const DevGraph& g, uint2 r, uint32_t entry) {
+  const uint32_t buckets = r.y >> 2;
+  const uint32_t* tab = g.htab + 2ull * r.x;
+  uint32_t s = row_bucket(entry, buckets);
+#pragma unroll 1
+  for (uint32_t n = 0; n < buckets; n++) {
+    const RowBucket b = ld_bucket(tab + 8ull * s);
+    uint32_t hit = kSlotEmpty;
+    bool open = false;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      if ((b.k[i] & ~kSlotTouched) == entry) hit = b.k[i];
+      open = open || b.k[i] == kSlotEmpty;
+    }
+    if (hit != kSlotEmpty || open) return hit;
+    if (++s == buckets) s = 0;
   }
-  return false;
+  return kSlotEmpty;
 }
 
 __device__ __forceinline__ uint32_t fold_label(const uint32_t* sorted, uint32_t n, uint32_t l) {
   uint32_t lo = 0, hi = n;
+#pragma unroll 1
   while (lo < hi) {
     uint32_t mid = (lo + hi) >> 1;
     if (sorted[mid] < l) lo = mid + 1; else hi = mid;
@@ -164,13 +209,14 @@ __device__ __forceinline__ uint32_t combo_of(const DevGraph& g, uint32_t vl, uin
 // Segment [lo, hi) of combo c in row v, as absolute pool offsets.
 __device__ __forceinline__ void segment(const DevGraph& g, uint32_t v, uint32_t c, uint64_t& lo, uint64_t& hi) {
   const uint32_t* d = g.dir + (size_t)v * (g.nc + 1) + c;
-  const uint64_t base = g.row_off[v];
+  const uint64_t base = g.row[v].x;
   lo = base + d[0];
   hi = base + d[1];
 }
 
 // lower_bound over a sorted uint32 range; returns the first index with a[i] >= x.
 __device__ __forceinline__ uint64_t lower_bound_u32(const uint32_t* a, uint64_t lo, uint64_t hi, uint32_t x) {
+#pragma unroll 1
   while (lo < hi) {
     uint64_t mid = (lo + hi) >> 1;
     if (a[mid] < x) lo = mid + 1; else hi = mid;
@@ -186,6 +232,7 @@ __device__ __forceinline__ bool contains_u32(const uint32_t* a, uint64_t lo, uin
 // Finds edge (x, y) in the union graph; returns its folded label or kNone.
 __device__ __forceinline__ uint32_t find_label(const DevGraph& g, const uint32_t* pool, uint32_t x, uint32_t y) {
   const uint32_t ly = g.vlabel[y];
+#pragma unroll 1
   for (uint32_t l = 0; l < g.n_el; l++) {
     uint64_t lo, hi;
     segment(g, x, ly * g.n_el + l, lo, hi);
@@ -194,24 +241,47 @@ __device__ __forceinline__ uint32_t find_label(const DevGraph& g, const uint32_t
   return kNone;
 }
 
-// Is edge (v, w) with combo c present at batch time t?  Only called for
-// edges found in the union graph; edges not touched in this batch are present.
-__device__ __forceinline__ bool present_at(const DevGraph& g, uint32_t v, uint32_t c, uint32_t w, int32_t t) {
-  const uint32_t cnt = g.t_count[v];
-  if (cnt == 0) return true;
-  const uint64_t key = g.kb.pack(v, c, w);
-  uint32_t lo = g.t_start[v], hi = lo + cnt;
-  while (lo < hi) {
-    uint32_t mid = (lo + hi) >> 1;
-    if (g.t_key[mid] < key) lo = mid + 1; else hi = mid;
+// Temporal table: a hash set (linear probing, empty key kTempEmpty) that holds,
+// for every touched entry (v, c, w) of the batch, its presence, and for every
+// segment (v, c) with touched entries -- key (v, c, all ones) -- the run of
+// them in t_key: first index, and length in the upper half.  An entry's value
+// is its one interval (start + 1, end), or, when it has several, kTempMany and
+// the run of t_span indices (first, and length in the upper half).
+constexpr uint64_t kTempEmpty = ~0ULL, kTempMany = 1ULL << 63;
+__device__ __forceinline__ uint64_t temporal_head(const DevGraph& g, uint32_t v, uint32_t c) {
+  return g.kb.pack(v, c, (uint32_t)((1ULL << g.kb.yb) - 1));
+}
+__device__ __forceinline__ uint32_t temporal_slot(uint64_t key, uint32_t mask) {
+  uint64_t h = key * 0x9E3779B97F4A7C15ULL;
+  h ^= h >> 32;
+  return (uint32_t)h & mask;
+}
+// Value of a key, or kTempEmpty.
+__device__ __forceinline__ uint64_t temporal_find(const DevGraph& g, uint64_t key) {
+  uint32_t s = temporal_slot(key, g.t_mask);
+#pragma unroll 1
+  for (;; s = (s + 1) & g.t_mask) {  // at most a quarter full: an empty slot ends it
+    const ulonglong2 e = g.t_tab[s];
+    if (e.x == key) return e.y;
+    if (e.x == kTempEmpty) return kTempEmpty;
   }
-  const uint32_t end = g.t_start[v] + cnt;
-  if (lo >= end || g.t_key[lo] != key) return true;
-  for (uint32_t i = lo; i < end && g.t_key[i] == key; i++) {
-    int2 s = g.t_span[i];
+}
+__device__ __forceinline__ bool temporal_present(const DevGraph& g, uint64_t val, int32_t t) {
+  if (!(val & kTempMany)) return (int32_t)(uint32_t)val - 1 <= t && t <= (int32_t)(val >> 32);
+  const uint32_t beg = (uint32_t)val, n = (uint32_t)((val & ~kTempMany) >> 32);
+#pragma unroll 1
+  for (uint32_t i = beg; i < beg + n; i++) {
+    const int2 s = g.t_span[i];
     if (s.x <= t && t <= s.y) return true;
   }
   return false;
+}
+
+// Is edge (v, w) with combo c present at batch time t?  Only called for
+// edges found in the union graph; edges not touched in this batch are present.
+__device__ __forceinline__ bool touched_present(const DevGraph& g, uint32_t v, uint32_t c, uint32_t w, int32_t t) {
+  const uint64_t val = temporal_find(g, g.kb.pack(v, c, w));
+  return val == kTempEmpty || temporal_present(g, val, t);
 }
 
 // Number of entries of segment (v, c) present at batch time t, given its
@@ -220,18 +290,15 @@ __device__ __forceinline__ bool present_at(const DevGraph& g, uint32_t v, uint32
 __device__ __forceinline__ uint32_t seg_size_at(const DevGraph& g, uint32_t v, uint32_t c, uint64_t lo, uint64_t hi,
                                                 int32_t t) {
   uint32_t size = (uint32_t)(hi - lo);
-  const uint32_t cnt = g.t_count[v];
-  if (cnt == 0 || size == 0) return size;
-  const uint32_t beg = g.t_start[v], end = beg + cnt;
-  const uint64_t k0 = g.kb.pack(v, c, 0);
-  uint32_t a = beg, b = end;
-  while (a < b) {
-    uint32_t mid = (a + b) >> 1;
-    if (g.t_key[mid] < k0) a = mid + 1; else b = mid;
-  }
-  for (uint32_t i = a; i < end && g.kb.x_of(g.t_key[i]) == v && g.kb.c_of(g.t_key[i]) == c;) {
+  if (size == 0 || g.t_count[v] == 0) return size;
+  const uint64_t run = temporal_find(g, temporal_head(g, v, c));
+  if (run == kTempEmpty) return size;
+  const uint32_t beg = (uint32_t)run, end = beg + (uint32_t)(run >> 32);
+#pragma unroll 1
+  for (uint32_t i = beg; i < end;) {
     const uint64_t key = g.t_key[i];
     bool present = false;
+#pragma unroll 1
     for (; i < end && g.t_key[i] == key; i++) {
       const int2 sp = g.t_span[i];
       if (sp.x <= t && t <= sp.y) present = true;
@@ -274,6 +341,7 @@ struct PlanAnchor {
   PlanPos pos[kMaxQ];
   uint8_t back_pos[kMaxQE];
   uint16_t back_combo[kMaxQE];
+  uint8_t back_el[kMaxQE];   // folded edge label of each back entry
 };
 
 struct Plan {

@@ -10,6 +10,56 @@
 namespace csm {
 
 // ---------------------------------------------------------------------
+// row tables (DevGraph::htab)
+// ---------------------------------------------------------------------
+
+// Places an entry that is not in the table (the rows are sets); entries of one
+// row may be placed side by side.
+__device__ __forceinline__ void row_table_insert(const DevGraph& g, uint2 r, uint32_t entry) {
+  const uint32_t buckets = r.y >> 2;
+  uint32_t* tab = g.htab + 2ull * r.x;
+  uint32_t s = row_bucket(entry, buckets);
+  for (uint32_t n = 0; n < buckets; n++) {
+    const RowBucket b = ld_bucket(tab + 8ull * s);
+#pragma unroll
+    for (int i = 0; i < 8; i++)
+      if (b.k[i] == kSlotEmpty && atomicCAS(tab + 8ull * s + i, kSlotEmpty, entry) == kSlotEmpty) return;
+    if (++s == buckets) s = 0;
+  }
+  atomicExch(&g.ps->error, kErrEdgeTable);  // no empty slot left
+}
+
+// Slot of `entry` in a row table (offset from its start), or kSlotEmpty;
+// `open`: its bucket has an empty slot.
+__device__ __forceinline__ uint32_t row_locate(const uint32_t* tab, uint32_t buckets, uint32_t entry, bool& open) {
+  uint32_t s = row_bucket(entry, buckets);
+  for (uint32_t n = 0; n < buckets; n++) {
+    const RowBucket b = ld_bucket(tab + 8ull * s);
+    uint32_t at = kSlotEmpty;
+    open = false;
+#pragma unroll
+    for (int i = 0; i < 8; i++) {
+      if ((b.k[i] & ~kSlotTouched) == entry) at = 8u * s + (uint32_t)i;
+      open = open || b.k[i] == kSlotEmpty;
+    }
+    if (at != kSlotEmpty || open) return at;
+    if (++s == buckets) s = 0;
+  }
+  return kSlotEmpty;
+}
+
+// A slot of a bucket that was never full is free again; in a full one a
+// deleted slot keeps the searches going that run over it, and is counted.
+__device__ __forceinline__ void row_table_delete(const DevGraph& g, uint32_t x, uint2 r, uint32_t entry) {
+  uint32_t* tab = g.htab + 2ull * r.x;
+  bool open = false;
+  const uint32_t s = row_locate(tab, r.y >> 2, entry, open);
+  if (s == kSlotEmpty) return;
+  tab[s] = open ? kSlotEmpty : kSlotTomb;
+  if (!open) atomicAdd(&g.htomb[x], 1u);
+}
+
+// ---------------------------------------------------------------------
 // load-time CSR build
 // ---------------------------------------------------------------------
 
@@ -76,8 +126,8 @@ __global__ void k_load_count(const uint64_t* dkey, uint64_t M, KeyBits kb, uint3
   }
 }
 
-__device__ __forceinline__ uint32_t slack_cap(uint32_t d) { return d == 0 ? 0u : d + max(2u, d >> 2); }
-__device__ __forceinline__ uint32_t grow_cap(uint32_t d) { return d + max(8u, d >> 1); }
+__device__ __forceinline__ uint32_t slack_cap(uint32_t d) { return d == 0 ? 0u : row_round(d + max(2u, d >> 2)); }
+__device__ __forceinline__ uint32_t grow_cap(uint32_t d) { return row_round(d + max(8u, d >> 1)); }
 
 __global__ void k_load_caps(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t* cap, uint64_t* cap64) {
   uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
@@ -87,14 +137,24 @@ __global__ void k_load_caps(const uint32_t* dir, uint32_t n_cap, uint32_t nc, ui
   cap64[v] = c;
 }
 
-__global__ void k_load_scatter(const uint64_t* dkey, uint64_t M, KeyBits kb, const uint64_t* first,
-                               const uint64_t* row_off, uint32_t* pool) {
+__global__ void k_load_rows(const uint64_t* off, const uint32_t* cap, uint32_t n_cap, uint2* row) {
+  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v < n_cap) row[v] = make_uint2((uint32_t)off[v], cap[v]);
+}
+
+// One thread per directed entry: its place in the row and its slot in the row
+// table (emptied before).  Taking the entries side by side, each with its
+// combo in the key, needs no search for the combo and no loop over long rows.
+__global__ void k_load_scatter(const uint64_t* dkey, uint64_t M, const uint64_t* first, DevGraph g, uint32_t* pool) {
+  const KeyBits kb = g.kb;
   uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= M) return;
   const uint64_t k = dkey[j];
   if (!kb.real(k)) return;
-  const uint32_t x = kb.x_of(k);
-  pool[row_off[x] + (j - first[x])] = kb.y_of(k);
+  const uint32_t x = kb.x_of(k), y = kb.y_of(k);
+  const uint2 r = g.row[x];
+  pool[r.x + (j - first[x])] = y;
+  if (g.htab) row_table_insert(g, r, row_entry(y, kb.c_of(k) % g.n_el, g.hlb));
 }
 
 // Turns per-combo counts into row-relative segment offsets; dir[nc] = degree.
@@ -227,18 +287,66 @@ __global__ void k_ranges(const uint64_t* key, uint32_t cap, KeyBits kb, VRange* 
   ranges[i] = VRange{x, j, t - j, big};
 }
 
-__global__ void k_temporal_set(const VRange* ranges, const unsigned int* n_ranges, DevGraph g) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= *n_ranges) return;
-  const VRange r = ranges[i];
-  g.t_start[r.x] = r.start;
-  g.t_count[r.x] = r.count;
+__device__ __forceinline__ void temporal_put(const DevGraph& g, uint64_t key, uint64_t val) {
+  uint32_t s = temporal_slot(key, g.t_mask);
+  for (uint32_t n = 0; n <= g.t_mask; n++, s = (s + 1) & g.t_mask) {
+    if (atomicCAS((unsigned long long*)&g.t_tab[s].x, (unsigned long long)kTempEmpty, (unsigned long long)key) ==
+        kTempEmpty) {
+      g.t_tab[s].y = val;
+      return;
+    }
+  }
+  atomicExch(&g.ps->error, kErrListOverflow);  // no empty slot: more entries than the batch can have
 }
 
-__global__ void k_temporal_clear(const VRange* ranges, const unsigned int* n_ranges, DevGraph g) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= *n_ranges) return;
-  g.t_count[ranges[i].x] = 0;
+// Temporal entries of the batch (g.t_key, sorted): their number for each row,
+// the temporal table (emptied before), and the touched bit of every entry in
+// its row table, so that the search asks for an edge's presence only where it
+// can be in question.  Runs on the union graph, which holds every touched
+// entry.
+__global__ void k_temporal_set(uint32_t L, DevGraph g) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= L) return;
+  const uint64_t k = g.t_key[j];
+  if (!g.kb.real(k)) return;
+  const uint32_t x = g.kb.x_of(k);
+  if (g.htab && (j == 0 || g.t_key[j - 1] != k)) {
+    const uint2 r = g.row[x];
+    uint32_t* tab = g.htab + 2ull * r.x;
+    bool open;
+    const uint32_t s = row_locate(tab, r.y >> 2, row_entry(g.kb.y_of(k), g.kb.c_of(k) % g.n_el, g.hlb), open);
+    if (s != kSlotEmpty) tab[s] |= kSlotTouched;
+  }
+  const uint64_t before = j > 0 ? g.t_key[j - 1] : ~0ULL;
+  if (before != k) {  // the entry's intervals
+    uint32_t n = 1;
+    while (j + n < L && g.t_key[j + n] == k) n++;
+    const int2 s = g.t_span[j];
+    temporal_put(g, k, n == 1 ? (uint64_t)(uint32_t)(s.x + 1) | ((uint64_t)(uint32_t)s.y << 32)
+                              : kTempMany | (uint64_t)j | ((uint64_t)n << 32));
+  }
+  if (j > 0 && (before >> g.kb.yb) == (k >> g.kb.yb)) return;
+  uint32_t n = 1;  // the segment's entries
+  while (j + n < L && (g.t_key[j + n] >> g.kb.yb) == (k >> g.kb.yb)) n++;
+  temporal_put(g, temporal_head(g, x, g.kb.c_of(k)), (uint64_t)j | ((uint64_t)n << 32));
+  atomicAdd(&g.t_count[x], n);
+}
+
+// After the batch: the entries still in the graph lose the touched bit.
+__global__ void k_temporal_clear(uint32_t L, DevGraph g) {
+  const uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
+  if (j >= L) return;
+  const uint64_t k = g.t_key[j];
+  if (!g.kb.real(k)) return;
+  const uint32_t x = g.kb.x_of(k);
+  if (g.htab && (j == 0 || g.t_key[j - 1] != k)) {
+    const uint2 r = g.row[x];
+    uint32_t* tab = g.htab + 2ull * r.x;
+    bool open;
+    const uint32_t s = row_locate(tab, r.y >> 2, row_entry(g.kb.y_of(k), g.kb.c_of(k) % g.n_el, g.hlb), open);
+    if (s != kSlotEmpty) tab[s] &= ~kSlotTouched;
+  }
+  if (j == 0 || g.kb.x_of(g.t_key[j - 1]) != x) g.t_count[x] = 0;
 }
 
 __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges, DevGraph g) {
@@ -247,7 +355,7 @@ __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges,
   if (i < *n_ranges) {
     const VRange r = ranges[i];
     const uint32_t deg = g.dir[(size_t)r.x * (g.nc + 1) + g.nc];
-    if (deg + r.count > g.row_cap[r.x]) need = grow_cap(deg + r.count);
+    if (deg + r.count > g.row[r.x].y) need = grow_cap(deg + r.count);
   }
   // warp-aggregated add
   for (int o = 16; o; o >>= 1) need += __shfl_down_sync(0xffffffffu, need, o);
@@ -260,8 +368,43 @@ __global__ void k_compact_check(DevGraph g) {
   ps->compact = (ps->need > free_slots) ? 1u : 0u;
 }
 
+// Combo of the row-relative entry index i: upper_bound(dir, i) - 1.
+__device__ __forceinline__ uint32_t combo_at(const uint32_t* dirx, uint32_t nc, uint32_t i) {
+  uint32_t lo = 0, hi = nc;  // find last c with dirx[c] <= i
+  while (lo < hi) {
+    uint32_t mid = (lo + hi + 1) >> 1;
+    if (dirx[mid] <= i) lo = mid; else hi = mid - 1;
+  }
+  return lo;
+}
+
+// Barrier of a group of G threads (a warp or a block).
+template <int G>
+__device__ __forceinline__ void group_sync() {
+  if (G == 32) __syncwarp(); else __syncthreads();
+}
+
+// Builds row x's table from the row's entries (dirx: its directory, deg of
+// them), by G threads; no thread of another group touches the region.
+template <int G>
+__device__ __forceinline__ void row_table_build(const DevGraph& g, const uint32_t* pool, uint32_t x, uint2 row,
+                                                const uint32_t* dirx, uint32_t deg, uint32_t lane) {
+  uint32_t* tab = g.htab + 2ull * row.x;
+  for (uint32_t i = lane; i < 2u * row.y; i += G) tab[i] = kSlotEmpty;
+  if (lane == 0) g.htomb[x] = 0;
+  group_sync<G>();
+  for (uint32_t i = lane; i < deg; i += G)
+    row_table_insert(g, row, row_entry(pool[(uint64_t)row.x + i], combo_at(dirx, g.nc, i) % g.n_el, g.hlb));
+}
+
+// Deleted slots a row's table may hold before a deletion builds it afresh: a
+// quarter of the row's capacity keeps the table (twice the capacity) below
+// two thirds full, so that most buckets keep an empty slot.
+__device__ __forceinline__ uint32_t tomb_limit(uint32_t cap) { return max(4u, cap >> 2); }
+
 // Copies every row into the other pool with fresh slack (runs only when the
-// active pool cannot absorb this batch's relocations).
+// active pool cannot absorb this batch's relocations) and builds its table at
+// its new place; each warp moves the 32 rows its threads sized.
 __global__ void k_compact_copy(DevGraph g) {
   PoolState* ps = g.ps;
   if (!ps->compact) return;
@@ -270,6 +413,7 @@ __global__ void k_compact_copy(DevGraph g) {
   uint32_t* dp = g.pools[dst];
   __shared__ unsigned long long base;
   __shared__ uint32_t scan[1024];
+  const uint32_t lane = threadIdx.x & 31;
   for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x; v0 < g.n_cap; v0 += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t v = v0 + threadIdx.x;
     uint32_t deg = 0, cap = 0;
@@ -284,16 +428,22 @@ __global__ void k_compact_copy(DevGraph g) {
     }
     if (threadIdx.x == blockDim.x - 1) base = atomicAdd(&ps->top[dst], (unsigned long long)scan[threadIdx.x]);
     __syncthreads();
-    if (v < g.n_cap) {
-      const uint64_t off = base + scan[threadIdx.x] - cap;
-      if (off + cap > g.pool_cap) {
-        atomicExch(&ps->error, kErrPoolFull);
-      } else {
-        const uint64_t so = g.row_off[v];
-        for (uint32_t i = 0; i < deg; i++) dp[off + i] = sp[so + i];
-        g.row_off[v] = off;
-        g.row_cap[v] = cap;
-      }
+    const unsigned long long off = base + scan[threadIdx.x] - cap;
+    const bool fits = off + cap <= g.pool_cap;
+    if (!fits) atomicExch(&ps->error, kErrPoolFull);
+    const uint64_t so = (fits && v < g.n_cap) ? g.row[v].x : 0;
+    for (uint32_t r = 0; r < 32; r++) {
+      const uint32_t rdeg = __shfl_sync(0xffffffffu, fits ? deg : 0u, r), rcap = __shfl_sync(0xffffffffu, cap, r);
+      const uint32_t roff = (uint32_t)__shfl_sync(0xffffffffu, off, r), rso = (uint32_t)__shfl_sync(0xffffffffu, so, r);
+      for (uint32_t i = lane; i < rdeg; i += 32) dp[(uint64_t)roff + i] = sp[(uint64_t)rso + i];
+      __syncwarp();
+      const uint64_t x = v - lane + r;
+      if (rdeg && g.htab)
+        row_table_build<32>(g, dp, (uint32_t)x, make_uint2(roff, rcap), g.dir + x * (g.nc + 1), rdeg, lane);
+    }
+    if (v < g.n_cap && fits) {
+      g.row[v] = make_uint2((uint32_t)off, cap);
+      if (deg == 0 && g.htab) g.htomb[v] = 0;
     }
     __syncthreads();
   }
@@ -309,16 +459,6 @@ __global__ void k_compact_finish(DevGraph g) {
   ps->need = 0;
 }
 
-// Combo of the row-relative entry index i: upper_bound(dir, i) - 1.
-__device__ __forceinline__ uint32_t combo_at(const uint32_t* dirx, uint32_t nc, uint32_t i) {
-  uint32_t lo = 0, hi = nc;  // find last c with dirx[c] <= i
-  while (lo < hi) {
-    uint32_t mid = (lo + hi + 1) >> 1;
-    if (dirx[mid] <= i) lo = mid; else hi = mid - 1;
-  }
-  return lo;
-}
-
 __device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t* a, uint32_t lo, uint32_t hi, uint64_t x) {
   while (lo < hi) {
     uint32_t mid = (lo + hi) >> 1;
@@ -331,10 +471,6 @@ __device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t* a, uint32_t 
 // round reads G entries into registers before any thread writes, so a move
 // that overlaps its source is safe when left moves run front to back and
 // right moves back to front.
-template <int G>
-__device__ __forceinline__ void group_sync() {
-  if (G == 32) __syncwarp(); else __syncthreads();
-}
 template <int G>
 __device__ __forceinline__ void group_move_left(uint32_t* pool, uint64_t src, uint64_t dst, uint32_t n,
                                                 uint32_t lane) {
@@ -387,11 +523,12 @@ __global__ void k_mut_insert_g(const VRange* ranges, const unsigned int* n_range
     const uint32_t x = r.x, s = r.start, k = r.count;
     uint32_t* dirx = g.dir + (size_t)x * (g.nc + 1);
     const uint32_t deg = dirx[g.nc];
-    const uint64_t off = g.row_off[x];
+    const uint2 old = g.row[x];
+    const uint64_t off = old.x;
     const uint32_t new_deg = deg + k;
     uint64_t dst_off = off;
     uint32_t new_cap = 0;
-    if (new_deg > g.row_cap[x]) {
+    if (new_deg > old.y) {
       new_cap = grow_cap(new_deg);
       if (lane == 0) {
         unsigned long long o = atomicAdd(&ps->top[ps->active], (unsigned long long)new_cap);
@@ -431,8 +568,23 @@ __global__ void k_mut_insert_g(const VRange* ranges, const unsigned int* n_range
       const uint32_t add = lower_bound_u64(ins_key, s, s + k, g.kb.pack(x, 0, 0) + ((uint64_t)c << g.kb.yb)) - s;
       dirx[c] += add;
     }
-    if (lane == 0 && new_cap) { g.row_off[x] = dst_off; g.row_cap[x] = new_cap; }
+    const uint2 now = new_cap ? make_uint2((uint32_t)dst_off, new_cap) : old;
+    if (lane == 0 && new_cap) g.row[x] = now;
+    const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread before the build below clears it
     group_sync<G>();
+    // 5. row table: the new entries, or the whole table when the row moved or
+    // deleted slots would fill it past three quarters
+    if (g.htab) {
+      if (new_cap || new_deg + tomb > now.y + now.y / 2) {
+        row_table_build<G>(g, pool, x, now, dirx, new_deg, lane);
+      } else {
+        for (uint32_t j = lane; j < k; j += G) {
+          const uint64_t key = ins_key[s + j];
+          row_table_insert(g, now, row_entry(g.kb.y_of(key), g.kb.c_of(key) % g.n_el, g.hlb));
+        }
+      }
+      group_sync<G>();
+    }
   }
 }
 
@@ -456,17 +608,22 @@ __global__ void k_mut_delete_g(const VRange* ranges, const unsigned int* n_range
     const uint32_t x = r.x, s = r.start, k = r.count;
     uint32_t* dirx = g.dir + (size_t)x * (g.nc + 1);
     const uint32_t deg = dirx[g.nc];
-    const uint64_t off = g.row_off[x];
+    const uint2 row = g.row[x];
+    const uint64_t off = row.x;
     for (uint32_t j = lane; j < k; j += G) {
       const uint64_t key = del_key[s + j];
       const uint32_t c = g.kb.c_of(key), y = g.kb.y_of(key);
       del_pos[s + j] = (uint32_t)lower_bound_u32(pool + off, dirx[c], dirx[c + 1], y);
+      if (g.htab) row_table_delete(g, x, row, row_entry(y, c % g.n_el, g.hlb));
     }
     group_sync<G>();
+    const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread well before a build clears it
+    bool whole = true;
     for (uint32_t j = 0; j < k; j++) {
       const uint32_t a = del_pos[s + j] + 1, b = (j + 1 < k) ? del_pos[s + j + 1] : deg;
       if (a < j + 1 || a > deg) {  // a deleted entry missing from its row: leave the row, report
         if (lane == 0) atomicExch(&g.ps->error, kErrRowState);
+        whole = false;
         break;
       }
       if (b > a) group_move_left<G>(pool, off + a, off + a - (j + 1), b - a, lane);
@@ -476,6 +633,10 @@ __global__ void k_mut_delete_g(const VRange* ranges, const unsigned int* n_range
       dirx[c] -= sub;
     }
     group_sync<G>();
+    if (whole && tomb > tomb_limit(row.y)) {
+      row_table_build<G>(g, pool, x, row, dirx, deg - k, lane);
+      group_sync<G>();
+    }
   }
 }
 
@@ -492,73 +653,6 @@ void launch_mut_delete(const VRange* ranges, const unsigned int* n_ranges, const
                        cudaStream_t st) {
   k_mut_delete_g<32><<<warp_blocks, 256, 0, st>>>(ranges, n_ranges, del_key, del_pos, g);
   k_mut_delete_g<256><<<big_blocks, 256, 0, st>>>(ranges, n_ranges, del_key, del_pos, g);
-}
-
-// ------------------------------------------------------------ edge table
-
-__device__ __forceinline__ void edge_insert(const DevGraph& g, uint64_t key) {
-  uint64_t slot = edge_slot(key, g.emask);
-  for (uint64_t n = 0; n <= g.emask; n++) {
-    const uint64_t k = g.ekeys[slot];
-    if (k == key) return;
-    if (k == kEdgeEmpty) {
-      const unsigned long long prev =
-          atomicCAS((unsigned long long*)&g.ekeys[slot], (unsigned long long)kEdgeEmpty, (unsigned long long)key);
-      if (prev == kEdgeEmpty || prev == key) return;  // placed here, or by another thread inserting the same key
-    }
-    slot = (slot + 1) & g.emask;
-  }
-  atomicExch(&g.ps->error, kErrEdgeTable);  // no empty slot left
-}
-
-__device__ __forceinline__ void edge_delete(const DevGraph& g, uint64_t key) {
-  uint64_t slot = edge_slot(key, g.emask);
-  for (uint64_t n = 0; n <= g.emask; n++) {
-    const uint64_t k = g.ekeys[slot];
-    if (k == key) {
-      atomicCAS((unsigned long long*)&g.ekeys[slot], (unsigned long long)key, (unsigned long long)kEdgeTomb);
-      return;
-    }
-    if (k == kEdgeEmpty) return;
-    slot = (slot + 1) & g.emask;
-  }
-}
-
-// One warp per row: the lanes take the row's entries 32 at a time and find
-// each entry's combo by a binary search in the row's directory, so that a
-// row's insertions run side by side (combos hold a few entries each: looping
-// over combos left most lanes idle and the insertions one after another).
-__global__ void k_edge_fill(DevGraph g) {
-  const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  const uint32_t* pool = g.pools[g.ps->active];
-  for (uint32_t v = warp; v < g.n; v += nwarps) {
-    const uint32_t* dirv = g.dir + (size_t)v * (g.nc + 1);
-    const uint32_t total = dirv[g.nc];
-    if (total == 0) continue;
-    const uint64_t off = g.row_off[v];
-    for (uint32_t i = lane; i < total; i += 32) {
-      uint32_t lo = 0, hi = g.nc - 1;  // the last combo c with dirv[c] <= i: its segment holds entry i
-      while (lo < hi) {
-        const uint32_t mid = (lo + hi + 1) >> 1;
-        if (dirv[mid] <= i) lo = mid; else hi = mid - 1;
-      }
-      const uint32_t w = pool[off + i];
-      if (v < w) edge_insert(g, edge_key(v, w, lo % g.n_el));
-    }
-  }
-}
-
-__global__ void k_edge_list(const uint64_t* keys, uint32_t L, DevGraph g, uint32_t del) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= L) return;
-  const uint64_t k = keys[i];
-  if (!g.kb.real(k)) return;
-  const uint32_t x = g.kb.x_of(k), y = g.kb.y_of(k);
-  if (x >= y) return;
-  const uint64_t ek = edge_key(x, y, g.kb.c_of(k) % g.n_el);
-  if (del) edge_delete(g, ek); else edge_insert(g, ek);
 }
 
 // ------------------------------------------------- one update per launch
@@ -604,7 +698,7 @@ __global__ void k_plain_resolve(const csm_update* up, DevGraph g, UpdInfo* info,
           for (int k = 0; k < 2; k++) {
             const uint32_t v = ends[k];
             const uint32_t deg = g.dir[(size_t)v * (g.nc + 1) + g.nc];
-            if (deg + 1 > g.row_cap[v]) need += grow_cap(deg + 1);
+            if (deg + 1 > g.row[v].y) need += grow_cap(deg + 1);
           }
           ps->need = need;
           ps->compact = (need > g.pool_cap - ps->top[ps->active]) ? 1u : 0u;
@@ -647,7 +741,9 @@ __global__ void __launch_bounds__(256) k_plain_mutate(DevGraph g, const UpdInfo*
       const uint32_t x = g.kb.x_of(key), c = g.kb.c_of(key), y = g.kb.y_of(key);
       uint32_t* dirx = g.dir + (size_t)x * (g.nc + 1);
       const uint32_t deg = dirx[g.nc];
-      const uint64_t off = g.row_off[x];
+      const uint2 old = g.row[x];
+      const uint64_t off = old.x;
+      const uint32_t entry = row_entry(y, c % g.n_el, g.hlb);
       if (lane == 0) {
         s_pos = (uint32_t)lower_bound_u32(pool + off, dirx[c], dirx[c + 1], y);
         s_bad = 0;
@@ -662,7 +758,7 @@ __global__ void __launch_bounds__(256) k_plain_mutate(DevGraph g, const UpdInfo*
       if (add) {
         uint64_t dst = off;
         uint32_t new_cap = 0;
-        if (deg + 1 > g.row_cap[x]) {
+        if (deg + 1 > old.y) {
           new_cap = grow_cap(deg + 1);
           if (lane == 0) {
             unsigned long long o = atomicAdd(&ps->top[ps->active], (unsigned long long)new_cap);
@@ -679,18 +775,28 @@ __global__ void __launch_bounds__(256) k_plain_mutate(DevGraph g, const UpdInfo*
         }
         if (lane == 0) pool[dst + p] = y;
         for (uint32_t cc = c + 1 + lane; cc <= g.nc; cc += 256) dirx[cc] += 1;
-        if (lane == 0 && new_cap) { g.row_off[x] = dst; g.row_cap[x] = new_cap; }
+        const uint2 now = new_cap ? make_uint2((uint32_t)dst, new_cap) : old;
+        if (lane == 0 && new_cap) g.row[x] = now;
+        const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread before the build below clears it
+        __syncthreads();
+        if (g.htab) {  // the row table follows, as in k_mut_insert_g
+          if (new_cap || deg + 1 + tomb > now.y + now.y / 2)
+            row_table_build<256>(g, pool, x, now, dirx, deg + 1, lane);
+          else if (lane == 0)
+            row_table_insert(g, now, entry);
+        }
       } else {
         group_move_left<256>(pool, off + p + 1, off + p, deg - p - 1, lane);
         for (uint32_t cc = c + 1 + lane; cc <= g.nc; cc += 256) dirx[cc] -= 1;
+        const uint32_t tomb = g.htab ? g.htomb[x] + 1u : 0u;
+        __syncthreads();
+        if (tomb > tomb_limit(old.y))
+          row_table_build<256>(g, pool, x, old, dirx, deg - 1, lane);
+        else if (g.htab && lane == 0)
+          row_table_delete(g, x, old, entry);
       }
       __syncthreads();
     }
-  }
-  if (g.emask && (inf.flags & UF_MUT) && lane == 0) {  // the edge table follows the rows
-    const uint64_t k0 = keys[0];
-    const uint64_t ek = edge_key(g.kb.x_of(k0), g.kb.y_of(k0), g.kb.c_of(k0) % g.n_el);
-    if (inf.flags & UF_ADD) edge_insert(g, ek); else edge_delete(g, ek);
   }
   if (out && lane == 0) {
     // an update whose label triple matches no query edge: nothing to count
@@ -713,7 +819,7 @@ __global__ void k_vdel_keys(DevGraph g, uint32_t v, uint32_t deg, uint64_t* keys
   if (i >= deg) return;
   const uint32_t* pool = g.pools[g.ps->active];
   const uint32_t* dirv = g.dir + (size_t)v * (g.nc + 1);
-  const uint32_t y = pool[g.row_off[v] + i];
+  const uint32_t y = pool[(uint64_t)g.row[v].x + i];
   const uint32_t c = combo_at(dirv, g.nc, i);
   const uint32_t el = c % g.n_el;
   keys[2 * i] = g.kb.pack(v, c, y);

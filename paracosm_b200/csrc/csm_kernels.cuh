@@ -19,8 +19,8 @@ __global__ void k_load_directed(const uint64_t* ukey, const uint64_t* uidx, uint
 __global__ void k_load_count(const uint64_t* dkey, uint64_t M, KeyBits kb, uint32_t nc, uint32_t* dir,
                              uint64_t* first, unsigned long long* n_valid);
 __global__ void k_load_caps(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t* cap, uint64_t* cap64);
-__global__ void k_load_scatter(const uint64_t* dkey, uint64_t M, KeyBits kb, const uint64_t* first,
-                               const uint64_t* row_off, uint32_t* pool);
+__global__ void k_load_rows(const uint64_t* off, const uint32_t* cap, uint32_t n_cap, uint2* row);
+__global__ void k_load_scatter(const uint64_t* dkey, uint64_t M, const uint64_t* first, DevGraph g, uint32_t* pool);
 __global__ void k_dir_scan(uint32_t* dir, uint32_t n_cap, uint32_t nc);
 
 // ---- batch preparation ----
@@ -37,8 +37,16 @@ __global__ void k_resolve(const uint64_t* skey, const uint32_t* sseq, uint32_t B
 constexpr uint32_t kBigRow = 4096;  // rows longer than this are mutated by a whole block
 __global__ void k_ranges(const uint64_t* key, uint32_t cap, KeyBits kb, VRange* ranges, unsigned int* n_ranges,
                          const uint32_t* dir, uint32_t nc);
-__global__ void k_temporal_set(const VRange* ranges, const unsigned int* n_ranges, DevGraph g);
-__global__ void k_temporal_clear(const VRange* ranges, const unsigned int* n_ranges, DevGraph g);
+__global__ void k_temporal_set(uint32_t L, DevGraph g);
+__global__ void k_temporal_clear(uint32_t L, DevGraph g);
+// Slots of the temporal table (DevGraph::t_tab) for a batch of B updates: a
+// power of two, at most a quarter full (two directed entries an update, and a
+// head for each of their segments).
+__host__ __device__ inline uint32_t temporal_slots(uint32_t B) {
+  uint32_t s = 64;
+  while (s < 16u * B) s <<= 1;
+  return s;
+}
 __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges, DevGraph g);
 __global__ void k_compact_check(DevGraph g);
 __global__ void k_compact_copy(DevGraph g);
@@ -50,15 +58,6 @@ void launch_mut_delete(const VRange* ranges, const unsigned int* n_ranges, const
                        uint32_t* del_pos, const DevGraph& g, uint32_t warp_blocks, uint32_t big_blocks,
                        cudaStream_t st);
 __global__ void k_vdel_keys(DevGraph g, uint32_t v, uint32_t deg, uint64_t* keys);
-
-// ---- edge table (csm_kernels.cu) ----
-// Inserts every (edge, label) of the CSR (one warp per row, from the row of
-// the smaller endpoint).
-__global__ void k_edge_fill(DevGraph g);
-// Inserts (del = 0) or deletes (del = 1) the edges of a packed-key list of
-// directed entries (x, combo, y) (the batch lists; each edge appears in both
-// directions and is taken from x < y).
-__global__ void k_edge_list(const uint64_t* keys, uint32_t L, DevGraph g, uint32_t del);
 
 // ---- one edge update per launch sequence (the plain form; csm_kernels.cu) ----
 // keys[0..1]: the update's two directed entries (sentinels when the graph does
@@ -81,7 +80,8 @@ struct DTask {
   uint16_t anchor;
   uint8_t orient;
   uint8_t depth;
-  uint32_t dlo, dn, dsel;
+  uint32_t dlo, dn;
+  uint32_t sel;  // driver and first join (back entries; LevelSM::dsel, jsel in bits 8 and up)
   uint32_t m[kMaxQ];
   uint32_t pad[3];
 };
@@ -94,9 +94,13 @@ static_assert(sizeof(DTask) == 160, "DTask is 160 bytes");
 // so records go to waiting warps in ticket order and tail never passes head.
 // `pending` counts this launch's tasks (root and donated) that are not
 // finished, and waiting warps exit when it reaches zero.
+// The words lie on cache lines of their own: waiting warps read `pending` all
+// the time, busy ones read and write the others.
 struct SearchQueue {
-  unsigned long long head, tail;
-  unsigned int hungry, pending;
+  alignas(128) unsigned long long head;
+  alignas(128) unsigned long long tail;
+  alignas(128) unsigned int hungry;
+  alignas(128) unsigned int pending;
 };
 
 // Cumulative search counters (device memory, read by csm_gpu_stats).
@@ -166,14 +170,21 @@ struct SearchParams {
   // nonzero: count each anchor's independent tail (PlanAnchor::tail_at)
   // instead of enumerating it; only for counts without hashes or match sets
   uint32_t tail;
+  uint32_t levels, warp_bytes;  // SearchShape
 };
 __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* plan, const uint64_t* d2,
                        uint64_t d2_words, Task* tasks, unsigned int* n_tasks, uint32_t task_cap,
                        uint32_t* safe, unsigned int* error, uint32_t shard_rank = 0, uint32_t shard_count = 1,
                        uint32_t turboflux_compat = 0, uint32_t dup_zero = 0);
-size_t search_smem_bytes(uint32_t n_q, uint32_t warps);
-uint32_t search_max_blocks(uint32_t n_q, uint32_t warps, int mode = 0);  // mode: 0 plain, 1 match sets, 2 tail counting
-void launch_search(const SearchParams& p, uint32_t n_q, uint32_t blocks, uint32_t warps, cudaStream_t s);
+// mode: 0 plain, 1 match sets, 2 tail counting
+struct SearchShape {
+  uint32_t levels;      // levels of a warp's walk
+  uint32_t warp_bytes;  // shared memory of a warp
+};
+SearchShape search_shape_of(const Plan& plan, int mode);
+uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode);
+int search_mode(const SearchParams& p);
+void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s);
 __global__ void k_finalize(uint32_t B, const UpdInfo* info, const unsigned long long* count,
                            const unsigned long long* hash, const unsigned long long* bytes, const uint32_t* safe,
                            const unsigned int* stop, uint64_t cap, int want_hash, csm_result* out,

@@ -34,6 +34,7 @@ struct CtxView {
   uint64_t cap;
   int homo, want_hash;
   uint32_t warps, bps;
+  SearchShape shape;
   uint32_t dup_zero;       // CaLiG: an insertion of a present edge counts 0
   cudaEvent_t owner_end;   // attached query: end of the owner's last submit (null otherwise)
 };
@@ -180,7 +181,9 @@ extern "C" int csm_gpu_probe_noalloc(csm_ctx* ctx, uint32_t n, const csm_update*
   sp.task_limit_ns = 20ull * 1000000000ull;
   sp.batch = n;
   sp.sstat = sstat;
-  launch_search(sp, v.nq, (uint32_t)v.sm_count * v.bps, v.warps, v.st);
+  sp.levels = v.shape.levels;
+  sp.warp_bytes = v.shape.warp_bytes;
+  launch_search(sp, (uint32_t)v.sm_count * v.bps, v.warps, v.st);
   k_probe_out<<<nb, 256, 0, v.st>>>(n, info, count, v.cap, d_counts);
   e = cudaGetLastError();
   if (e != cudaSuccess) return set_err(CSM_ECUDA, "probe launch: %s", cudaGetErrorString(e));

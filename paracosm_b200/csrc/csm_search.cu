@@ -14,29 +14,58 @@
 // level holds up to 32 partial matches at once: to extend level d the warp
 // takes the next 32 (entry, driver element) pairs of level d's entries -- the
 // driver being the smallest back-neighbour segment -- so lanes stay busy even
-// when segments are a few elements long.  Every lane checks its candidate
-// against the other back-neighbour segments (binary search), the same-label
-// matched vertices (injectivity), the candidate filter, and the batch-time
-// presence of every back edge; survivors are compacted with a ballot into
-// level d + 1 together with the driver segment of their own next level
-// (an empty next-level segment prunes them right away).  Leaves are only
-// counted.
+// when segments are a few elements long.  A step first applies the two tests
+// that settle most candidates and need nothing but the entry -- the candidate
+// filter's bit and one probe of a row table -- and only the candidates left
+// rebuild their prefix for the other joins, the same-label matched vertices
+// (injectivity) and the batch-time presence of every back edge; survivors are
+// compacted with a ballot into level d + 1 together with the driver segment
+// of their own next level (an empty next-level segment prunes them right
+// away).  Leaves are only counted.
+#include <algorithm>
+
 #include "csm_kernels.cuh"
 
 namespace csm {
 
+// One level of a warp's walk: up to 32 partial matches, each with the driver
+// segment of the next position.  The segments are laid end to end, so the
+// level's work is the range [cur, total) of (entry, driver element) pairs and
+// a pair's pool offset is base[entry] + its place in the range.
+// Level 1 has one entry: v[0] is position 1's vertex, and its parent, v[1],
+// position 0's.
 struct LevelSM {
   uint32_t v[32];     // data vertex of this level's position
-  uint32_t dlo[32];   // driver segment of the next position: pool offset
-  uint32_t dn[32];    //   and length
+  uint32_t incl[32];  // end of each entry's driver segment in the range
+  uint32_t base[32];  // pool offset of the segment minus its start in the range
+  uint32_t jv[32];    // matched vertex of the entry's first join
   uint8_t par[32];    // entry index in the previous level
   uint8_t dsel[32];   // back entry that is the driver
-  uint32_t cnt, cur_e, cur_k, pad;
+  uint8_t jsel[32];   // back entry of the first join: the smallest segment but the driver's
+  uint32_t cnt, cur, total, pad;
 };
 
-size_t search_smem_bytes(uint32_t n_q, uint32_t warps) {
-  const uint32_t levels = n_q > 2 ? n_q - 2 : 1;
-  return (size_t)warps * levels * sizeof(LevelSM);
+// Levels a walk of this plan may use: 1 .. n - 2, or, where every order's
+// independent tail is counted, up to the tail with the class counters of
+// tail_stage above it.
+static uint32_t search_levels(const Plan& plan, int mode) {
+  const uint32_t n = plan.n;
+  uint32_t levels = n > 2 ? n - 2 : 1;
+  if (mode != 2) return levels;
+  constexpr uint32_t kCounters = (((1u << kTailGroup) - 1u) * 32u * 4u + sizeof(LevelSM) - 1) / sizeof(LevelSM);
+  uint32_t need = 1;
+  for (uint32_t a = 0; a < plan.n_anchor; a++)
+    need = std::max<uint32_t>(need, plan.anchors[a].tail_at ? plan.anchors[a].tail_at + kCounters : levels);
+  return need;
+}
+
+// Shared memory of one warp: its levels, then its walk's plan (WalkPlan).
+SearchShape search_shape_of(const Plan& plan, int mode) {
+  SearchShape s;
+  s.levels = search_levels(plan, mode);
+  const uint32_t words = 3 * plan.n + (plan.n_anchor ? plan.n_anchor - 1 : 0);  // every query edge but the anchor is a back entry once
+  s.warp_bytes = s.levels * (uint32_t)sizeof(LevelSM) + ((4 * words + 15) & ~15u);
+  return s;
 }
 
 __device__ __forceinline__ bool d2_bit(const uint64_t* d2, uint64_t words, uint32_t q, uint32_t v) {
@@ -92,178 +121,185 @@ __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
   return v;
 }
 
-// Bounds of up to four back segments of one position for one prefix, with
-// the batch touch count of each row (0: the row holds no entry inserted or
-// deleted in this batch, so every entry of it is present at every batch time).
-struct SegQuad {
-  uint32_t v[4], c[4], lo[4], hi[4], tc[4];
+// A walk's order in the warp's shared memory, copied from the plan when a task
+// starts: three words a position (query vertex, back entries and the first
+// one; same-label positions; positions with a back entry), then one word a
+// back entry (position, edge label, combo).  Every step reads it, and L1 is
+// swept by the search's random loads.
+struct WalkPlan {
+  const uint32_t* w;
+  uint32_t n;
+  __device__ __forceinline__ uint32_t qv(uint32_t pos) const { return w[3 * pos] & 0xffu; }
+  __device__ __forceinline__ uint32_t nb(uint32_t pos) const { return (w[3 * pos] >> 8) & 0xffu; }
+  __device__ __forceinline__ uint32_t samelab(uint32_t pos) const { return w[3 * pos + 1]; }
+  __device__ __forceinline__ uint32_t backmask(uint32_t pos) const { return w[3 * pos + 2]; }
+  __device__ __forceinline__ uint32_t back(uint32_t pos, uint32_t b) const {
+    return w[3 * n + (w[3 * pos] >> 16) + b];
+  }
 };
+__device__ __forceinline__ uint32_t back_el(uint32_t w) { return (w >> 8) & 0xffu; }
+__device__ __forceinline__ uint32_t back_combo(uint32_t w) { return w >> 16; }
 
-// Loads back entries b0 .. b0 + 3 of position P for prefix m: all loads are
-// independent, so the quad costs one round trip to L2.  The bounds of entry
-// `skip` are not loaded (the driver: the candidate came from it), but its
-// touch count is (its edge still needs the batch-time presence test).
-__device__ __forceinline__ void load_quad(const DevGraph& g, const PlanAnchor* A, const PlanPos& P, uint32_t b0,
-                                          const uint32_t* m, uint32_t skip, SegQuad& s) {
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t b = b0 + (uint32_t)i;
-    s.v[i] = 0; s.c[i] = 0; s.lo[i] = 0; s.hi[i] = 0; s.tc[i] = 0;
-    if (b < P.nb) {
-      s.v[i] = m[A->back_pos[P.boff + b]];
-      s.c[i] = A->back_combo[P.boff + b];
-      if (b != skip) {
-        const uint32_t* d = g.dir + (size_t)s.v[i] * (g.nc + 1) + s.c[i];
-        const uint32_t base = (uint32_t)g.row_off[s.v[i]];
-        s.lo[i] = base + d[0];
-        s.hi[i] = base + d[1];
-      }
-      s.tc[i] = g.t_count[s.v[i]];
-    }
+// `same`: the same-label positions an injectivity test looks at (none under
+// homomorphism; only those before the tail when it is counted).
+__device__ __forceinline__ void load_walk_plan(uint32_t* w, const PlanAnchor* A, uint32_t n, uint32_t same,
+                                               uint32_t lane) {
+  uint32_t backs = 0;
+  if (lane < n) {
+    const PlanPos P = A->pos[lane];
+    uint32_t bm = 0;
+#pragma unroll 1
+    for (uint32_t b = 0; b < P.nb; b++) bm |= 1u << A->back_pos[P.boff + b];
+    w[3 * lane] = (uint32_t)P.qv | ((uint32_t)P.nb << 8) | ((uint32_t)P.boff << 16);
+    w[3 * lane + 1] = P.samelab & same;
+    w[3 * lane + 2] = bm;
+    backs = (uint32_t)P.boff + P.nb;
+  }
+  backs = __reduce_max_sync(0xffffffffu, backs);
+  for (uint32_t i = lane; i < backs; i += 32)
+    w[3 * n + i] = (uint32_t)A->back_pos[i] | ((uint32_t)A->back_el[i] << 8) | ((uint32_t)A->back_combo[i] << 16);
+  __syncwarp();
+}
+
+// Visits (position, data vertex) of the prefix of entry e of level d, the
+// last position first.  Every position is read from the levels when it is
+// needed: a copy of the prefix per lane would be local memory, and the random
+// loads leave it no room in L1.
+template <class F>
+__device__ __forceinline__ void walk_prefix(const LevelSM* lv, int d, uint32_t e, F visit) {
+#pragma unroll 1
+  for (int j = d; j >= 0; --j) {
+    const LevelSM& S = lv[j ? j : 1];
+    visit((uint32_t)j, S.v[e]);
+    e = S.par[e];
   }
 }
 
-// Is x in each loaded segment of the quad (every entry but `skip`), and is
-// every back edge of the quad present at batch time t?  The lower-bound
-// searches of the four segments advance in lockstep (one round trip per
-// round); a probe that lands on x ends that search, so no separate load
-// confirms the final position (if x is in the segment, the search must probe
-// its slot before it can end there).
-__device__ __forceinline__ bool quad_joins(const DevGraph& g, const uint32_t* pool, const PlanPos& P, uint32_t b0,
-                                           uint32_t skip, uint32_t x, int32_t t, SegQuad& s) {
-  uint32_t need = 0, found = 0;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    const uint32_t b = b0 + (uint32_t)i;
-    if (b < P.nb && b != skip) need |= 1u << i;
-  }
-  for (;;) {
-    bool more = false;
-#pragma unroll
-    for (int i = 0; i < 4; i++) {
-      if (s.lo[i] < s.hi[i]) {
-        const uint32_t mid = (s.lo[i] + s.hi[i]) >> 1;
-        const uint32_t val = pool[mid];
-        if (val < x) s.lo[i] = mid + 1;
-        else if (val > x) s.hi[i] = mid;
-        else { found |= 1u << i; s.hi[i] = s.lo[i]; }
-        more = true;
-      }
-    }
-    if (!more) break;
-  }
-  if ((found & need) != need) return false;
-#pragma unroll
-  for (int i = 0; i < 4; i++) {
-    if (b0 + (uint32_t)i >= P.nb || s.tc[i] == 0) continue;
-    if (!present_at(g, s.v[i], s.c[i], x, t)) return false;
-  }
-  return true;
+// Candidate filter bit of x for query vertex qv.
+__device__ __forceinline__ bool filter_bit(const SearchParams& p, uint32_t qv, uint32_t x) {
+  return !p.d2 || ((ld_gather(p.d2 + (uint64_t)qv * p.d2_words + (x >> 6)) >> (x & 63)) & 1ULL);
 }
 
-// Full candidate check of data vertex x for position `pos` given the matched
-// prefix m[0 .. pos-1]; `dsel` is the back entry whose segment produced x and
-// q0 the first quad of pos's back entries, already loaded (load_quad with
-// skip = dsel).  The candidate-filter word is loaded before the first join
-// round and tested after it, so the two round trips overlap.
-__device__ __forceinline__ bool check_candidate_q(const SearchParams& p, const uint32_t* pool, const PlanAnchor* A,
-                                                  uint32_t pos, uint32_t x, const uint32_t* m, uint32_t dsel,
-                                                  int32_t t, SegQuad& q0, uint32_t lab_mask = 0xffffffffu) {
-  const PlanPos P = A->pos[pos];
-  const uint64_t fw = p.d2 ? p.d2[(uint64_t)P.qv * p.d2_words + (x >> 6)] : ~0ULL;
-  bool ok = true;
-  if (!p.homo) {
-    for (uint32_t mk = P.samelab & lab_mask; mk; mk &= mk - 1) ok &= m[__ffs(mk) - 1] != x;
-  }
-  if (!ok) return false;
-  ok = quad_joins(p.g, pool, P, 0, dsel, x, t, q0);
-  if (!((fw >> (x & 63)) & 1ULL)) return false;
-  if (!ok) return false;
-  for (uint32_t b0 = 4; b0 < P.nb; b0 += 4) {
-    SegQuad q;
-    load_quad(p.g, A, P, b0, m, dsel, q);
-    if (!quad_joins(p.g, pool, P, b0, dsel, x, t, q)) return false;
-  }
-  return true;
+// The paths few candidates take are functions of their own: inlined and
+// unrolled into every use they made the search 290 KB of code, several times
+// the instruction cache, and warps waited for instructions as long as for
+// data (7.8 of 33 cycles per instruction on a graph that stays in L2).
+__device__ __noinline__ bool present_slow(const SearchParams& p, uint32_t v, uint32_t c, uint32_t w, int32_t t) {
+  return touched_present(p.g, v, c, w, t);
+}
+__device__ __noinline__ uint32_t seg_size_slow(const SearchParams& p, uint32_t v, uint32_t c, uint32_t lo, uint32_t hi,
+                                               int32_t t) {
+  return seg_size_at(p.g, v, c, lo, hi, t);
+}
+// Join without row tables: a binary search in v's segment.
+__device__ __noinline__ uint32_t join_search(const SearchParams& p, const uint32_t* pool, uint32_t v, uint32_t c,
+                                             uint32_t x) {
+  uint64_t lo, hi;
+  segment(p.g, v, c, lo, hi);
+  if (!contains_u32(pool, lo, hi, x)) return kSlotEmpty;
+  return p.g.t_count[v] ? kSlotTouched : 0u;
 }
 
-// The same check with the edge table (DevGraph::ekeys): each join is one
-// probe for the key of edge (m[b], x) with back entry b's edge label.  The
-// candidate-filter word comes first (the filter is small and stays in L2),
-// then the joins one at a time, stopping at the first that fails: the table
-// is larger than L2, every probe of it is a random line fetched from HBM, and
-// HBM is what bounds this search -- most candidates fail their first join,
-// and probing all back entries at once (four in flight) fetched three times
-// the lines for a candidate that one probe settles.  The batch-time presence
-// of the back edges is tested for the candidates that pass.
-__device__ __forceinline__ bool check_candidate_h(const SearchParams& p, const PlanAnchor* A, uint32_t pos,
-                                                  uint32_t x, const uint32_t* m, uint32_t dsel, int32_t t,
-                                                  uint32_t lab_mask = 0xffffffffu) {
-  const PlanPos P = A->pos[pos];
+// Is x a neighbour of v over back entry bw?  kSlotEmpty when it is not, else
+// a word whose touched bit says that the edge's presence intervals must be
+// asked.  One probe of v's row table, or a binary search in v's segment where
+// the graph has no tables.
+__device__ __forceinline__ uint32_t join_find(const SearchParams& p, const uint32_t* pool, uint32_t v, uint32_t bw,
+                                              uint32_t x) {
+  if (p.g.htab) return row_find(p.g, p.g.row[v], row_entry(x, back_el(bw), p.g.hlb));
+  return join_search(p, pool, v, back_combo(bw), x);
+}
+
+// The tests of candidate x for position `pos` beyond the filter bit, for the
+// prefix of entry e of level d: injectivity, every join, the batch-time
+// presence of every back edge.  `dsel` is the back entry whose segment
+// produced x (0xff: none) and `joined` one that was found before, with word
+// jhit (0xff: none).  The joins run one at a time and stop at the first that
+// fails.
+__device__ __forceinline__ bool check_rest(const SearchParams& p, const uint32_t* pool, const LevelSM* lv,
+                                           const WalkPlan& wp, int d, uint32_t e, uint32_t pos, uint32_t x,
+                                           uint32_t dsel, uint32_t joined, uint32_t jhit, int32_t t) {
   const DevGraph& g = p.g;
-  const uint64_t fw = p.d2 ? ld_stream(p.d2 + (uint64_t)P.qv * p.d2_words + (x >> 6)) : ~0ULL;
+  const uint32_t same = wp.samelab(pos), bm = wp.backmask(pos);
+  uint32_t b = wp.nb(pos);
   bool ok = true;
-  if (!p.homo) {
-    for (uint32_t mk = P.samelab & lab_mask; mk; mk &= mk - 1) ok &= m[__ffs(mk) - 1] != x;
-  }
-  if (!ok) return false;
-  if (!((fw >> (x & 63)) & 1ULL)) return false;
-  for (uint32_t b = 0; b < P.nb; b++) {
-    if (b == dsel) continue;
-    const uint64_t key = edge_key(m[A->back_pos[P.boff + b]], x, A->back_combo[P.boff + b] % g.n_el);
-    const uint64_t slot = edge_slot(key, g.emask);
-    if (!edge_probe_rest(g, key, slot, ld_stream(g.ekeys + slot))) return false;
-  }
-  for (uint32_t b = 0; b < P.nb; b++) {
-    const uint32_t v = m[A->back_pos[P.boff + b]];
-    if (g.t_count[v] && !present_at(g, v, A->back_combo[P.boff + b], x, t)) return false;
-  }
-  return true;
+  walk_prefix(lv, d, e, [&](uint32_t j, uint32_t v) {
+    if ((same >> j) & 1u) ok = ok && v != x;
+    if ((bm >> j) & 1u) {
+      --b;
+      if (ok && (b != dsel || g.t_count[v])) {
+        const uint32_t bw = wp.back(pos, b);
+        const uint32_t hit = b == joined ? jhit : join_find(p, pool, v, bw, x);
+        ok = hit != kSlotEmpty && (!(hit & kSlotTouched) || present_slow(p, v, back_combo(bw), x, t));
+      }
+    }
+  });
+  return ok;
 }
 
-// The same check when no quad was prefetched.
-__device__ __forceinline__ bool check_candidate(const SearchParams& p, const uint32_t* pool, const PlanAnchor* A,
-                                                uint32_t pos, uint32_t x, const uint32_t* m, uint32_t dsel,
-                                                int32_t t, uint32_t lab_mask = 0xffffffffu) {
-  if (p.g.emask) return check_candidate_h(p, A, pos, x, m, dsel, t, lab_mask);
-  SegQuad q0;
-  load_quad(p.g, A, A->pos[pos], 0, m, dsel, q0);
-  return check_candidate_q(p, pool, A, pos, x, m, dsel, t, q0, lab_mask);
-}
-
-// Number of entries of segment (v, c) = [lo, hi) present at batch time t,
-// given the row's touch count tc (seg_size_at with the count already loaded).
-__device__ __forceinline__ uint32_t seg_size_tc(const DevGraph& g, uint32_t v, uint32_t c, uint32_t lo, uint32_t hi,
-                                                uint32_t tc, int32_t t) {
-  if (tc == 0 || hi == lo) return hi - lo;
-  return seg_size_at(g, v, c, lo, hi, t);
-}
-
-// Driver segment of position np for prefix m (the smallest union-graph back
-// segment); false if some back segment is empty at batch time t.  `bytes`
-// receives 4 B x the sizes at time t of all back segments: the algorithmic
-// bytes of expanding this node.  Segment bounds and touch counts are loaded
-// four back entries at a time.
-__device__ __forceinline__ bool pick_driver(const SearchParams& p, const PlanAnchor* A, uint32_t np,
-                                            const uint32_t* m, int32_t t, uint32_t& dlo, uint32_t& dn,
-                                            uint32_t& dsel, unsigned long long& bytes) {
-  const PlanPos P = A->pos[np];
-  uint32_t best = 0xffffffffu;
+// Driver of position np (the smallest union-graph back segment, the first of
+// equals) for the prefix of entry e of level d, continued by x at position
+// d + 1 when `with_x`; false if some back segment is empty at batch time t.
+// `jsel` and `jv` are the first join -- the back entry of the smallest segment
+// but the driver's, and its vertex: the row most likely to lack a candidate,
+// and the row table whose lines a warp's lanes share most -- and `bytes`
+// receives 4 B x the sizes at time t of all back segments: the
+// algorithmic bytes of expanding this node.  Segment bounds and touch counts
+// are loaded four back entries at a time, all loads independent.
+__device__ __forceinline__ bool pick_driver(const SearchParams& p, const LevelSM* lv, const WalkPlan& wp, int d,
+                                            uint32_t e, bool with_x, uint32_t x, uint32_t np, int32_t t,
+                                            uint32_t& dlo, uint32_t& dn, uint32_t& dsel, uint32_t& jsel,
+                                            uint32_t& jv, unsigned long long& bytes) {
+  const DevGraph& g = p.g;
+  const uint32_t nb = wp.nb(np), bm = wp.backmask(np);
+  uint32_t best = 0xffffffffu, second = 0xffffffffu, dv = 0;
+  jsel = 0; jv = 0;
   bool empty = false;
   unsigned long long b4 = 0;
-  for (uint32_t b0 = 0; b0 < P.nb; b0 += 4) {
-    SegQuad q;
-    load_quad(p.g, A, P, b0, m, 0xffffffffu, q);
+#pragma unroll 1
+  for (uint32_t end = nb; end > 0;) {
+    const uint32_t beg = end > 4u ? end - 4u : 0u;
+    uint32_t v[4] = {0, 0, 0, 0};
+    uint32_t b = nb;
+    auto visit = [&](uint32_t j, uint32_t u) {
+      if ((bm >> j) & 1u) {
+        --b;
 #pragma unroll
-    for (int i = 0; i < 4; i++) {
-      const uint32_t b = b0 + (uint32_t)i;
-      if (b >= P.nb) continue;
-      const uint32_t sz = q.hi[i] - q.lo[i];
-      const uint32_t szt = seg_size_tc(p.g, q.v[i], q.c[i], q.lo[i], q.hi[i], q.tc[i], t);
-      b4 += 4ull * szt;
-      if (szt == 0) empty = true;
-      if (sz < best) { best = sz; dsel = b; dlo = q.lo[i]; }
+        for (uint32_t i = 0; i < 4; i++)
+          if (b == beg + i && b < end) v[i] = u;
+      }
+    };
+    if (with_x) visit((uint32_t)d + 1u, x);
+    walk_prefix(lv, d, e, visit);
+    uint32_t lo[4], hi[4], tc[4], c[4];
+#pragma unroll
+    for (uint32_t i = 0; i < 4; i++) {
+      lo[i] = 0; hi[i] = 0; tc[i] = 0; c[i] = 0;
+      if (beg + i < end) {
+        c[i] = back_combo(wp.back(np, beg + i));
+        const uint32_t* dir = g.dir + (size_t)v[i] * (g.nc + 1) + c[i];
+        const uint32_t base = g.row[v[i]].x;
+        lo[i] = base + dir[0];
+        hi[i] = base + dir[1];
+        tc[i] = g.t_count[v[i]];
+      }
     }
+#pragma unroll
+    for (int i = 3; i >= 0; i--) {
+      if (beg + (uint32_t)i < end) {
+        const uint32_t sz = hi[i] - lo[i];
+        const uint32_t szt = (tc[i] == 0 || sz == 0) ? sz : seg_size_slow(p, v[i], c[i], lo[i], hi[i], t);
+        b4 += 4ull * szt;
+        if (szt == 0) empty = true;
+        if (sz <= best) {
+          second = best; jsel = dsel; jv = dv;
+          best = sz; dsel = beg + (uint32_t)i; dv = v[i]; dlo = lo[i];
+        } else if (sz <= second) {
+          second = sz; jsel = beg + (uint32_t)i; jv = v[i];
+        }
+      }
+    }
+    end = beg;
   }
   dn = best;
   bytes = b4;
@@ -276,38 +312,50 @@ __device__ __forceinline__ unsigned long long global_ns() {
   return t;
 }
 
-// Per-task accumulators, flushed to the update's counters when the task ends.
+// Per-task accumulators, flushed to the update's counters when the task ends;
+// bytes are each lane's own until then.
 struct TaskAcc {
-  unsigned long long cnt, hash, bytes, iters, checks, checks_hungry;
+  unsigned long long cnt, hash, bytes;
+  uint32_t iters;
 };
 
 // Hands unexpanded work at the shallowest level with work left to idle warps:
 // whole entries from the end of that level's buffer, or, when only the entry
-// in progress is left, the upper half of its remaining driver range.  Each
+// in progress is left, parts of its remaining driver range.  Each
 // donated task is a partial match (positions 0..L) plus a driver range for
-// position L + 1.  Returns the number of tasks handed over.
-__device__ uint32_t donate(const SearchParams& p, LevelSM* lv, int d, uint32_t lane, uint32_t idle_now,
-                           uint32_t t, const Task& T, uint32_t m0, uint32_t m1, int tail_level) {
+// position L + 1.
+__device__ __noinline__ void donate(const SearchParams& p, LevelSM* lv, int d, uint32_t lane, uint32_t idle_now,
+                                    uint32_t t, uint32_t anchor, uint32_t orient, int tail_level) {
   // Ranges are split down to two elements near the root (where every element
-  // heads a large subtree) and only from 64 elements further down.
+  // heads a large subtree) and only from 64 elements further down.  Lane L
+  // looks at level L; the shallowest level that has something to give wins.
   const int n = (int)p.plan->n;
-  int Ls = 0;
-  uint32_t mode = 0;  // 1: whole entries, 2: split the entry in progress
-  for (int L = 1; L <= d && L <= n - 2; L++) {
-    const uint32_t cnt = lv[L].cnt, ce = lv[L].cur_e;
-    if (ce >= cnt) continue;
-    if (cnt - ce >= 2) { Ls = L; mode = 1; break; }
-    if (L == tail_level) continue;  // the tail stage takes whole entries only
-    const uint32_t min_split = (L + 5 <= n) ? 2u : (p.split_deep ? p.split_deep : 64u);
-    if (lv[L].dn[ce] - lv[L].cur_k >= min_split) { Ls = L; mode = 2; break; }
+  const int me = (int)lane;
+  uint32_t give = 0;  // 1: whole entries, 2: split the entry in progress
+  if (me >= 1 && me <= d && me <= n - 2) {
+    const LevelSM& S = lv[me];
+    const uint32_t cnt = S.cnt, cur = S.cur, total = S.total;
+    if (cur < total) {
+      const uint32_t min_split = (me + 5 <= n) ? 2u : (p.split_deep ? p.split_deep : 64u);
+      if (cnt >= 2 && cur < S.incl[cnt - 2]) give = 1;
+      else if (me != tail_level && total - cur >= min_split) give = 2;  // the tail stage takes whole entries only
+    }
   }
-  if (!mode) {
+  const uint32_t who = __ballot_sync(0xffffffffu, give != 0);
+  if (!who) {
     if (lane == 0) atomicAdd(&p.sstat->starved, 1ULL);
-    return 0;
+    return;
   }
+  const int Ls = __ffs((int)who) - 1;
+  const uint32_t mode = __shfl_sync(0xffffffffu, give, Ls);
   LevelSM& S = lv[Ls];
-  const uint32_t cnt = S.cnt, ce = S.cur_e;
-  const uint32_t avail = mode == 1 ? min(cnt - ce - 1, 32u) : 1u;
+  const uint32_t cnt = S.cnt, cur = S.cur, total = S.total;
+  // the entry in progress
+  const uint32_t ce = __popc(__ballot_sync(0xffffffffu, lane < cnt && S.incl[lane] <= cur));
+  // a range in progress is cut into up to 16 parts of at least half the
+  // smallest range worth splitting; the first stays here
+  const uint32_t floor_part = (Ls + 5 <= n) ? 1u : max(1u, (p.split_deep ? p.split_deep : 64u) / 2);
+  const uint32_t avail = mode == 1 ? min(cnt - ce - 1, 32u) : min((total - cur) / floor_part - 1u, 15u);
   // take up to `avail` units of hunger (idle warps not yet promised a
   // record; a signed count): one subtraction, the excess given back, no
   // retries however many warps donate at once
@@ -325,18 +373,25 @@ __device__ uint32_t donate(const SearchParams& p, LevelSM* lv, int d, uint32_t l
     }
   }
   k = __shfl_sync(0xffffffffu, k, 0);
-  if (k == 0) return 0;
+  if (k == 0) return;
   base = __shfl_sync(0xffffffffu, base, 0);
   // entry handed to lane j and its driver range
   uint32_t e = 0, dlo = 0, dn = 0;
+  const uint32_t rem = total - cur;
+  const uint32_t beg = (uint32_t)((unsigned long long)rem * (lane + 1u) / (k + 1u));  // part lane + 1 of k + 1
+  const uint32_t end = (uint32_t)((unsigned long long)rem * (lane + 2u) / (k + 1u));
+  const uint32_t keep = rem / (k + 1u);
   if (mode == 1) {
     e = cnt - k + lane;
-    if (lane < k) { dlo = S.dlo[e]; dn = S.dn[e]; }
+    if (lane < k) {
+      const uint32_t start = S.incl[e - 1];  // e > ce
+      dlo = S.base[e] + start;
+      dn = S.incl[e] - start;
+    }
   } else {
     e = ce;
-    const uint32_t rem = S.dn[ce] - S.cur_k, keep = rem >> 1;
-    dlo = S.dlo[ce] + S.cur_k + keep;
-    dn = rem - keep;
+    dlo = S.base[ce] + cur + beg;
+    dn = end - beg;
   }
   if (lane < k) {
     const unsigned long long ticket = base + lane;
@@ -351,21 +406,24 @@ __device__ uint32_t donate(const SearchParams& p, LevelSM* lv, int d, uint32_t l
     }
     DTask* D = p.dq + slot;
     uint32_t idx = e;
-    for (int L = Ls; L >= 2; --L) { D->m[L] = lv[L].v[idx]; idx = lv[L].par[idx]; }
-    D->m[0] = m0; D->m[1] = m1;
+#pragma unroll 1
+    for (int L = Ls; L >= 0; --L) {
+      const LevelSM& X = lv[L ? L : 1];
+      D->m[L] = X.v[idx];
+      idx = X.par[idx];
+    }
     D->upd = ok ? t : 0xffffffffu;  // a record that could not be placed is published as void
-    D->anchor = T.anchor; D->orient = T.orient; D->depth = (uint8_t)Ls;
-    D->dlo = dlo; D->dn = dn; D->dsel = S.dsel[e];
+    D->anchor = (uint16_t)anchor; D->orient = (uint8_t)orient; D->depth = (uint8_t)Ls;
+    D->dlo = dlo; D->dn = dn; D->sel = (uint32_t)S.dsel[e] | ((uint32_t)S.jsel[e] << 8);
     __threadfence();
     *sq = ticket + 1;  // publish
   }
   __syncwarp();
   if (lane == 0) {
-    if (mode == 1) S.cnt = cnt - k;
-    else S.dn[ce] = S.cur_k + ((S.dn[ce] - S.cur_k) >> 1);
+    if (mode == 1) { S.cnt = cnt - k; S.total = S.incl[cnt - k - 1]; }
+    else S.total = cur + keep;
   }
   __syncwarp();
-  return k;
 }
 
 // ---------------------------------------------------------------- tail stage
@@ -387,8 +445,10 @@ __device__ __noinline__ unsigned long long group_assignments(uint32_t g, const u
   const uint32_t full = (1u << g) - 1u;
   if (homo) {
     unsigned long long prod = 1;
+#pragma unroll 1
     for (uint32_t i = 0; i < g; i++) {
       unsigned long long c = 0;
+#pragma unroll 1
       for (uint32_t M = 1; M <= full; M++)
         if ((M >> i) & 1u) c = min(kTailSat, c + N[M]);
       prod = sat_mul(prod, c);
@@ -397,14 +457,18 @@ __device__ __noinline__ unsigned long long group_assignments(uint32_t g, const u
   }
   unsigned long long f[1u << kTailGroup], h[1u << kTailGroup];
   for (uint32_t S = 0; S <= full; S++) f[S] = S == 0 ? 1ull : 0ull;
+#pragma unroll 1
   for (uint32_t M = 1; M <= full; M++) {
     if (!N[M]) continue;
     for (uint32_t S = 0; S <= full; S++) h[S] = 0;
+#pragma unroll 1
     for (uint32_t S = 0; S <= full; S++) {
       if (!f[S]) continue;
       const uint32_t fr = M & ~S;
+#pragma unroll 1
       for (uint32_t R = fr;; R = (R - 1u) & fr) {  // every subset of fr, the empty one last
         unsigned long long ways = 1;
+#pragma unroll 1
         for (uint32_t r = 0, k = (uint32_t)__popc(R); r < k; r++) ways = sat_mul(ways, N[M] > r ? N[M] - r : 0ull);
         if (ways) h[S | R] = min(kTailSat, h[S | R] + sat_mul(f[S], ways));
         if (R == 0) break;
@@ -415,14 +479,6 @@ __device__ __noinline__ unsigned long long group_assignments(uint32_t g, const u
   return f[full];
 }
 
-// Prefix m[0 .. L] of entry e of level L.
-__device__ __forceinline__ void load_prefix(uint32_t* m, const LevelSM* lv, int L, uint32_t e, uint32_t m0,
-                                            uint32_t m1) {
-  m[0] = m0; m[1] = m1;
-  uint32_t idx = e;
-  for (int l2 = L; l2 >= 2; --l2) { m[l2] = lv[l2].v[idx]; idx = lv[l2].par[idx]; }
-}
-
 // Counts the completions of the entries of level L (= the anchor's tail_at:
 // complete matches of the positions before the independent tail).  For each
 // label group of the tail, every member's candidates are listed from its
@@ -431,56 +487,59 @@ __device__ __forceinline__ void load_prefix(uint32_t* m, const LevelSM* lv, int 
 // counted under the first member it belongs to, in per-entry class counters
 // kept in the unused levels above L.  Each entry's completions are the
 // product over groups of group_assignments.  A group is not looked at for
-// entries whose product is already 0.  Returns false when the update was
-// stopped (cap, deadline or stop flag).
-__device__ __forceinline__ bool tail_stage(const SearchParams& p, const uint32_t* pool, LevelSM* lv, int L,
-                                        uint32_t lane, const Task& T, const PlanAnchor* A, uint32_t m0,
-                                        uint32_t m1, TaskAcc& acc) {
-  const uint32_t t = T.upd;
+// entries whose product is already 0.  Not inlined: it runs once per 32 prefixes
+// and would take registers from the walk.
+struct TailOut {
+  unsigned long long sum, bytes;  // completions (all lanes), bytes (this lane's)
+  uint32_t iters;
+  bool stopped;                   // the update was stopped (deadline or stop flag)
+};
+__device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t* pool, LevelSM* lv,
+                                           const uint32_t* plan_words, uint32_t n, int L, uint32_t lane, uint32_t t,
+                                           uint32_t anchor) {
+  const PlanAnchor* A = &p.plan->anchors[anchor];
+  const WalkPlan wp{plan_words, n};
   volatile unsigned int* stop = p.stop;
-  LevelSM& S = lv[L];
-  const uint32_t ce = S.cur_e, cnt = S.cnt, ck = S.cur_k;
-  const uint32_t ne = cnt > ce ? cnt - ce : 0u;
-  const bool has = lane < ne;
-  const uint32_t e_mine = ce + (has ? lane : 0u);
+  const LevelSM& S = lv[L];
+  const bool has = lane < S.cnt;
+  const uint32_t e_mine = has ? lane : 0u;
   uint32_t* cntr = reinterpret_cast<uint32_t*>(&lv[L + 1]);  // [class][entry], levels L+1.. are unused here
-  const uint32_t pmask = A->prefix_mask;
-  uint32_t m[kMaxQ];
-  unsigned long long prod = has ? 1ull : 0ull, bytes = 0;
-  bool stopped = false;
-  uint32_t gp = 0, it = 0;
+  TailOut out{0, 0, 0, false};
+  unsigned long long prod = has ? 1ull : 0ull;
+  uint32_t gp = 0;
+#pragma unroll 1
   for (uint32_t gi = 0; gi < A->n_groups; gi++) {
     const uint32_t g = A->gsize[gi];
     const uint32_t ncls = (1u << g) - 1u;
     for (uint32_t c = 0; c < ncls; c++) cntr[c * 32 + lane] = 0;
     __syncwarp();
-    for (uint32_t j = 0; j < g && !stopped; j++) {
+#pragma unroll 1
+    for (uint32_t j = 0; j < g && !out.stopped; j++) {
       const uint32_t ps = A->gpos[gp + j];
-      uint32_t dlo = 0, dn = 0, dsel = 0;
+      uint32_t dlo = 0, dn = 0, dsel = 0, jsel = 0, jv = 0;
       if (prod) {
         if (ps == (uint32_t)L + 1) {  // the entry's own driver, found when it was pushed
-          const uint32_t skip = lane == 0 ? ck : 0u;
-          dlo = S.dlo[e_mine] + skip; dn = S.dn[e_mine] - skip; dsel = S.dsel[e_mine];
+          const uint32_t start = e_mine ? S.incl[e_mine - 1] : 0u;
+          dlo = S.base[e_mine] + start; dn = S.incl[e_mine] - start; dsel = S.dsel[e_mine];
+          jsel = S.jsel[e_mine]; jv = S.jv[e_mine];
         } else {
-          load_prefix(m, lv, L, e_mine, m0, m1);
           unsigned long long b4 = 0;
-          if (!pick_driver(p, A, ps, m, (int32_t)t, dlo, dn, dsel, b4)) dn = 0;
-          bytes += b4;
+          if (!pick_driver(p, lv, wp, L, e_mine, false, 0u, ps, (int32_t)t, dlo, dn, dsel, jsel, jv, b4)) dn = 0;
+          out.bytes += b4;
         }
       }
       const uint32_t incl = warp_incl_scan(dn, lane);
       const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
       for (uint32_t base = 0; base < total; base += 32) {
-        if ((++it & 63) == 0) {
+        if ((++out.iters & 63) == 0) {
           unsigned int st = 0;
           if (lane == 0) {
             if (p.deadline_ns && global_ns() - p.sstat->launch_t0 > p.deadline_ns)
               atomicCAS(const_cast<unsigned int*>(stop) + t, 0u, kStopDeadline);
             st = stop[t];
           }
-          if (__shfl_sync(0xffffffffu, st, 0)) { stopped = true; break; }
+          if (__shfl_sync(0xffffffffu, st, 0)) { out.stopped = true; break; }
         }
-        acc.iters++;
         const uint32_t gidx = base + lane;
         uint32_t owner = 0;
 #pragma unroll
@@ -491,16 +550,27 @@ __device__ __forceinline__ bool tail_stage(const SearchParams& p, const uint32_t
         const uint32_t own = owner & 31u;
         const uint32_t prev = __shfl_sync(0xffffffffu, incl, (owner - 1u) & 31u);
         const uint32_t o_dlo = __shfl_sync(0xffffffffu, dlo, own);
-        const uint32_t o_dsel = __shfl_sync(0xffffffffu, dsel, own);
+        const uint32_t o_sel = __shfl_sync(0xffffffffu, dsel | (jsel << 8), own);
+        const uint32_t o_dsel = o_sel & 0xffu;
+        const uint32_t o_jv = __shfl_sync(0xffffffffu, jv, own);
         if (gidx < total) {
-          const uint32_t kk = gidx - (owner ? prev : 0u);
-          const uint32_t x = ld_stream(pool + (uint64_t)o_dlo + kk);
-          load_prefix(m, lv, L, ce + owner, m0, m1);
-          if (check_candidate(p, pool, A, ps, x, m, o_dsel, (int32_t)t, pmask)) {
+          const uint32_t x = ld_stream(pool + (uint64_t)o_dlo + (gidx - (owner ? prev : 0u)));
+          uint32_t joined = 0xffu, jhit = 0;
+          bool ok = filter_bit(p, wp.qv(ps), x);
+          if (ok && wp.nb(ps) > 1) {
+            joined = o_sel >> 8;
+            jhit = join_find(p, pool, o_jv, wp.back(ps, joined), x);
+            ok = jhit != kSlotEmpty;
+          }
+          if (ok && check_rest(p, pool, lv, wp, L, owner, ps, x, o_dsel, joined, jhit, (int32_t)t)) {
             uint32_t M = 1u << j;
             bool seen = false;
+#pragma unroll 1
             for (uint32_t i = 0; i < g && !seen; i++) {
-              if (i == j || !check_candidate(p, pool, A, A->gpos[gp + i], x, m, 0xffu, (int32_t)t, pmask)) continue;
+              const uint32_t pi = A->gpos[gp + i];
+              if (i == j || !filter_bit(p, wp.qv(pi), x) ||
+                  !check_rest(p, pool, lv, wp, L, owner, pi, x, 0xffu, 0xffu, 0u, (int32_t)t))
+                continue;
               if (i < j) seen = true;
               else M |= 1u << i;
             }
@@ -511,7 +581,7 @@ __device__ __forceinline__ bool tail_stage(const SearchParams& p, const uint32_t
       __syncwarp();
     }
     gp += g;
-    if (stopped) break;
+    if (out.stopped) break;
     if (prod) {
       unsigned long long N[1u << kTailGroup];
       N[0] = 0;
@@ -521,217 +591,266 @@ __device__ __forceinline__ bool tail_stage(const SearchParams& p, const uint32_t
     __syncwarp();
     if (!__any_sync(0xffffffffu, prod != 0)) break;
   }
-#pragma unroll
-  for (int o = 16; o; o >>= 1) bytes += __shfl_xor_sync(0xffffffffu, bytes, o);
-  acc.bytes += bytes;
-  if (stopped) return false;
   unsigned long long sum = prod;
 #pragma unroll
   for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
-  if (lane == 0) S.cur_e = cnt;
-  __syncwarp();
-  acc.cnt += sum;
-  if (sum && p.cap) {
-    unsigned int hit = 0;
-    if (lane == 0) {
-      const unsigned long long old = atomicAdd(&p.count[t], acc.cnt);
-      acc.cnt = 0;
-      if (old + sum >= p.cap) { stop[t] = kStopCap; hit = 1; }
-    }
-    if (__shfl_sync(0xffffffffu, hit, 0)) return false;
-  }
-  return true;
+  out.sum = out.stopped ? 0ull : sum;
+  return out;
 }
 
+// A warp's counters of one launch.
+struct WarpStat {
+  unsigned long long busy, idle, root, last_root, longest, iters, checks, hungry;
+  unsigned long long began;  // start of the current task
+};
+
 // Depth-first walk over chunked levels starting at level `d` (see the file
-// comment); positions 0 and 1 hold m0 and m1.  MODE 1 compiles the
-// match-set append in, MODE 2 the tail stage; each is a separate
-// instantiation so that the plain counting kernel (MODE 0) keeps its
-// register budget.
+// comment).  MODE 1 compiles the match-set append in, MODE 2 the tail stage;
+// each is a separate instantiation so that the others keep their registers.
+//
+// What bounds a step is how many cache lines the SM can have in flight: its
+// loads are scattered over the lanes, and with 24 warps of 80 registers the
+// spilled ones swept through L1 with them and came back from L2.  Sixteen
+// warps of 128 registers spill nothing (12,000 -> 4,200 cycles a step, and the
+// search of a 65,536-update batch on the 2^22-vertex stream 131 -> 68 ms).  So
+// the common step -- no candidate survives -- reads little: the level's cursor
+// and segment ends live in registers, the range layout of LevelSM needs no
+// scan, the order of the joins is in shared memory (WalkPlan), and nothing of
+// the prefix is touched before a candidate has passed its first join and the
+// filter.  Those that have are few (1.4 of 30 a step there, in 70 % of the
+// steps), and what they need next is a long chain of loads: they are gathered
+// over the level's steps in `wait` (x; entry, touched bit of the first join)
+// and go through it 32 at a time.
 template <int MODE>
-__device__ void run_levels(const SearchParams& p, const uint32_t* pool, LevelSM* lv, int d, uint32_t lane,
-                           const Task& T, const PlanAnchor* A, uint32_t m0, uint32_t m1, TaskAcc& acc) {
-  const uint32_t n = p.plan->n;
+__device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t* pool, LevelSM* lv,
+                                           const WalkPlan& wp, uint2* wait, int d, uint32_t lane, const Task& T,
+                                           WarpStat& ws, TaskAcc& acc) {
+  const uint32_t n = wp.n;
   const uint32_t t = T.upd;
+  const DevGraph& g = p.g;
   volatile unsigned int* stop = p.stop;
   uint32_t iter = 0;
-  const unsigned long long t_start = global_ns();
   constexpr bool EN = MODE == 1;
-  const int tail_level = (MODE == 2 && p.tail && A->tail_at) ? (int)A->tail_at : -1;
-  uint32_t seen_stop = 0, seen_hungry = 0;  // lane 0: flags loaded in the previous iteration
-  while (d >= 1) {
-    ++iter;
-    if ((iter & 63) == 0 && p.deadline_ns) {
-      unsigned int late = 0;
-      if (lane == 0 && global_ns() - p.sstat->launch_t0 > p.deadline_ns) {
-        atomicCAS(const_cast<unsigned int*>(stop) + t, 0u, kStopDeadline);
-        late = 1;
+  const int tail_level = (MODE == 2 && p.tail && p.plan->anchors[T.anchor].tail_at) ? (int)p.plan->anchors[T.anchor].tail_at : -1;
+  uint32_t seen_stop = 0, seen_hungry = 0;  // flags loaded at the previous check
+  const uint32_t every = p.donate_every ? p.donate_every : 1u;  // steps between hand-over checks (a power of two)
+  bool enter = true;
+  uint32_t cur = 0, total = 0, my_incl = 0, qv = 0, held = 0;
+  bool joins = false;
+  // the pair of this lane at cur, loaded a step ahead: entry, candidate, and
+  // the row of the entry's first join; `fresh` when they are cur's
+  bool fresh = false;
+  uint32_t own = 0, x = 0;
+  uint2 jrow = make_uint2(0, 0);
+  auto fetch = [&](uint32_t c) {
+    const uint32_t at = c + lane;
+    own = __popc(__ballot_sync(0xffffffffu, my_incl <= c));
+    if (__popc(__ballot_sync(0xffffffffu, my_incl <= c + 31u)) != (int)own) {
+      // the pairs span several entries: the first whose end lies beyond `at`
+      own = 0;
+#pragma unroll
+      for (uint32_t step = 16; step; step >>= 1) {
+        const uint32_t v = __shfl_sync(0xffffffffu, my_incl, own + step - 1);
+        if (v <= at) own += step;
       }
-      if (__shfl_sync(0xffffffffu, late, 0)) break;
     }
+    if (at < total) {
+      const LevelSM& L = lv[d];
+      x = ld_stream(pool + (L.base[own] + at));
+      if (joins) jrow = g.row[L.jv[own]];
+    }
+  };
+  for (;;) {
+    if (enter) {
+      // the level's cursor and segment ends (lane e: entry e's)
+      const LevelSM& L = lv[d];
+      cur = L.cur;
+      total = L.total;
+      my_incl = lane < L.cnt ? L.incl[lane] : 0xffffffffu;
+      qv = wp.qv((uint32_t)d + 1u);
+      joins = wp.nb((uint32_t)d + 1u) > 1 && g.htab != nullptr;
+      enter = false;
+      fresh = false;
+    }
+    ++iter;
     if ((iter & 63) == 0) {
-      unsigned int expired = (lane == 0) ? (global_ns() - t_start > p.task_limit_ns) : 0u;
-      if (__shfl_sync(0xffffffffu, expired, 0)) {
-        if (lane == 0) {
+      unsigned int quit = 0;
+      if (lane == 0) {
+        const unsigned long long now = global_ns();
+        if (p.deadline_ns && now - p.sstat->launch_t0 > p.deadline_ns) {
+          atomicCAS(const_cast<unsigned int*>(stop) + t, 0u, kStopDeadline);
+          quit = 1;
+        }
+        if (now - ws.began > p.task_limit_ns) {
+          quit = 1;
           atomicExch(p.error, kErrTaskGuard);
           if (atomicCAS(&p.sstat->guard_set, 0u, 1u) == 0u) {
             p.sstat->guard_d = (unsigned)d; p.sstat->guard_upd = t; p.sstat->guard_iters = iter;
+#pragma unroll 1
             for (int L = 1; L <= d && L <= 16; L++) {
-              const uint32_t ce = lv[L].cur_e;
               p.sstat->guard_lv[4 * (L - 1) + 0] = lv[L].cnt;
-              p.sstat->guard_lv[4 * (L - 1) + 1] = ce;
-              p.sstat->guard_lv[4 * (L - 1) + 2] = lv[L].cur_k;
-              p.sstat->guard_lv[4 * (L - 1) + 3] = ce < 32 ? lv[L].dn[ce] : 0xffffffffu;
+              p.sstat->guard_lv[4 * (L - 1) + 1] = lv[L].cur;
+              p.sstat->guard_lv[4 * (L - 1) + 2] = lv[L].total;
+              p.sstat->guard_lv[4 * (L - 1) + 3] = lv[L].incl[0];
             }
           }
         }
-        break;
+      }
+      if (__shfl_sync(0xffffffffu, quit, 0)) break;
+    }
+    if ((iter & (every - 1)) == 0 && p.dq) {
+      const uint32_t idle_now = __shfl_sync(0xffffffffu, seen_hungry, 0);
+      if (idle_now) {
+        if (lane == 0) { lv[d].cur = cur; ws.hungry++; }
+        __syncwarp();
+        donate(p, lv, d, lane, idle_now, t, T.anchor, T.orient, tail_level);
+        total = lv[d].total;
+        if (lane >= lv[d].cnt) my_incl = 0xffffffffu;
       }
     }
-    if ((iter & 7) == 0) {
+    // the stop flag and the idle-warp count are loaded every fourth step, each
+    // a round trip to a line other warps update, and looked at later, so that
+    // the trip overlaps the steps between; lane 0's view decides for the warp
+    if ((iter & 3) == 0) {
       if (__shfl_sync(0xffffffffu, seen_stop, 0)) break;
-    }
-    if ((iter & (p.donate_every ? p.donate_every - 1 : 0u)) == 0 && p.dq) {
-      const uint32_t idle_now = __shfl_sync(0xffffffffu, seen_hungry, 0);
-      acc.checks++;
-      if (idle_now) acc.checks_hungry++;
-      if (idle_now) donate(p, lv, d, lane, idle_now, t, T, m0, m1, tail_level);
-    }
-    // the stop flag and the idle-warp count the checks above read are loaded
-    // one iteration ahead, so their round trip to L2 overlaps a step's work
-    // instead of preceding it (a step late is soon enough for both), and only
-    // before the iterations that read them: each load is a round trip to a
-    // line other warps update
-    if (lane == 0 && (iter & 3) == 3) {
-      seen_stop = stop[t];
-      seen_hungry = p.dq ? (uint32_t)max((int)*(volatile unsigned int*)&p.q->hungry, 0) : 0u;
+      if (lane == 0) {
+        seen_stop = stop[t];
+        seen_hungry = p.dq ? (uint32_t)max((int)*(volatile unsigned int*)&p.q->hungry, 0) : 0u;
+      }
     }
     if constexpr (MODE == 2) {
       if (d == tail_level) {
-        if (!tail_stage(p, pool, lv, d, lane, T, A, m0, m1, acc)) break;
-        d--;
-        continue;
+        const TailOut r = tail_stage(p, pool, lv, wp.w, n, d, lane, t, T.anchor);
+        acc.bytes += r.bytes;
+        acc.iters += r.iters;
+        acc.cnt += r.sum;
+        if (r.stopped) break;
+        if (r.sum && p.cap) {
+          unsigned int hit = 0;
+          if (lane == 0) {
+            const unsigned long long old = atomicAdd(&p.count[t], acc.cnt);
+            if (old + r.sum >= p.cap) { stop[t] = kStopCap; hit = 1; }
+          }
+          acc.cnt = 0;
+          if (__shfl_sync(0xffffffffu, hit, 0)) break;
+        }
+        cur = total;  // the stage took every entry
       }
     }
-    LevelSM& L = lv[d];
-    const uint32_t cnt = L.cnt, ce = L.cur_e, ck = L.cur_k;
-    if (ce >= cnt) { d--; continue; }
+    if (cur >= total) {  // level done (and none of its candidates waits)
+      if (--d < 1) break;
+      enter = true;
+      continue;
+    }
     acc.iters++;
-    // the next 32 (entry, driver element) pairs of this level
-    const uint32_t el = ce + lane;
-    const uint32_t rem = (el < cnt) ? L.dn[el] - (lane == 0 ? ck : 0u) : 0u;
-    const uint32_t incl = warp_incl_scan(rem, lane);
-    const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
-    uint32_t owner = 0;
-#pragma unroll
-    for (uint32_t step = 16; step; step >>= 1) {
-      const uint32_t v = __shfl_sync(0xffffffffu, incl, owner + step - 1);
-      if (v <= lane) owner += step;
-    }
-    const uint32_t prev = __shfl_sync(0xffffffffu, incl, owner > 0 ? (owner - 1) & 31 : 0);
-    const bool active = lane < total;
-    const uint32_t e = ce + owner;
-    const uint32_t kk = lane - (owner > 0 ? prev : 0u) + (owner == 0 ? ck : 0u);
-    uint32_t nce, nck;
-    if (total <= 32) {
-      nce = ce + min(32u, cnt - ce); nck = 0;
-    } else {
-      const uint32_t o31 = __shfl_sync(0xffffffffu, owner, 31);
-      const uint32_t k31 = __shfl_sync(0xffffffffu, kk, 31);
-      const uint32_t e31 = ce + o31;
-      if (k31 + 1 >= L.dn[e31]) { nce = e31 + 1; nck = 0; } else { nce = e31; nck = k31 + 1; }
-    }
+    // the next 32 (entry, driver element) pairs of this level: the first join,
+    // then the filter bit of those it leaves.  This order reads fewest lines:
+    // on the 2^22-vertex stream the join leaves 7 % and the filter 66 %
+    // (filter first 234 ms of search, join first 211 ms, both at once 268 ms).
+    // The following pairs are fetched between the two.
     const uint32_t pos = (uint32_t)d + 1;
-    bool valid = false;
-    uint32_t x = 0, ndlo = 0, ndn = 0, ndsel = 0;
-    unsigned long long nb4 = 0;
-    uint32_t m[kMaxQ];
-    bool act = active;
-    if (act && (e >= cnt || kk >= L.dn[e])) {  // lanes disagree on the level state: flag it, read nothing
-      atomicExch(p.error, kErrBadTask);
-      act = false;
+    if (!fresh) fetch(cur);
+    const uint32_t cx = x;
+    uint32_t meta = own;
+    bool valid = cur + lane < total;
+    if (valid && joins) {
+      const uint32_t el = back_el(wp.back(pos, lv[d].jsel[own]));
+      const uint32_t hit = row_find(g, jrow, row_entry(cx, el, g.hlb));
+      valid = hit != kSlotEmpty;
+      meta |= (hit & kSlotTouched) >> 15;
     }
-    if (act) {
-      // the candidate and the first back segments of its position are loaded
-      // together: the segments depend on the prefix only
-      x = ld_stream(pool + (uint64_t)L.dlo[e] + kk);
-      m[0] = m0; m[1] = m1;
-      uint32_t idx = e;
-      for (int l2 = d; l2 >= 2; --l2) { m[l2] = lv[l2].v[idx]; idx = lv[l2].par[idx]; }
-      const uint32_t ds = L.dsel[e];
-      if (p.g.emask) {
-        valid = check_candidate_h(p, A, pos, x, m, ds, (int32_t)t);
-      } else {
-        SegQuad q0;
-        load_quad(p.g, A, A->pos[pos], 0, m, ds, q0);
-        valid = check_candidate_q(p, pool, A, pos, x, m, ds, (int32_t)t, q0);
-      }
-      if (valid && pos + 1 < n) {
-        m[pos] = x;
-        valid = pick_driver(p, A, pos + 1, m, (int32_t)t, ndlo, ndn, ndsel, nb4);
-      }
-    }
+    fresh = cur + 32u < total;
+    if (fresh) fetch(cur + 32u);
+    if (valid) valid = filter_bit(p, qv, cx);
+    // the candidates left wait until 32 of them, or all of the level's, are
+    // together; a step that finds more than there is room for ends before the
+    // first of those
+    const uint32_t found = __ballot_sync(0xffffffffu, valid);
+    const uint32_t rank = held + __popc(found & ((1u << lane) - 1u));
+    const uint32_t over = __ballot_sync(0xffffffffu, valid && rank >= 32u);
+    if (valid && rank < 32u) wait[rank] = make_uint2(cx, meta);
+    cur += over ? (uint32_t)__ffs((int)over) - 1u : 32u;
+    fresh = fresh && !over;
+    held = over ? 32u : held + __popc(found);
+    if (held == 0 || (held < 32u && cur < total)) continue;
     __syncwarp();
-    if (lane == 0) { L.cur_e = nce; L.cur_k = nck; }
-    __syncwarp();  // the cursor must be visible to every lane before the next iteration reads it
-    const uint32_t mask = __ballot_sync(0xffffffffu, valid);
-    if (pos + 1 < n) {
-#pragma unroll
-      for (int o = 16; o; o >>= 1) nb4 += __shfl_xor_sync(0xffffffffu, nb4, o);
-      acc.bytes += nb4;
+    // injectivity, remaining joins, presence, next driver
+    uint32_t ndlo = 0, ndn = 0, ndsel = 0, njsel = 0, njv = 0;
+    uint32_t wx = 0, wown = 0;
+    valid = lane < held;
+    if (valid) {
+      const uint2 w = wait[lane];
+      wx = w.x;
+      wown = w.y & 31u;
+      const uint32_t wsel = lv[d].dsel[wown];
+      valid = check_rest(p, pool, lv, wp, d, wown, pos, wx, wsel, joins ? lv[d].jsel[wown] : 0xffu,
+                         (w.y << 15) & kSlotTouched, (int32_t)t);
+      if (valid && pos + 1 < n) {
+        unsigned long long nb4 = 0;
+        valid = pick_driver(p, lv, wp, d, wown, true, wx, pos + 1, (int32_t)t, ndlo, ndn, ndsel, njsel, njv, nb4);
+        acc.bytes += nb4;
+      }
     }
+    held = 0;
+    const uint32_t mask = __ballot_sync(0xffffffffu, valid);
+    if (!mask) continue;
     if (pos == n - 1) {
       const uint32_t c = __popc(mask);
       if (EN) {
         unsigned long long base = 0;
-        if (lane == 0 && c) base = atomicAdd(p.enum_n, (unsigned long long)c);
+        if (lane == 0) base = atomicAdd(p.enum_n, (unsigned long long)c);
         base = __shfl_sync(0xffffffffu, base, 0);
         if (valid) {
           const unsigned long long r = base + __popc(mask & ((1u << lane) - 1u));
           if (r < p.enum_cap) {
             uint32_t* rec = p.enum_buf + r * p.enum_stride;
             rec[0] = p.enum_base + t;
-            rec[1 + A->pos[pos].qv] = x;
-            for (uint32_t q = 0; q < pos; q++) rec[1 + A->pos[q].qv] = m[q];
+            rec[1 + qv] = wx;
+            walk_prefix(lv, d, wown, [&](uint32_t j, uint32_t v) { rec[1 + wp.qv(j)] = v; });
           }
         }
       }
-      if (p.want_hash) {
-        unsigned long long h = 0;
-        if (valid) {
-          uint64_t s = pair_hash(A->pos[pos].qv, x);
-          for (uint32_t q = 0; q < pos; q++) s += pair_hash(A->pos[q].qv, m[q]);
-          h = mix64(s);
-        }
-#pragma unroll
-        for (int o = 16; o; o >>= 1) h += __shfl_xor_sync(0xffffffffu, h, o);
-        acc.hash += h;
+      if (MODE != 2 && p.want_hash && valid) {
+        uint64_t s = pair_hash(qv, wx);
+        walk_prefix(lv, d, wown, [&](uint32_t j, uint32_t v) { s += pair_hash(wp.qv(j), v); });
+        acc.hash += mix64(s);
       }
       acc.cnt += c;
-      if (c && p.cap) {
+      if (p.cap) {
         unsigned int hit = 0;
         if (lane == 0) {
           const unsigned long long old = atomicAdd(&p.count[t], acc.cnt);
-          acc.cnt = 0;
           if (old + c >= p.cap) { stop[t] = kStopCap; hit = 1; }
         }
+        acc.cnt = 0;
         if (__shfl_sync(0xffffffffu, hit, 0)) break;
       }
     } else {
+      // survivors become level pos, their driver segments laid end to end
       LevelSM& N = lv[pos];
+      const uint32_t mine = valid ? ndn : 0u;
+      const uint32_t incl = warp_incl_scan(mine, lane);
       if (valid) {
         const uint32_t slot = __popc(mask & ((1u << lane) - 1u));
-        N.v[slot] = x; N.par[slot] = (uint8_t)e; N.dlo[slot] = ndlo; N.dn[slot] = ndn;
-        N.dsel[slot] = (uint8_t)ndsel;
+        N.v[slot] = wx; N.par[slot] = (uint8_t)wown; N.dsel[slot] = (uint8_t)ndsel;
+        N.jsel[slot] = (uint8_t)njsel; N.jv[slot] = njv;
+        N.incl[slot] = incl; N.base[slot] = ndlo - (incl - mine);
       }
-      if (lane == 0) { N.cnt = __popc(mask); N.cur_e = 0; N.cur_k = 0; }
+      if (lane == 31) { N.cnt = __popc(mask); N.cur = 0; N.total = incl; lv[d].cur = cur; }
       __syncwarp();
-      if (mask) d = (int)pos;
+      d = (int)pos;
+      enter = true;
     }
   }
+  if (lane == 0 && p.dq) ws.checks += iter / every;
 }
 
 __device__ __forceinline__ void flush_acc(const SearchParams& p, uint32_t t, uint32_t lane, TaskAcc& acc) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) {
+    acc.bytes += __shfl_xor_sync(0xffffffffu, acc.bytes, o);
+    if (p.want_hash) acc.hash += __shfl_xor_sync(0xffffffffu, acc.hash, o);
+  }
   if (lane == 0) {
     if (acc.cnt) {
       const unsigned long long old = atomicAdd(&p.count[t], acc.cnt);
@@ -744,19 +863,26 @@ __device__ __forceinline__ void flush_acc(const SearchParams& p, uint32_t t, uin
   __syncwarp();
 }
 
+// Same-label positions the injectivity tests of this anchor's walk look at: all,
+// or those before a counted tail (whose own vertices are told apart by their
+// classes); none under homomorphism.
+__device__ __forceinline__ uint32_t same_mask(const SearchParams& p, const PlanAnchor* A) {
+  if (p.homo) return 0u;
+  return p.tail ? A->prefix_mask : 0xffffffffu;
+}
+
 // Root task: positions 0 and 1 are the updated edge; level 1 holds the driver
-// segment of position 2.
+// segment of position 2.  Returns false when there is nothing to walk.
 template <int MODE>
-__device__ void run_root(const SearchParams& p, const uint32_t* pool, LevelSM* lv, uint32_t lane, const Task& T,
-                         TaskAcc& acc) {
-  const uint32_t n = p.plan->n;
+__device__ __forceinline__ bool setup_root(const SearchParams& p, LevelSM* lv, uint32_t* plan_words, uint32_t n,
+                                           uint32_t lane, const Task& T, TaskAcc& acc) {
   const uint32_t t = T.upd;
   const PlanAnchor* A = &p.plan->anchors[T.anchor];
   const UpdInfo U = p.info[t];
   const uint32_t m0 = T.orient ? U.v2 : U.v1, m1 = T.orient ? U.v1 : U.v2;
   if (n == 2) {
+    acc.cnt += 1;
     if (lane == 0) {
-      acc.cnt += 1;
       if (p.want_hash) acc.hash += mix64(pair_hash(A->pos[0].qv, m0) + pair_hash(A->pos[1].qv, m1));
       if (MODE == 1) {
         const unsigned long long r = atomicAdd(p.enum_n, 1ull);
@@ -768,87 +894,85 @@ __device__ void run_root(const SearchParams& p, const uint32_t* pool, LevelSM* l
         }
       }
     }
-    return;
+    return false;
   }
   const PlanPos P2 = A->pos[2];
   uint32_t sz = 0xffffffffu, szt = 1;
   uint64_t lo = 0, hi = 0;
-  unsigned long long rb = 0;
   if (lane < P2.nb) {
     const uint32_t j = A->back_pos[P2.boff + lane], c = A->back_combo[P2.boff + lane];
     const uint32_t v = j == 0 ? m0 : m1;
     segment(p.g, v, c, lo, hi);
     sz = (uint32_t)(hi - lo);
-    szt = seg_size_at(p.g, v, c, lo, hi, (int32_t)t);
-    rb = 4ull * szt;
+    szt = seg_size_slow(p, v, c, (uint32_t)lo, (uint32_t)hi, (int32_t)t);
+    acc.bytes += 4ull * szt;
   }
-  const bool root_empty = __any_sync(0xffffffffu, szt == 0);
-#pragma unroll
-  for (int o = 16; o; o >>= 1) rb += __shfl_xor_sync(0xffffffffu, rb, o);
-  acc.bytes += rb;
+  if (__any_sync(0xffffffffu, szt == 0)) return false;
   uint64_t key = ((uint64_t)sz << 32) | lane;
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
     uint64_t other = __shfl_xor_sync(0xffffffffu, key, o);
     key = other < key ? other : key;
   }
-  const uint32_t minsz = root_empty ? 0u : (uint32_t)(key >> 32), sel = (uint32_t)key;
+  const uint32_t minsz = (uint32_t)(key >> 32), sel = (uint32_t)key;
+  const uint32_t other = sel == 0 ? 1u : 0u;  // position 2 has one back entry or two
   const uint32_t dlo0 = (uint32_t)__shfl_sync(0xffffffffu, lo, sel);
-  if (minsz == 0) return;
   if (lane == 0) {
-    lv[1].cnt = 1; lv[1].cur_e = 0; lv[1].cur_k = 0;
-    lv[1].dlo[0] = dlo0; lv[1].dn[0] = minsz; lv[1].dsel[0] = (uint8_t)sel;
+    lv[1].cnt = 1; lv[1].cur = 0; lv[1].total = minsz;
+    lv[1].incl[0] = minsz; lv[1].base[0] = dlo0; lv[1].dsel[0] = (uint8_t)sel;
+    lv[1].v[0] = m1; lv[1].par[0] = 1; lv[1].v[1] = m0;
+    lv[1].jsel[0] = (uint8_t)other;
+    lv[1].jv[0] = P2.nb > 1 ? (A->back_pos[P2.boff + other] == 0 ? m0 : m1) : 0u;
   }
-  __syncwarp();
-  run_levels<MODE>(p, pool, lv, 1, lane, T, A, m0, m1, acc);
+  load_walk_plan(plan_words, A, n, same_mask(p, A), lane);
+  return true;
 }
 
 // Donated task: rebuild the chain of the partial match (exhausted levels
 // 1 .. depth-1) and continue from level `depth`.  `hw` holds record words
-// 0..4 in lanes 0..4 and `mv` holds m[lane] (see DTask).
-template <int MODE>
-__device__ void run_donated(const SearchParams& p, const uint32_t* pool, LevelSM* lv, uint32_t lane, uint32_t hw,
-                            uint32_t mv, TaskAcc& acc, uint32_t& upd_out, unsigned long long ticket,
-                            unsigned long long seen_seq) {
+// 0..4 in lanes 0..4 and `mv` holds m[lane] (see DTask).  Returns the level
+// to start from, 0 when there is nothing to walk.
+__device__ __forceinline__ int setup_donated(const SearchParams& p, LevelSM* lv, uint32_t* plan_words, uint32_t n,
+                                             uint32_t lane, uint32_t hw, uint32_t mv, Task& T,
+                                             unsigned long long ticket, unsigned long long seen_seq) {
   const uint32_t upd = __shfl_sync(0xffffffffu, hw, 0);
   const uint32_t w1 = __shfl_sync(0xffffffffu, hw, 1);
   const uint32_t dlo = __shfl_sync(0xffffffffu, hw, 2);
   const uint32_t dn = __shfl_sync(0xffffffffu, hw, 3);
-  const uint32_t dsel = __shfl_sync(0xffffffffu, hw, 4);
+  const uint32_t w4 = __shfl_sync(0xffffffffu, hw, 4), dsel = w4 & 0xffu;
   const uint32_t anchor = w1 & 0xffffu, orient = (w1 >> 16) & 0xffu, depth = w1 >> 24;
-  const uint32_t n = p.plan->n;
-  upd_out = upd;
-  if (upd == 0xffffffffu) return;  // void record (its donor flagged an error)
-  if (upd >= p.batch || anchor >= p.plan->n_anchor || depth < 1 || depth + 2 > n || dn == 0 ||
+  T = Task{upd, (uint16_t)anchor, (uint8_t)orient, 0};
+  if (upd == 0xffffffffu) return 0;  // void record (its donor flagged an error)
+  if (upd >= p.batch || anchor >= p.plan->n_anchor || depth < 1 || depth + 2 > n || depth > p.levels || dn == 0 ||
       (unsigned long long)dlo + dn > p.g.pool_cap) {
     if (lane == 0) {
       atomicExch(p.error, kErrBadTask);
       if (atomicCAS(&p.sstat->bad_set, 0u, 1u) == 0u) {
         p.sstat->bad_ticket = ticket; p.sstat->bad_seq = seen_seq; p.sstat->bad_batch = p.batch;
         p.sstat->bad_words[0] = upd; p.sstat->bad_words[1] = w1; p.sstat->bad_words[2] = dlo;
-        p.sstat->bad_words[3] = dn; p.sstat->bad_words[4] = dsel;
+        p.sstat->bad_words[3] = dn; p.sstat->bad_words[4] = w4;
       }
     }
-    upd_out = 0xffffffffu;
-    return;
+    T.upd = 0xffffffffu;
+    return 0;
   }
-  Task T{upd, (uint16_t)anchor, (uint8_t)orient, 0};
-  const PlanAnchor* A = &p.plan->anchors[anchor];
-  const uint32_t m0 = __shfl_sync(0xffffffffu, mv, 0), m1 = __shfl_sync(0xffffffffu, mv, 1);
-  for (uint32_t L = 1; L <= depth; L++) {
-    const uint32_t v = __shfl_sync(0xffffffffu, mv, L);
-    if (lane == 0) {
-      LevelSM& S = lv[L];
-      S.cnt = 1; S.cur_k = 0; S.v[0] = v; S.par[0] = 0;
-      S.cur_e = (L < depth) ? 1u : 0u;
-      if (L == depth) { S.dlo[0] = dlo; S.dn[0] = dn; S.dsel[0] = (uint8_t)dsel; }
-    }
-  }
-  __syncwarp();
   const unsigned int stopped =
       __shfl_sync(0xffffffffu, lane == 0 ? *(volatile unsigned int*)(p.stop + upd) : 0u, 0);
-  if (stopped) return;
-  run_levels<MODE>(p, pool, lv, (int)depth, lane, T, A, m0, m1, acc);
+  if (stopped) return 0;
+  const PlanAnchor* A = &p.plan->anchors[anchor];
+  const uint32_t jsel = w4 >> 8;
+  const PlanPos N = A->pos[depth + 1];
+  const uint32_t jv = __shfl_sync(0xffffffffu, mv, N.nb > 1 ? A->back_pos[N.boff + min(jsel, N.nb - 1u)] : 0);
+  if (lane >= 1 && lane <= depth) {
+    LevelSM& S = lv[lane];
+    S.cnt = 1; S.cur = 0; S.v[0] = mv; S.par[0] = lane == 1 ? 1 : 0;
+    S.total = lane < depth ? 0u : dn;
+    S.incl[0] = dn; S.base[0] = dlo; S.dsel[0] = (uint8_t)dsel;
+    S.jsel[0] = (uint8_t)jsel; S.jv[0] = jv;
+  }
+  if (lane == 0) lv[1].v[1] = mv;
+  load_walk_plan(plan_words, A, n, same_mask(p, A), lane);
+  return (int)depth;
 }
 
 // Per launch: tickets keep counting up across launches (the ring's slot
@@ -870,120 +994,135 @@ template <int W, int MODE>
 __device__ __forceinline__ void search_body(const SearchParams& p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint4 task_scratch[W * 10];  // one 160-byte record per warp
+  __shared__ uint2 waiting[W][32];         // candidates past their first join (run_levels)
+  __shared__ WarpStat stats[W];
   const uint32_t lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const uint32_t n = p.plan->n;
-  const uint32_t nlev = n > 2 ? n - 2 : 1;
-  LevelSM* lv = reinterpret_cast<LevelSM*>(smem_raw) + (size_t)warp * nlev - 1;  // levels 1 .. n-2
+  unsigned char* mine = smem_raw + (size_t)warp * p.warp_bytes;
+  LevelSM* lv = reinterpret_cast<LevelSM*>(mine) - 1;  // levels 1 .. p.levels
+  uint32_t* plan_words = reinterpret_cast<uint32_t*>(mine + (size_t)p.levels * sizeof(LevelSM));
+  const WalkPlan wp{plan_words, n};
   const uint32_t* pool = p.g.pools[p.g.ps->active];
   const uint32_t ntask = min(*p.n_tasks, p.task_cap);
   volatile unsigned int* stop = p.stop;
-  TaskAcc acc{0, 0, 0, 0, 0, 0};
-  unsigned long long root_ns = 0, last_root = 0, max_task = 0;
-  unsigned long long busy_ns = 0, idle_ns = 0;
-
-  // 1. root tasks, in claim order
-  for (;;) {
-    uint32_t ti = 0;
-    if (lane == 0) ti = atomicAdd(p.task_next, 1u);
-    ti = __shfl_sync(0xffffffffu, ti, 0);
-    if (ti >= ntask) break;
-    const Task T = p.tasks[ti];
-    const unsigned long long tb = global_ns();
-    if (lane == 0 && p.deadline_ns && tb - p.sstat->launch_t0 > p.deadline_ns)
-      atomicCAS(const_cast<unsigned int*>(stop) + T.upd, 0u, kStopDeadline);
-    // stop flags change under our feet: one lane reads, the warp follows it
-    const unsigned int stopped = __shfl_sync(0xffffffffu, lane == 0 ? stop[T.upd] : 0u, 0);
-    if (!stopped) run_root<MODE>(p, pool, lv, lane, T, acc);
-    const unsigned long long te = global_ns();
-    busy_ns += te - tb;
-    root_ns += te - tb;
-    last_root = te;
-    max_task = max(max_task, te - tb);
-    flush_acc(p, T.upd, lane, acc);
-    if (lane == 0 && p.dq) atomicSub(&p.q->pending, 1u);
-  }
-  if (lane == 0) {
-    atomicAdd(&p.sstat->root_busy_ns, root_ns);
-    if (last_root) atomicMax(&p.sstat->last_root_ns, last_root - p.sstat->launch_t0);
-  }
-  if (!p.dq) {
-    if (lane == 0) { atomicAdd(&p.sstat->busy_ns, busy_ns); atomicAdd(&p.sstat->iters, acc.iters); }
-    return;
-  }
-  // 2. donated tasks until every task is done.  The queue is a bounded ring
-  // of DTask slots with per-slot sequence numbers: slot (ticket % qcap) holds
-  // ticket T's record once seq == T + 1, and is free for ticket T + qcap once
-  // its reader stores seq = T + qcap.  Claims take a ticket by fetch-and-add:
-  // a compare-and-swap on the head, retried by thousands of idle warps at
-  // once, took most of the warps' time late in a batch.
   volatile SearchQueue* q = p.q;
-  for (;;) {
-    unsigned long long claimed = ~0ULL, seen = 0;
-    if (lane == 0) {
-      const unsigned long long t0 = global_ns();
-      // this warp's ticket, and one unit of hunger for it: donors fill the
-      // tickets in order, one per unit they take
-      const unsigned long long tk = atomicAdd((unsigned long long*)&p.q->head, 1ull);
-      atomicAdd(&p.q->hungry, 1u);
-      unsigned int nap = 32;
-      for (;;) {
-        const unsigned long long sv = *(volatile unsigned long long*)(p.qseq + (tk & (p.qcap - 1)));
-        if (sv == tk + 1) { claimed = tk; seen = sv; break; }
-        if (q->pending == 0) break;
-        __nanosleep(nap);
-        nap = min(nap * 2, 1024u);
-        if (global_ns() - t0 > p.wait_limit_ns) { atomicExch(p.error, kErrWaitTimeout); break; }
+  WarpStat& ws = stats[warp];
+  if (lane == 0) ws = WarpStat{};
+  bool roots = ntask > 0;
+  while (ntask) {
+    TaskAcc acc{0, 0, 0, 0};
+    Task T;
+    int d = 0;
+    unsigned long long tb = 0;
+    const bool root = roots;
+    if (roots) {
+      // 1. root tasks, in claim order
+      uint32_t ti = 0;
+      if (lane == 0) ti = atomicAdd(p.task_next, 1u);
+      ti = __shfl_sync(0xffffffffu, ti, 0);
+      if (ti >= ntask) {
+        roots = false;
+        if (!p.dq) break;
+        continue;
       }
-      idle_ns += global_ns() - t0;
-    }
-    claimed = __shfl_sync(0xffffffffu, claimed, 0);
-    if (claimed == ~0ULL) break;
-    // lane 0 copies the record through L2 (records share cache lines with other
-    // slots) into the warp's scratch, and only then frees the slot for reuse
-    uint4* scratch = task_scratch + warp * 10;
-    if (lane == 0) {
-      __threadfence();
-      const uint32_t slot = (uint32_t)(claimed & (p.qcap - 1));
-      const uint4* src = reinterpret_cast<const uint4*>(p.dq + slot);
+      T = p.tasks[ti];
+      tb = global_ns();
+      if (lane == 0 && p.deadline_ns && tb - p.sstat->launch_t0 > p.deadline_ns)
+        atomicCAS(const_cast<unsigned int*>(stop) + T.upd, 0u, kStopDeadline);
+      // stop flags change under our feet: one lane reads, the warp follows it
+      const unsigned int stopped = __shfl_sync(0xffffffffu, lane == 0 ? stop[T.upd] : 0u, 0);
+      if (!stopped) d = setup_root<MODE>(p, lv, plan_words, n, lane, T, acc) ? 1 : 0;
+    } else {
+      // 2. donated tasks until every task is done.  The queue is a bounded ring
+      // of DTask slots with per-slot sequence numbers: slot (ticket % qcap) holds
+      // ticket T's record once seq == T + 1, and is free for ticket T + qcap once
+      // its reader stores seq = T + qcap.  Claims take a ticket by fetch-and-add:
+      // a compare-and-swap on the head, retried by thousands of idle warps at
+      // once, took most of the warps' time late in a batch.  A warp that finds
+      // no task pending takes no ticket.
+      unsigned long long claimed = ~0ULL, seen = 0;
+      if (lane == 0 && q->pending != 0) {
+        const unsigned long long t0 = global_ns();
+        // this warp's ticket, and one unit of hunger for it: donors fill the
+        // tickets in order, one per unit they take
+        const unsigned long long tk = atomicAdd((unsigned long long*)&p.q->head, 1ull);
+        atomicAdd(&p.q->hungry, 1u);
+        unsigned int nap = 32;
+        for (uint32_t poll = 0;; poll++) {
+          const unsigned long long sv = *(volatile unsigned long long*)(p.qseq + (tk & (p.qcap - 1)));
+          if (sv == tk + 1) { claimed = tk; seen = sv; break; }
+          if ((poll & 3u) == 0 && q->pending == 0) break;  // the one word every waiting warp reads
+          __nanosleep(nap);
+          nap = min(nap * 2, 1024u);
+          if (global_ns() - t0 > p.wait_limit_ns) { atomicExch(p.error, kErrWaitTimeout); break; }
+        }
+        ws.idle += global_ns() - t0;
+      }
+      claimed = __shfl_sync(0xffffffffu, claimed, 0);
+      if (claimed == ~0ULL) break;
+      // lane 0 copies the record through L2 (records share cache lines with other
+      // slots) into the warp's scratch, and only then frees the slot for reuse
+      uint4* scratch = task_scratch + warp * 10;
+      if (lane == 0) {
+        __threadfence();
+        const uint32_t slot = (uint32_t)(claimed & (p.qcap - 1));
+        const uint4* src = reinterpret_cast<const uint4*>(p.dq + slot);
 #pragma unroll
-      for (int i = 0; i < 10; i++) scratch[i] = __ldcg(src + i);
-      __threadfence();
-      *(volatile unsigned long long*)(p.qseq + slot) = claimed + p.qcap;
+        for (int i = 0; i < 10; i++) scratch[i] = __ldcg(src + i);
+        __threadfence();
+        *(volatile unsigned long long*)(p.qseq + slot) = claimed + p.qcap;
+      }
+      __syncwarp();
+      const uint32_t* Dw = reinterpret_cast<const uint32_t*>(scratch);
+      const uint32_t hw = lane < 5 ? Dw[lane] : 0u;
+      const uint32_t mv = Dw[5 + lane];
+      __syncwarp();
+      tb = global_ns();
+      d = setup_donated(p, lv, plan_words, n, lane, hw, mv, T, claimed, seen);
+    }
+    if (lane == 0) ws.began = tb;
+    if (d > 0) run_levels<MODE>(p, pool, lv, wp, waiting[warp], d, lane, T, ws, acc);
+    if (T.upd < p.batch) flush_acc(p, T.upd, lane, acc);
+    if (lane == 0) {
+      if (p.dq) atomicSub(&p.q->pending, 1u);
+      const unsigned long long te = global_ns(), took = te - ws.began;
+      ws.busy += took;
+      ws.longest = max(ws.longest, took);
+      if (root) { ws.root += took; ws.last_root = te; }
+      ws.iters += acc.iters;
     }
     __syncwarp();
-    const uint32_t* Dw = reinterpret_cast<const uint32_t*>(scratch);
-    const uint32_t hw = lane < 5 ? Dw[lane] : 0u;
-    const uint32_t mv = Dw[5 + lane];
-    __syncwarp();
-    uint32_t t = 0;
-    const unsigned long long tb = global_ns();
-    run_donated<MODE>(p, pool, lv, lane, hw, mv, acc, t, claimed, seen);
-    busy_ns += global_ns() - tb;
-    max_task = max(max_task, global_ns() - tb);
-    if (t < p.batch) flush_acc(p, t, lane, acc);
-    if (lane == 0) atomicSub(&p.q->pending, 1u);
   }
-  if (lane == 0) {
-    atomicAdd(&p.sstat->busy_ns, busy_ns);
-    atomicAdd(&p.sstat->idle_ns, idle_ns);
-    atomicAdd(&p.sstat->iters, acc.iters);
-    atomicAdd(&p.sstat->checks, acc.checks);
-    atomicAdd(&p.sstat->checks_hungry, acc.checks_hungry);
-    atomicMax(&p.sstat->max_task_ns, max_task);
+  // one set of counter updates per block
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    WarpStat s{};
+    for (int i = 0; i < W; i++) {
+      s.busy += stats[i].busy; s.idle += stats[i].idle; s.root += stats[i].root;
+      s.last_root = max(s.last_root, stats[i].last_root); s.longest = max(s.longest, stats[i].longest);
+      s.iters += stats[i].iters; s.checks += stats[i].checks; s.hungry += stats[i].hungry;
+    }
+    if (s.busy) atomicAdd(&p.sstat->busy_ns, s.busy);
+    if (s.idle) atomicAdd(&p.sstat->idle_ns, s.idle);
+    if (s.root) atomicAdd(&p.sstat->root_busy_ns, s.root);
+    if (s.last_root) atomicMax(&p.sstat->last_root_ns, s.last_root - p.sstat->launch_t0);
+    if (s.longest) atomicMax(&p.sstat->max_task_ns, s.longest);
+    if (s.iters) atomicAdd(&p.sstat->iters, s.iters);
+    if (s.checks) atomicAdd(&p.sstat->checks, s.checks);
+    if (s.hungry) atomicAdd(&p.sstat->checks_hungry, s.hungry);
   }
 }
 
-// Blocks of the search kernel that can be resident on one SM for this query
-// size (registers, shared memory and warp slots), from the occupancy API.
+// Sixteen warps per SM, 128 registers a thread (run_levels says why).
+constexpr int min_blocks(int w) { return w == 16 ? 1 : 16 / w; }
+
 template <int W, bool EN>
-__global__ void __launch_bounds__(W * 32) k_search(SearchParams p) {
+__global__ void __launch_bounds__(W * 32, min_blocks(W)) k_search(const __grid_constant__ SearchParams p) {
   search_body<W, EN ? 1 : 0>(p);
 }
 
-// The tail-counting variant keeps the plain kernel's resident blocks (three
-// of 8 warps, two of 16) under a register bound.
 template <int W>
-__global__ void __launch_bounds__(W * 32, W == 16 ? 2 : 768 / (W * 32)) k_search_tail(SearchParams p) {
+__global__ void __launch_bounds__(W * 32, min_blocks(W)) k_search_tail(const __grid_constant__ SearchParams p) {
   search_body<W, 2>(p);
 }
 
@@ -1020,12 +1159,12 @@ void search_launch(const SearchParams& p, uint32_t blocks, size_t smem, cudaStre
 
 }  // namespace
 
-// Blocks of the search kernel that can be resident on one SM for this query
-// size (registers, shared memory and warp slots), from the occupancy API.
-// `mode` selects the instantiation: 0 plain counting (and hashes), 1 match
+// Blocks of the search kernel that can be resident on one SM for walks of
+// this shape (registers, shared memory and warp slots), from the
+// occupancy API.  `mode` selects the instantiation: 0 plain counting (and hashes), 1 match
 // sets, 2 tail counting.
-uint32_t search_max_blocks(uint32_t n_q, uint32_t warps, int mode) {
-  const size_t smem = search_smem_bytes(n_q, warps);
+uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode) {
+  const size_t smem = (size_t)shape.warp_bytes * warps;
   int nb = 0;
   cudaError_t e = cudaSuccess;
   switch (warps) {
@@ -1039,8 +1178,8 @@ uint32_t search_max_blocks(uint32_t n_q, uint32_t warps, int mode) {
 
 int search_mode(const SearchParams& p) { return p.enum_buf ? 1 : (p.tail ? 2 : 0); }
 
-void launch_search(const SearchParams& p, uint32_t n_q, uint32_t blocks, uint32_t warps, cudaStream_t s) {
-  const size_t smem = search_smem_bytes(n_q, warps);
+void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s) {
+  const size_t smem = (size_t)p.warp_bytes * warps;
   if (p.q) k_search_prep<<<1, 1, 0, s>>>(p.q, p.n_tasks, p.task_cap, p.sstat, p.error);
   const int mode = search_mode(p);
   switch (warps) {

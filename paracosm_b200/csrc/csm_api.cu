@@ -1120,12 +1120,23 @@ __global__ void k_init_count(DevGraph g, uint32_t la, uint32_t combo, unsigned l
   cnt[v] = c;
 }
 
-// Seeds [first, first + B) of the entry enumeration: info and one task each.
+// Seeds of one search launch where memory allows.  A launch of one seed -- the
+// batch size of a context that runs one update per launch -- leaves all but a
+// few warps idle and pays the launch sequence for every seed: the about 4,000
+// seeds of a 2^13-vertex graph's 6-vertex query take 253 ms that way and
+// 3.0 ms in one launch.
+constexpr uint32_t kInitSeeds = 1u << 16;
+
+// Seeds [first, first + B) of the entry enumeration: info and one task each,
+// and the launch's counters cleared (cnt[6]: tasks, cnt[7]: next task).
 __global__ void k_init_fill(DevGraph g, uint32_t combo, uint32_t label, const unsigned long long* off,
                             unsigned long long first, uint32_t B, uint32_t stride, uint32_t rank, UpdInfo* info,
-                            Task* tasks) {
+                            Task* tasks, unsigned long long* count, unsigned long long* bytes, unsigned int* stop,
+                            unsigned int* cnt) {
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
+  if (i == 0) { cnt[6] = B; cnt[7] = 0; }
   if (i >= B) return;
+  count[i] = 0; bytes[i] = 0; stop[i] = 0;
   const unsigned long long e = (first + i) * stride + rank;  // this shard's seeds
   uint32_t lo = 0, hi = g.n_cap;  // last x with off[x] <= e
   while (hi - lo > 1) {
@@ -1156,19 +1167,44 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
   const PlanAnchor& A = ctx->h_plan->anchors[0];
   const uint32_t combo = A.lb * g.n_el + A.el;
   const uint64_t n_cap = g.n_cap;
-  unsigned long long *cnt = nullptr, *off = nullptr, *total = nullptr;
-  void* tmp = nullptr;
+  // working memory of the call, in one allocation: entry counts and offsets of
+  // the vertices, scan scratch, and the seeds' search buffers (the batch
+  // buffers where there is no room for those)
   size_t tb = 0;
-  CK(cub::DeviceScan::ExclusiveSum(nullptr, tb, cnt, off, (int64_t)n_cap, st));
-  int rc = ctx->mem.alloc((void**)&cnt, 8ull * n_cap);
-  if (!rc) rc = ctx->mem.alloc((void**)&off, 8ull * n_cap);
-  if (!rc) rc = ctx->mem.alloc((void**)&total, 64);
-  if (!rc) rc = ctx->mem.alloc(&tmp, tb);
-  auto release = [&]() {
-    ctx->mem.release(cnt, 8ull * n_cap); ctx->mem.release(off, 8ull * n_cap);
-    ctx->mem.release(total, 64); ctx->mem.release(tmp, tb);
-  };
-  if (rc) { release(); return rc; }
+  {
+    unsigned long long* none = nullptr;
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, tb, none, none, (int64_t)n_cap, st));
+  }
+  tb = (tb + 255) & ~(size_t)255;
+  const size_t vbytes = 16ull * n_cap + 256 + tb;
+  constexpr size_t kPerSeed = 8 + 8 + sizeof(UpdInfo) + sizeof(Task) + 4;
+  uint32_t chunk = std::max<uint32_t>(kInitSeeds, ctx->bmax);
+  unsigned char* mem = nullptr;
+  size_t mem_bytes = vbytes + kPerSeed * chunk;
+  int rc = ctx->mem.alloc((void**)&mem, mem_bytes);
+  if (rc) {
+    chunk = ctx->bmax;
+    mem_bytes = vbytes;
+    rc = ctx->mem.alloc((void**)&mem, mem_bytes);
+    if (rc) return rc;
+    set_err(CSM_OK, "");
+  }
+  auto release = [&]() { ctx->mem.release(mem, mem_bytes); };
+  unsigned long long* cnt = reinterpret_cast<unsigned long long*>(mem);
+  unsigned long long* off = cnt + n_cap;
+  unsigned long long* total = off + n_cap;
+  void* tmp = mem + 16ull * n_cap + 256;
+  unsigned long long *s_count = ctx->d_count, *s_bytes = ctx->d_bytes;
+  UpdInfo* s_info = ctx->d_info;
+  Task* s_tasks = ctx->d_tasks;
+  unsigned int* s_stop = ctx->d_stop;
+  if (mem_bytes > vbytes) {
+    s_count = reinterpret_cast<unsigned long long*>(mem + vbytes);
+    s_bytes = s_count + chunk;
+    s_info = reinterpret_cast<UpdInfo*>(s_bytes + chunk);
+    s_tasks = reinterpret_cast<Task*>(s_info + chunk);
+    s_stop = reinterpret_cast<unsigned int*>(s_tasks + chunk);
+  }
   k_init_count<<<blocks_for(n_cap, 256), 256, 0, st>>>(g, A.la, combo, cnt); CKL();
   CK(cub::DeviceScan::ExclusiveSum(tmp, tb, cnt, off, (int64_t)n_cap, st));
   CK(cudaMemsetAsync(total, 0, 64, st));
@@ -1183,20 +1219,15 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
   const unsigned long long n_seeds = n_all > rank ? (n_all - rank + stride - 1) / stride : 0ull;
   uint32_t warps, bps;
   search_shape(ctx, warps, bps);
-  for (unsigned long long first = 0; first < n_seeds; first += ctx->bmax) {
-    const uint32_t B = (uint32_t)std::min<unsigned long long>(ctx->bmax, n_seeds - first);
-    unsigned int* c = ctx->d_cnt;
-    CK(cudaMemsetAsync(c, 0, 64, st));
-    CK(cudaMemcpyAsync(c + 6, &B, 4, cudaMemcpyHostToDevice, st));
-    CK(cudaMemsetAsync(ctx->d_count, 0, 8ull * B, st));
-    CK(cudaMemsetAsync(ctx->d_bytes, 0, 8ull * B, st));
-    CK(cudaMemsetAsync(ctx->d_stop, 0, 4ull * B, st));
-    k_init_fill<<<blocks_for(B, 256), 256, 0, st>>>(g, combo, A.el, off, first, B, stride, rank, ctx->d_info,
-                                                    ctx->d_tasks); CKL();
+  unsigned int* c = ctx->d_cnt;
+  for (unsigned long long first = 0; first < n_seeds; first += chunk) {
+    const uint32_t B = (uint32_t)std::min<unsigned long long>(chunk, n_seeds - first);
+    k_init_fill<<<blocks_for(B, 256), 256, 0, st>>>(g, combo, A.el, off, first, B, stride, rank, s_info, s_tasks,
+                                                    s_count, s_bytes, s_stop, c); CKL();
     SearchParams sp{};
-    sp.g = g; sp.plan = ctx->d_plan; sp.tasks = ctx->d_tasks; sp.n_tasks = c + 6; sp.task_cap = ctx->task_cap;
-    sp.task_next = c + 7; sp.info = ctx->d_info; sp.count = ctx->d_count; sp.hash = ctx->d_hash;
-    sp.bytes = ctx->d_bytes; sp.stop = ctx->d_stop;
+    sp.g = g; sp.plan = ctx->d_plan; sp.tasks = s_tasks; sp.n_tasks = c + 6; sp.task_cap = B;
+    sp.task_next = c + 7; sp.info = s_info; sp.count = s_count; sp.hash = ctx->d_hash;
+    sp.bytes = s_bytes; sp.stop = s_stop;
     sp.d2 = ctx->index.d2; sp.d2_words = ctx->index.words; sp.cap = 0;
     sp.homo = ctx->cfg.homomorphism; sp.want_hash = 0; sp.error = &g.ps->error;
     sp.q = ctx->d_q; sp.dq = ctx->d_dq; sp.qseq = ctx->d_qseq; sp.qcap = ctx->qcap;
@@ -1209,7 +1240,7 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
     set_search_shape(sp, *ctx->h_plan);
     launch_search(sp, (uint32_t)ctx->sm_count * bps, warps, st); CKL();
     ctx->search_launches++;
-    k_init_sum<<<std::min<uint32_t>(blocks_for(B, 256), 1024), 256, 0, st>>>(B, ctx->d_count, total); CKL();
+    k_init_sum<<<std::min<uint32_t>(blocks_for(B, 256), 1024), 256, 0, st>>>(B, s_count, total); CKL();
     ctx->launches += 3;
   }
   unsigned long long h = 0;

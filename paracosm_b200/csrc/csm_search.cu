@@ -40,7 +40,7 @@ struct LevelSM {
   uint32_t base[32];  // pool offset of the segment minus its start in the range
   uint32_t jv[32];    // matched vertex of the entry's first join
   uint8_t par[32];    // entry index in the previous level
-  uint8_t dsel[32];   // back entry that is the driver
+  uint8_t dsel[32];   // back entry that is the driver (kSelTouched: its row has touched entries)
   uint8_t jsel[32];   // back entry of the first join: the smallest segment but the driver's
   uint32_t cnt, cur, total, pad;
 };
@@ -161,16 +161,19 @@ __device__ __forceinline__ void load_walk_plan(uint32_t* w, const PlanAnchor* A,
   __syncwarp();
 }
 
-// Visits (position, data vertex) of the prefix of entry e of level d, the
-// last position first.  Every position is read from the levels when it is
-// needed: a copy of the prefix per lane would be local memory, and the random
-// loads leave it no room in L1.
+// Visits (position, data vertex) of the prefix of entry e of level d at the
+// positions of `mask`, the last one first.  Every position is read from the
+// levels when it is needed: a copy of the prefix per lane would be local
+// memory, and the random loads leave it no room in L1.
 template <class F>
-__device__ __forceinline__ void walk_prefix(const LevelSM* lv, int d, uint32_t e, F visit) {
+__device__ __forceinline__ void walk_prefix(const LevelSM* lv, int d, uint32_t e, uint32_t mask, F visit) {
 #pragma unroll 1
-  for (int j = d; j >= 0; --j) {
+  for (int j = d; mask; --j) {
     const LevelSM& S = lv[j ? j : 1];
-    visit((uint32_t)j, S.v[e]);
+    if ((mask >> j) & 1u) {
+      visit((uint32_t)j, S.v[e]);
+      mask &= ~(1u << j);
+    }
     e = S.par[e];
   }
 }
@@ -210,35 +213,38 @@ __device__ __forceinline__ uint32_t join_find(const SearchParams& p, const uint3
   return join_search(p, pool, v, back_combo(bw), x);
 }
 
+// LevelSM::dsel: the driver, and whether its row has entries touched in this
+// batch (else every entry of the segment is present at every batch time).
+constexpr uint32_t kSelMask = 0x1fu, kSelTouched = 0x80u, kSelNone = 0xffu;
+
 // The tests of candidate x for position `pos` beyond the filter bit, for the
 // prefix of entry e of level d: injectivity, every join, the batch-time
-// presence of every back edge.  `dsel` is the back entry whose segment
-// produced x (0xff: none) and `joined` one that was found before, with word
-// jhit (0xff: none).  The joins run one at a time and stop at the first that
-// fails.
+// presence of every back edge.  `dsel` (LevelSM::dsel) is the back entry whose
+// segment produced x (kSelNone: none) and `joined` one that was found before,
+// with word jhit (0xff: none).  The joins run one at a time and stop at the
+// first that fails; where no test needs the prefix, it is not walked.
 __device__ __forceinline__ bool check_rest(const SearchParams& p, const uint32_t* pool, const LevelSM* lv,
                                            const WalkPlan& wp, int d, uint32_t e, uint32_t pos, uint32_t x,
                                            uint32_t dsel, uint32_t joined, uint32_t jhit, int32_t t) {
-  const DevGraph& g = p.g;
   const uint32_t same = wp.samelab(pos), bm = wp.backmask(pos);
-  uint32_t b = wp.nb(pos);
+  uint32_t joins = bm;
+  if (dsel != kSelNone && !(dsel & kSelTouched)) joins &= ~(1u << (wp.back(pos, dsel & kSelMask) & 0xffu));
+  if (joined != 0xffu && !(jhit & kSlotTouched)) joins &= ~(1u << (wp.back(pos, joined) & 0xffu));
   bool ok = true;
-  walk_prefix(lv, d, e, [&](uint32_t j, uint32_t v) {
+  walk_prefix(lv, d, e, same | joins, [&](uint32_t j, uint32_t v) {
     if ((same >> j) & 1u) ok = ok && v != x;
-    if ((bm >> j) & 1u) {
-      --b;
-      if (ok && (b != dsel || g.t_count[v])) {
-        const uint32_t bw = wp.back(pos, b);
-        const uint32_t hit = b == joined ? jhit : join_find(p, pool, v, bw, x);
-        ok = hit != kSlotEmpty && (!(hit & kSlotTouched) || present_slow(p, v, back_combo(bw), x, t));
-      }
+    if (((joins >> j) & 1u) && ok) {
+      const uint32_t b = __popc(bm & ((1u << j) - 1u));
+      const uint32_t bw = wp.back(pos, b);
+      const uint32_t hit = b == joined ? jhit : join_find(p, pool, v, bw, x);
+      ok = hit != kSlotEmpty && (!(hit & kSlotTouched) || present_slow(p, v, back_combo(bw), x, t));
     }
   });
   return ok;
 }
 
 // Driver of position np (the smallest union-graph back segment, the first of
-// equals) for the prefix of entry e of level d, continued by x at position
+// equals; with kSelTouched) for the prefix of entry e of level d, continued by x at position
 // d + 1 when `with_x`; false if some back segment is empty at batch time t.
 // `jsel` and `jv` are the first join -- the back entry of the smallest segment
 // but the driver's, and its vertex: the row most likely to lack a candidate,
@@ -260,17 +266,14 @@ __device__ __forceinline__ bool pick_driver(const SearchParams& p, const LevelSM
   for (uint32_t end = nb; end > 0;) {
     const uint32_t beg = end > 4u ? end - 4u : 0u;
     uint32_t v[4] = {0, 0, 0, 0};
-    uint32_t b = nb;
     auto visit = [&](uint32_t j, uint32_t u) {
-      if ((bm >> j) & 1u) {
-        --b;
+      const uint32_t b = __popc(bm & ((1u << j) - 1u));
 #pragma unroll
-        for (uint32_t i = 0; i < 4; i++)
-          if (b == beg + i && b < end) v[i] = u;
-      }
+      for (uint32_t i = 0; i < 4; i++)
+        if (b == beg + i && b < end) v[i] = u;
     };
-    if (with_x) visit((uint32_t)d + 1u, x);
-    walk_prefix(lv, d, e, visit);
+    if (with_x && (bm >> (d + 1)) & 1u) visit((uint32_t)d + 1u, x);
+    walk_prefix(lv, d, e, bm & ((2u << d) - 1u), visit);
     uint32_t lo[4], hi[4], tc[4], c[4];
 #pragma unroll
     for (uint32_t i = 0; i < 4; i++) {
@@ -292,8 +295,8 @@ __device__ __forceinline__ bool pick_driver(const SearchParams& p, const LevelSM
         b4 += 4ull * szt;
         if (szt == 0) empty = true;
         if (sz <= best) {
-          second = best; jsel = dsel; jv = dv;
-          best = sz; dsel = beg + (uint32_t)i; dv = v[i]; dlo = lo[i];
+          second = best; jsel = dsel & kSelMask; jv = dv;
+          best = sz; dsel = (beg + (uint32_t)i) | (tc[i] ? kSelTouched : 0u); dv = v[i]; dlo = lo[i];
         } else if (sz <= second) {
           second = sz; jsel = beg + (uint32_t)i; jv = v[i];
         }
@@ -569,7 +572,7 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
             for (uint32_t i = 0; i < g && !seen; i++) {
               const uint32_t pi = A->gpos[gp + i];
               if (i == j || !filter_bit(p, wp.qv(pi), x) ||
-                  !check_rest(p, pool, lv, wp, L, owner, pi, x, 0xffu, 0xffu, 0u, (int32_t)t))
+                  !check_rest(p, pool, lv, wp, L, owner, pi, x, kSelNone, 0xffu, 0u, (int32_t)t))
                 continue;
               if (i < j) seen = true;
               else M |= 1u << i;
@@ -806,13 +809,13 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
             uint32_t* rec = p.enum_buf + r * p.enum_stride;
             rec[0] = p.enum_base + t;
             rec[1 + qv] = wx;
-            walk_prefix(lv, d, wown, [&](uint32_t j, uint32_t v) { rec[1 + wp.qv(j)] = v; });
+            walk_prefix(lv, d, wown, (2u << d) - 1u, [&](uint32_t j, uint32_t v) { rec[1 + wp.qv(j)] = v; });
           }
         }
       }
       if (MODE != 2 && p.want_hash && valid) {
         uint64_t s = pair_hash(qv, wx);
-        walk_prefix(lv, d, wown, [&](uint32_t j, uint32_t v) { s += pair_hash(wp.qv(j), v); });
+        walk_prefix(lv, d, wown, (2u << d) - 1u, [&](uint32_t j, uint32_t v) { s += pair_hash(wp.qv(j), v); });
         acc.hash += mix64(s);
       }
       acc.cnt += c;
@@ -897,13 +900,14 @@ __device__ __forceinline__ bool setup_root(const SearchParams& p, LevelSM* lv, u
     return false;
   }
   const PlanPos P2 = A->pos[2];
-  uint32_t sz = 0xffffffffu, szt = 1;
+  uint32_t sz = 0xffffffffu, szt = 1, touched = 0;
   uint64_t lo = 0, hi = 0;
   if (lane < P2.nb) {
     const uint32_t j = A->back_pos[P2.boff + lane], c = A->back_combo[P2.boff + lane];
     const uint32_t v = j == 0 ? m0 : m1;
     segment(p.g, v, c, lo, hi);
     sz = (uint32_t)(hi - lo);
+    touched = p.g.t_count[v];
     szt = seg_size_slow(p, v, c, (uint32_t)lo, (uint32_t)hi, (int32_t)t);
     acc.bytes += 4ull * szt;
   }
@@ -915,11 +919,13 @@ __device__ __forceinline__ bool setup_root(const SearchParams& p, LevelSM* lv, u
     key = other < key ? other : key;
   }
   const uint32_t minsz = (uint32_t)(key >> 32), sel = (uint32_t)key;
+  touched = __shfl_sync(0xffffffffu, touched, sel);
   const uint32_t other = sel == 0 ? 1u : 0u;  // position 2 has one back entry or two
   const uint32_t dlo0 = (uint32_t)__shfl_sync(0xffffffffu, lo, sel);
   if (lane == 0) {
     lv[1].cnt = 1; lv[1].cur = 0; lv[1].total = minsz;
-    lv[1].incl[0] = minsz; lv[1].base[0] = dlo0; lv[1].dsel[0] = (uint8_t)sel;
+    lv[1].incl[0] = minsz; lv[1].base[0] = dlo0;
+    lv[1].dsel[0] = (uint8_t)(sel | (touched ? kSelTouched : 0u));
     lv[1].v[0] = m1; lv[1].par[0] = 1; lv[1].v[1] = m0;
     lv[1].jsel[0] = (uint8_t)other;
     lv[1].jv[0] = P2.nb > 1 ? (A->back_pos[P2.boff + other] == 0 ? m0 : m1) : 0u;

@@ -642,14 +642,14 @@ static int run_plain_edge(csm_ctx* ctx, const csm_update* d_up, const csm_update
   } else if (h.is_add) {
     k_plain_mutate<<<1, 256, 0, st>>>(g, ctx->d_info, keys, nullptr, nullptr, 16u);
     CKL();
-    rc = index_apply_edge_one(ctx->index, g, keys, st, &ctx->launches);
+    rc = index_apply_edges(ctx->index, g, keys, 2, st, &ctx->launches);
     if (!rc) rc = query_seed_search(ctx, ctx, 1, out);
   } else {
     rc = query_seed_search(ctx, ctx, 1, out);
     if (rc) return rc;
     k_plain_mutate<<<1, 256, 0, st>>>(g, ctx->d_info, keys, nullptr, nullptr, 16u);
     CKL();
-    rc = index_apply_edge_one(ctx->index, g, keys, st, &ctx->launches);
+    rc = index_apply_edges(ctx->index, g, keys, 2, st, &ctx->launches);
   }
   if (rc) return rc;
   ctx->batches++;

@@ -4,15 +4,13 @@
 // Kernels (all integer work, bound by L2/HBM latency of the segment reads):
 //   k_ix_freq   query-edge frequencies and label counts that choose the root
 //               (ParaCOSM/CSM/matching/SymBi/symbi.cpp:116-195)
-//   k_ix_seed   marks the endpoints of changed directed entries for
-//               re-evaluation (the reference's per-edge Insertion/Deletion
-//               TopDown/BottomUp entry, symbi.cpp:679-735)
-//   k_ix_prop   marks the DAG-neighbour-side neighbours of vertices whose
-//               flag changed (the Q1 / Q2 propagation loops, symbi.cpp:714-735)
-//   k_ix_eval   re-evaluates marked flags of one query vertex from their
-//               definition: one warp per 64-vertex word; short segments are
-//               scanned by one lane each, long ones by the whole warp with
-//               an early exit on the first supporting neighbour
+//   k_ix_eval   evaluates every flag of one query vertex (index build)
+//   k_ix_round  one round after edges or a vertex changed: marks the vertices
+//               concerned (the reference's per-edge Insertion/Deletion
+//               TopDown/BottomUp entry, symbi.cpp:679-735), re-evaluates marked
+//               flags query vertex by query vertex in DAG order, and marks the
+//               DAG-neighbour-side neighbours of vertices whose flag changed
+//               (the Q1 / Q2 propagation loops, symbi.cpp:714-735)
 #include <cooperative_groups.h>
 
 #include <algorithm>
@@ -93,219 +91,217 @@ __global__ void k_ix_freq(DevGraph g, uint32_t ne, const uint32_t* __restrict__ 
     if (s_lc[i]) atomicAdd(&lcount[i], s_lc[i]);
 }
 
-// Marks, for every changed directed entry x -> y (combo = (L(y), l)) and every
-// DAG edge p -> c with L(p) = L(x), L(c) = L(y) and label l: y for d1 of c,
-// x for d2 of p.  The reverse entry y -> x covers the other orientation.
-__global__ void k_ix_seed(const uint64_t* __restrict__ keys, uint32_t L, DevGraph g, const IxDag* __restrict__ dag,
-                          IxBits b) {
-  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= L) return;
-  const uint64_t k = keys[i];
-  if (!g.kb.real(k)) return;
-  const uint32_t x = g.kb.x_of(k), c = g.kb.c_of(k), y = g.kb.y_of(k);
-  const uint32_t ly = c / g.n_el, el = c % g.n_el;
-  const uint32_t lx = g.vlabel[x];
-  const uint32_t ne = dag->n_edges;
-  for (uint32_t e = 0; e < ne; e++) {
-    if (dag->eel[e] != el) continue;
-    const uint32_t p = dag->ep[e], ch = dag->ec[e];
-    if (dag->qlab[p] != lx || dag->qlab[ch] != ly) continue;
-    atomicOr((unsigned long long*)&b.m1[(uint64_t)ch * b.words + (y >> 6)], 1ull << (y & 63));
-    atomicOr((unsigned long long*)&b.m2[(uint64_t)p * b.words + (x >> 6)], 1ull << (x & 63));
-    *b.active = 1u;
-  }
-}
-
-// A new vertex: mark it for every query vertex (only its d1 at the root can
-// become set; the evaluation decides).
-__global__ void k_ix_seed_vertex(uint32_t v, const IxDag* __restrict__ dag, IxBits b) {
-  const uint32_t u = threadIdx.x;
-  if (u >= dag->nq) return;
-  if (u == 0) *b.active = 1u;
-  b.m1[(uint64_t)u * b.words + (v >> 6)] |= 1ull << (v & 63);
-  b.m2[(uint64_t)u * b.words + (v >> 6)] |= 1ull << (v & 63);
-}
-
-// Phase 1 (d1 of u): for each parent p, every vertex w whose d1[p] changed
-// marks its neighbours in S(w, L(u), l(u,p)).  Phase 2 (d2 of u): the same
-// from each child c through d2[c] changes.  One warp per word of changes.
-__device__ __forceinline__ void ix_prop(const DevGraph& g, const IxDag* __restrict__ dag, const IxBits& b, uint32_t u,
-                                        uint32_t phase, uint32_t lane, uint32_t warp, uint32_t nwarps) {
-  const uint32_t* pool = g.pools[g.ps->active];
-  const uint32_t nsrc = phase == 1 ? dag->npar[u] : dag->nchd[u];
-  uint64_t* dst = (phase == 1 ? b.m1 : b.m2) + (uint64_t)u * b.words;
-  for (uint32_t s = 0; s < nsrc; s++) {
+// Does v keep its flag for query vertex u (phase 1: d1, phase 2: d2)?  One lane;
+// `far` instead when a segment is too long for one.
+__device__ __forceinline__ bool ix_lane_eval(const DevGraph& g, const uint32_t* pool, const IxDag* __restrict__ dag,
+                                             const IxBits& b, uint32_t u, uint32_t phase, uint32_t v, bool& far) {
+  const uint32_t nchk = phase == 1 ? dag->npar[u] : dag->nchd[u];
+  const uint64_t* sup = (phase == 1 || dag->lighting) ? b.d1 : b.d2;
+  const uint32_t nreq = (phase == 1 && dag->lighting) ? dag->nreq[u] : 0u;
+  bool ok = phase == 1 ? g.vlabel[v] == dag->qlab[u] : bit_of(b.d1 + (uint64_t)u * b.words, v);
+  for (uint32_t r = 0; r < nreq && ok; r++) ok = seg_count(g, v, dag->req_combo[u][r]) >= dag->req_mult[u][r];
+  for (uint32_t s = 0; s < nchk && ok; s++) {
     const uint32_t q = phase == 1 ? dag->par[u][s] : dag->chd[u][s];
-    const uint32_t combo = phase == 1 ? dag->par_ucombo[u][s] : dag->chd_ucombo[u][s];
-    const uint64_t* src = (phase == 1 || dag->lighting ? b.c1 : b.c2) + (uint64_t)q * b.words;
-    for (uint64_t wi = warp; wi < b.words; wi += nwarps) {
-      uint64_t word = src[wi];
-      while (word) {
-        const uint32_t w = (uint32_t)(wi * 64 + (uint64_t)(__ffsll((long long)word) - 1));
-        word &= word - 1;
-        uint64_t lo, hi;
-        segment(g, w, combo, lo, hi);
-        for (uint64_t k = lo + lane; k < hi; k += 32) {
-          const uint32_t v = pool[k];
-          atomicOr((unsigned long long*)&dst[v >> 6], 1ull << (v & 63));
-        }
-      }
-    }
+    uint64_t lo, hi;
+    segment(g, v, phase == 1 ? dag->par_vcombo[u][s] : dag->chd_vcombo[u][s], lo, hi);
+    if (hi - lo > kLaneScanMax) { far = true; break; }
+    ok = lane_support(pool, lo, hi, sup + (uint64_t)q * b.words);
   }
+  return ok;
 }
 
-__global__ void k_ix_prop(DevGraph g, const IxDag* __restrict__ dag, IxBits b, uint32_t u, uint32_t phase) {
-  if (!*b.active) return;
-  ix_prop(g, dag, b, u, phase, threadIdx.x & 31, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-          (gridDim.x * blockDim.x) >> 5);
+// The same by a whole warp.  Lane s looks up segment s, all at once; then the
+// warp scans them one after another.
+__device__ __forceinline__ bool ix_warp_eval(const DevGraph& g, const uint32_t* pool, const IxDag* __restrict__ dag,
+                                             const IxBits& b, uint32_t u, uint32_t phase, uint32_t v, uint32_t lane) {
+  const uint32_t nchk = phase == 1 ? dag->npar[u] : dag->nchd[u];
+  const uint64_t* sup = (phase == 1 || dag->lighting) ? b.d1 : b.d2;
+  const uint32_t nreq = (phase == 1 && dag->lighting) ? dag->nreq[u] : 0u;
+  bool ok = phase == 1 ? g.vlabel[v] == dag->qlab[u] : bit_of(b.d1 + (uint64_t)u * b.words, v);
+  if (lane < nreq) ok = ok && seg_count(g, v, dag->req_combo[u][lane]) >= dag->req_mult[u][lane];
+  uint64_t lo = 0, hi = 0;
+  uint32_t q = 0;
+  if (lane < nchk) {
+    q = phase == 1 ? dag->par[u][lane] : dag->chd[u][lane];
+    segment(g, v, phase == 1 ? dag->par_vcombo[u][lane] : dag->chd_vcombo[u][lane], lo, hi);
+    ok = ok && lo < hi;
+  }
+  if (!__all_sync(0xffffffffu, ok)) return false;
+  for (uint32_t s = 0; s < nchk; s++) {
+    const uint64_t* flag = sup + (uint64_t)__shfl_sync(0xffffffffu, q, s) * b.words;
+    if (!warp_support(pool, __shfl_sync(0xffffffffu, lo, s), __shfl_sync(0xffffffffu, hi, s), flag, lane)) return false;
+  }
+  return true;
 }
 
-// Re-evaluates the marked flags of query vertex u (phase 1: d1, phase 2: d2).
-// full = 1 evaluates every vertex of u's label (index build).  Each warp owns
-// whole words of the target bitset, so its updates need no atomics.
-__device__ __forceinline__ void ix_eval(const DevGraph& g, const IxDag* __restrict__ dag, const IxBits& b, uint32_t u,
-                                        uint32_t phase, uint32_t full, uint32_t lane, uint32_t warp,
-                                        uint32_t nwarps) {
+// Every flag of query vertex u from its definition (index build).  Each warp
+// owns whole words of the target bitset, so its updates need no atomics.
+__global__ void k_ix_eval(DevGraph g, const IxDag* __restrict__ dag, IxBits b, uint32_t u, uint32_t phase) {
+  const uint32_t lane = threadIdx.x & 31, warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
   const uint32_t* pool = g.pools[g.ps->active];
   const uint32_t lu = dag->qlab[u];
   const uint64_t off = (uint64_t)u * b.words;
   uint64_t* target = (phase == 1 ? b.d1 : b.d2) + off;
-  uint64_t* mark = (phase == 1 ? b.m1 : b.m2) + off;
-  uint64_t* chg = (phase == 1 ? b.c1 : b.c2) + off;
-  const uint64_t* d1u = b.d1 + off;
-  const uint32_t nchk = phase == 1 ? dag->npar[u] : dag->nchd[u];
-  // support flags of the checked neighbours: d1 of parents; d2 of children,
-  // or their d1 in lighting mode
-  const uint64_t* sup = (phase == 1 || dag->lighting) ? b.d1 : b.d2;
-  const uint32_t nreq = (phase == 1 && dag->lighting) ? dag->nreq[u] : 0u;
   for (uint64_t wi = warp; wi < b.words; wi += nwarps) {
     uint64_t cand;
-    if (full) {
-      if (phase == 1) {
-        const uint64_t v0 = wi * 64 + lane, v1 = v0 + 32;
-        const bool a = v0 < g.n && g.vlabel[v0] == lu;
-        const bool c = v1 < g.n && g.vlabel[v1] == lu;
-        cand = (uint64_t)__ballot_sync(0xffffffffu, a) | ((uint64_t)__ballot_sync(0xffffffffu, c) << 32);
-      } else {
-        cand = d1u[wi];
-      }
+    if (phase == 1) {
+      const uint64_t v0 = wi * 64 + lane, v1 = v0 + 32;
+      const bool a = v0 < g.n && g.vlabel[v0] == lu;
+      const bool c = v1 < g.n && g.vlabel[v1] == lu;
+      cand = (uint64_t)__ballot_sync(0xffffffffu, a) | ((uint64_t)__ballot_sync(0xffffffffu, c) << 32);
     } else {
-      cand = mark[wi];
-      if (phase == 2) cand |= b.c1[off + wi];
-      __syncwarp();
-      if (cand && lane == 0) mark[wi] = 0;
+      cand = b.d1[off + wi];
     }
     if (!cand) continue;
-    const uint64_t old = target[wi];
-    // pass 1: one candidate per lane (the j-th set bit goes to lane j % 32)
-    uint64_t mine = 0, defer = 0;
-    {
-      uint64_t rest = cand;
-      uint32_t j = 0;
-      while (rest) {
-        const uint32_t bitpos = (uint32_t)(__ffsll((long long)rest) - 1);
-        rest &= rest - 1;
-        if ((j++ & 31) != lane) continue;
-        const uint32_t v = (uint32_t)(wi * 64 + bitpos);
-        bool ok;
-        bool long_seg = false;
-        if (phase == 1) ok = g.vlabel[v] == lu;
-        else ok = bit_of(d1u, v);
-        for (uint32_t r = 0; r < nreq && ok; r++) ok = seg_count(g, v, dag->req_combo[u][r]) >= dag->req_mult[u][r];
-        for (uint32_t s = 0; s < nchk && ok; s++) {
-          const uint32_t q = phase == 1 ? dag->par[u][s] : dag->chd[u][s];
-          const uint32_t combo = phase == 1 ? dag->par_vcombo[u][s] : dag->chd_vcombo[u][s];
-          const uint64_t* flag = sup + (uint64_t)q * b.words;
-          uint64_t lo, hi;
-          segment(g, v, combo, lo, hi);
-          if (hi - lo > kLaneScanMax) { long_seg = true; break; }
-          ok = lane_support(pool, lo, hi, flag);
-        }
-        if (long_seg) defer |= 1ull << bitpos;
-        else if (ok) mine |= 1ull << bitpos;
-      }
+    // one candidate per lane (the j-th set bit goes to lane j % 32), then the
+    // vertices with a long segment by the whole warp
+    uint64_t mine = 0, defer = 0, rest = cand;
+    for (uint32_t j = 0; rest; j++) {
+      const uint32_t bitpos = (uint32_t)(__ffsll((long long)rest) - 1);
+      rest &= rest - 1;
+      if ((j & 31) != lane) continue;
+      bool far = false;
+      const bool ok = ix_lane_eval(g, pool, dag, b, u, phase, (uint32_t)(wi * 64 + bitpos), far);
+      if (far) defer |= 1ull << bitpos;
+      else if (ok) mine |= 1ull << bitpos;
     }
-    uint64_t newbits = warp_or64(mine);
+    uint64_t bits = warp_or64(mine);
     defer = warp_or64(defer);
-    // pass 2: vertices with a long segment, by the whole warp
-    while (defer) {
+    for (; defer; defer &= defer - 1) {
       const uint32_t bitpos = (uint32_t)(__ffsll((long long)defer) - 1);
-      defer &= defer - 1;
-      const uint32_t v = (uint32_t)(wi * 64 + bitpos);
-      bool ok = phase == 1 ? (g.vlabel[v] == lu) : bit_of(d1u, v);
-      for (uint32_t r = 0; r < nreq && ok; r++) ok = seg_count(g, v, dag->req_combo[u][r]) >= dag->req_mult[u][r];
-      for (uint32_t s = 0; s < nchk && ok; s++) {
-        const uint32_t q = phase == 1 ? dag->par[u][s] : dag->chd[u][s];
-        const uint32_t combo = phase == 1 ? dag->par_vcombo[u][s] : dag->chd_vcombo[u][s];
-        const uint64_t* flag = sup + (uint64_t)q * b.words;
-        uint64_t lo, hi;
-        segment(g, v, combo, lo, hi);
-        ok = warp_support(pool, lo, hi, flag, lane);
-      }
-      if (ok) newbits |= 1ull << bitpos;
+      if (ix_warp_eval(g, pool, dag, b, u, phase, (uint32_t)(wi * 64 + bitpos), lane)) bits |= 1ull << bitpos;
     }
-    const uint64_t nw = (old & ~cand) | (newbits & cand);
-    if (lane == 0 && nw != old) {
-      target[wi] = nw;
-      chg[wi] |= nw ^ old;
-    }
+    if (lane == 0) target[wi] = bits;
     __syncwarp();
   }
 }
 
-__global__ void k_ix_eval(DevGraph g, const IxDag* __restrict__ dag, IxBits b, uint32_t u, uint32_t phase,
-                          uint32_t full) {
-  if (!*b.active) return;
-  ix_eval(g, dag, b, u, phase, full, threadIdx.x & 31, (blockIdx.x * blockDim.x + threadIdx.x) >> 5,
-          (gridDim.x * blockDim.x) >> 5);
+// Marks v for re-evaluation of its d1 (phase 1) or d2 (phase 2) flag of u.
+__device__ __forceinline__ void ix_mark(const IxBits& b, uint32_t nq, uint32_t phase, uint32_t u, uint32_t v) {
+  const uint64_t bit = 1ull << (v & 63);
+  uint64_t* word = (phase == 1 ? b.m1 : b.m2) + (uint64_t)u * b.words + (v >> 6);
+  if (atomicOr((unsigned long long*)word, bit) & bit) return;
+  const uint32_t row = (phase == 1 ? 0u : nq) + u;
+  const uint32_t i = atomicAdd(&b.count[row], 1u);
+  if (i < b.list_cap) b.list[(size_t)row * b.list_cap + i] = v;
 }
 
-// End of a round: the change bitsets start the next round empty.
-__global__ void k_ix_clear_changes(IxBits b, uint64_t n) {
-  if (!*b.active) return;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    b.c1[i] = 0;
-    b.c2[i] = 0;
+// Marks for DAG edge e and the changed directed entry k = x -> y (combo = (L(y),
+// l)), when its labels are the edge's: y for d1 of the child, x for d2 of the
+// parent.  The reverse entry y -> x covers the other orientation.
+__device__ __forceinline__ void ix_seed(const DevGraph& g, const IxDag* __restrict__ dag, const IxBits& b, uint64_t k,
+                                        uint32_t lx, uint32_t e) {
+  const uint32_t c = g.kb.c_of(k);
+  if (dag->eel[e] != c % g.n_el) return;
+  const uint32_t p = dag->ep[e], ch = dag->ec[e];
+  if (dag->qlab[p] != lx || dag->qlab[ch] != c / g.n_el) return;
+  ix_mark(b, dag->nq, 1, ch, g.kb.y_of(k));
+  ix_mark(b, dag->nq, 2, p, g.kb.x_of(k));
+}
+
+// Re-evaluates u's flag of vertex v in each lane with `has` (their marks are
+// taken off here), and marks what depends on the flags that changed.
+__device__ __forceinline__ void ix_items(const DevGraph& g, const uint32_t* pool, const IxDag* __restrict__ dag,
+                                         const IxBits& b, uint32_t u, uint32_t phase, bool has, uint32_t v,
+                                         bool by_lane, uint32_t lane) {
+  const uint64_t off = (uint64_t)u * b.words;
+  const uint64_t bit = 1ull << (v & 63);
+  unsigned long long* target = (unsigned long long*)((phase == 1 ? b.d1 : b.d2) + off + (v >> 6));
+  bool ok = false, far = !by_lane;
+  if (has && by_lane) ok = ix_lane_eval(g, pool, dag, b, u, phase, v, far);
+  for (uint32_t todo = __ballot_sync(0xffffffffu, has && far); todo; todo &= todo - 1) {
+    const uint32_t l = (uint32_t)__ffs((int)todo) - 1;
+    const bool r = ix_warp_eval(g, pool, dag, b, u, phase, __shfl_sync(0xffffffffu, v, l), lane);
+    if (l == lane) ok = r;
+  }
+  bool changed = false;
+  if (has) {
+    atomicAnd((unsigned long long*)((phase == 1 ? b.m1 : b.m2) + off + (v >> 6)), ~bit);
+    changed = ((*target & bit) != 0) != ok;  // no other lane has this vertex
+    if (changed) atomicXor(target, bit);
+    if (changed && phase == 1) ix_mark(b, dag->nq, 2, u, v);
+  }
+  // phase 1: the d1 of u's children (their d2 in lighting mode) over v's
+  // neighbours; phase 2: the d2 of u's parents
+  if (phase == 2 && dag->lighting) return;
+  const uint32_t n_to = phase == 1 ? dag->nchd[u] : dag->npar[u];
+  const uint32_t to_phase = (phase == 2 || dag->lighting) ? 2u : 1u;
+  for (uint32_t todo = __ballot_sync(0xffffffffu, changed); todo; todo &= todo - 1) {
+    const uint32_t w = __shfl_sync(0xffffffffu, v, (uint32_t)__ffs((int)todo) - 1);
+    for (uint32_t s = 0; s < n_to; s++) {
+      const uint32_t q = phase == 1 ? dag->chd[u][s] : dag->par[u][s];
+      uint64_t lo, hi;
+      segment(g, w, phase == 1 ? dag->chd_vcombo[u][s] : dag->par_vcombo[u][s], lo, hi);
+      for (uint64_t k = lo + lane; k < hi; k += 32) ix_mark(b, dag->nq, to_phase, q, pool[k]);
+    }
   }
 }
 
-// One incremental round over every query vertex in a single launch, for the
-// changes of one edge update (the plain form): the steps of
-// index_launch_round -- per query vertex in DAG order, propagation of the
-// parents' d1 changes and re-evaluation of d1, then in reverse order the
-// children's d2 changes and d2 -- separated by grid-wide barriers instead of
-// kernel boundaries.  Launched cooperatively (every block resident), with a
-// grid no larger than the occupancy allows.  Every block takes the same
-// branches, so every block reaches every barrier.
-__global__ void __launch_bounds__(256) k_ix_round_coop(DevGraph g, const IxDag* __restrict__ dag, IxBits b,
-                                                       IxOrder ord) {
-  if (!*b.active) return;  // nothing that the flags depend on changed: the same in every block
+// One incremental round in a single cooperative launch (every block resident),
+// for the changed directed entries keys[0, L) and, when it is not kNone, the
+// new or removed vertex `vert`.  The marks come first; then, query vertex by
+// query vertex in DAG order, the d1 flags on the work lists, and in reverse
+// order the d2 flags, each followed by a grid barrier.  An empty list costs
+// one load and no barrier: few of the 2 |V_Q| are not (the round of one edge
+// update took 2 |V_Q| + 52 barriers over whole bitsets before, 153 us for a
+// 13-vertex query on 2^19 vertices).  A list's length is read by every block
+// between the barrier after the last mark it can get and the one after its
+// own work, so all blocks take the same way.
+__global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __restrict__ dag, IxBits b, IxOrder ord,
+                                                  const uint64_t* __restrict__ keys, uint32_t L, uint32_t vert) {
   cg::grid_group grid = cg::this_grid();
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t warp = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-  const uint32_t nwarps = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t i = 0; i < ord.nq; i++) {
-    const uint32_t u = ord.order[i];
-    if (dag->npar[u] != 0) {  // the root's d1 is its label test: only new vertices change it
-      ix_prop(g, dag, b, u, 1, lane, warp, nwarps);
-      grid.sync();
+  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
+  const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
+  const uint32_t ne = dag->n_edges, nq = ord.nq;
+  const uint32_t* pool = g.pools[g.ps->active];
+  if (L <= 64) {  // a thread per (entry, DAG edge)
+    for (uint32_t i = tid; i < L * ne; i += nthreads) {
+      const uint64_t k = keys[i / ne];
+      if (g.kb.real(k)) ix_seed(g, dag, b, k, g.vlabel[g.kb.x_of(k)], i % ne);
     }
-    ix_eval(g, dag, b, u, 1, 0, lane, warp, nwarps);
-    grid.sync();
-  }
-  for (uint32_t i = ord.nq; i-- > 0;) {
-    const uint32_t u = ord.order[i];
-    if (dag->nchd[u] != 0) {
-      ix_prop(g, dag, b, u, 2, lane, warp, nwarps);
-      grid.sync();
+  } else {
+    for (uint32_t i = tid; i < L; i += nthreads) {
+      const uint64_t k = keys[i];
+      if (!g.kb.real(k)) continue;
+      const uint32_t lx = g.vlabel[g.kb.x_of(k)];
+      for (uint32_t e = 0; e < ne; e++) ix_seed(g, dag, b, k, lx, e);
     }
-    ix_eval(g, dag, b, u, 2, 0, lane, warp, nwarps);
-    grid.sync();
   }
-  const uint64_t n = (uint64_t)ord.nq * b.words;
-  for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
-    b.c1[i] = 0;
-    b.c2[i] = 0;
+  if (vert != kNone && tid < nq) {
+    ix_mark(b, nq, 1, tid, vert);
+    ix_mark(b, nq, 2, tid, vert);
+  }
+  grid.sync();
+  for (uint32_t i = 0; i < 2 * nq; i++) {
+    const uint32_t phase = i < nq ? 1u : 2u;
+    const uint32_t u = ord.order[phase == 1 ? i : 2 * nq - 1 - i];
+    const uint32_t row = (phase == 1 ? 0u : nq) + u;
+    const uint32_t n = *(volatile unsigned int*)&b.count[row];
+    if (n == 0) continue;
+    if (n <= b.list_cap) {
+      // as many items per warp as it takes to share them out; with several,
+      // each lane first tries its own
+      const uint32_t* list = b.list + (size_t)row * b.list_cap;
+      const uint32_t per = min(32u, (n + nwarps - 1) / nwarps);
+      for (uint32_t base = warp * per; base < n; base += nwarps * per) {
+        const bool has = lane < per && base + lane < n;
+        ix_items(g, pool, dag, b, u, phase, has, has ? __ldcg(list + base + lane) : 0u, per > 4, lane);
+      }
+    } else {
+      const uint64_t* mark = (phase == 1 ? b.m1 : b.m2) + (uint64_t)u * b.words;
+      for (uint64_t wi = warp; wi < b.words; wi += nwarps) {
+        const uint64_t word = __ldcg(mark + wi);
+        if (!word) continue;
+#pragma unroll 1
+        for (uint32_t half = 0; half < 2; half++)
+          ix_items(g, pool, dag, b, u, phase, (word >> (32u * half + lane)) & 1ULL, (uint32_t)(wi * 64 + 32u * half + lane),
+                   true, lane);
+      }
+    }
+    grid.sync();
+    if (tid == 0) b.count[row] = 0;
   }
 }
 
@@ -327,6 +323,15 @@ namespace {
     if (e_ != cudaSuccess) return set_err(CSM_ECUDA, "%s: %s", #x, cudaGetErrorString(e_)); \
   } while (0)
 
+// Work-list entries per query vertex and phase: 2 |V_Q| lists of 128 KB are a
+// small part of the bitsets of a large graph, and a batch of 65,536 updates
+// marks fewer vertices (a list that overflows is worked off from its marks).
+constexpr uint32_t kListCap = 32768;
+
+size_t list_bytes(const IndexState& ix) {
+  return 4ull * 2 * ix.h_dag.nq * ix.bits.list_cap + 8ull * ix.h_dag.nq;
+}
+
 // Root choice (ParaCOSM/CSM/matching/SymBi/symbi.cpp:116-195, identical in
 // TurboFlux/turboflux.cpp:82-149): the first query edge (u < u', adjacency
 // order) of least frequency; of its endpoints the one whose label is rarer in
@@ -346,30 +351,16 @@ uint32_t choose_root(const IndexQuery& q, const std::vector<std::pair<uint32_t, 
 
 }  // namespace
 
-static int index_launch_round(IndexState& ix, const DevGraph& g, cudaStream_t st, uint64_t* launches, bool full) {
+// The full first evaluation: per query vertex in DAG order d1, in reverse d2.
+static int index_launch_build(IndexState& ix, const DevGraph& g, cudaStream_t st, uint64_t* launches) {
   const uint32_t nq = ix.h_dag.nq;
   const uint64_t warps_needed = std::max<uint64_t>(ix.words, 1);
   const uint32_t blocks = (uint32_t)std::min<uint64_t>((warps_needed + 7) / 8, (uint64_t)ix.sm_count * 8);
-  for (uint32_t i = 0; i < nq; i++) {
-    const uint32_t u = ix.order[i];
-    if (!full && ix.h_dag.npar[u] == 0) {
-      // the root's d1 is its label test: only new vertices change it
-      k_ix_eval<<<blocks, 256, 0, st>>>(g, ix.d_dag, ix.bits, u, 1, 0);
-      (*launches)++;
-      continue;
-    }
-    if (!full) { k_ix_prop<<<blocks, 256, 0, st>>>(g, ix.d_dag, ix.bits, u, 1); (*launches)++; }
-    k_ix_eval<<<blocks, 256, 0, st>>>(g, ix.d_dag, ix.bits, u, 1, full ? 1u : 0u);
+  for (uint32_t i = 0; i < 2 * nq; i++) {
+    const uint32_t phase = i < nq ? 1u : 2u;
+    k_ix_eval<<<blocks, 256, 0, st>>>(g, ix.d_dag, ix.bits, ix.order[phase == 1 ? i : 2 * nq - 1 - i], phase);
     (*launches)++;
   }
-  for (uint32_t i = nq; i-- > 0;) {
-    const uint32_t u = ix.order[i];
-    if (!full && ix.h_dag.nchd[u]) { k_ix_prop<<<blocks, 256, 0, st>>>(g, ix.d_dag, ix.bits, u, 2); (*launches)++; }
-    k_ix_eval<<<blocks, 256, 0, st>>>(g, ix.d_dag, ix.bits, u, 2, full ? 1u : 0u);
-    (*launches)++;
-  }
-  k_ix_clear_changes<<<ix.sm_count * 2, 256, 0, st>>>(ix.bits, (uint64_t)nq * ix.words);
-  (*launches)++;
   IXCK(cudaGetLastError());
   return CSM_OK;
 }
@@ -529,26 +520,26 @@ static int index_finish(IndexState& ix, DevMem& mem, const DevGraph& g, const In
   ix.words = ((uint64_t)g.n_cap + 63) / 64;
   ix.words = (ix.words + 3) & ~3ull;
   const uint64_t fam = 8ull * nq * ix.words;
-  rc = mem.alloc((void**)&ix.bits.d1, 6 * fam);
+  ix.bits.list_cap = std::min<uint32_t>(g.n_cap, kListCap);
+  rc = mem.alloc((void**)&ix.bits.d1, 4 * fam);
   if (rc) return rc;
   ix.bits.d2 = ix.bits.d1 + nq * ix.words;
   ix.bits.m1 = ix.bits.d2 + nq * ix.words;
   ix.bits.m2 = ix.bits.m1 + nq * ix.words;
-  ix.bits.c1 = ix.bits.m2 + nq * ix.words;
-  ix.bits.c2 = ix.bits.c1 + nq * ix.words;
   ix.bits.words = ix.words;
   rc = mem.alloc((void**)&ix.d_dag, sizeof(IxDag));
   if (rc) return rc;
   rc = mem.alloc((void**)&ix.d_pop, 16);
   if (rc) return rc;
-  rc = mem.alloc((void**)&ix.bits.active, 16);
+  rc = mem.alloc((void**)&ix.bits.list, list_bytes(ix));
   if (rc) return rc;
-  IXCK(cudaMemsetAsync(ix.bits.active, 0xff, 4, st));  // the build evaluates everything
-  IXCK(cudaMemsetAsync(ix.bits.d1, 0, 6 * fam, st));
+  ix.bits.count = ix.bits.list + (size_t)2 * nq * ix.bits.list_cap;
+  IXCK(cudaMemsetAsync(ix.bits.count, 0, 8ull * nq, st));
+  IXCK(cudaMemsetAsync(ix.bits.d1, 0, 4 * fam, st));
   IXCK(cudaMemcpyAsync(ix.d_dag, &D, sizeof(IxDag), cudaMemcpyHostToDevice, st));
   ix.d2 = ix.bits.d2;
   ix.active = true;
-  rc = index_launch_round(ix, g, st, launches, true);
+  rc = index_launch_build(ix, g, st, launches);
   if (rc) return rc;
   IXCK(cudaStreamSynchronize(st));
   return CSM_OK;
@@ -598,54 +589,31 @@ int index_build(IndexState& ix, DevMem& mem, const DevGraph& g, const IndexQuery
   return rc;
 }
 
-// The incremental round as one cooperative launch (k_ix_round_coop).
-static int index_round_coop(IndexState& ix, const DevGraph& g, cudaStream_t st, uint64_t* launches) {
-  if (!ix.coop_blocks) {
-    int occ = 0;
-    IXCK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k_ix_round_coop, 256, 0));
-    const uint64_t warps_needed = std::max<uint64_t>(ix.words, 1);
-    ix.coop_blocks = (uint32_t)std::max<uint64_t>(
-        1, std::min<uint64_t>((warps_needed + 7) / 8, (uint64_t)ix.sm_count * (uint64_t)std::max(occ, 1)));
-  }
+// The incremental round (k_ix_round): one block per SM.
+static int index_round(IndexState& ix, const DevGraph& g, const uint64_t* keys, uint32_t L, uint32_t vert,
+                       cudaStream_t st, uint64_t* launches) {
   IxOrder ord{};
   ord.nq = ix.h_dag.nq;
   for (uint32_t i = 0; i < ord.nq; i++) ord.order[i] = ix.order[i];
   DevGraph gv = g;
   const IxDag* dag = ix.d_dag;
   IxBits bits = ix.bits;
-  void* args[] = {&gv, &dag, &bits, &ord};
-  IXCK(cudaLaunchCooperativeKernel((const void*)k_ix_round_coop, dim3(ix.coop_blocks), dim3(256), args, 0, st));
+  void* args[] = {&gv, &dag, &bits, &ord, &keys, &L, &vert};
+  IXCK(cudaLaunchCooperativeKernel((const void*)k_ix_round, dim3((unsigned)ix.sm_count), dim3(512), args, 0, st));
   (*launches)++;
   return CSM_OK;
 }
 
-// A batch's changed edges: the seed over all of them, then the round in one
-// launch (2 |V_Q| + 1 launches per batch before).
 int index_apply_edges(IndexState& ix, const DevGraph& g, const uint64_t* keys, uint32_t L, cudaStream_t st,
                       uint64_t* launches) {
   if (!ix.active || L == 0) return CSM_OK;
-  IXCK(cudaMemsetAsync(ix.bits.active, 0, 4, st));  // set by the seed when a changed entry matters
-  k_ix_seed<<<(L + 255) / 256, 256, 0, st>>>(keys, L, g, ix.d_dag, ix.bits);
-  (*launches)++;
-  return index_round_coop(ix, g, st, launches);
-}
-
-int index_apply_edge_one(IndexState& ix, const DevGraph& g, const uint64_t* keys, cudaStream_t st,
-                         uint64_t* launches) {
-  if (!ix.active) return CSM_OK;
-  IXCK(cudaMemsetAsync(ix.bits.active, 0, 4, st));  // set by the seed when a changed entry matters
-  k_ix_seed<<<1, 32, 0, st>>>(keys, 2, g, ix.d_dag, ix.bits);
-  (*launches)++;
-  return index_round_coop(ix, g, st, launches);
+  return index_round(ix, g, keys, L, kNone, st, launches);
 }
 
 int index_vertex_update(IndexState& ix, const DevGraph& g, const csm_update& h, cudaStream_t st, uint64_t* launches) {
   if (!ix.active) return CSM_OK;
   if (h.type != 'v' || h.id1 >= g.n_cap) return CSM_OK;  // a new or a removed vertex: re-evaluate its flags
-  IXCK(cudaMemsetAsync(ix.bits.active, 0, 4, st));
-  k_ix_seed_vertex<<<1, 32, 0, st>>>(h.id1, ix.d_dag, ix.bits);
-  (*launches)++;
-  return index_launch_round(ix, g, st, launches, false);
+  return index_round(ix, g, nullptr, 0, h.id1, st, launches);
 }
 
 int index_counts(IndexState& ix, cudaStream_t st, uint64_t* d1_count, uint64_t* d2_count) {
@@ -670,10 +638,10 @@ void index_stats(const IndexState& ix, uint64_t* entries, uint64_t* vertices) {
 }
 
 void index_free(IndexState& ix, DevMem& mem) {
-  if (ix.bits.d1) mem.release(ix.bits.d1, 6 * 8ull * ix.h_dag.nq * ix.words);
+  if (ix.bits.d1) mem.release(ix.bits.d1, 4 * 8ull * ix.h_dag.nq * ix.words);
   if (ix.d_dag) mem.release(ix.d_dag, sizeof(IxDag));
   if (ix.d_pop) mem.release(ix.d_pop, 16);
-  if (ix.bits.active) mem.release(ix.bits.active, 16);
+  if (ix.bits.list) mem.release(ix.bits.list, list_bytes(ix));
   ix.bits = IxBits{};
   ix.d_dag = nullptr;
   ix.d_pop = nullptr;

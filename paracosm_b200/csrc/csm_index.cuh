@@ -71,12 +71,16 @@ struct IxDag {
   uint8_t req_mult[kMaxQ][kMaxQ];
 };
 
-// Flag bitsets: [n_q][words] each.  m1 / m2 mark vertices to re-evaluate,
-// c1 / c2 record flags that changed in the current maintenance round.
+// Flag bitsets d1 / d2 and the marks m1 / m2 of vertices to re-evaluate:
+// [n_q][words] each.  A marked vertex is also on its query vertex's work list
+// (list [2][n_q][list_cap], lengths count [2][n_q], the d1 lists first) while
+// that has room; a list that overflowed is worked off from its marks.
 struct IxBits {
-  uint64_t *d1, *d2, *m1, *m2, *c1, *c2;
+  uint64_t *d1, *d2, *m1, *m2;
   uint64_t words;
-  unsigned int* active;  // nonzero when the current round marked anything; else its kernels return at once
+  uint32_t* list;
+  unsigned int* count;
+  uint32_t list_cap;
 };
 
 // Query vertices in DAG order, by value for a kernel argument.
@@ -87,7 +91,6 @@ struct IxOrder {
 
 struct IndexState {
   int algo = CSM_ALGO_GRAPHFLOW;
-  uint32_t coop_blocks = 0;  // grid of the single-launch round (0: not sized yet)
   bool active = false;
   uint64_t* d2 = nullptr;     // == bits.d2 (null: no index)
   uint64_t words = 0;
@@ -104,14 +107,10 @@ struct IndexState {
 int index_build(IndexState& ix, DevMem& mem, const DevGraph& g, const IndexQuery& q, int algo, int sm_count,
                 cudaStream_t st, uint64_t* launches);
 // Brings the flags to the CSR as it is now, after the directed entries in
-// keys[0, L) (packed (x, combo, y), sentinel-padded) changed.
+// keys[0, L) (packed (x, combo, y), sentinel-padded) changed: one cooperative
+// launch.
 int index_apply_edges(IndexState& ix, const DevGraph& g, const uint64_t* keys, uint32_t L, cudaStream_t st,
                       uint64_t* launches);
-// The same for the two directed entries keys[0..1] of one edge update, in two
-// launches: the marks, then every propagation and re-evaluation step in one
-// cooperative kernel.
-int index_apply_edge_one(IndexState& ix, const DevGraph& g, const uint64_t* keys, cudaStream_t st,
-                         uint64_t* launches);
 int index_vertex_update(IndexState& ix, const DevGraph& g, const csm_update& h, cudaStream_t st, uint64_t* launches);
 int index_counts(IndexState& ix, cudaStream_t st, uint64_t* d1_count, uint64_t* d2_count);
 void index_stats(const IndexState& ix, uint64_t* entries, uint64_t* vertices);

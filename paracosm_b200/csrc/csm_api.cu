@@ -412,13 +412,10 @@ static int batch_mutate_insert(csm_ctx* ctx, const csm_update* ups, uint32_t B, 
   g.t_span = reinterpret_cast<int2*>(ctx->d_ts2);
   // CSR -> union graph (relocating rows, and compacting the pools first if needed)
   k_reloc_need<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_rins, c + 3, g); CKL();
-  k_compact_check<<<1, 1, 0, st>>>(g); CKL();
-  k_compact_copy<<<ctx->sm_count * 4, 1024, 0, st>>>(g); CKL();
-  k_compact_finish<<<1, 1, 0, st>>>(g); CKL();
+  k_compact_copy<<<ctx->sm_count * 2, 1024, 0, st>>>(g); CKL();
   const uint32_t mut_blocks = std::min<uint32_t>(blocks_for(L * 32ull, 256), (uint32_t)ctx->sm_count * 16);
   launch_mut_insert(ctx->d_rins, c + 3, ctx->d_ins2, ctx->d_ins_dst, g, mut_blocks, (uint32_t)ctx->sm_count * 2, st);
   CKL();
-  ctx->launches++;
   g.t_mask = temporal_slots(B) - 1;
   CK(cudaMemsetAsync(g.t_tab, 0xff, sizeof(ulonglong2) * (size_t)(g.t_mask + 1), st));
   k_temporal_set<<<blocks_for(L, 256), 256, 0, st>>>(L, g); CKL();
@@ -569,7 +566,6 @@ static int run_edge_batch(csm_ctx* ctx, const csm_update* ups, uint32_t B, csm_r
   const uint32_t mut_blocks = std::min<uint32_t>(blocks_for(L * 32ull, 256), (uint32_t)ctx->sm_count * 16);
   launch_mut_delete(ctx->d_rdel, c + 4, ctx->d_del2, ctx->d_ins_dst, g, mut_blocks, (uint32_t)ctx->sm_count * 2, st);
   CKL();
-  ctx->launches++;
   for (csm_ctx* a : ctx->attached) {
     rc = stream_after(a->st, st, ctx->ev_fork);
     if (!rc) rc = index_apply_edges(a->index, g, ctx->d_del2, L, a->st, &a->launches);
@@ -632,22 +628,22 @@ static int run_plain_edge(csm_ctx* ctx, const csm_update* d_up, const csm_update
                                      ctx->d_stop);
   CKL();
   if (h.type == 'e' && h.is_add) {
-    k_compact_copy<<<ctx->sm_count * 4, 1024, 0, st>>>(g);  // returns at once unless the pool must be compacted
+    k_compact_copy<<<ctx->sm_count * 2, 1024, 0, st>>>(g);  // returns at once unless the pool must be compacted
     CKL();
   }
   int rc = CSM_OK;
   if (!plain_may_count(ctx, h)) {
-    k_plain_mutate<<<1, 256, 0, st>>>(g, ctx->d_info, keys, out, ctx->d_stamp, 16u);
+    k_plain_mutate<<<2, 256, 0, st>>>(g, ctx->d_info, keys, out, ctx->d_stamp, 16u);
     CKL();
   } else if (h.is_add) {
-    k_plain_mutate<<<1, 256, 0, st>>>(g, ctx->d_info, keys, nullptr, nullptr, 16u);
+    k_plain_mutate<<<2, 256, 0, st>>>(g, ctx->d_info, keys, nullptr, nullptr, 16u);
     CKL();
     rc = index_apply_edges(ctx->index, g, keys, 2, st, &ctx->launches);
     if (!rc) rc = query_seed_search(ctx, ctx, 1, out);
   } else {
     rc = query_seed_search(ctx, ctx, 1, out);
     if (rc) return rc;
-    k_plain_mutate<<<1, 256, 0, st>>>(g, ctx->d_info, keys, nullptr, nullptr, 16u);
+    k_plain_mutate<<<2, 256, 0, st>>>(g, ctx->d_info, keys, nullptr, nullptr, 16u);
     CKL();
     rc = index_apply_edges(ctx->index, g, keys, 2, st, &ctx->launches);
   }
@@ -694,7 +690,6 @@ static int run_vertex_delete(csm_ctx* ctx, uint32_t v) {
     launch_mut_delete(ranges, nr, keys2, reinterpret_cast<uint32_t*>(keys), g, mut_blocks, (uint32_t)ctx->sm_count * 2,
                       st);
     CKL();
-    ctx->launches++;
     for (csm_ctx* q : all) {
       if (q != ctx) { q->g = g; rc = stream_after(q->st, st, ctx->ev_fork); }
       if (!rc) rc = index_apply_edges(q->index, g, keys2, K, q->st, &q->launches);

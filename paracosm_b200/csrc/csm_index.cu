@@ -240,21 +240,23 @@ __device__ __forceinline__ void ix_items(const DevGraph& g, const uint32_t* pool
 
 // One incremental round in a single cooperative launch (every block resident),
 // for the changed directed entries keys[0, L) and, when it is not kNone, the
-// new or removed vertex `vert`.  The marks come first; then, query vertex by
-// query vertex in DAG order, the d1 flags on the work lists, and in reverse
-// order the d2 flags, each followed by a grid barrier.  An empty list costs
-// one load and no barrier: few of the 2 |V_Q| are not (the round of one edge
-// update took 2 |V_Q| + 52 barriers over whole bitsets before, 153 us for a
-// 13-vertex query on 2^19 vertices).  A list's length is read by every block
-// between the barrier after the last mark it can get and the one after its
-// own work, so all blocks take the same way.
+// new or removed vertex `vert`.  The marks come first; then, step by step of
+// the order, the flags on the work lists of the step's query vertices, d1
+// before d2, each step followed by a grid barrier.  Query vertices that do not
+// draw on one another's flags share a step, and a step of empty lists costs a
+// load each and no barrier.  What bounds a round is the number of barriers and
+// the chain of loads between two: for one edge update of a 13-vertex query on
+// 2^19 vertices 52 barriers over whole bitsets took 153 us, one barrier per
+// query vertex 29 us.  A list's length is read by every block between the
+// barrier after the last mark it can get and the one after its own work, so
+// all blocks take the same way.
 __global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __restrict__ dag, IxBits b, IxOrder ord,
                                                   const uint64_t* __restrict__ keys, uint32_t L, uint32_t vert) {
   cg::grid_group grid = cg::this_grid();
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
   const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
-  const uint32_t ne = dag->n_edges, nq = ord.nq;
+  const uint32_t ne = dag->n_edges, nq = dag->nq;
   const uint32_t* pool = g.pools[g.ps->active];
   if (L <= 64) {  // a thread per (entry, DAG edge)
     for (uint32_t i = tid; i < L * ne; i += nthreads) {
@@ -274,34 +276,46 @@ __global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __res
     ix_mark(b, nq, 2, tid, vert);
   }
   grid.sync();
-  for (uint32_t i = 0; i < 2 * nq; i++) {
-    const uint32_t phase = i < nq ? 1u : 2u;
-    const uint32_t u = ord.order[phase == 1 ? i : 2 * nq - 1 - i];
-    const uint32_t row = (phase == 1 ? 0u : nq) + u;
-    const uint32_t n = *(volatile unsigned int*)&b.count[row];
-    if (n == 0) continue;
-    if (n <= b.list_cap) {
-      // as many items per warp as it takes to share them out; with several,
-      // each lane first tries its own
-      const uint32_t* list = b.list + (size_t)row * b.list_cap;
-      const uint32_t per = min(32u, (n + nwarps - 1) / nwarps);
-      for (uint32_t base = warp * per; base < n; base += nwarps * per) {
-        const bool has = lane < per && base + lane < n;
-        ix_items(g, pool, dag, b, u, phase, has, has ? __ldcg(list + base + lane) : 0u, per > 4, lane);
-      }
-    } else {
-      const uint64_t* mark = (phase == 1 ? b.m1 : b.m2) + (uint64_t)u * b.words;
-      for (uint64_t wi = warp; wi < b.words; wi += nwarps) {
-        const uint64_t word = __ldcg(mark + wi);
-        if (!word) continue;
+  for (uint32_t phase = 1; phase <= 2; phase++) {
+    uint32_t beg = 0;
+    for (uint32_t step = 0; step < ord.steps[phase - 1]; step++) {
+      const uint32_t end = ord.end[phase - 1][step];
+      uint32_t used = 0;  // warps' shares given out in this step so far: the next list starts with the next warp
+      for (uint32_t i = beg; i < end; i++) {
+        const uint32_t u = ord.order[phase - 1][i];
+        const uint32_t row = (phase == 1 ? 0u : nq) + u;
+        const uint32_t n = *(volatile unsigned int*)&b.count[row];
+        if (n == 0) continue;
+        const uint32_t w0 = (warp + nwarps - used % nwarps) % nwarps;
+        if (n <= b.list_cap) {
+          // as many items per warp as it takes to share them out; with several,
+          // each lane first tries its own
+          const uint32_t* list = b.list + (size_t)row * b.list_cap;
+          const uint32_t per = min(32u, (n + nwarps - 1) / nwarps);
+          for (uint32_t base = w0 * per; base < n; base += nwarps * per) {
+            const bool has = lane < per && base + lane < n;
+            ix_items(g, pool, dag, b, u, phase, has, has ? __ldcg(list + base + lane) : 0u, per > 4, lane);
+          }
+          used += (n + per - 1) / per;
+        } else {
+          const uint64_t* mark = (phase == 1 ? b.m1 : b.m2) + (uint64_t)u * b.words;
+          for (uint64_t wi = w0; wi < b.words; wi += nwarps) {
+            const uint64_t word = __ldcg(mark + wi);
+            if (!word) continue;
 #pragma unroll 1
-        for (uint32_t half = 0; half < 2; half++)
-          ix_items(g, pool, dag, b, u, phase, (word >> (32u * half + lane)) & 1ULL, (uint32_t)(wi * 64 + 32u * half + lane),
-                   true, lane);
+            for (uint32_t half = 0; half < 2; half++)
+              ix_items(g, pool, dag, b, u, phase, (word >> (32u * half + lane)) & 1ULL,
+                       (uint32_t)(wi * 64 + 32u * half + lane), true, lane);
+          }
+          used += nwarps;
+        }
       }
+      if (used) {
+        grid.sync();
+        if (tid >= beg && tid < end) b.count[(phase == 1 ? 0u : nq) + ord.order[phase - 1][tid]] = 0;
+      }
+      beg = end;
     }
-    grid.sync();
-    if (tid == 0) b.count[row] = 0;
   }
 }
 
@@ -515,6 +529,23 @@ static int index_finish(IndexState& ix, DevMem& mem, const DevGraph& g, const In
   }
   ix.root = root;
   ix.order = order;
+  // steps of a round: by longest path from a vertex without parents (d1) and
+  // from one without children (d2); the lighting levels draw on no other
+  // vertex's flag of the same level
+  for (uint32_t f = 0; f < 2; f++) {
+    uint32_t level[kMaxQ] = {}, deepest = 0, k = 0;
+    for (uint32_t i = 0; i < nq && !D.lighting; i++) {
+      const uint32_t u = order[f == 0 ? i : nq - 1 - i];
+      for (uint32_t w : f == 0 ? par[u] : chd[u]) level[u] = std::max(level[u], level[w] + 1);
+      deepest = std::max(deepest, level[u]);
+    }
+    ix.rounds.steps[f] = deepest + 1;
+    for (uint32_t l = 0; l <= deepest; l++) {
+      for (uint32_t u = 0; u < nq; u++)
+        if (level[u] == l) ix.rounds.order[f][k++] = (uint8_t)u;
+      ix.rounds.end[f][l] = (uint8_t)k;
+    }
+  }
 
   // flag bitsets, 32-byte aligned rows
   ix.words = ((uint64_t)g.n_cap + 63) / 64;
@@ -592,9 +623,7 @@ int index_build(IndexState& ix, DevMem& mem, const DevGraph& g, const IndexQuery
 // The incremental round (k_ix_round): one block per SM.
 static int index_round(IndexState& ix, const DevGraph& g, const uint64_t* keys, uint32_t L, uint32_t vert,
                        cudaStream_t st, uint64_t* launches) {
-  IxOrder ord{};
-  ord.nq = ix.h_dag.nq;
-  for (uint32_t i = 0; i < ord.nq; i++) ord.order[i] = ix.order[i];
+  IxOrder ord = ix.rounds;
   DevGraph gv = g;
   const IxDag* dag = ix.d_dag;
   IxBits bits = ix.bits;

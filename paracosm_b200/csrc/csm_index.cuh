@@ -83,10 +83,14 @@ struct IxBits {
   uint32_t list_cap;
 };
 
-// Query vertices in DAG order, by value for a kernel argument.
+// Query vertices in the steps of a round, by value for a kernel argument:
+// phase f (0: d1, 1: d2) takes order[f][0 .. end[f][0]) together, then up to
+// end[f][1], and so on; a vertex comes in a later step than those whose flags
+// its own flag of that phase draws on.
 struct IxOrder {
-  uint32_t nq;
-  uint32_t order[kMaxQ];
+  uint32_t steps[2];
+  uint8_t order[2][kMaxQ];
+  uint8_t end[2][kMaxQ];
 };
 
 struct IndexState {
@@ -100,6 +104,7 @@ struct IndexState {
   uint64_t* d_pop = nullptr;  // popcount scratch
   uint32_t root = 0;
   std::vector<uint32_t> order;
+  IxOrder rounds{};
   int sm_count = 148;
   uint64_t entries = 0, vertices = 0;
 };

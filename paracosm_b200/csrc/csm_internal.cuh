@@ -68,7 +68,7 @@ struct PoolState {
   uint32_t active;            // index of the active pool
   uint32_t compact;           // set when this batch must compact first
   uint32_t error;             // nonzero: internal error code (see kErr*)
-  uint32_t pad;
+  uint32_t arrived;           // blocks of a kernel that have arrived (last_block)
 };
 enum : uint32_t { kErrNone = 0, kErrPoolFull = 1, kErrListOverflow = 2, kErrTaskOverflow = 3, kErrWaitTimeout = 4,
                   kErrBadTask = 5, kErrRingState = 6, kErrTaskGuard = 7, kErrRowState = 8, kErrEdgeTable = 9 };

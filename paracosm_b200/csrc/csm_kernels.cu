@@ -349,7 +349,24 @@ __global__ void k_temporal_clear(uint32_t L, DevGraph g) {
   if (j == 0 || g.kb.x_of(g.t_key[j - 1]) != x) g.t_count[x] = 0;
 }
 
+// True in every thread of the block that arrives last; *ctr is 0 before and after.
+__device__ __forceinline__ bool last_block(unsigned int* ctr) {
+  __shared__ bool last;
+  __syncthreads();
+  if (threadIdx.x == 0) {
+    __threadfence();
+    last = atomicAdd(ctr, 1u) + 1u == gridDim.x;
+    if (last) *ctr = 0;
+    __threadfence();
+  }
+  __syncthreads();
+  return last;
+}
+
+// Pool space that the batch's growing rows will take; the last block decides
+// whether the pools are compacted first.
 __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges, DevGraph g) {
+  PoolState* ps = g.ps;
   uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
   unsigned long long need = 0;
   if (i < *n_ranges) {
@@ -359,13 +376,11 @@ __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges,
   }
   // warp-aggregated add
   for (int o = 16; o; o >>= 1) need += __shfl_down_sync(0xffffffffu, need, o);
-  if ((threadIdx.x & 31) == 0 && need) atomicAdd(&g.ps->need, need);
-}
-
-__global__ void k_compact_check(DevGraph g) {
-  PoolState* ps = g.ps;
-  const unsigned long long free_slots = g.pool_cap - ps->top[ps->active];
-  ps->compact = (ps->need > free_slots) ? 1u : 0u;
+  if ((threadIdx.x & 31) == 0 && need) atomicAdd(&ps->need, need);
+  if (last_block(&ps->arrived) && threadIdx.x == 0) {
+    const unsigned long long all = atomicExch(&ps->need, 0ULL);
+    ps->compact = all > g.pool_cap - ps->top[ps->active] ? 1u : 0u;
+  }
 }
 
 // Combo of the row-relative entry index i: upper_bound(dir, i) - 1.
@@ -447,16 +462,11 @@ __global__ void k_compact_copy(DevGraph g) {
     }
     __syncthreads();
   }
-}
-
-__global__ void k_compact_finish(DevGraph g) {
-  PoolState* ps = g.ps;
-  if (ps->compact) {
-    ps->top[ps->active] = 0;
-    ps->active = 1u - ps->active;
+  if (last_block(&ps->arrived) && threadIdx.x == 0) {  // every row has moved
+    ps->top[src] = 0;
+    ps->active = dst;
     ps->compact = 0;
   }
-  ps->need = 0;
 }
 
 __device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t* a, uint32_t lo, uint32_t hi, uint64_t x) {
@@ -467,58 +477,108 @@ __device__ __forceinline__ uint32_t lower_bound_u64(const uint64_t* a, uint32_t 
   return lo;
 }
 
-// Group copies of n pool entries by G threads (a warp or a block).  Each
-// round reads G entries into registers before any thread writes, so a move
-// that overlaps its source is safe when left moves run front to back and
-// right moves back to front.
+// Number of the k ascending positions in pos that are at most (below) i.
+__device__ __forceinline__ uint32_t count_le(const uint32_t* pos, uint32_t k, uint32_t i) {
+  uint32_t lo = 0, hi = k;
+#pragma unroll 1
+  while (lo < hi) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (pos[mid] <= i) lo = mid + 1; else hi = mid;
+  }
+  return lo;
+}
+
+// Row moves by G threads (a warp or a block), eight entries a thread and round:
+// a round's entries are all in registers before any is stored, so a move
+// within a row is safe when rounds go from the back for a move to the right and
+// from the front for a move to the left.  An entry's place follows from its
+// rank among the k changed positions, whatever k is: moving the blocks between
+// changed positions one after another cost two barriers per change (a batch
+// of 65,536 updates changes hub rows in hundreds of places: 508 us inserting
+// and 549 us deleting on the 2^22-vertex graph, against 105 and 83 us).
+constexpr uint32_t kMoveUnroll = 8;
+
+// Entries [from, deg) of the row at src go to dst + i + (changed positions <= i).
 template <int G>
-__device__ __forceinline__ void group_move_left(uint32_t* pool, uint64_t src, uint64_t dst, uint32_t n,
-                                                uint32_t lane) {
-  for (uint32_t b = 0; b < n; b += G) {
-    const uint32_t i = b + lane;
-    uint32_t v = 0;
-    if (i < n) v = pool[src + i];
+__device__ __forceinline__ void group_insert_move(uint32_t* pool, uint64_t src, uint64_t dst, uint32_t from,
+                                                  uint32_t deg, const uint32_t* pos, uint32_t k, uint32_t lane) {
+  for (uint32_t end = deg; end > from;) {
+    const uint32_t beg = end - from > G * kMoveUnroll ? end - G * kMoveUnroll : from;
+    uint32_t val[kMoveUnroll];
+#pragma unroll
+    for (uint32_t u = 0; u < kMoveUnroll; u++) {
+      const uint32_t i = beg + u * G + lane;
+      if (i < end) val[u] = pool[src + i];
+    }
     group_sync<G>();
-    if (i < n) pool[dst + i] = v;
+#pragma unroll
+    for (uint32_t u = 0; u < kMoveUnroll; u++) {
+      const uint32_t i = beg + u * G + lane;
+      if (i < end) pool[dst + i + count_le(pos, k, i)] = val[u];
+    }
     group_sync<G>();
+    end = beg;
   }
 }
+
+// Entries (pos[0], deg) but those at the changed positions move left by the
+// number of changed positions before them.
 template <int G>
-__device__ __forceinline__ void group_move_right(uint32_t* pool, uint64_t src, uint64_t dst, uint32_t n,
-                                                 uint32_t lane) {
-  for (uint32_t b = n; b > 0;) {
-    const uint32_t cnt = min((uint32_t)G, b);
-    b -= cnt;
-    uint32_t v = 0;
-    if (lane < cnt) v = pool[src + b + lane];
+__device__ __forceinline__ void group_delete_move(uint32_t* pool, uint64_t off, uint32_t deg, const uint32_t* pos,
+                                                  uint32_t k, uint32_t lane) {
+  for (uint32_t beg = pos[0]; beg < deg; beg += G * kMoveUnroll) {
+    uint32_t val[kMoveUnroll];
+#pragma unroll
+    for (uint32_t u = 0; u < kMoveUnroll; u++) {
+      const uint32_t i = beg + u * G + lane;
+      if (i < deg) val[u] = pool[off + i];
+    }
     group_sync<G>();
-    if (lane < cnt) pool[dst + b + lane] = v;
+#pragma unroll
+    for (uint32_t u = 0; u < kMoveUnroll; u++) {
+      const uint32_t i = beg + u * G + lane;
+      if (i >= deg) continue;
+      const uint32_t le = count_le(pos, k, i);
+      if (pos[le - 1] != i) pool[off + i - le] = val[u];  // le >= 1: i is not before the first
+    }
     group_sync<G>();
   }
 }
 
+// lower_bound of x in the sorted range a[lo, hi) by a warp: 32 probes a round.
+__device__ __forceinline__ uint32_t warp_lower_bound(const uint32_t* a, uint32_t lo, uint32_t hi, uint32_t x,
+                                                     uint32_t lane) {
+  while (hi - lo > 32) {
+    const uint32_t step = (hi - lo + 31) / 32;
+    const uint32_t at = lo + lane * step;
+    const uint32_t less = __popc(__ballot_sync(0xffffffffu, at < hi && a[at] < x));
+    if (less == 0) return lo;
+    const uint32_t last = lo + (less - 1) * step;  // the last probe below x
+    hi = min(hi, last + step);
+    lo = last + 1;
+  }
+  return lo + __popc(__ballot_sync(0xffffffffu, lo + lane < hi && a[lo + lane] < x));
+}
+
 // Merges each vertex's sorted insert list into its row; G = 32: one warp per
 // row of at most kBigRow entries, G = blockDim: one block per longer row.
-// Insert j (sorted by combo, then id) goes to row position p_j (its
-// lower_bound in the old row); old entries in [p_j, p_{j+1}) then shift by
-// j + 1, so the row moves as k + 1 contiguous blocks -- in place (last block
-// first, back to front) or into a larger row elsewhere.
+// Insert j (sorted by combo, then id) goes to row position p_j + j, p_j being
+// its lower_bound in the old row; an old entry i shifts by the inserts with
+// p_j <= i -- in place, or into a larger row elsewhere.
 template <int G>
-__global__ void k_mut_insert_g(const VRange* ranges, const unsigned int* n_ranges, const uint64_t* ins_key,
-                               uint32_t* ins_dst, DevGraph g) {
+__device__ __forceinline__ void mut_insert(const VRange* ranges, uint32_t nr, const uint64_t* ins_key,
+                                           uint32_t* ins_dst, const DevGraph& g, unsigned long long* s_off,
+                                           uint32_t block, uint32_t blocks) {
   const uint32_t lane = threadIdx.x % G;
   const uint32_t groups_per_block = blockDim.x / G;
-  const uint32_t nr = *n_ranges;
   PoolState* ps = g.ps;
   uint32_t* pool = g.pools[ps->active];
-  __shared__ unsigned long long s_off[8];
-  for (uint32_t w = blockIdx.x * groups_per_block + threadIdx.x / G; w - threadIdx.x / G < nr;
-       w += gridDim.x * groups_per_block) {
+  for (uint32_t w = block * groups_per_block + threadIdx.x / G; w - threadIdx.x / G < nr;
+       w += blocks * groups_per_block) {
     // every thread of a block-sized group walks the same w; warps of a
     // warp-sized group skip ranges of the other kind
     const bool mine = w < nr && ranges[w].pad == (G == 32 ? 0u : 1u);
-    if (G == 32 && !mine) continue;
-    if (G != 32 && !mine) { __syncthreads(); continue; }
+    if (!mine) continue;
     const VRange r = ranges[w];
     const uint32_t x = r.x, s = r.start, k = r.count;
     uint32_t* dirx = g.dir + (size_t)x * (g.nc + 1);
@@ -526,6 +586,7 @@ __global__ void k_mut_insert_g(const VRange* ranges, const unsigned int* n_range
     const uint2 old = g.row[x];
     const uint64_t off = old.x;
     const uint32_t new_deg = deg + k;
+    const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread before a build clears it
     uint64_t dst_off = off;
     uint32_t new_cap = 0;
     if (new_deg > old.y) {
@@ -547,20 +608,8 @@ __global__ void k_mut_insert_g(const VRange* ranges, const unsigned int* n_range
       ins_dst[s + j] = (uint32_t)lower_bound_u32(pool + off, dirx[c], dirx[c + 1], y);
     }
     group_sync<G>();
-    // 2. old entries, block by block
-    if (dst_off == off) {
-      for (int64_t j = (int64_t)k - 1; j >= 0; j--) {
-        const uint32_t a = ins_dst[s + j], b = (j + 1 < (int64_t)k) ? ins_dst[s + j + 1] : deg;
-        if (b > a) group_move_right<G>(pool, off + a, off + a + (uint64_t)j + 1, b - a, lane);
-      }
-    } else {
-      group_move_left<G>(pool, off, dst_off, ins_dst[s], lane);  // different rows: no overlap
-      for (uint32_t j = 0; j < k; j++) {
-        const uint32_t a = ins_dst[s + j], b = (j + 1 < k) ? ins_dst[s + j + 1] : deg;
-        if (b > a) group_move_left<G>(pool, off + a, dst_off + a + j + 1, b - a, lane);
-      }
-    }
-    // 3. inserted entries
+    // 2. old entries, 3. inserted ones
+    group_insert_move<G>(pool, off, dst_off, dst_off == off ? ins_dst[s] : 0u, deg, ins_dst + s, k, lane);
     for (uint32_t j = lane; j < k; j += G) pool[dst_off + ins_dst[s + j] + j] = g.kb.y_of(ins_key[s + j]);
     group_sync<G>();
     // 4. directory: a combo's segment starts after the inserts of smaller combos
@@ -570,7 +619,6 @@ __global__ void k_mut_insert_g(const VRange* ranges, const unsigned int* n_range
     }
     const uint2 now = new_cap ? make_uint2((uint32_t)dst_off, new_cap) : old;
     if (lane == 0 && new_cap) g.row[x] = now;
-    const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread before the build below clears it
     group_sync<G>();
     // 5. row table: the new entries, or the whole table when the row moved or
     // deleted slots would fill it past three quarters
@@ -589,70 +637,83 @@ __global__ void k_mut_insert_g(const VRange* ranges, const unsigned int* n_range
 }
 
 // Removes each vertex's sorted delete list from its row in place (G as
-// above).  Delete j sits at row position q_j; the old entries between q_j and
-// q_{j+1} move left by j + 1, blocks front to back.  `del_pos` is scratch of
-// the delete list's length.
+// above).  Delete j sits at row position q_j; an old entry moves left by the
+// deletes before it.  `del_pos` is scratch of the delete list's length.
 template <int G>
-__global__ void k_mut_delete_g(const VRange* ranges, const unsigned int* n_ranges, const uint64_t* del_key,
-                               uint32_t* del_pos, DevGraph g) {
+__device__ __forceinline__ void mut_delete(const VRange* ranges, uint32_t nr, const uint64_t* del_key,
+                                           uint32_t* del_pos, const DevGraph& g, uint32_t block, uint32_t blocks) {
   const uint32_t lane = threadIdx.x % G;
   const uint32_t groups_per_block = blockDim.x / G;
-  const uint32_t nr = *n_ranges;
   uint32_t* pool = g.pools[g.ps->active];
-  for (uint32_t w = blockIdx.x * groups_per_block + threadIdx.x / G; w - threadIdx.x / G < nr;
-       w += gridDim.x * groups_per_block) {
+  for (uint32_t w = block * groups_per_block + threadIdx.x / G; w - threadIdx.x / G < nr;
+       w += blocks * groups_per_block) {
     const bool mine = w < nr && ranges[w].pad == (G == 32 ? 0u : 1u);
-    if (G == 32 && !mine) continue;
-    if (G != 32 && !mine) { __syncthreads(); continue; }
+    if (!mine) continue;
     const VRange r = ranges[w];
     const uint32_t x = r.x, s = r.start, k = r.count;
     uint32_t* dirx = g.dir + (size_t)x * (g.nc + 1);
     const uint32_t deg = dirx[g.nc];
     const uint2 row = g.row[x];
     const uint64_t off = row.x;
+    bool missing = false;
     for (uint32_t j = lane; j < k; j += G) {
       const uint64_t key = del_key[s + j];
       const uint32_t c = g.kb.c_of(key), y = g.kb.y_of(key);
-      del_pos[s + j] = (uint32_t)lower_bound_u32(pool + off, dirx[c], dirx[c + 1], y);
-      if (g.htab) row_table_delete(g, x, row, row_entry(y, c % g.n_el, g.hlb));
+      const uint32_t q = (uint32_t)lower_bound_u32(pool + off, dirx[c], dirx[c + 1], y);
+      del_pos[s + j] = q;
+      if (q >= dirx[c + 1] || pool[off + q] != y) missing = true;
+      else if (g.htab) row_table_delete(g, x, row, row_entry(y, c % g.n_el, g.hlb));
     }
-    group_sync<G>();
+    // a deleted entry missing from its row: leave the row, report
+    if (G == 32) { __syncwarp(); missing = __any_sync(0xffffffffu, missing); }
+    else missing = __syncthreads_or(missing);
+    if (missing) {
+      if (lane == 0) atomicExch(&g.ps->error, kErrRowState);
+      continue;
+    }
     const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread well before a build clears it
-    bool whole = true;
-    for (uint32_t j = 0; j < k; j++) {
-      const uint32_t a = del_pos[s + j] + 1, b = (j + 1 < k) ? del_pos[s + j + 1] : deg;
-      if (a < j + 1 || a > deg) {  // a deleted entry missing from its row: leave the row, report
-        if (lane == 0) atomicExch(&g.ps->error, kErrRowState);
-        whole = false;
-        break;
-      }
-      if (b > a) group_move_left<G>(pool, off + a, off + a - (j + 1), b - a, lane);
-    }
+    group_delete_move<G>(pool, off, deg, del_pos + s, k, lane);
     for (uint32_t c = lane; c <= g.nc; c += G) {
       const uint32_t sub = lower_bound_u64(del_key, s, s + k, g.kb.pack(x, 0, 0) + ((uint64_t)c << g.kb.yb)) - s;
       dirx[c] -= sub;
     }
     group_sync<G>();
-    if (whole && tomb > tomb_limit(row.y)) {
+    if (tomb > tomb_limit(row.y)) {
       row_table_build<G>(g, pool, x, row, dirx, deg - k, lane);
       group_sync<G>();
     }
   }
 }
 
-// Both row kinds of a batch: rows up to kBigRow entries by warps, longer rows
-// by 256-thread blocks.
+// Both row kinds in one launch: the first warp_blocks blocks take the rows of
+// up to kBigRow entries warp by warp, the others the longer rows.
+__global__ void __launch_bounds__(256) k_mut_insert(const VRange* ranges, const unsigned int* n_ranges,
+                                                    const uint64_t* ins_key, uint32_t* ins_dst, DevGraph g,
+                                                    uint32_t warp_blocks) {
+  __shared__ unsigned long long s_off[8];
+  if (blockIdx.x < warp_blocks)
+    mut_insert<32>(ranges, *n_ranges, ins_key, ins_dst, g, s_off, blockIdx.x, warp_blocks);
+  else
+    mut_insert<256>(ranges, *n_ranges, ins_key, ins_dst, g, s_off, blockIdx.x - warp_blocks, gridDim.x - warp_blocks);
+}
+__global__ void __launch_bounds__(256) k_mut_delete(const VRange* ranges, const unsigned int* n_ranges,
+                                                    const uint64_t* del_key, uint32_t* del_pos, DevGraph g,
+                                                    uint32_t warp_blocks) {
+  if (blockIdx.x < warp_blocks)
+    mut_delete<32>(ranges, *n_ranges, del_key, del_pos, g, blockIdx.x, warp_blocks);
+  else
+    mut_delete<256>(ranges, *n_ranges, del_key, del_pos, g, blockIdx.x - warp_blocks, gridDim.x - warp_blocks);
+}
+
 void launch_mut_insert(const VRange* ranges, const unsigned int* n_ranges, const uint64_t* ins_key,
                        uint32_t* ins_dst, const DevGraph& g, uint32_t warp_blocks, uint32_t big_blocks,
                        cudaStream_t st) {
-  k_mut_insert_g<32><<<warp_blocks, 256, 0, st>>>(ranges, n_ranges, ins_key, ins_dst, g);
-  k_mut_insert_g<256><<<big_blocks, 256, 0, st>>>(ranges, n_ranges, ins_key, ins_dst, g);
+  k_mut_insert<<<warp_blocks + big_blocks, 256, 0, st>>>(ranges, n_ranges, ins_key, ins_dst, g, warp_blocks);
 }
 void launch_mut_delete(const VRange* ranges, const unsigned int* n_ranges, const uint64_t* del_key,
                        uint32_t* del_pos, const DevGraph& g, uint32_t warp_blocks, uint32_t big_blocks,
                        cudaStream_t st) {
-  k_mut_delete_g<32><<<warp_blocks, 256, 0, st>>>(ranges, n_ranges, del_key, del_pos, g);
-  k_mut_delete_g<256><<<big_blocks, 256, 0, st>>>(ranges, n_ranges, del_key, del_pos, g);
+  k_mut_delete<<<warp_blocks + big_blocks, 256, 0, st>>>(ranges, n_ranges, del_key, del_pos, g, warp_blocks);
 }
 
 // ------------------------------------------------- one update per launch
@@ -664,141 +725,135 @@ void launch_mut_delete(const VRange* ranges, const unsigned int* n_ranges, const
 // preparation is one kernel and its row mutation another (plus the
 // compaction copy when an insertion's relocation does not fit).
 
+// One warp: the labels an edge may have are looked up side by side (one thread
+// trying them in turn took 5.4 us).
 __global__ void k_plain_resolve(const csm_update* up, DevGraph g, UpdInfo* info, uint64_t* keys, unsigned int* cnt,
                                 unsigned long long* count, unsigned long long* hash, unsigned long long* bytes,
                                 unsigned int* stop) {
-  if (blockIdx.x != 0 || threadIdx.x != 0) return;
+  const uint32_t lane = threadIdx.x;
   const csm_update u = *up;
-  UpdInfo inf;
-  inf.v1 = u.id1; inf.v2 = u.id2; inf.label = fold_elabel(g, u.label); inf.flags = 0;
-  keys[0] = ~0ULL; keys[1] = ~0ULL;
-  for (int i = 0; i < 16; i++) cnt[i] = 0;
-  count[0] = 0; hash[0] = 0; bytes[0] = 0; stop[0] = 0;
   PoolState* ps = g.ps;
-  ps->need = 0;
-  ps->compact = 0;
-  if (u.type == 'e') {
-    const bool ok = u.id1 < g.n && u.id2 < g.n && u.id1 != u.id2 && g.vlabel[u.id1] != kNone &&
-                    g.vlabel[u.id2] != kNone;
-    if (!ok) {
-      inf.flags = UF_INVALID;
-    } else {
-      inf.flags = UF_VALID | (u.is_add ? UF_ADD : 0u);
-      const uint32_t l0 = find_label(g, g.pools[ps->active], u.id1, u.id2);
-      const uint32_t x = min(u.id1, u.id2), y = max(u.id1, u.id2);
-      if (u.is_add) {
-        if (l0 != kNone) {
-          inf.flags |= UF_DUP;  // graph unchanged; counted with the given label
+  const bool ids = u.type == 'e' && u.id1 < g.n && u.id2 < g.n && u.id1 != u.id2;
+  const uint32_t x = min(u.id1, u.id2), y = max(u.id1, u.id2);
+  uint32_t lx = kNone, ly = kNone;
+  if (ids) { lx = g.vlabel[x]; ly = g.vlabel[y]; }
+  const bool ok = ids && lx != kNone && ly != kNone;
+  if (lane < 16) cnt[lane] = 0;
+  uint32_t l0 = kNone;
+  if (ok) {
+    const uint2 rx = g.row[x];
+    const uint32_t* pool = g.pools[ps->active];
+    for (uint32_t base = 0; base < g.n_el; base += 32) {
+      const uint32_t l = base + lane;
+      bool found = false;
+      if (l < g.n_el) {
+        if (g.htab) {
+          found = row_find(g, rx, row_entry(y, l, g.hlb)) != kSlotEmpty;
         } else {
-          inf.flags |= UF_MUT;
-          keys[0] = g.kb.pack(x, g.vlabel[y] * g.n_el + inf.label, y);
-          keys[1] = g.kb.pack(y, g.vlabel[x] * g.n_el + inf.label, x);
-          unsigned long long need = 0;
-          const uint32_t ends[2] = {x, y};
-          for (int k = 0; k < 2; k++) {
-            const uint32_t v = ends[k];
-            const uint32_t deg = g.dir[(size_t)v * (g.nc + 1) + g.nc];
-            if (deg + 1 > g.row[v].y) need += grow_cap(deg + 1);
-          }
-          ps->need = need;
-          ps->compact = (need > g.pool_cap - ps->top[ps->active]) ? 1u : 0u;
+          uint64_t lo, hi;
+          segment(g, x, ly * g.n_el + l, lo, hi);
+          found = contains_u32(pool, lo, hi, y);
         }
-      } else if (l0 == kNone) {
-        inf.flags |= UF_INVALID;  // deleting a missing edge
-      } else {
-        inf.label = l0;  // a deletion counts with the edge's own label
-        inf.flags |= UF_MUT;
-        keys[0] = g.kb.pack(x, g.vlabel[y] * g.n_el + l0, y);
-        keys[1] = g.kb.pack(y, g.vlabel[x] * g.n_el + l0, x);
       }
+      const uint32_t hit = __ballot_sync(0xffffffffu, found);
+      if (hit) { l0 = base + (uint32_t)__ffs((int)hit) - 1u; break; }
     }
   }
-  info[0] = inf;
+  UpdInfo inf;
+  inf.v1 = u.id1; inf.v2 = u.id2; inf.label = fold_elabel(g, u.label); inf.flags = 0;
+  if (u.type == 'e') {
+    if (!ok) inf.flags = UF_INVALID;
+    else if (u.is_add)  // an edge that is there: graph unchanged, counted with the given label
+      inf.flags = UF_VALID | UF_ADD | (l0 != kNone ? UF_DUP : UF_MUT);
+    else if (l0 == kNone)
+      inf.flags = UF_VALID | UF_INVALID;  // deleting a missing edge
+    else {
+      inf.label = l0;  // a deletion counts with the edge's own label
+      inf.flags = UF_VALID | UF_MUT;
+    }
+  }
+  unsigned long long need = 0;
+  if (lane < 2 && (inf.flags & UF_MUT) && u.is_add) {
+    const uint32_t v = lane ? y : x;
+    const uint32_t deg = g.dir[(size_t)v * (g.nc + 1) + g.nc];
+    if (deg + 1 > g.row[v].y) need = grow_cap(deg + 1);
+  }
+  need += __shfl_xor_sync(0xffffffffu, need, 1);
+  if (lane == 0) {
+    const bool mut = (inf.flags & UF_MUT) != 0;
+    keys[0] = mut ? g.kb.pack(x, ly * g.n_el + inf.label, y) : ~0ULL;
+    keys[1] = mut ? g.kb.pack(y, lx * g.n_el + inf.label, x) : ~0ULL;
+    count[0] = 0; hash[0] = 0; bytes[0] = 0; stop[0] = 0;
+    ps->compact = need > g.pool_cap - ps->top[ps->active] ? 1u : 0u;
+    info[0] = inf;
+  }
 }
 
+// One block per row (the two ends of the edge).
 __global__ void __launch_bounds__(256) k_plain_mutate(DevGraph g, const UpdInfo* info, const uint64_t* keys,
                                                       csm_result* out, const unsigned long long* stamp,
                                                       uint32_t mut_bytes) {
   PoolState* ps = g.ps;
   const uint32_t lane = threadIdx.x;
   __shared__ unsigned long long s_off;
-  __shared__ uint32_t s_pos, s_bad;
-  if (lane == 0) {
-    if (ps->compact) {  // k_compact_copy moved every row to the other pool (k_compact_finish's step)
-      ps->top[ps->active] = 0;
-      ps->active = 1u - ps->active;
-      ps->compact = 0;
-    }
-    ps->need = 0;
-  }
-  __syncthreads();
+  __shared__ uint32_t s_pos;
   const UpdInfo inf = info[0];
-  uint32_t* pool = g.pools[ps->active];
   if (inf.flags & UF_MUT) {
+    uint32_t* pool = g.pools[ps->active];
+    const uint64_t key = keys[blockIdx.x];
+    const uint32_t x = g.kb.x_of(key), c = g.kb.c_of(key), y = g.kb.y_of(key);
+    uint32_t* dirx = g.dir + (size_t)x * (g.nc + 1);
+    const uint32_t deg = dirx[g.nc];
+    const uint2 old = g.row[x];
+    const uint64_t off = old.x;
+    const uint32_t entry = row_entry(y, c % g.n_el, g.hlb);
+    const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread before a build clears it
     const bool add = (inf.flags & UF_ADD) != 0;
-    for (int k = 0; k < 2; k++) {
-      const uint64_t key = keys[k];
-      const uint32_t x = g.kb.x_of(key), c = g.kb.c_of(key), y = g.kb.y_of(key);
-      uint32_t* dirx = g.dir + (size_t)x * (g.nc + 1);
-      const uint32_t deg = dirx[g.nc];
-      const uint2 old = g.row[x];
-      const uint64_t off = old.x;
-      const uint32_t entry = row_entry(y, c % g.n_el, g.hlb);
+    uint32_t new_cap = 0;
+    if (lane < 32) {
+      const uint32_t end = dirx[c + 1];
+      const uint32_t p = warp_lower_bound(pool + off, dirx[c], end, y, lane);
+      if (lane == 0) s_pos = !add && (p >= end || pool[off + p] != y) ? kNone : p;  // a deleted entry must be there
+    }
+    if (add && deg + 1 > old.y) {
+      new_cap = grow_cap(deg + 1);
       if (lane == 0) {
-        s_pos = (uint32_t)lower_bound_u32(pool + off, dirx[c], dirx[c + 1], y);
-        s_bad = 0;
-        if (!add && (s_pos >= dirx[c + 1] || pool[off + s_pos] != y)) s_bad = 1;  // the entry must be there
+        unsigned long long o = atomicAdd(&ps->top[ps->active], (unsigned long long)new_cap);
+        if (o + new_cap > g.pool_cap) { atomicExch(&ps->error, kErrPoolFull); o = ~0ULL; }
+        s_off = o;
       }
+    }
+    __syncthreads();
+    const uint32_t p = s_pos;
+    const uint64_t dst = new_cap ? s_off : off;
+    if (p == kNone) {
+      if (lane == 0) atomicExch(&ps->error, kErrRowState);
+    } else if (add && dst != ~0ULL) {
+      const uint2 now = new_cap ? make_uint2((uint32_t)dst, new_cap) : old;
+      group_insert_move<256>(pool, off, dst, new_cap ? 0u : p, deg, &s_pos, 1, lane);
+      if (lane == 0) pool[dst + p] = y;
+      for (uint32_t cc = c + 1 + lane; cc <= g.nc; cc += 256) dirx[cc] += 1;
+      if (lane == 0 && new_cap) g.row[x] = now;
       __syncthreads();
-      const uint32_t p = s_pos;
-      if (s_bad) {
-        if (lane == 0) atomicExch(&ps->error, kErrRowState);
-        break;
+      if (g.htab) {  // the row table follows, as in mut_insert
+        if (new_cap || deg + 1 + tomb > now.y + now.y / 2)
+          row_table_build<256>(g, pool, x, now, dirx, deg + 1, lane);
+        else if (lane == 0)
+          row_table_insert(g, now, entry);
       }
-      if (add) {
-        uint64_t dst = off;
-        uint32_t new_cap = 0;
-        if (deg + 1 > old.y) {
-          new_cap = grow_cap(deg + 1);
-          if (lane == 0) {
-            unsigned long long o = atomicAdd(&ps->top[ps->active], (unsigned long long)new_cap);
-            if (o + new_cap > g.pool_cap) { atomicExch(&ps->error, kErrPoolFull); o = ~0ULL; }
-            s_off = o;
-          }
-          __syncthreads();
-          dst = s_off;
-          if (dst == ~0ULL) break;  // the same value in every thread
-          group_move_left<256>(pool, off, dst, p, lane);                 // different rows: no overlap
-          group_move_left<256>(pool, off + p, dst + p + 1, deg - p, lane);
-        } else {
-          group_move_right<256>(pool, off + p, off + p + 1, deg - p, lane);
-        }
-        if (lane == 0) pool[dst + p] = y;
-        for (uint32_t cc = c + 1 + lane; cc <= g.nc; cc += 256) dirx[cc] += 1;
-        const uint2 now = new_cap ? make_uint2((uint32_t)dst, new_cap) : old;
-        if (lane == 0 && new_cap) g.row[x] = now;
-        const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread before the build below clears it
-        __syncthreads();
-        if (g.htab) {  // the row table follows, as in k_mut_insert_g
-          if (new_cap || deg + 1 + tomb > now.y + now.y / 2)
-            row_table_build<256>(g, pool, x, now, dirx, deg + 1, lane);
-          else if (lane == 0)
-            row_table_insert(g, now, entry);
-        }
-      } else {
-        group_move_left<256>(pool, off + p + 1, off + p, deg - p - 1, lane);
-        for (uint32_t cc = c + 1 + lane; cc <= g.nc; cc += 256) dirx[cc] -= 1;
-        const uint32_t tomb = g.htab ? g.htomb[x] + 1u : 0u;
-        __syncthreads();
-        if (tomb > tomb_limit(old.y))
+    } else if (!add) {
+      group_delete_move<256>(pool, off, deg, &s_pos, 1, lane);
+      for (uint32_t cc = c + 1 + lane; cc <= g.nc; cc += 256) dirx[cc] -= 1;
+      __syncthreads();
+      if (g.htab) {
+        if (tomb + 1 > tomb_limit(old.y))
           row_table_build<256>(g, pool, x, old, dirx, deg - 1, lane);
-        else if (g.htab && lane == 0)
+        else if (lane == 0)
           row_table_delete(g, x, old, entry);
       }
-      __syncthreads();
     }
   }
-  if (out && lane == 0) {
+  if (out && blockIdx.x == 0 && lane == 0) {
     // an update whose label triple matches no query edge: nothing to count
     csm_result r;
     r.pos = 0; r.neg = 0; r.hash = 0;

@@ -48,9 +48,7 @@ __host__ __device__ inline uint32_t temporal_slots(uint32_t B) {
   return s;
 }
 __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges, DevGraph g);
-__global__ void k_compact_check(DevGraph g);
 __global__ void k_compact_copy(DevGraph g);
-__global__ void k_compact_finish(DevGraph g);
 void launch_mut_insert(const VRange* ranges, const unsigned int* n_ranges, const uint64_t* ins_key,
                        uint32_t* ins_dst, const DevGraph& g, uint32_t warp_blocks, uint32_t big_blocks,
                        cudaStream_t st);
@@ -65,9 +63,9 @@ __global__ void k_vdel_keys(DevGraph g, uint32_t v, uint32_t deg, uint64_t* keys
 __global__ void k_plain_resolve(const csm_update* up, DevGraph g, UpdInfo* info, uint64_t* keys, unsigned int* cnt,
                                 unsigned long long* count, unsigned long long* hash, unsigned long long* bytes,
                                 unsigned int* stop);
-// Applies the update's row insertion or deletion (one 256-thread block), after
-// finishing a compaction k_compact_copy ran; with `out`, also writes the
-// result of an update that needs no search (latency from stamp[0]).
+// Applies the update's row insertion or deletion (two 256-thread blocks); with
+// `out`, also writes the result of an update that needs no search (latency
+// from stamp[0]).
 __global__ void k_plain_mutate(DevGraph g, const UpdInfo* info, const uint64_t* keys, csm_result* out,
                                const unsigned long long* stamp, uint32_t mut_bytes);
 __global__ void k_vertex_update(const csm_update* ups, uint32_t B, DevGraph g, UpdInfo* info);

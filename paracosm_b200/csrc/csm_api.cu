@@ -91,7 +91,7 @@ struct csm_ctx {
   uint64_t *d_tk = nullptr, *d_tk2 = nullptr, *d_ts = nullptr, *d_ts2 = nullptr;
   VRange *d_rins = nullptr, *d_rdel = nullptr;
   uint32_t* d_ins_dst = nullptr;
-  unsigned int* d_cnt = nullptr;  // [0] n_ins [1] n_del [2] n_t [3] n_rins [4] n_rdel [6] n_tasks [7] task_next
+  unsigned int* d_cnt = nullptr;  // [0] n_ins [1] n_del [2] n_t [3] n_rins [4] n_rdel [6] n_tasks [7] task_next [8] search blocks ended
   Task* d_tasks = nullptr;
   unsigned long long *d_count = nullptr, *d_hash = nullptr, *d_bytes = nullptr;
   unsigned int* d_stop = nullptr;
@@ -480,11 +480,13 @@ static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out
   cudaStream_t st = q->st;
   const DevGraph& g = o->g;
   unsigned int* c = q->d_cnt;
-  k_seed<<<blocks_for(B, 128), 128, 0, st>>>(B, o->d_info, g, q->d_plan, q->index.d2, q->index.words,
-                                              q->d_tasks, c + 6, q->task_cap, q->d_safe, &g.ps->error,
-                                              q->cfg.shard_rank, q->cfg.shard_count,
-                                              (uint32_t)q->cfg.turboflux_compat,
-                                              q->cfg.algorithm == CSM_ALGO_CALIG ? 1u : 0u); CKL();
+  const bool one = B == 1;  // the seeds' one warp prepares the search's queue too
+  k_seed<<<blocks_for(B, 4), one ? 32 : 128, 0, st>>>(B, o->d_info, g, q->d_plan, q->index.d2, q->index.words,
+                                                      q->d_tasks, c + 6, q->task_cap, q->d_safe, &g.ps->error,
+                                                      q->cfg.shard_rank, q->cfg.shard_count,
+                                                      (uint32_t)q->cfg.turboflux_compat,
+                                                      q->cfg.algorithm == CSM_ALGO_CALIG ? 1u : 0u,
+                                                      one ? q->d_q : nullptr, one ? q->d_sstat : nullptr); CKL();
   SearchParams sp{};
   sp.g = g; sp.plan = q->d_plan; sp.tasks = q->d_tasks; sp.n_tasks = c + 6; sp.task_cap = q->task_cap;
   sp.task_next = c + 7; sp.info = o->d_info; sp.count = q->d_count; sp.hash = q->d_hash; sp.bytes = q->d_bytes;
@@ -509,8 +511,14 @@ static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out
   set_search_shape(sp, *q->h_plan);
   uint32_t warps, bps;
   search_shape(q, warps, bps);
+  const ResultArgs ra{o->d_info, q->d_count, q->d_hash, q->d_bytes, q->d_safe, q->d_stop, q->cfg.max_results,
+                      q->cfg.want_hash, out, (q->cfg.shard_count > 1 && q->cfg.shard_rank) ? 0u : 16u, o->d_stamp};
+  if (B <= kFuseResults) {
+    sp.result = ra;
+    sp.ended = q->d_cnt + 8;  // cleared with the batch's counters
+  }
   if (o->capturing) {  // replays are not timed per search
-    launch_search(sp, (uint32_t)q->sm_count * bps, warps, st); CKL();
+    launch_search(sp, (uint32_t)q->sm_count * bps, warps, st, one); CKL();
   } else {
     if (q->sev_used == q->sev.size()) {
       cudaEvent_t a, b;
@@ -519,15 +527,11 @@ static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out
       q->sev.emplace_back(a, b);
     }
     CK(cudaEventRecord(q->sev[q->sev_used].first, st));
-    launch_search(sp, (uint32_t)q->sm_count * bps, warps, st); CKL();
+    launch_search(sp, (uint32_t)q->sm_count * bps, warps, st, one); CKL();
     CK(cudaEventRecord(q->sev[q->sev_used].second, st));
     q->sev_used++;
   }
-  k_finalize<<<blocks_for(B, 256), 256, 0, st>>>(B, o->d_info, q->d_count, q->d_hash, q->d_bytes,
-                                                  q->d_safe, q->d_stop, q->cfg.max_results, q->cfg.want_hash,
-                                                  out, (q->cfg.shard_count > 1 && q->cfg.shard_rank) ? 0u : 16u,
-                                                  o->d_stamp);
-  CKL();
+  if (B > kFuseResults) { k_finalize<<<blocks_for(B, 256), 256, 0, st>>>(B, ra); CKL(); }
   return CSM_OK;
 }
 
@@ -594,11 +598,9 @@ static int run_edge_batch(csm_ctx* ctx, const csm_update* ups, uint32_t B, csm_r
 // with the edge's own label, which the host does not know, so a deletion is
 // only decided this way when no query edge has its vertex-label pair.
 // Launches per update:
-//   no matching query edge: resolve, [compaction copy,] mutate        2-3
-//   insertion:  resolve, compaction copy, mutate, index marks + round,
-//               seeds, search queue + search, results                 9
-//   deletion:   resolve, seeds, search queue + search, results,
-//               mutate, index marks + round                           8
+//   no matching query edge: resolve, [compaction copy,] mutate              2-3
+//   insertion:  resolve, compaction copy, mutate, index round, seeds, search  6
+//   deletion:   resolve, seeds, search, mutate, index round                   5
 // (the compaction copy returns at once unless the insertion's relocation
 // does not fit; GraphFlow has no index rounds).
 
@@ -722,7 +724,10 @@ static int run_vertex_update(csm_ctx* ctx, const csm_update* ups, const csm_upda
   }
   k_vertex_update<<<1, 32, 0, st>>>(ups, 1, ctx->g, ctx->d_info); CKL();
   CK(cudaMemsetAsync(ctx->d_safe, 0xff, 4, st));
-  k_finalize<<<1, 32, 0, st>>>(1, ctx->d_info, ctx->d_count, ctx->d_hash, nullptr, nullptr, nullptr, 0, 0, out); CKL();
+  ResultArgs ra{};
+  ra.info = ctx->d_info;
+  ra.out = out;
+  k_finalize<<<1, 32, 0, st>>>(1, ra); CKL();
   int rc = index_vertex_update(ctx->index, ctx->g, h, st, &ctx->launches);
   if (rc) return rc;
   for (size_t k = 0; k < ctx->attached.size(); k++) {
@@ -730,8 +735,8 @@ static int run_vertex_update(csm_ctx* ctx, const csm_update* ups, const csm_upda
     a->g = ctx->g;
     rc = stream_after(a->st, st, ctx->ev_fork);
     if (rc) return rc;
-    k_finalize<<<1, 32, 0, a->st>>>(1, ctx->d_info, a->d_count, a->d_hash, nullptr, nullptr, nullptr, 0, 0,
-                                    out_q[k]);
+    ra.out = out_q[k];
+    k_finalize<<<1, 32, 0, a->st>>>(1, ra);
     a->launches++;
     CK(cudaGetLastError());
     rc = index_vertex_update(a->index, ctx->g, h, a->st, &a->launches);
@@ -1020,7 +1025,7 @@ static int tune_run(csm_ctx* ctx, uint32_t B, uint32_t warps, uint32_t bps, floa
   CK(cudaMemsetAsync(ctx->d_count, 0, 8ull * B, st));
   CK(cudaMemsetAsync(ctx->d_bytes, 0, 8ull * B, st));
   CK(cudaMemsetAsync(ctx->d_stop, 0, 4ull * B, st));
-  k_seed<<<blocks_for(B, 128), 128, 0, st>>>(B, ctx->d_info, g, ctx->d_plan, ctx->index.d2, ctx->index.words,
+  k_seed<<<blocks_for(B, 4), 128, 0, st>>>(B, ctx->d_info, g, ctx->d_plan, ctx->index.d2, ctx->index.words,
                                               ctx->d_tasks, c + 6, ctx->task_cap, ctx->d_safe, &g.ps->error); CKL();
   SearchParams sp{};
   sp.g = g; sp.plan = ctx->d_plan; sp.tasks = ctx->d_tasks; sp.n_tasks = c + 6; sp.task_cap = ctx->task_cap;

@@ -494,8 +494,9 @@ __device__ __forceinline__ uint32_t count_le(const uint32_t* pos, uint32_t k, ui
 // from the front for a move to the left.  An entry's place follows from its
 // rank among the k changed positions, whatever k is: moving the blocks between
 // changed positions one after another cost two barriers per change (a batch
-// of 65,536 updates changes hub rows in hundreds of places: 508 us inserting
-// and 549 us deleting on the 2^22-vertex graph, against 105 and 83 us).
+// of 65,536 updates changes hub rows in hundreds of places: 634 us inserting
+// and 691 us deleting on the 2^22-vertex graph, against 448 and 469 us, the
+// time one block takes to move its longest row).
 constexpr uint32_t kMoveUnroll = 8;
 
 // Entries [from, deg) of the row at src go to dst + i + (changed positions <= i).

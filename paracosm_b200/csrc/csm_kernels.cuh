@@ -124,6 +124,19 @@ struct SearchStats {
   unsigned int guard_lv[4 * 16];  // per level 1..16: cnt, cur_e, cur_k, dn[cur_e]
 };
 
+// What the results of a batch's updates are made of.
+struct ResultArgs {
+  const UpdInfo* info;
+  const unsigned long long *count, *hash, *bytes;
+  const uint32_t* safe;
+  const unsigned int* stop;
+  uint64_t cap;
+  int want_hash;
+  csm_result* out;
+  uint32_t mut_bytes;               // bytes of an applied mutation (0 on secondary shards)
+  const unsigned long long* stamp;  // non-null: latency from stamp[0]
+};
+
 struct SearchParams {
   DevGraph g;
   const Plan* plan;
@@ -169,11 +182,17 @@ struct SearchParams {
   // instead of enumerating it; only for counts without hashes or match sets
   uint32_t tail;
   uint32_t levels, warp_bytes;  // SearchShape
+  // non-null result.out: the launch's last block writes the batch's results
+  // (a launch less; for a few updates, which one block writes in no time)
+  ResultArgs result;
+  unsigned int* ended;          // blocks that have ended; 0 between launches
 };
+constexpr uint32_t kFuseResults = 1024;  // updates of a batch up to which it does
 __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* plan, const uint64_t* d2,
                        uint64_t d2_words, Task* tasks, unsigned int* n_tasks, uint32_t task_cap,
                        uint32_t* safe, unsigned int* error, uint32_t shard_rank = 0, uint32_t shard_count = 1,
-                       uint32_t turboflux_compat = 0, uint32_t dup_zero = 0);
+                       uint32_t turboflux_compat = 0, uint32_t dup_zero = 0, SearchQueue* q = nullptr,
+                       SearchStats* ss = nullptr);
 // mode: 0 plain, 1 match sets, 2 tail counting
 struct SearchShape {
   uint32_t levels;      // levels of a warp's walk
@@ -182,12 +201,9 @@ struct SearchShape {
 SearchShape search_shape_of(const Plan& plan, int mode);
 uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode);
 int search_mode(const SearchParams& p);
-void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s);
-__global__ void k_finalize(uint32_t B, const UpdInfo* info, const unsigned long long* count,
-                           const unsigned long long* hash, const unsigned long long* bytes, const uint32_t* safe,
-                           const unsigned int* stop, uint64_t cap, int want_hash, csm_result* out,
-                           uint32_t mut_bytes = 16,  // bytes of an applied mutation (0 on secondary shards)
-                           const unsigned long long* stamp = nullptr);  // non-null: latency from stamp[0]
+// `prepared`: k_seed has prepared the queue.
+void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s, bool prepared = false);
+__global__ void k_finalize(uint32_t B, ResultArgs a);
 // stop[] values: 1 = the cap was reached, 2 = the deadline passed first
 constexpr unsigned int kStopCap = 1u, kStopDeadline = 2u;
 __global__ void k_classify(uint64_t n, const csm_update* ups, DevGraph g, const Plan* plan, uint8_t* safe);

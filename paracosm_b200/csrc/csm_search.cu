@@ -72,14 +72,41 @@ __device__ __forceinline__ bool d2_bit(const uint64_t* d2, uint64_t words, uint3
   return (d2[(uint64_t)q * words + (v >> 6)] >> (v & 63)) & 1ULL;
 }
 
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
+  return t;
+}
+
+// Per launch: tickets keep counting up across launches (the ring's slot
+// sequence numbers stay consistent); hunger and pending start afresh, and the
+// tickets that warps still waiting at the end of the last launch held (never
+// filled) are handed out again.
+__device__ __forceinline__ void search_prep(SearchQueue* q, SearchStats* ss, uint32_t tasks, unsigned int* error) {
+  if (q->head < q->tail) atomicExch(error, kErrRingState);
+  q->head = q->tail;  // tickets that waiting warps held when the last launch ended were never filled
+  q->hungry = 0;
+  q->pending = tasks;
+  ss->launch_t0 = global_ns();
+}
+__global__ void k_search_prep(SearchQueue* q, const unsigned int* n_tasks, uint32_t task_cap, SearchStats* ss,
+                              unsigned int* error) {
+  search_prep(q, ss, min(*n_tasks, task_cap), error);
+}
+
+// One warp per update, a lane per anchor (one thread trying the anchors in
+// turn took 9.6 us for a single update of a 35-edge query, its loads one
+// after another).  With `q` (one update only) the warp also prepares the
+// search's queue, as k_search_prep does.
 __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* plan, const uint64_t* d2,
                        uint64_t d2_words, Task* tasks, unsigned int* n_tasks, uint32_t task_cap,
                        uint32_t* safe, unsigned int* error, uint32_t shard_rank, uint32_t shard_count,
-                       uint32_t turboflux_compat, uint32_t dup_zero) {
-  uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+                       uint32_t turboflux_compat, uint32_t dup_zero, SearchQueue* q, SearchStats* ss) {
+  const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= B) return;
   const UpdInfo u = info[s];
-  uint32_t sf = 1;
+  bool matches = false;
+  uint32_t made = 0;
   // dup_zero: an insertion of a present edge counts nothing (CaLiG skips it,
   // ParaCOSM/CSM/matching/Parallel_CaLiG/parallel_calig.cpp:1249)
   if ((u.flags & UF_VALID) && !(u.flags & UF_INVALID) && !(dup_zero && (u.flags & UF_DUP))) {
@@ -89,13 +116,13 @@ __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* 
     // labels match, whatever its edge label, and filters the endpoints by d2
     // only on spanning-tree edges (ParaCOSM/CSM/matching/TurboFlux/turboflux.cpp:966-1022)
     const bool compat_del = turboflux_compat && !(u.flags & UF_ADD);
-    for (uint32_t a = 0; a < na; a++) {
+    for (uint32_t a = lane; a < na; a += 32) {
       const PlanAnchor* A = &plan->anchors[a];
-      if (A->el != l && !compat_del) continue;
-      const bool o0 = A->la == L1 && A->lb == L2;
-      const bool o1 = A->la == L2 && A->lb == L1;
-      if (!(o0 || o1)) continue;
-      sf = 0;
+      const uint32_t el = A->el, la = A->la, lb = A->lb;
+      if (el != l && !compat_del) continue;
+      const bool o0 = la == L1 && lb == L2;
+      const bool o1 = la == L2 && lb == L1;
+      matches = matches || o0 || o1;
       for (int o = 0; o < 2; o++) {
         if (!(o ? o1 : o0)) continue;
         const uint32_t x = o ? u.v2 : u.v1, y = o ? u.v1 : u.v2;
@@ -106,10 +133,16 @@ __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* 
         unsigned int i = atomicAdd(n_tasks, 1u);
         if (i >= task_cap) { atomicExch(error, kErrTaskOverflow); continue; }
         tasks[i] = Task{s, (uint16_t)a, (uint8_t)o, 0};
+        made++;
       }
     }
   }
-  safe[s] = sf;
+  matches = __any_sync(0xffffffffu, matches);
+  if (lane == 0) safe[s] = matches ? 0u : 1u;
+  if (q) {
+    made = __reduce_add_sync(0xffffffffu, made);
+    if (lane == 0) search_prep(q, ss, made, error);
+  }
 }
 
 __device__ __forceinline__ uint32_t warp_incl_scan(uint32_t v, uint32_t lane) {
@@ -307,12 +340,6 @@ __device__ __forceinline__ bool pick_driver(const SearchParams& p, const LevelSM
   dn = best;
   bytes = b4;
   return !empty;
-}
-
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(t));
-  return t;
 }
 
 // Per-task accumulators, flushed to the update's counters when the task ends;
@@ -599,6 +626,27 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
   for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   out.sum = out.stopped ? 0ull : sum;
   return out;
+}
+
+// Result of update s once its search is done.
+__device__ __forceinline__ void write_result(const ResultArgs& a, uint32_t s) {
+  const UpdInfo u = a.info[s];
+  csm_result r;
+  r.pos = 0; r.neg = 0; r.hash = 0; r.work_bytes = 0; r.latency_ns = 0;
+  r.status = CSM_ST_OK; r.safe = a.safe ? a.safe[s] : 1u;
+  if ((u.flags & UF_INVALID) || !(u.flags & UF_VALID)) {
+    r.status = (u.flags & UF_INVALID) ? CSM_ST_INVALID : CSM_ST_OK;  // vertex updates count nothing
+    r.safe = 1;
+  } else {
+    unsigned long long c = __ldcg(a.count + s);
+    if (a.cap && c >= a.cap) { c = a.cap; r.status = CSM_ST_CAPPED; }
+    else if (a.stop && __ldcg(a.stop + s) == kStopDeadline) r.status = CSM_ST_TIMED_OUT;  // c is a lower bound
+    if (u.flags & UF_ADD) r.pos = c; else r.neg = c;
+    if (a.want_hash && r.status == CSM_ST_OK) r.hash = __ldcg(a.hash + s);
+    r.work_bytes = (a.bytes ? __ldcg(a.bytes + s) : 0ull) + ((u.flags & UF_MUT) ? (unsigned long long)a.mut_bytes : 0ull);
+  }
+  if (a.stamp) r.latency_ns = global_ns() - a.stamp[0];
+  a.out[s] = r;
 }
 
 // A warp's counters of one launch.
@@ -981,19 +1029,6 @@ __device__ __forceinline__ int setup_donated(const SearchParams& p, LevelSM* lv,
   return (int)depth;
 }
 
-// Per launch: tickets keep counting up across launches (the ring's slot
-// sequence numbers stay consistent); hunger and pending start afresh, and the
-// tickets that warps still waiting at the end of the last launch held (never
-// filled) are handed out again.
-__global__ void k_search_prep(SearchQueue* q, const unsigned int* n_tasks, uint32_t task_cap, SearchStats* ss,
-                              unsigned int* error) {
-  if (q->head < q->tail) atomicExch(error, kErrRingState);
-  q->head = q->tail;  // tickets that waiting warps held when the last launch ended were never filled
-  q->hungry = 0;
-  q->pending = min(*n_tasks, task_cap);
-  ss->launch_t0 = global_ns();
-}
-
 // Kernel body; MODE 0 counts (and hashes), 1 also appends match sets, 2
 // counts independent tails (tail_stage).
 template <int W, int MODE>
@@ -1117,6 +1152,19 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
     if (s.checks) atomicAdd(&p.sstat->checks, s.checks);
     if (s.hungry) atomicAdd(&p.sstat->checks_hungry, s.hungry);
   }
+  // the results, by the block that ends last (small batches: SearchParams)
+  if (p.result.out) {
+    __shared__ bool last;
+    if (threadIdx.x == 0) {
+      __threadfence();
+      last = atomicAdd(p.ended, 1u) + 1u == gridDim.x;
+      if (last) *p.ended = 0;
+      __threadfence();
+    }
+    __syncthreads();
+    if (last)
+      for (uint32_t i = threadIdx.x; i < p.batch; i += W * 32) write_result(p.result, i);
+  }
 }
 
 // Sixteen warps per SM, 128 registers a thread (run_levels says why).
@@ -1184,9 +1232,9 @@ uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode) {
 
 int search_mode(const SearchParams& p) { return p.enum_buf ? 1 : (p.tail ? 2 : 0); }
 
-void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s) {
+void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s, bool prepared) {
   const size_t smem = (size_t)p.warp_bytes * warps;
-  if (p.q) k_search_prep<<<1, 1, 0, s>>>(p.q, p.n_tasks, p.task_cap, p.sstat, p.error);
+  if (p.q && !prepared) k_search_prep<<<1, 1, 0, s>>>(p.q, p.n_tasks, p.task_cap, p.sstat, p.error);
   const int mode = search_mode(p);
   switch (warps) {
     case 4: search_launch<4>(p, blocks, smem, s, mode); break;
@@ -1195,29 +1243,9 @@ void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaS
   }
 }
 
-__global__ void k_finalize(uint32_t B, const UpdInfo* info, const unsigned long long* count,
-                           const unsigned long long* hash, const unsigned long long* bytes, const uint32_t* safe,
-                           const unsigned int* stop, uint64_t cap, int want_hash, csm_result* out,
-                           uint32_t mut_bytes, const unsigned long long* stamp) {
+__global__ void k_finalize(uint32_t B, ResultArgs a) {
   uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
-  if (s >= B) return;
-  const UpdInfo u = info[s];
-  csm_result r;
-  r.pos = 0; r.neg = 0; r.hash = 0; r.work_bytes = 0; r.latency_ns = 0;
-  r.status = CSM_ST_OK; r.safe = safe ? safe[s] : 1u;
-  if ((u.flags & UF_INVALID) || !(u.flags & UF_VALID)) {
-    r.status = (u.flags & UF_INVALID) ? CSM_ST_INVALID : CSM_ST_OK;  // vertex updates count nothing
-    r.safe = 1;
-  } else {
-    unsigned long long c = count[s];
-    if (cap && c >= cap) { c = cap; r.status = CSM_ST_CAPPED; }
-    else if (stop && stop[s] == kStopDeadline) r.status = CSM_ST_TIMED_OUT;  // c is a lower bound
-    if (u.flags & UF_ADD) r.pos = c; else r.neg = c;
-    if (want_hash && r.status == CSM_ST_OK) r.hash = hash[s];
-    r.work_bytes = (bytes ? bytes[s] : 0ull) + ((u.flags & UF_MUT) ? (unsigned long long)mut_bytes : 0ull);
-  }
-  if (stamp) r.latency_ns = global_ns() - stamp[0];
-  out[s] = r;
+  if (s < B) write_result(a, s);
 }
 
 __global__ void k_classify(uint64_t n, const csm_update* ups, DevGraph g, const Plan* plan, uint8_t* safe) {

@@ -68,8 +68,8 @@ extern "C" {
 /* ---- execution modes ------------------------------------------------ */
 #define CSM_MODE_BATCHED 0   /* many updates per launch sequence (default) */
 #define CSM_MODE_PLAIN 1     /* one update per launch sequence: 2-3 launches for an update whose label
-                                triple matches no query edge, about 9 otherwise (index marks and one
-                                cooperative index round, seeds, search, results) */
+                                triple matches no query edge, 5-6 otherwise (row changes, one
+                                cooperative index round, seeds, search) */
 
 typedef struct csm_cfg {
   int32_t algorithm;          /* CSM_ALGO_* */

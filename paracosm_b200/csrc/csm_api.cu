@@ -109,6 +109,16 @@ struct csm_ctx {
   uint64_t updates_done = 0, v_updates = 0, e_updates = 0, batches = 0;
   uint64_t tot_pos = 0, tot_neg = 0, tot_unsafe = 0;
   bool totals_dirty = false;
+  // what a caller asks for after a submit -- the device's error word and, of a
+  // small submit, the results -- is copied to pinned memory behind it, so that
+  // waiting for the stream is all that is left to do
+  static constexpr uint32_t kSmall = 1024;
+  struct Pinned {
+    PoolState ps;
+    csm_result res[kSmall];
+  };
+  Pinned* pin = nullptr;
+  bool pin_ps = false, pin_res = false;  // the copies of the last submit have been queued
   std::vector<csm_result> h_last;  // host copy of the last submit's results (filled lazily)
   bool h_last_valid = false;
   cudaEvent_t ev_start = nullptr, ev_end = nullptr;
@@ -279,6 +289,12 @@ static int build_plan(csm_ctx* ctx) {
 
 // --------------------------------------------------------- batch buffers
 
+// Empty hand-over ring: slot i is free for ticket i.
+__global__ void k_ring_init(SearchQueue* q, unsigned long long* seq, uint32_t qcap) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *q = SearchQueue{};
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < qcap; i += gridDim.x * blockDim.x) seq[i] = i;
+}
+
 static int ensure_batch_buffers(csm_ctx* ctx) {
   if (ctx->d_ukey) return CSM_OK;
   const uint32_t B = ctx->bmax;
@@ -286,9 +302,19 @@ static int ensure_batch_buffers(csm_ctx* ctx) {
   ctx->lcap = L;
   const uint32_t na = std::max<uint32_t>(1, (uint32_t)(ctx->qe.size() / 3));
   ctx->task_cap = B * 2 * na;
-  DevMem& m = ctx->mem;
-  int rc = 0;
-#define AL(p, sz) do { rc = m.alloc((void**)&(p), (sz)); if (rc) return rc; } while (0)
+  // CUB scratch: the largest of the sorts issued per batch
+  size_t b1 = 0, b2 = 0, b3 = 0;
+  {
+    uint64_t* k = nullptr;
+    uint32_t* v = nullptr;
+    CK(cub::DeviceRadixSort::SortPairs(nullptr, b1, k, k, v, v, (int)B, 0, 64, ctx->st));
+    CK(cub::DeviceRadixSort::SortKeys(nullptr, b2, k, k, (int)L, 0, 64, ctx->st));
+    CK(cub::DeviceRadixSort::SortPairs(nullptr, b3, k, k, k, k, (int)L, 0, 64, ctx->st));
+  }
+  ctx->cub_bytes = std::max(b1, std::max(b2, b3));
+  ctx->qcap = 1u << 16;  // outstanding handed-over tasks never exceed the idle warps
+  DevBlock blk;
+#define AL(p, sz) blk.add(p, sz)
   AL(ctx->d_ukey, 8ull * B); AL(ctx->d_ukey2, 8ull * B);
   AL(ctx->d_useq, 4ull * B); AL(ctx->d_useq2, 4ull * B);
   AL(ctx->d_info, sizeof(UpdInfo) * (size_t)B);
@@ -303,46 +329,32 @@ static int ensure_batch_buffers(csm_ctx* ctx) {
   AL(ctx->d_count, 8ull * B); AL(ctx->d_hash, 8ull * B); AL(ctx->d_bytes, 8ull * B);
   AL(ctx->d_stop, 4ull * B); AL(ctx->d_safe, 4ull * B);
   AL(ctx->d_stamp, 64);
-  AL(ctx->d_gups, sizeof(csm_update) * (size_t)B);
-  AL(ctx->d_gres, sizeof(csm_result) * (size_t)B);
-  AL(ctx->d_gpad, sizeof(csm_update) * (size_t)B);
+  if (ctx->cfg.graphs == CSM_GRAPHS_ON) {
+    AL(ctx->d_gups, sizeof(csm_update) * (size_t)B);
+    AL(ctx->d_gres, sizeof(csm_result) * (size_t)B);
+    AL(ctx->d_gpad, sizeof(csm_update) * (size_t)B);
+  }
   if (ctx->cfg.enum_capacity) {
     AL(ctx->d_enum, 4ull * (1 + ctx->nq) * ctx->cfg.enum_capacity);
     AL(ctx->d_enum_n, 16);
-    CK(cudaMemsetAsync(ctx->d_enum_n, 0, 16, ctx->st));
   }
-  {
+  AL(ctx->d_q, sizeof(SearchQueue));
+  AL(ctx->d_sstat, sizeof(SearchStats));
+  AL(ctx->d_dq, sizeof(DTask) * (size_t)ctx->qcap);
+  AL(ctx->d_qseq, 8ull * ctx->qcap);
+  AL(ctx->d_cub, ctx->cub_bytes);
+#undef AL
+  void* base = nullptr;
+  int rc = blk.alloc(ctx->mem, &base);
+  if (rc) return rc;
+  if (ctx->d_enum_n) CK(cudaMemsetAsync(ctx->d_enum_n, 0, 16, ctx->st));
+  if (ctx->d_gpad) {
     std::vector<csm_update> pad(B, csm_update{'e', 1, 0, 0, 0, 0});
     CK(cudaMemcpyAsync(ctx->d_gpad, pad.data(), sizeof(csm_update) * (size_t)B, cudaMemcpyHostToDevice, ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
   }
-  ctx->qcap = 1u << 16;  // outstanding handed-over tasks never exceed the idle warps
-  AL(ctx->d_q, sizeof(SearchQueue));
-  AL(ctx->d_sstat, sizeof(SearchStats));
   CK(cudaMemsetAsync(ctx->d_sstat, 0, sizeof(SearchStats), ctx->st));
-  AL(ctx->d_dq, sizeof(DTask) * (size_t)ctx->qcap);
-  AL(ctx->d_qseq, 8ull * ctx->qcap);
-  CK(cudaMemsetAsync(ctx->d_q, 0, sizeof(SearchQueue), ctx->st));
-  {
-    std::vector<unsigned long long> seq(ctx->qcap);
-    for (uint32_t i = 0; i < ctx->qcap; i++) seq[i] = i;
-    CK(cudaMemcpyAsync(ctx->d_qseq, seq.data(), 8ull * ctx->qcap, cudaMemcpyHostToDevice, ctx->st));
-    CK(cudaStreamSynchronize(ctx->st));
-  }
-#undef AL
-  // CUB scratch: the largest of the sorts issued per batch
-  size_t b1 = 0, b2 = 0, b3 = 0;
-  CK(cub::DeviceRadixSort::SortPairs(nullptr, b1, ctx->d_ukey, ctx->d_ukey2, ctx->d_useq, ctx->d_useq2, (int)B, 0, 64, ctx->st));
-  CK(cub::DeviceRadixSort::SortKeys(nullptr, b2, ctx->d_ins, ctx->d_ins2, (int)L, 0, 64, ctx->st));
-  CK(cub::DeviceRadixSort::SortPairs(nullptr, b3, ctx->d_tk, ctx->d_tk2, ctx->d_ts, ctx->d_ts2, (int)L, 0, 64, ctx->st));
-  const size_t need = std::max(b1, std::max(b2, b3));
-  if (need > ctx->cub_bytes) {
-    if (ctx->d_cub) ctx->mem.release(ctx->d_cub, ctx->cub_bytes);
-    ctx->d_cub = nullptr;
-    rc = ctx->mem.alloc(&ctx->d_cub, need);
-    if (rc) return rc;
-    ctx->cub_bytes = need;
-  }
+  k_ring_init<<<64, 256, 0, ctx->st>>>(ctx->d_q, ctx->d_qseq, ctx->qcap); CKL();
   return CSM_OK;
 }
 
@@ -621,13 +633,13 @@ static bool plain_may_count(const csm_ctx* ctx, const csm_update& u) {
 }
 
 // One edge update of the plain form (no attached queries); d_up is the record
-// in device memory, h its host copy.
-static int run_plain_edge(csm_ctx* ctx, const csm_update* d_up, const csm_update& h, csm_result* out) {
+// in device memory, h its host copy.  `stamp`: note the submit's time.
+static int run_plain_edge(csm_ctx* ctx, const csm_update* d_up, const csm_update& h, csm_result* out, bool stamp) {
   cudaStream_t st = ctx->st;
   const DevGraph& g = ctx->g;
   uint64_t* keys = ctx->d_ins2;
   k_plain_resolve<<<1, 32, 0, st>>>(d_up, g, ctx->d_info, keys, ctx->d_cnt, ctx->d_count, ctx->d_hash, ctx->d_bytes,
-                                     ctx->d_stop);
+                                     ctx->d_stop, stamp ? ctx->d_stamp : nullptr);
   CKL();
   if (h.type == 'e' && h.is_add) {
     k_compact_copy<<<ctx->sm_count * 2, 1024, 0, st>>>(g);  // returns at once unless the pool must be compacted
@@ -826,6 +838,10 @@ static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, cons
   rc = ensure_results(ctx, n);
   if (rc) return rc;
   cudaStream_t st = ctx->st;
+  if (!ctx->pin && cudaMallocHost((void**)&ctx->pin, sizeof(csm_ctx::Pinned)) != cudaSuccess) {
+    cudaGetLastError();
+    ctx->pin = nullptr;  // the copies are then made when asked for
+  }
   for (csm_ctx* a : ctx->attached) {
     rc = ensure_results(a, n);
     if (!rc) rc = stream_after(st, a->st, a->ev_join);  // work issued on it outside a submit
@@ -835,7 +851,9 @@ static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, cons
   if (ctx->d_enum_n) CK(cudaMemsetAsync(ctx->d_enum_n, 0, 16, st));
   for (csm_ctx* a : ctx->attached)
     if (a->d_enum_n) CK(cudaMemsetAsync(a->d_enum_n, 0, 16, st));  // before the fork below
-  k_stamp<<<1, 1, 0, st>>>(ctx->d_stamp); CKL();
+  const bool plain = ctx->cfg.mode == CSM_MODE_PLAIN && ctx->attached.empty() && !ctx->d_enum;
+  bool stamp = plain && h_ups && h_ups[0].type == 'e';  // the first update's own kernel takes the time
+  if (!stamp) { k_stamp<<<1, 1, 0, st>>>(ctx->d_stamp); CKL(); }
   for (csm_ctx* a : ctx->attached) {
     rc = stream_after(a->st, st, ctx->ev_fork);
     if (rc) return rc;
@@ -870,8 +888,9 @@ static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, cons
       i++;
       continue;
     }
-    if (ctx->cfg.mode == CSM_MODE_PLAIN && ctx->attached.empty() && !ctx->d_enum) {
-      rc = run_plain_edge(ctx, d_ups + i, h[i], ctx->d_results + i);
+    if (plain) {
+      rc = run_plain_edge(ctx, d_ups + i, h[i], ctx->d_results + i, stamp);
+      stamp = false;
       if (rc) return rc;
       ctx->e_updates++;
       i++;
@@ -899,6 +918,15 @@ static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, cons
     q->updates_done += n;
     q->totals_dirty = true;
     q->h_last_valid = false;
+    q->pin_ps = q->pin_res = false;
+  }
+  if (ctx->pin) {
+    CK(cudaMemcpyAsync(&ctx->pin->ps, ctx->g.ps, sizeof(PoolState), cudaMemcpyDeviceToHost, st));
+    ctx->pin_ps = true;
+    if (n <= csm_ctx::kSmall) {
+      CK(cudaMemcpyAsync(ctx->pin->res, ctx->d_results, n * sizeof(csm_result), cudaMemcpyDeviceToHost, st));
+      ctx->pin_res = true;
+    }
   }
   return CSM_OK;
 }
@@ -906,16 +934,19 @@ static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, cons
 // Puts the hand-over ring back into its initial state (after a failed launch).
 static int reset_ring(csm_ctx* ctx) {
   if (!ctx->d_q) return CSM_OK;
-  CK(cudaMemsetAsync(ctx->d_q, 0, sizeof(SearchQueue), ctx->st));
-  std::vector<unsigned long long> seq(ctx->qcap);
-  for (uint32_t i = 0; i < ctx->qcap; i++) seq[i] = i;
-  CK(cudaMemcpyAsync(ctx->d_qseq, seq.data(), 8ull * ctx->qcap, cudaMemcpyHostToDevice, ctx->st));
+  k_ring_init<<<64, 256, 0, ctx->st>>>(ctx->d_q, ctx->d_qseq, ctx->qcap);
+  CK(cudaGetLastError());
   CK(cudaStreamSynchronize(ctx->st));
   return CSM_OK;
 }
 
+// After the context's stream has been waited for.
 static int check_device_error(csm_ctx* ctx) {
   PoolState ps;
+  if (ctx->pin_ps) {
+    if (ctx->pin->ps.error == 0) return CSM_OK;
+    ctx->pin_ps = false;  // reported (and cleared on the device) once
+  }
   CK(cudaMemcpy(&ps, ctx->g.ps, sizeof(PoolState), cudaMemcpyDeviceToHost));
   if (ps.error) {
     static const char* names[] = {"none", "row pool exhausted", "batch list overflow", "task list overflow",
@@ -970,7 +1001,9 @@ static int fetch_last(csm_ctx* ctx) {
   int rc = check_device_error(ctx);
   if (rc) return rc;
   ctx->h_last.resize(ctx->last_n);
-  if (ctx->last_n) {
+  if (ctx->pin_res) {
+    memcpy(ctx->h_last.data(), ctx->pin->res, ctx->last_n * sizeof(csm_result));
+  } else if (ctx->last_n) {
     CK(cudaMemcpyAsync(ctx->h_last.data(), ctx->d_results, ctx->last_n * sizeof(csm_result), cudaMemcpyDeviceToHost,
                        ctx->st));
     CK(cudaStreamSynchronize(ctx->st));
@@ -1018,6 +1051,7 @@ __global__ void k_tune_prep(const csm_update* edges, uint32_t n, DevGraph g, Upd
 
 static int tune_run(csm_ctx* ctx, uint32_t B, uint32_t warps, uint32_t bps, float* ms, uint32_t donate_every = 0,
                     uint32_t split_deep = 0) {
+  ctx->pin_ps = false;  // the error word is read again below
   cudaStream_t st = ctx->st;
   const DevGraph& g = ctx->g;
   unsigned int* c = ctx->d_cnt;
@@ -1162,6 +1196,7 @@ __global__ void k_init_sum(uint32_t B, const unsigned long long* count, unsigned
 }
 
 static int initial_match(csm_ctx* ctx, uint64_t* out) {
+  ctx->pin_ps = false;  // the error word is read again below
   cudaStream_t st = ctx->st;
   DevGraph& g = ctx->g;
   const PlanAnchor& A = ctx->h_plan->anchors[0];
@@ -1294,15 +1329,17 @@ int csm_gpu_create(const csm_cfg* cfg, csm_ctx** out) {
   if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return set_err(CSM_ECUDA, "no CUDA device");
   if (cfg->device < 0 || cfg->device >= ndev) return set_err(CSM_EINVAL, "bad device %d", cfg->device);
   CK(cudaSetDevice(cfg->device));
-  cudaDeviceProp prop;
-  CK(cudaGetDeviceProperties(&prop, cfg->device));
-  if (prop.major < 10) return set_err(CSM_EUNSUPPORTED, "needs an sm_100 device, found sm_%d%d", prop.major, prop.minor);
+  int major = 0, minor = 0, sms = 0;  // the whole property record takes 2.6 ms to fetch
+  CK(cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, cfg->device));
+  CK(cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, cfg->device));
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, cfg->device));
+  if (major < 10) return set_err(CSM_EUNSUPPORTED, "needs an sm_100 device, found sm_%d%d", major, minor);
   csm_ctx* ctx = new csm_ctx();
   ctx->cfg = *cfg;
   if (!ctx->cfg.max_batch) ctx->cfg.max_batch = kMaxBatch;
   ctx->bmax = ctx->cfg.mode == CSM_MODE_PLAIN ? 1u : ctx->cfg.max_batch;
   ctx->dev = cfg->device;
-  ctx->sm_count = prop.multiProcessorCount;
+  ctx->sm_count = sms;
   size_t free_b = 0, total_b = 0;
   cudaMemGetInfo(&free_b, &total_b);
   ctx->mem.budget = cfg->hbm_budget_bytes ? cfg->hbm_budget_bytes : (uint64_t)(0.9 * (double)free_b);
@@ -1491,14 +1528,19 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   g.n = n_v; g.n_cap = n_cap; g.n_vl = n_vl; g.n_el = n_el; g.nc = (uint32_t)nc; g.kb = kb;
   DevMem& m = ctx->mem;
   int rc = 0;
-#define AL(p, sz) do { rc = m.alloc((void**)&(p), (sz)); if (rc) return rc; } while (0)
-  AL(g.vlabel, 4ull * n_cap);
-  AL(g.row, 8ull * n_cap);
-  AL(g.dir, 4ull * n_cap * (nc + 1));
-  AL(g.t_tab, sizeof(ulonglong2) * (size_t)temporal_slots(ctx->bmax));
-  AL(g.t_count, 4ull * n_cap);
-  AL(g.ps, sizeof(PoolState));
-  AL(ctx->d_qlab, 4ull * (ctx->qlab_v.size() + ctx->qlab_e.size()));
+  {
+    DevBlock blk;
+    blk.add(g.vlabel, 4ull * n_cap);
+    blk.add(g.row, 8ull * n_cap);
+    blk.add(g.dir, 4ull * n_cap * (nc + 1));
+    blk.add(g.t_tab, sizeof(ulonglong2) * (size_t)temporal_slots(ctx->bmax));
+    blk.add(g.t_count, 4ull * n_cap);
+    blk.add(g.ps, sizeof(PoolState));
+    blk.add(ctx->d_qlab, 4ull * (ctx->qlab_v.size() + ctx->qlab_e.size()));
+    void* base = nullptr;
+    rc = blk.alloc(m, &base);
+    if (rc) return rc;
+  }
   CK(cudaMemcpyAsync(ctx->d_qlab, ctx->qlab_v.data(), 4ull * ctx->qlab_v.size(), cudaMemcpyHostToDevice, st));
   CK(cudaMemcpyAsync(ctx->d_qlab + ctx->qlab_v.size(), ctx->qlab_e.data(), 4ull * ctx->qlab_e.size(),
                      cudaMemcpyHostToDevice, st));
@@ -1509,31 +1551,59 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   CK(cudaMemsetAsync(g.vlabel, 0xff, 4ull * n_cap, st));
   CK(cudaMemcpyAsync(g.vlabel, vlabels, 4ull * n_v, cudaMemcpyHostToDevice, st));
   ctx->h_vlabel.assign(n_cap, kNone);
-  for (uint32_t v = 0; v < n_v; v++)
-    if (vlabels[v] != kNone) ctx->h_vlabel[v] = fold_host(ctx->qlab_v, vlabels[v]);
+  {
+    // folded label of every label up to the largest kept one, where that is small
+    std::vector<uint32_t> table;
+    if (!ctx->qlab_v.empty() && ctx->qlab_v.back() < (1u << 16)) {
+      table.assign(ctx->qlab_v.back() + 1, (uint32_t)ctx->qlab_v.size());
+      for (uint32_t i = 0; i < ctx->qlab_v.size(); i++) table[ctx->qlab_v[i]] = i;
+    }
+    const uint32_t inert = (uint32_t)ctx->qlab_v.size();
+    for (uint32_t v = 0; v < n_v; v++) {
+      const uint32_t l = vlabels[v];
+      if (l == kNone) continue;
+      ctx->h_vlabel[v] = table.empty() ? fold_host(ctx->qlab_v, l) : l < table.size() ? table[l] : inert;
+    }
+  }
   if (n_v) { k_fold_vlabels<<<blocks_for(n_v, 256), 256, 0, st>>>(g.vlabel, n_v, g); CKL(); }
   CK(cudaMemsetAsync(g.dir, 0, 4ull * n_cap * (nc + 1), st));
   CK(cudaMemsetAsync(g.t_count, 0, 4ull * n_cap, st));
   CK(cudaMemsetAsync(g.ps, 0, sizeof(PoolState), st));
-  // temporaries
-  uint32_t* d_e = nullptr; uint64_t *ukey = nullptr, *ukey2 = nullptr, *uidx = nullptr, *uidx2 = nullptr;
-  uint64_t *dkey = nullptr, *dkey2 = nullptr, *first = nullptr, *cap64 = nullptr, *off64 = nullptr;
-  uint32_t* cap32 = nullptr;
-  unsigned long long* d_small = nullptr;
+  // temporaries, in two allocations: the input edges with their sort buffers
+  // (dkey takes the place of ukey and uidx), and what is needed to the end
   const uint64_t M = 2 * n_e;
-  AL(d_e, 12ull * n_e);
-  AL(ukey, 8ull * n_e); AL(ukey2, 8ull * n_e); AL(uidx, 8ull * n_e); AL(uidx2, 8ull * n_e);
-  AL(d_small, 64);
+  size_t tb = 0, tb2 = 0, tb3 = 0;
+  {
+    uint64_t* k = nullptr;
+    CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, k, k, k, k, (int64_t)n_e, 0, 64, st));
+    CK(cub::DeviceRadixSort::SortKeys(nullptr, tb2, k, k, (int64_t)M, 0, (int)kb.total(), st));
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, tb3, k, k, (int64_t)n_cap, st));
+  }
+  const size_t tbmax = std::max(tb, std::max(tb2, tb3));
+  uint32_t *d_e = nullptr, *cap32 = nullptr;
+  uint64_t *dkey = nullptr, *ukey2 = nullptr, *uidx2 = nullptr, *dkey2 = nullptr;
+  uint64_t *first = nullptr, *cap64 = nullptr, *off64 = nullptr;
+  unsigned long long* d_small = nullptr;
+  void *tmp = nullptr, *early = nullptr, *late = nullptr;
+  DevBlock blk1, blk2;
+  blk1.add(d_e, 12ull * n_e);
+  blk1.add(dkey, 8ull * M);
+  blk1.add(ukey2, 8ull * n_e);
+  blk1.add(uidx2, 8ull * n_e);
+  blk2.add(tmp, tbmax);
+  blk2.add(d_small, 64);
+  blk2.add(dkey2, 8ull * M);
+  blk2.add(first, 8ull * n_cap);
+  blk2.add(cap64, 8ull * n_cap);
+  blk2.add(off64, 8ull * n_cap);
+  blk2.add(cap32, 4ull * n_cap);
+  rc = blk1.alloc(m, &early);
+  if (!rc) rc = blk2.alloc(m, &late);
+  if (rc) { m.release(early, blk1.total); return rc; }
+  uint64_t *ukey = dkey, *uidx = dkey + n_e;
   CK(cudaMemcpyAsync(d_e, edges, 12ull * n_e, cudaMemcpyHostToDevice, st));
   CK(cudaMemsetAsync(d_small, 0, 64, st));
   if (n_e) { k_load_edge_keys<<<blocks_for(n_e, 256), 256, 0, st>>>(d_e, n_e, g.vlabel, n_v, ukey, uidx, d_small); CKL(); }
-  void* tmp = nullptr; size_t tb = 0, tb2 = 0;
-  CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, ukey, ukey2, uidx, uidx2, (int64_t)n_e, 0, 64, st));
-  CK(cub::DeviceRadixSort::SortKeys(nullptr, tb2, dkey, dkey2, (int64_t)M, 0, (int)kb.total(), st));
-  size_t tb3 = 0;
-  CK(cub::DeviceScan::ExclusiveSum(nullptr, tb3, cap64, off64, (int64_t)n_cap, st));
-  const size_t tbmax = std::max(tb, std::max(tb2, tb3));
-  AL(tmp, tbmax);
   if (n_e) {
     tb = tbmax;
     CK(cub::DeviceRadixSort::SortPairs(tmp, tb, ukey, ukey2, uidx, uidx2, (int64_t)n_e, 0, 64, st));
@@ -1541,19 +1611,16 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   unsigned long long bad = 0;
   CK(cudaMemcpyAsync(&bad, d_small, 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  m.release(ukey, 8ull * n_e); m.release(uidx, 8ull * n_e);
-  if (bad) { m.release(d_e, 12ull * n_e); m.release(ukey2, 8ull * n_e); m.release(uidx2, 8ull * n_e);
-             m.release(tmp, tbmax); m.release(d_small, 64);
-             return set_err(CSM_EINVAL, "%llu edges touch a vertex id without a label line", bad); }
-  AL(dkey, 8ull * std::max<uint64_t>(M, 1)); AL(dkey2, 8ull * std::max<uint64_t>(M, 1));
+  if (bad) {
+    m.release(early, blk1.total);
+    m.release(late, blk2.total);
+    return set_err(CSM_EINVAL, "%llu edges touch a vertex id without a label line", bad);
+  }
   if (n_e) { k_load_directed<<<blocks_for(n_e, 256), 256, 0, st>>>(ukey2, uidx2, n_e, d_e, g, dkey); CKL(); }
-  m.release(ukey2, 8ull * n_e); m.release(uidx2, 8ull * n_e); m.release(d_e, 12ull * n_e);
   if (M) {
     tb = tbmax;
     CK(cub::DeviceRadixSort::SortKeys(tmp, tb, dkey, dkey2, (int64_t)M, 0, (int)kb.total(), st));
   }
-  m.release(dkey, 8ull * std::max<uint64_t>(M, 1));
-  AL(first, 8ull * n_cap); AL(cap64, 8ull * n_cap); AL(off64, 8ull * n_cap); AL(cap32, 4ull * n_cap);
   if (M) { k_load_count<<<blocks_for(M, 256), 256, 0, st>>>(dkey2, M, kb, (uint32_t)nc, g.dir, first, d_small + 1); CKL(); }
   k_dir_scan<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc); CKL();
   k_load_caps<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc, cap32, cap64); CKL();
@@ -1567,10 +1634,13 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   CK(cudaStreamSynchronize(st));
   const uint64_t used = last_off + last_cap;
   const uint64_t pool_cap = 2 * used + 16ull * ctx->bmax + (1ull << 20);  // a multiple of four, as every row's capacity
-  if (pool_cap >= (1ull << 32)) return set_err(CSM_EUNSUPPORTED, "graph too large for 32-bit pool offsets");
+  m.release(early, blk1.total);  // before the pools: they are the peak
+  auto fail = [&](int code) { m.release(late, blk2.total); return code; };
+  if (pool_cap >= (1ull << 32)) return fail(set_err(CSM_EUNSUPPORTED, "graph too large for 32-bit pool offsets"));
   g.pool_cap = pool_cap;
-  AL(g.pools[0], 4ull * pool_cap);
-  AL(g.pools[1], 4ull * pool_cap);
+  rc = m.alloc((void**)&g.pools[0], 4ull * pool_cap);
+  if (!rc) rc = m.alloc((void**)&g.pools[1], 4ull * pool_cap);
+  if (rc) return fail(rc);
   // row tables: two slots per row slot.  Without room for them, or when an id
   // and a folded edge label do not fit in 31 bits, the search joins by binary
   // search in the rows instead
@@ -1594,10 +1664,7 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   CK(cudaMemcpyAsync(g.ps, &ps, sizeof(ps), cudaMemcpyHostToDevice, st));
   if (M) { k_load_scatter<<<blocks_for(M, 256), 256, 0, st>>>(dkey2, M, first, g, g.pools[0]); CKL(); }
   CK(cudaStreamSynchronize(st));
-  m.release(dkey2, 8ull * std::max<uint64_t>(M, 1)); m.release(first, 8ull * n_cap); m.release(cap64, 8ull * n_cap);
-  m.release(off64, 8ull * n_cap); m.release(cap32, 4ull * n_cap);
-  m.release(tmp, tbmax); m.release(d_small, 64);
-#undef AL
+  m.release(late, blk2.total);
   ctx->num_edges = n_valid / 2;
   ctx->has_graph = true;
   return CSM_OK;
@@ -1877,6 +1944,7 @@ void csm_gpu_destroy(csm_ctx* ctx) {
   index_free(ctx->index, ctx->mem);
   ctx->mem.free_all();
   for (auto& e : ctx->sev) { cudaEventDestroy(e.first); cudaEventDestroy(e.second); }
+  if (ctx->pin) cudaFreeHost(ctx->pin);
   if (ctx->ev_start) cudaEventDestroy(ctx->ev_start);
   if (ctx->ev_end) cudaEventDestroy(ctx->ev_end);
   if (ctx->st) cudaStreamDestroy(ctx->st);

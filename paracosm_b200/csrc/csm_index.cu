@@ -342,10 +342,6 @@ namespace {
 // marks fewer vertices (a list that overflows is worked off from its marks).
 constexpr uint32_t kListCap = 32768;
 
-size_t list_bytes(const IndexState& ix) {
-  return 4ull * 2 * ix.h_dag.nq * ix.bits.list_cap + 8ull * ix.h_dag.nq;
-}
-
 // Root choice (ParaCOSM/CSM/matching/SymBi/symbi.cpp:116-195, identical in
 // TurboFlux/turboflux.cpp:82-149): the first query edge (u < u', adjacency
 // order) of least frequency; of its endpoints the one whose label is rarer in
@@ -401,10 +397,12 @@ static int dag_for(const IndexQuery& q, const DevGraph& g, int algo,
   }
   uint32_t* d_e = nullptr;
   unsigned long long* d_f = nullptr;
-  int rc = mem.alloc((void**)&d_e, 12ull * ne);
+  DevBlock blk;
+  blk.add(d_e, 12ull * ne);
+  blk.add(d_f, 8ull * (ne + kMaxQ + 1));
+  void* tmp = nullptr;
+  const int rc = blk.alloc(mem, &tmp);
   if (rc) return rc;
-  rc = mem.alloc((void**)&d_f, 8ull * (ne + kMaxQ + 1));
-  if (rc) { mem.release(d_e, 12ull * ne); return rc; }
   IXCK(cudaMemcpyAsync(d_e, h_eu.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
   IXCK(cudaMemcpyAsync(d_e + ne, h_ec.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
   IXCK(cudaMemcpyAsync(d_e + 2 * ne, h_el.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
@@ -415,8 +413,7 @@ static int dag_for(const IndexQuery& q, const DevGraph& g, int algo,
   std::vector<unsigned long long> freq(ne + kMaxQ + 1);
   IXCK(cudaMemcpyAsync(freq.data(), d_f, 8ull * (ne + kMaxQ + 1), cudaMemcpyDeviceToHost, st));
   IXCK(cudaStreamSynchronize(st));
-  mem.release(d_e, 12ull * ne);
-  mem.release(d_f, 8ull * (ne + kMaxQ + 1));
+  mem.release(tmp, blk.total);
   std::vector<unsigned long long> lcount(freq.begin() + ne, freq.end());
   freq.resize(ne);
   root = choose_root(q, edges, freq, lcount);
@@ -552,19 +549,19 @@ static int index_finish(IndexState& ix, DevMem& mem, const DevGraph& g, const In
   ix.words = (ix.words + 3) & ~3ull;
   const uint64_t fam = 8ull * nq * ix.words;
   ix.bits.list_cap = std::min<uint32_t>(g.n_cap, kListCap);
-  rc = mem.alloc((void**)&ix.bits.d1, 4 * fam);
+  ix.bits.words = ix.words;
+  DevBlock blk;
+  blk.add(ix.bits.d1, 4 * fam);
+  blk.add(ix.d_dag, sizeof(IxDag));
+  blk.add(ix.d_pop, 16);
+  blk.add(ix.bits.list, 4ull * 2 * nq * ix.bits.list_cap);
+  blk.add(ix.bits.count, 8ull * nq);
+  rc = blk.alloc(mem, &ix.block);
   if (rc) return rc;
+  ix.block_bytes = blk.total;
   ix.bits.d2 = ix.bits.d1 + nq * ix.words;
   ix.bits.m1 = ix.bits.d2 + nq * ix.words;
   ix.bits.m2 = ix.bits.m1 + nq * ix.words;
-  ix.bits.words = ix.words;
-  rc = mem.alloc((void**)&ix.d_dag, sizeof(IxDag));
-  if (rc) return rc;
-  rc = mem.alloc((void**)&ix.d_pop, 16);
-  if (rc) return rc;
-  rc = mem.alloc((void**)&ix.bits.list, list_bytes(ix));
-  if (rc) return rc;
-  ix.bits.count = ix.bits.list + (size_t)2 * nq * ix.bits.list_cap;
   IXCK(cudaMemsetAsync(ix.bits.count, 0, 8ull * nq, st));
   IXCK(cudaMemsetAsync(ix.bits.d1, 0, 4 * fam, st));
   IXCK(cudaMemcpyAsync(ix.d_dag, &D, sizeof(IxDag), cudaMemcpyHostToDevice, st));
@@ -667,10 +664,8 @@ void index_stats(const IndexState& ix, uint64_t* entries, uint64_t* vertices) {
 }
 
 void index_free(IndexState& ix, DevMem& mem) {
-  if (ix.bits.d1) mem.release(ix.bits.d1, 4 * 8ull * ix.h_dag.nq * ix.words);
-  if (ix.d_dag) mem.release(ix.d_dag, sizeof(IxDag));
-  if (ix.d_pop) mem.release(ix.d_pop, 16);
-  if (ix.bits.list) mem.release(ix.bits.list, list_bytes(ix));
+  if (ix.block) mem.release(ix.block, ix.block_bytes);
+  ix.block = nullptr;
   ix.bits = IxBits{};
   ix.d_dag = nullptr;
   ix.d_pop = nullptr;

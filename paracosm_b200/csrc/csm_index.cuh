@@ -102,6 +102,8 @@ struct IndexState {
   IxDag h_dag{};
   IxDag* d_dag = nullptr;
   uint64_t* d_pop = nullptr;  // popcount scratch
+  void* block = nullptr;      // the one allocation behind bits, d_dag and d_pop
+  size_t block_bytes = 0;
   uint32_t root = 0;
   std::vector<uint32_t> order;
   IxOrder rounds{};

@@ -106,24 +106,24 @@ __global__ void k_load_directed(const uint64_t* ukey, const uint64_t* uidx, uint
   dkey[2 * j + 1] = kb.pack(y, vlabel[x] * n_el + l, x);
 }
 
-// Per (vertex, combo) run lengths (into dir, scanned later) and the first
-// position of each vertex in the sorted keys.
+// Per (vertex, combo) run lengths (into dir, cleared before and scanned later)
+// and the first position of each vertex in the sorted keys.  A run's first
+// entry subtracts its place and its last adds the place after it (modulo
+// 2^32): no thread walks a run (a hub's runs are long: 518 us on 2^19
+// vertices and 4.2M edges).
 __global__ void k_load_count(const uint64_t* dkey, uint64_t M, KeyBits kb, uint32_t nc, uint32_t* dir,
                              uint64_t* first, unsigned long long* n_valid) {
   uint64_t j = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= M) return;
   const uint64_t k = dkey[j];
   if (!kb.real(k)) return;
-  const uint32_t x = kb.x_of(k), c = kb.c_of(k);
-  if ((j + 1 == M) || !kb.real(dkey[j + 1])) *n_valid = j + 1;
-  const bool head_x = (j == 0) || kb.x_of(dkey[j - 1]) != x;
-  if (head_x) first[x] = j;
-  const bool head_c = head_x || kb.c_of(dkey[j - 1]) != c;
-  if (head_c) {
-    uint64_t t = j;  // walk to the end of this (x, c) run
-    while (t + 1 < M && kb.real(dkey[t + 1]) && kb.x_of(dkey[t + 1]) == x && kb.c_of(dkey[t + 1]) == c) t++;
-    dir[(size_t)x * (nc + 1) + c] = (uint32_t)(t - j + 1);
-  }
+  const uint64_t before = j ? dkey[j - 1] : ~0ULL, after = j + 1 < M ? dkey[j + 1] : ~0ULL;
+  if (!kb.real(after)) *n_valid = j + 1;
+  const uint32_t x = kb.x_of(k);
+  uint32_t* run = dir + (size_t)x * (nc + 1) + kb.c_of(k);
+  if (j == 0 || kb.x_of(before) != x) first[x] = j;
+  if (j == 0 || (before >> kb.yb) != (k >> kb.yb)) atomicSub(run, (uint32_t)j);
+  if (!kb.real(after) || (after >> kb.yb) != (k >> kb.yb)) atomicAdd(run, (uint32_t)(j + 1));
 }
 
 __device__ __forceinline__ uint32_t slack_cap(uint32_t d) { return d == 0 ? 0u : row_round(d + max(2u, d >> 2)); }
@@ -730,8 +730,13 @@ void launch_mut_delete(const VRange* ranges, const unsigned int* n_ranges, const
 // trying them in turn took 5.4 us).
 __global__ void k_plain_resolve(const csm_update* up, DevGraph g, UpdInfo* info, uint64_t* keys, unsigned int* cnt,
                                 unsigned long long* count, unsigned long long* hash, unsigned long long* bytes,
-                                unsigned int* stop) {
+                                unsigned int* stop, unsigned long long* stamp) {
   const uint32_t lane = threadIdx.x;
+  if (stamp && lane == 0) {
+    unsigned long long now;
+    asm volatile("mov.u64 %0, %%globaltimer;" : "=l"(now));
+    stamp[0] = now;
+  }
   const csm_update u = *up;
   PoolState* ps = g.ps;
   const bool ids = u.type == 'e' && u.id1 < g.n && u.id2 < g.n && u.id1 != u.id2;

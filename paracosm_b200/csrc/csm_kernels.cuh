@@ -59,10 +59,11 @@ __global__ void k_vdel_keys(DevGraph g, uint32_t v, uint32_t deg, uint64_t* keys
 
 // ---- one edge update per launch sequence (the plain form; csm_kernels.cu) ----
 // keys[0..1]: the update's two directed entries (sentinels when the graph does
-// not change); cnt[0..15], count/hash/bytes/stop[0]: cleared for the search.
+// not change); cnt[0..15], count/hash/bytes/stop[0]: cleared for the search;
+// stamp[0] (unless null): the time.
 __global__ void k_plain_resolve(const csm_update* up, DevGraph g, UpdInfo* info, uint64_t* keys, unsigned int* cnt,
                                 unsigned long long* count, unsigned long long* hash, unsigned long long* bytes,
-                                unsigned int* stop);
+                                unsigned int* stop, unsigned long long* stamp);
 // Applies the update's row insertion or deletion (two 256-thread blocks); with
 // `out`, also writes the result of an update that needs no search (latency
 // from stamp[0]).

@@ -42,6 +42,7 @@ struct LevelSM {
   uint8_t par[32];    // entry index in the previous level
   uint8_t dsel[32];   // back entry that is the driver (kSelTouched: its row has touched entries)
   uint8_t jsel[32];   // back entry of the first join: the smallest segment but the driver's
+  uint8_t jel[32];    // its edge label
   uint32_t cnt, cur, total, pad;
 };
 
@@ -683,11 +684,13 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
   uint32_t iter = 0;
   constexpr bool EN = MODE == 1;
   const int tail_level = (MODE == 2 && p.tail && p.plan->anchors[T.anchor].tail_at) ? (int)p.plan->anchors[T.anchor].tail_at : -1;
-  uint32_t seen_stop = 0, seen_hungry = 0;  // flags loaded at the previous check
+  uint32_t seen_stop = 0, seen_hungry = 0;  // lane 0: flags loaded at the last check
+  uint32_t hungry = 0;                      // idle warps seen
   const uint32_t every = p.donate_every ? p.donate_every : 1u;  // steps between hand-over checks (a power of two)
   bool enter = true;
   uint32_t cur = 0, total = 0, my_incl = 0, qv = 0, held = 0;
   bool joins = false;
+  const uint64_t* filter = nullptr;  // candidate filter of the level's next position
   // the pair of this lane at cur, loaded a step ahead: entry, candidate, and
   // the row of the entry's first join; `fresh` when they are cur's
   bool fresh = false;
@@ -695,22 +698,20 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
   uint2 jrow = make_uint2(0, 0);
   auto fetch = [&](uint32_t c) {
     const uint32_t at = c + lane;
-    own = __popc(__ballot_sync(0xffffffffu, my_incl <= c));
-    if (__popc(__ballot_sync(0xffffffffu, my_incl <= c + 31u)) != (int)own) {
-      // the pairs span several entries: the first whose end lies beyond `at`
-      own = 0;
-#pragma unroll
-      for (uint32_t step = 16; step; step >>= 1) {
-        const uint32_t v = __shfl_sync(0xffffffffu, my_incl, own + step - 1);
-        if (v <= at) own += step;
-      }
-    }
+    // bit i of `ends`: an entry ends before the pair of lane i
+    const uint32_t end = my_incl - c;
+    const uint32_t ends = __reduce_or_sync(0xffffffffu, end - 1u < 31u ? 1u << end : 0u);
+    own = __popc(__ballot_sync(0xffffffffu, my_incl <= c)) + __popc(ends & (0xffffffffu >> (31u - lane)));
     if (at < total) {
       const LevelSM& L = lv[d];
       x = ld_stream(pool + (L.base[own] + at));
       if (joins) jrow = g.row[L.jv[own]];
     }
   };
+  // a single update's own range is handed over at once, while every other warp
+  // waits (its calls take 4 to 8 % less; in batches it only breaks up work)
+  if (lane == 0 && p.dq && p.batch == 1 && lv[d].total > 32u)
+    seen_hungry = (uint32_t)max((int)*(volatile unsigned int*)&p.q->hungry, 0);
   for (;;) {
     if (enter) {
       // the level's cursor and segment ends (lane e: entry e's)
@@ -719,6 +720,7 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
       total = L.total;
       my_incl = lane < L.cnt ? L.incl[lane] : 0xffffffffu;
       qv = wp.qv((uint32_t)d + 1u);
+      filter = p.d2 ? p.d2 + (uint64_t)qv * p.d2_words : nullptr;
       joins = wp.nb((uint32_t)d + 1u) > 1 && g.htab != nullptr;
       enter = false;
       fresh = false;
@@ -749,25 +751,22 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
       }
       if (__shfl_sync(0xffffffffu, quit, 0)) break;
     }
-    if ((iter & (every - 1)) == 0 && p.dq) {
-      const uint32_t idle_now = __shfl_sync(0xffffffffu, seen_hungry, 0);
-      if (idle_now) {
-        if (lane == 0) { lv[d].cur = cur; ws.hungry++; }
-        __syncwarp();
-        donate(p, lv, d, lane, idle_now, t, T.anchor, T.orient, tail_level);
-        total = lv[d].total;
-        if (lane >= lv[d].cnt) my_incl = 0xffffffffu;
-      }
-    }
     // the stop flag and the idle-warp count are loaded every fourth step, each
-    // a round trip to a line other warps update, and looked at later, so that
-    // the trip overlaps the steps between; lane 0's view decides for the warp
-    if ((iter & 3) == 0) {
+    // a round trip to a line other warps update, and looked at a step later, so
+    // that the trip overlaps a step; lane 0's view decides for the warp
+    if ((iter & 3) == 1) {
       if (__shfl_sync(0xffffffffu, seen_stop, 0)) break;
-      if (lane == 0) {
-        seen_stop = stop[t];
-        seen_hungry = p.dq ? (uint32_t)max((int)*(volatile unsigned int*)&p.q->hungry, 0) : 0u;
-      }
+      hungry = __shfl_sync(0xffffffffu, seen_hungry, 0);
+    } else if ((iter & 3) == 0 && lane == 0) {
+      seen_stop = stop[t];
+      seen_hungry = p.dq ? (uint32_t)max((int)*(volatile unsigned int*)&p.q->hungry, 0) : 0u;
+    }
+    if (hungry && (iter & (every - 1)) == 0) {
+      if (lane == 0) { lv[d].cur = cur; ws.hungry++; }
+      __syncwarp();
+      donate(p, lv, d, lane, hungry, t, T.anchor, T.orient, tail_level);
+      total = lv[d].total;
+      if (lane >= lv[d].cnt) my_incl = 0xffffffffu;
     }
     if constexpr (MODE == 2) {
       if (d == tail_level) {
@@ -805,24 +804,30 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
     uint32_t meta = own;
     bool valid = cur + lane < total;
     if (valid && joins) {
-      const uint32_t el = back_el(wp.back(pos, lv[d].jsel[own]));
-      const uint32_t hit = row_find(g, jrow, row_entry(cx, el, g.hlb));
+      const uint32_t hit = row_find(g, jrow, row_entry(cx, lv[d].jel[own], g.hlb));
       valid = hit != kSlotEmpty;
       meta |= (hit & kSlotTouched) >> 15;
     }
     fresh = cur + 32u < total;
     if (fresh) fetch(cur + 32u);
-    if (valid) valid = filter_bit(p, qv, cx);
+    if (valid && filter) valid = (ld_gather(filter + (cx >> 6)) >> (cx & 63u)) & 1ULL;
     // the candidates left wait until 32 of them, or all of the level's, are
     // together; a step that finds more than there is room for ends before the
     // first of those
     const uint32_t found = __ballot_sync(0xffffffffu, valid);
+    if (found == 0 && (held == 0 || cur + 32u < total)) {
+      cur += 32u;
+      continue;
+    }
     const uint32_t rank = held + __popc(found & ((1u << lane) - 1u));
-    const uint32_t over = __ballot_sync(0xffffffffu, valid && rank >= 32u);
     if (valid && rank < 32u) wait[rank] = make_uint2(cx, meta);
-    cur += over ? (uint32_t)__ffs((int)over) - 1u : 32u;
-    fresh = fresh && !over;
-    held = over ? 32u : held + __popc(found);
+    held += __popc(found);
+    cur += 32u;
+    if (held > 32u) {
+      cur += (uint32_t)__ffs((int)__ballot_sync(0xffffffffu, valid && rank >= 32u)) - 33u;
+      held = 32u;
+      fresh = false;
+    }
     if (held == 0 || (held < 32u && cur < total)) continue;
     __syncwarp();
     // injectivity, remaining joins, presence, next driver
@@ -884,7 +889,7 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
       if (valid) {
         const uint32_t slot = __popc(mask & ((1u << lane) - 1u));
         N.v[slot] = wx; N.par[slot] = (uint8_t)wown; N.dsel[slot] = (uint8_t)ndsel;
-        N.jsel[slot] = (uint8_t)njsel; N.jv[slot] = njv;
+        N.jsel[slot] = (uint8_t)njsel; N.jel[slot] = (uint8_t)back_el(wp.back(pos + 1, njsel)); N.jv[slot] = njv;
         N.incl[slot] = incl; N.base[slot] = ndlo - (incl - mine);
       }
       if (lane == 31) { N.cnt = __popc(mask); N.cur = 0; N.total = incl; lv[d].cur = cur; }
@@ -924,17 +929,21 @@ __device__ __forceinline__ uint32_t same_mask(const SearchParams& p, const PlanA
 
 // Root task: positions 0 and 1 are the updated edge; level 1 holds the driver
 // segment of position 2.  Returns false when there is nothing to walk.
+struct RootOut {
+  unsigned long long cnt, hash, bytes;  // of the whole (two-vertex) query; bytes of the first node
+  bool walk;
+};
 template <int MODE>
-__device__ __forceinline__ bool setup_root(const SearchParams& p, LevelSM* lv, uint32_t* plan_words, uint32_t n,
-                                           uint32_t lane, const Task& T, TaskAcc& acc) {
-  const uint32_t t = T.upd;
-  const PlanAnchor* A = &p.plan->anchors[T.anchor];
+__device__ __noinline__ RootOut setup_root(const SearchParams& p, LevelSM* lv, uint32_t* plan_words, uint32_t n,
+                                           uint32_t lane, uint32_t t, uint32_t anchor, uint32_t orient) {
+  RootOut out{0, 0, 0, false};
+  const PlanAnchor* A = &p.plan->anchors[anchor];
   const UpdInfo U = p.info[t];
-  const uint32_t m0 = T.orient ? U.v2 : U.v1, m1 = T.orient ? U.v1 : U.v2;
+  const uint32_t m0 = orient ? U.v2 : U.v1, m1 = orient ? U.v1 : U.v2;
   if (n == 2) {
-    acc.cnt += 1;
+    out.cnt = 1;
     if (lane == 0) {
-      if (p.want_hash) acc.hash += mix64(pair_hash(A->pos[0].qv, m0) + pair_hash(A->pos[1].qv, m1));
+      if (p.want_hash) out.hash = mix64(pair_hash(A->pos[0].qv, m0) + pair_hash(A->pos[1].qv, m1));
       if (MODE == 1) {
         const unsigned long long r = atomicAdd(p.enum_n, 1ull);
         if (r < p.enum_cap) {
@@ -945,7 +954,7 @@ __device__ __forceinline__ bool setup_root(const SearchParams& p, LevelSM* lv, u
         }
       }
     }
-    return false;
+    return out;
   }
   const PlanPos P2 = A->pos[2];
   uint32_t sz = 0xffffffffu, szt = 1, touched = 0;
@@ -957,9 +966,9 @@ __device__ __forceinline__ bool setup_root(const SearchParams& p, LevelSM* lv, u
     sz = (uint32_t)(hi - lo);
     touched = p.g.t_count[v];
     szt = seg_size_slow(p, v, c, (uint32_t)lo, (uint32_t)hi, (int32_t)t);
-    acc.bytes += 4ull * szt;
+    out.bytes = 4ull * szt;
   }
-  if (__any_sync(0xffffffffu, szt == 0)) return false;
+  if (__any_sync(0xffffffffu, szt == 0)) return out;
   uint64_t key = ((uint64_t)sz << 32) | lane;
 #pragma unroll
   for (int o = 16; o; o >>= 1) {
@@ -976,18 +985,24 @@ __device__ __forceinline__ bool setup_root(const SearchParams& p, LevelSM* lv, u
     lv[1].dsel[0] = (uint8_t)(sel | (touched ? kSelTouched : 0u));
     lv[1].v[0] = m1; lv[1].par[0] = 1; lv[1].v[1] = m0;
     lv[1].jsel[0] = (uint8_t)other;
+    lv[1].jel[0] = P2.nb > 1 ? A->back_el[P2.boff + other] : 0;
     lv[1].jv[0] = P2.nb > 1 ? (A->back_pos[P2.boff + other] == 0 ? m0 : m1) : 0u;
   }
   load_walk_plan(plan_words, A, n, same_mask(p, A), lane);
-  return true;
+  out.walk = true;
+  return out;
 }
 
 // Donated task: rebuild the chain of the partial match (exhausted levels
 // 1 .. depth-1) and continue from level `depth`.  `hw` holds record words
 // 0..4 in lanes 0..4 and `mv` holds m[lane] (see DTask).  Returns the level
 // to start from, 0 when there is nothing to walk.
-__device__ __forceinline__ int setup_donated(const SearchParams& p, LevelSM* lv, uint32_t* plan_words, uint32_t n,
-                                             uint32_t lane, uint32_t hw, uint32_t mv, Task& T,
+struct DonatedOut {
+  Task task;
+  int depth;  // level to start from; 0: nothing to walk
+};
+__device__ __noinline__ DonatedOut setup_donated(const SearchParams& p, LevelSM* lv, uint32_t* plan_words, uint32_t n,
+                                             uint32_t lane, uint32_t hw, uint32_t mv,
                                              unsigned long long ticket, unsigned long long seen_seq) {
   const uint32_t upd = __shfl_sync(0xffffffffu, hw, 0);
   const uint32_t w1 = __shfl_sync(0xffffffffu, hw, 1);
@@ -995,8 +1010,8 @@ __device__ __forceinline__ int setup_donated(const SearchParams& p, LevelSM* lv,
   const uint32_t dn = __shfl_sync(0xffffffffu, hw, 3);
   const uint32_t w4 = __shfl_sync(0xffffffffu, hw, 4), dsel = w4 & 0xffu;
   const uint32_t anchor = w1 & 0xffffu, orient = (w1 >> 16) & 0xffu, depth = w1 >> 24;
-  T = Task{upd, (uint16_t)anchor, (uint8_t)orient, 0};
-  if (upd == 0xffffffffu) return 0;  // void record (its donor flagged an error)
+  DonatedOut out{Task{upd, (uint16_t)anchor, (uint8_t)orient, 0}, 0};
+  if (upd == 0xffffffffu) return out;  // void record (its donor flagged an error)
   if (upd >= p.batch || anchor >= p.plan->n_anchor || depth < 1 || depth + 2 > n || depth > p.levels || dn == 0 ||
       (unsigned long long)dlo + dn > p.g.pool_cap) {
     if (lane == 0) {
@@ -1007,12 +1022,12 @@ __device__ __forceinline__ int setup_donated(const SearchParams& p, LevelSM* lv,
         p.sstat->bad_words[3] = dn; p.sstat->bad_words[4] = w4;
       }
     }
-    T.upd = 0xffffffffu;
-    return 0;
+    out.task.upd = 0xffffffffu;
+    return out;
   }
   const unsigned int stopped =
       __shfl_sync(0xffffffffu, lane == 0 ? *(volatile unsigned int*)(p.stop + upd) : 0u, 0);
-  if (stopped) return 0;
+  if (stopped) return out;
   const PlanAnchor* A = &p.plan->anchors[anchor];
   const uint32_t jsel = w4 >> 8;
   const PlanPos N = A->pos[depth + 1];
@@ -1022,11 +1037,12 @@ __device__ __forceinline__ int setup_donated(const SearchParams& p, LevelSM* lv,
     S.cnt = 1; S.cur = 0; S.v[0] = mv; S.par[0] = lane == 1 ? 1 : 0;
     S.total = lane < depth ? 0u : dn;
     S.incl[0] = dn; S.base[0] = dlo; S.dsel[0] = (uint8_t)dsel;
-    S.jsel[0] = (uint8_t)jsel; S.jv[0] = jv;
+    S.jsel[0] = (uint8_t)jsel; S.jel[0] = A->back_el[N.boff + min(jsel, N.nb - 1u)]; S.jv[0] = jv;
   }
   if (lane == 0) lv[1].v[1] = mv;
   load_walk_plan(plan_words, A, n, same_mask(p, A), lane);
-  return (int)depth;
+  out.depth = (int)depth;
+  return out;
 }
 
 // Kernel body; MODE 0 counts (and hashes), 1 also appends match sets, 2
@@ -1072,7 +1088,11 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
         atomicCAS(const_cast<unsigned int*>(stop) + T.upd, 0u, kStopDeadline);
       // stop flags change under our feet: one lane reads, the warp follows it
       const unsigned int stopped = __shfl_sync(0xffffffffu, lane == 0 ? stop[T.upd] : 0u, 0);
-      if (!stopped) d = setup_root<MODE>(p, lv, plan_words, n, lane, T, acc) ? 1 : 0;
+      if (!stopped) {
+        const RootOut r = setup_root<MODE>(p, lv, plan_words, n, lane, T.upd, T.anchor, T.orient);
+        acc.cnt = r.cnt; acc.hash = r.hash; acc.bytes = r.bytes;
+        d = r.walk ? 1 : 0;
+      }
     } else {
       // 2. donated tasks until every task is done.  The queue is a bounded ring
       // of DTask slots with per-slot sequence numbers: slot (ticket % qcap) holds
@@ -1119,7 +1139,9 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
       const uint32_t mv = Dw[5 + lane];
       __syncwarp();
       tb = global_ns();
-      d = setup_donated(p, lv, plan_words, n, lane, hw, mv, T, claimed, seen);
+      const DonatedOut r = setup_donated(p, lv, plan_words, n, lane, hw, mv, claimed, seen);
+      T = r.task;
+      d = r.depth;
     }
     if (lane == 0) ws.began = tb;
     if (d > 0) run_levels<MODE>(p, pool, lv, wp, waiting[warp], d, lane, T, ws, acc);

@@ -87,8 +87,8 @@ struct csm_ctx {
   uint64_t *d_ukey = nullptr, *d_ukey2 = nullptr;
   uint32_t *d_useq = nullptr, *d_useq2 = nullptr;
   UpdInfo* d_info = nullptr;
-  uint64_t *d_ins = nullptr, *d_ins2 = nullptr, *d_del = nullptr, *d_del2 = nullptr;
-  uint64_t *d_tk = nullptr, *d_tk2 = nullptr, *d_ts = nullptr, *d_ts2 = nullptr;
+  uint64_t *d_lists = nullptr;  // insert, delete and temporal keys as emitted; *2: sorted
+  uint64_t *d_ins2 = nullptr, *d_del2 = nullptr, *d_tk2 = nullptr, *d_ts = nullptr, *d_ts2 = nullptr;
   VRange *d_rins = nullptr, *d_rdel = nullptr;
   uint32_t* d_ins_dst = nullptr;
   unsigned int* d_cnt = nullptr;  // [0] n_ins [1] n_del [2] n_t [3] n_rins [4] n_rdel [6] n_tasks [7] task_next [8] search blocks ended
@@ -289,6 +289,12 @@ static int build_plan(csm_ctx* ctx) {
 
 // --------------------------------------------------------- batch buffers
 
+// Slots of a batch's lists of directed entries: an edge's updates give rise to
+// at most as many row insertions, row deletions and presence intervals each
+// (an inserted label, a label that leaves and an interval's end take an update
+// of their own), in both directions.
+static uint32_t list_slots(uint32_t B) { return 2 * B + 64; }
+
 // Empty hand-over ring: slot i is free for ticket i.
 __global__ void k_ring_init(SearchQueue* q, unsigned long long* seq, uint32_t qcap) {
   if (blockIdx.x == 0 && threadIdx.x == 0) *q = SearchQueue{};
@@ -298,7 +304,7 @@ __global__ void k_ring_init(SearchQueue* q, unsigned long long* seq, uint32_t qc
 static int ensure_batch_buffers(csm_ctx* ctx) {
   if (ctx->d_ukey) return CSM_OK;
   const uint32_t B = ctx->bmax;
-  const uint32_t L = 4 * B + 64;
+  const uint32_t L = list_slots(B);
   ctx->lcap = L;
   const uint32_t na = std::max<uint32_t>(1, (uint32_t)(ctx->qe.size() / 3));
   ctx->task_cap = B * 2 * na;
@@ -318,9 +324,8 @@ static int ensure_batch_buffers(csm_ctx* ctx) {
   AL(ctx->d_ukey, 8ull * B); AL(ctx->d_ukey2, 8ull * B);
   AL(ctx->d_useq, 4ull * B); AL(ctx->d_useq2, 4ull * B);
   AL(ctx->d_info, sizeof(UpdInfo) * (size_t)B);
-  AL(ctx->d_ins, 8ull * L); AL(ctx->d_ins2, 8ull * L);
-  AL(ctx->d_del, 8ull * L); AL(ctx->d_del2, 8ull * L);
-  AL(ctx->d_tk, 8ull * L); AL(ctx->d_tk2, 8ull * L);
+  AL(ctx->d_lists, 24ull * L);
+  AL(ctx->d_ins2, 8ull * L); AL(ctx->d_del2, 8ull * L); AL(ctx->d_tk2, 8ull * L);
   AL(ctx->d_ts, 8ull * L); AL(ctx->d_ts2, 8ull * L);
   AL(ctx->d_rins, sizeof(VRange) * (size_t)L); AL(ctx->d_rdel, sizeof(VRange) * (size_t)L);
   AL(ctx->d_ins_dst, 4ull * L);
@@ -401,23 +406,22 @@ static int batch_mutate_insert(csm_ctx* ctx, const csm_update* ups, uint32_t B, 
   cudaStream_t st = ctx->st;
   DevGraph& g = ctx->g;
   const KeyBits kb = g.kb;
-  CK(cudaMemsetAsync(ctx->d_cnt, 0, 64, st));
-  CK(cudaMemsetAsync(ctx->d_ins, 0xff, 8ull * L, st));
-  CK(cudaMemsetAsync(ctx->d_del, 0xff, 8ull * L, st));
-  CK(cudaMemsetAsync(ctx->d_tk, 0xff, 8ull * L, st));
+  // the three lists, one after another, all unused slots
+  uint64_t *ins = ctx->d_lists, *del = ins + L, *tk = del + L;
+  CK(cudaMemsetAsync(ins, 0xff, 24ull * L, st));
   unsigned int* c = ctx->d_cnt;
-  k_batch_init<<<blocks_for(B, 256), 256, 0, st>>>(ups, B, g, ctx->d_ukey, ctx->d_useq, ctx->d_info); CKL();
+  k_batch_init<<<blocks_for(B, 256), 256, 0, st>>>(ups, B, g, ctx->d_ukey, ctx->d_useq, ctx->d_info, c); CKL();
   size_t tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, ctx->d_ukey, ctx->d_ukey2, ctx->d_useq, ctx->d_useq2, (int)B, 0, 64, st));
-  ResolveOut ro{ctx->d_ins, c + 0, ctx->d_del, c + 1, ctx->d_tk, ctx->d_ts, c + 2, L};
+  CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, ctx->d_ukey, ctx->d_ukey2, ctx->d_useq, ctx->d_useq2, (int)B, 0, (int)(2 * kb.yb), st));
+  ResolveOut ro{ins, c + 0, del, c + 1, tk, ctx->d_ts, c + 2, L};
   k_resolve<<<blocks_for(B, 128), 128, 0, st>>>(ctx->d_ukey2, ctx->d_useq2, B, g, ups, ctx->d_info, ro); CKL();
   const int end_bit = (int)kb.total();
   tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, ctx->d_ins, ctx->d_ins2, (int)L, 0, end_bit, st));
+  CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, ins, ctx->d_ins2, (int)L, 0, end_bit, st));
   tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, ctx->d_del, ctx->d_del2, (int)L, 0, end_bit, st));
+  CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, del, ctx->d_del2, (int)L, 0, end_bit, st));
   tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, ctx->d_tk, ctx->d_tk2, ctx->d_ts, ctx->d_ts2, (int)L, 0, end_bit, st));
+  CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, tk, ctx->d_tk2, ctx->d_ts, ctx->d_ts2, (int)L, 0, end_bit, st));
   k_ranges<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_ins2, L, kb, ctx->d_rins, c + 3, g.dir, g.nc); CKL();
   k_ranges<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_del2, L, kb, ctx->d_rdel, c + 4, g.dir, g.nc); CKL();
   g.t_key = ctx->d_tk2;
@@ -474,10 +478,6 @@ static int batch_query_search(csm_ctx* q, csm_ctx* o, uint32_t B, uint32_t L, cs
   csm_ctx* ctx = q;  // launches are counted on the query's context
   cudaStream_t st = q->st;
   const DevGraph& g = o->g;
-  CK(cudaMemsetAsync(q->d_count, 0, 8ull * B, st));
-  CK(cudaMemsetAsync(q->d_bytes, 0, 8ull * B, st));
-  CK(cudaMemsetAsync(q->d_stop, 0, 4ull * B, st));
-  if (q->cfg.want_hash) CK(cudaMemsetAsync(q->d_hash, 0, 8ull * B, st));
   unsigned int* c = q->d_cnt;
   if (q != o) CK(cudaMemsetAsync(c, 0, 64, st));
   int rc = index_apply_edges(q->index, g, o->d_ins2, L, st, &q->launches);
@@ -495,6 +495,7 @@ static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out
   const bool one = B == 1;  // the seeds' one warp prepares the search's queue too
   k_seed<<<blocks_for(B, 4), one ? 32 : 128, 0, st>>>(B, o->d_info, g, q->d_plan, q->index.d2, q->index.words,
                                                       q->d_tasks, c + 6, q->task_cap, q->d_safe, &g.ps->error,
+                                                      Counters{q->d_count, q->d_hash, q->d_bytes, q->d_stop},
                                                       q->cfg.shard_rank, q->cfg.shard_count,
                                                       (uint32_t)q->cfg.turboflux_compat,
                                                       q->cfg.algorithm == CSM_ALGO_CALIG ? 1u : 0u,
@@ -559,7 +560,7 @@ static int stream_after(cudaStream_t waiter, cudaStream_t signaller, cudaEvent_t
 static int run_edge_batch(csm_ctx* ctx, const csm_update* ups, uint32_t B, csm_result* out,
                           const std::vector<csm_result*>& out_q) {
   cudaStream_t st = ctx->st;
-  const uint32_t L = std::min<uint32_t>(ctx->lcap, 4 * B + 64);
+  const uint32_t L = std::min<uint32_t>(ctx->lcap, list_slots(B));
   int rc = batch_mutate_insert(ctx, ups, B, L);
   if (rc) return rc;
   // every query: index to the union graph, then search
@@ -1056,11 +1057,9 @@ static int tune_run(csm_ctx* ctx, uint32_t B, uint32_t warps, uint32_t bps, floa
   const DevGraph& g = ctx->g;
   unsigned int* c = ctx->d_cnt;
   CK(cudaMemsetAsync(c, 0, 64, st));
-  CK(cudaMemsetAsync(ctx->d_count, 0, 8ull * B, st));
-  CK(cudaMemsetAsync(ctx->d_bytes, 0, 8ull * B, st));
-  CK(cudaMemsetAsync(ctx->d_stop, 0, 4ull * B, st));
   k_seed<<<blocks_for(B, 4), 128, 0, st>>>(B, ctx->d_info, g, ctx->d_plan, ctx->index.d2, ctx->index.words,
-                                              ctx->d_tasks, c + 6, ctx->task_cap, ctx->d_safe, &g.ps->error); CKL();
+                                              ctx->d_tasks, c + 6, ctx->task_cap, ctx->d_safe, &g.ps->error,
+                                           Counters{ctx->d_count, ctx->d_hash, ctx->d_bytes, ctx->d_stop}); CKL();
   SearchParams sp{};
   sp.g = g; sp.plan = ctx->d_plan; sp.tasks = ctx->d_tasks; sp.n_tasks = c + 6; sp.task_cap = ctx->task_cap;
   sp.task_next = c + 7; sp.info = ctx->d_info; sp.count = ctx->d_count; sp.hash = ctx->d_hash;

@@ -171,20 +171,24 @@ __global__ void k_dir_scan(uint32_t* dir, uint32_t n_cap, uint32_t nc) {
 // batch preparation
 // ---------------------------------------------------------------------
 
+// Sort key of a record that is no valid edge update (ids are below 2^yb - 1).
+__device__ __forceinline__ uint64_t edge_sort_none(const KeyBits& kb) { return (1ULL << (2 * kb.yb)) - 1; }
+
 __global__ void k_batch_init(const csm_update* ups, uint32_t B, DevGraph g, uint64_t* ukey, uint32_t* useq,
-                             UpdInfo* info) {
+                             UpdInfo* info, unsigned int* cnt) {
   uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+  if (s < 16) cnt[s] = 0;
   if (s >= B) return;
   const csm_update u = ups[s];
   UpdInfo inf;
   inf.v1 = u.id1; inf.v2 = u.id2; inf.label = fold_elabel(g, u.label); inf.flags = 0;
   useq[s] = s;
-  uint64_t key = ~0ULL;
+  uint64_t key = edge_sort_none(g.kb);
   if (u.type == 'e') {
     const bool ok = u.id1 < g.n && u.id2 < g.n && u.id1 != u.id2 && g.vlabel[u.id1] != kNone &&
                     g.vlabel[u.id2] != kNone;
     if (ok) {
-      key = ((uint64_t)min(u.id1, u.id2) << 32) | (uint64_t)max(u.id1, u.id2);
+      key = ((uint64_t)min(u.id1, u.id2) << g.kb.yb) | (uint64_t)max(u.id1, u.id2);
       inf.flags = UF_VALID | (u.is_add ? UF_ADD : 0u);
     } else {
       inf.flags = UF_INVALID;
@@ -213,8 +217,8 @@ __global__ void k_resolve(const uint64_t* skey, const uint32_t* sseq, uint32_t B
   uint32_t j = blockIdx.x * blockDim.x + threadIdx.x;
   if (j >= B) return;
   const uint64_t k = skey[j];
-  if (k == ~0ULL || (j > 0 && skey[j - 1] == k)) return;
-  const uint32_t x = (uint32_t)(k >> 32), y = (uint32_t)k;
+  if (k == edge_sort_none(g.kb) || (j > 0 && skey[j - 1] == k)) return;
+  const uint32_t x = (uint32_t)(k >> g.kb.yb), y = (uint32_t)(k & ((1ULL << g.kb.yb) - 1));
   const uint32_t lx = g.vlabel[x], ly = g.vlabel[y];
   const uint32_t* pool = g.pools[g.ps->active];
   const uint32_t l0 = find_label(g, pool, x, y);

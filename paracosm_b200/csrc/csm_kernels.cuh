@@ -24,8 +24,10 @@ __global__ void k_load_scatter(const uint64_t* dkey, uint64_t M, const uint64_t*
 __global__ void k_dir_scan(uint32_t* dir, uint32_t n_cap, uint32_t nc);
 
 // ---- batch preparation ----
+// ukey: the update's edge (smaller end, larger end; yb bits each), for sorting;
+// cnt[0..15] cleared.
 __global__ void k_batch_init(const csm_update* ups, uint32_t B, DevGraph g, uint64_t* ukey, uint32_t* useq,
-                             UpdInfo* info);
+                             UpdInfo* info, unsigned int* cnt);
 struct ResolveOut {
   uint64_t* ins_key; unsigned int* n_ins;
   uint64_t* del_key; unsigned int* n_del;
@@ -189,9 +191,15 @@ struct SearchParams {
   unsigned int* ended;          // blocks that have ended; 0 between launches
 };
 constexpr uint32_t kFuseResults = 1024;  // updates of a batch up to which it does
+// Per-update counters of a search.
+struct Counters {
+  unsigned long long *count, *hash, *bytes;
+  unsigned int* stop;
+};
+// Root tasks of B updates; clears their counters.
 __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* plan, const uint64_t* d2,
                        uint64_t d2_words, Task* tasks, unsigned int* n_tasks, uint32_t task_cap,
-                       uint32_t* safe, unsigned int* error, uint32_t shard_rank = 0, uint32_t shard_count = 1,
+                       uint32_t* safe, unsigned int* error, Counters ctr, uint32_t shard_rank = 0, uint32_t shard_count = 1,
                        uint32_t turboflux_compat = 0, uint32_t dup_zero = 0, SearchQueue* q = nullptr,
                        SearchStats* ss = nullptr);
 // mode: 0 plain, 1 match sets, 2 tail counting

@@ -169,7 +169,7 @@ extern "C" int csm_gpu_probe_noalloc(csm_ctx* ctx, uint32_t n, const csm_update*
   }
   k_probe_prep<<<nb, 256, 0, v.st>>>(d_edges, n, v.g, info, count, hash, bytes, stop, words, sstat);
   k_seed<<<(n + 3) / 4, 128, 0, v.st>>>(n, info, v.g, v.plan, v.d2, v.d2_words, tasks, words + 0, task_cap, safe,
-                                             words + 2, 0, 1, 0, v.dup_zero);
+                                             words + 2, Counters{count, hash, bytes, stop}, 0, 1, 0, v.dup_zero);
   SearchParams sp{};
   sp.g = v.g; sp.plan = v.plan; sp.tasks = tasks; sp.n_tasks = words + 0; sp.task_cap = task_cap;
   sp.task_next = words + 1; sp.info = info; sp.count = count; sp.hash = hash; sp.bytes = bytes; sp.stop = stop;

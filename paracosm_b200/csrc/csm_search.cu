@@ -101,7 +101,7 @@ __global__ void k_search_prep(SearchQueue* q, const unsigned int* n_tasks, uint3
 // search's queue, as k_search_prep does.
 __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* plan, const uint64_t* d2,
                        uint64_t d2_words, Task* tasks, unsigned int* n_tasks, uint32_t task_cap,
-                       uint32_t* safe, unsigned int* error, uint32_t shard_rank, uint32_t shard_count,
+                       uint32_t* safe, unsigned int* error, Counters ctr, uint32_t shard_rank, uint32_t shard_count,
                        uint32_t turboflux_compat, uint32_t dup_zero, SearchQueue* q, SearchStats* ss) {
   const uint32_t s = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
   if (s >= B) return;
@@ -139,7 +139,10 @@ __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* 
     }
   }
   matches = __any_sync(0xffffffffu, matches);
-  if (lane == 0) safe[s] = matches ? 0u : 1u;
+  if (lane == 0) {
+    safe[s] = matches ? 0u : 1u;
+    ctr.count[s] = 0; ctr.hash[s] = 0; ctr.bytes[s] = 0; ctr.stop[s] = 0;
+  }
   if (q) {
     made = __reduce_add_sync(0xffffffffu, made);
     if (lane == 0) search_prep(q, ss, made, error);

@@ -93,7 +93,7 @@ __global__ void k_ix_freq(DevGraph g, uint32_t ne, const uint32_t* __restrict__ 
 
 // Does v keep its flag for query vertex u (phase 1: d1, phase 2: d2)?  One lane;
 // `far` instead when a segment is too long for one.
-__device__ __forceinline__ bool ix_lane_eval(const DevGraph& g, const uint32_t* pool, const IxDag* __restrict__ dag,
+__device__ __forceinline__ bool ix_lane_eval(const DevGraph& g, const uint32_t* pool, const IxDag* dag,
                                              const IxBits& b, uint32_t u, uint32_t phase, uint32_t v, bool& far) {
   const uint32_t nchk = phase == 1 ? dag->npar[u] : dag->nchd[u];
   const uint64_t* sup = (phase == 1 || dag->lighting) ? b.d1 : b.d2;
@@ -110,9 +110,10 @@ __device__ __forceinline__ bool ix_lane_eval(const DevGraph& g, const uint32_t* 
   return ok;
 }
 
-// The same by a whole warp.  Lane s looks up segment s, all at once; then the
-// warp scans them one after another.
-__device__ __forceinline__ bool ix_warp_eval(const DevGraph& g, const uint32_t* pool, const IxDag* __restrict__ dag,
+// The same by a whole warp.  Lane s looks up segment s, all at once, and the
+// first few entries of every segment are tried together; what that leaves open
+// is scanned segment by segment.
+__device__ __forceinline__ bool ix_warp_eval(const DevGraph& g, const uint32_t* pool, const IxDag* dag,
                                              const IxBits& b, uint32_t u, uint32_t phase, uint32_t v, uint32_t lane) {
   const uint32_t nchk = phase == 1 ? dag->npar[u] : dag->nchd[u];
   const uint64_t* sup = (phase == 1 || dag->lighting) ? b.d1 : b.d2;
@@ -127,9 +128,21 @@ __device__ __forceinline__ bool ix_warp_eval(const DevGraph& g, const uint32_t* 
     ok = ok && lo < hi;
   }
   if (!__all_sync(0xffffffffu, ok)) return false;
-  for (uint32_t s = 0; s < nchk; s++) {
-    const uint64_t* flag = sup + (uint64_t)__shfl_sync(0xffffffffu, q, s) * b.words;
-    if (!warp_support(pool, __shfl_sync(0xffffffffu, lo, s), __shfl_sync(0xffffffffu, hi, s), flag, lane)) return false;
+  if (nchk == 0) return true;
+  const uint32_t few = 32u / nchk;  // entries of each segment tried together; nchk <= 31
+  const uint32_t s = lane / few, k = lane % few;
+  const uint64_t slo = __shfl_sync(0xffffffffu, lo, s & 31u), shi = __shfl_sync(0xffffffffu, hi, s & 31u);
+  const uint32_t sq = __shfl_sync(0xffffffffu, q, s & 31u);
+  const bool hit = s < nchk && slo + k < shi && bit_of(sup + (uint64_t)sq * b.words, pool[slo + k]);
+  const uint32_t found = __reduce_or_sync(0xffffffffu, hit ? 1u << s : 0u);
+  const uint32_t over = __ballot_sync(0xffffffffu, lane < nchk && hi - lo <= few);  // wholly tried
+  const uint32_t all = 0xffffffffu >> (32u - nchk);
+  if (over & ~found) return false;
+  for (uint32_t open = all & ~found; open; open &= open - 1) {
+    const uint32_t i = (uint32_t)__ffs((int)open) - 1;
+    const uint64_t* flag = sup + (uint64_t)__shfl_sync(0xffffffffu, q, i) * b.words;
+    if (!warp_support(pool, __shfl_sync(0xffffffffu, lo, i) + few, __shfl_sync(0xffffffffu, hi, i), flag, lane))
+      return false;
   }
   return true;
 }
@@ -190,7 +203,7 @@ __device__ __forceinline__ void ix_mark(const IxBits& b, uint32_t nq, uint32_t p
 // Marks for DAG edge e and the changed directed entry k = x -> y (combo = (L(y),
 // l)), when its labels are the edge's: y for d1 of the child, x for d2 of the
 // parent.  The reverse entry y -> x covers the other orientation.
-__device__ __forceinline__ void ix_seed(const DevGraph& g, const IxDag* __restrict__ dag, const IxBits& b, uint64_t k,
+__device__ __forceinline__ void ix_seed(const DevGraph& g, const IxDag* dag, const IxBits& b, uint64_t k,
                                         uint32_t lx, uint32_t e) {
   const uint32_t c = g.kb.c_of(k);
   if (dag->eel[e] != c % g.n_el) return;
@@ -202,7 +215,7 @@ __device__ __forceinline__ void ix_seed(const DevGraph& g, const IxDag* __restri
 
 // Re-evaluates u's flag of vertex v in each lane with `has` (their marks are
 // taken off here), and marks what depends on the flags that changed.
-__device__ __forceinline__ void ix_items(const DevGraph& g, const uint32_t* pool, const IxDag* __restrict__ dag,
+__device__ __forceinline__ void ix_items(const DevGraph& g, const uint32_t* pool, const IxDag* dag,
                                          const IxBits& b, uint32_t u, uint32_t phase, bool has, uint32_t v,
                                          bool by_lane, uint32_t lane) {
   const uint64_t off = (uint64_t)u * b.words;
@@ -247,12 +260,18 @@ __device__ __forceinline__ void ix_items(const DevGraph& g, const uint32_t* pool
 // load each and no barrier.  What bounds a round is the number of barriers and
 // the chain of loads between two: for one edge update of a 13-vertex query on
 // 2^19 vertices 52 barriers over whole bitsets took 153 us, one barrier per
-// query vertex 29 us.  A list's length is read by every block between the
+// step 33 us, and 28 us with the DAG in shared memory and a warp trying all
+// segments of a vertex at once (a batch of 100: 289, 95 and 77 us).  A list's length is read by every block between the
 // barrier after the last mark it can get and the one after its own work, so
 // all blocks take the same way.
-__global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __restrict__ dag, IxBits b, IxOrder ord,
+__global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __restrict__ gdag, IxBits b, IxOrder ord,
                                                   const uint64_t* __restrict__ keys, uint32_t L, uint32_t vert) {
   cg::grid_group grid = cg::this_grid();
+  __shared__ __align__(16) IxDag sdag;  // every step's chain of loads starts in it
+  for (uint32_t i = threadIdx.x; i < sizeof(IxDag) / 4; i += blockDim.x)
+    reinterpret_cast<uint32_t*>(&sdag)[i] = reinterpret_cast<const uint32_t*>(gdag)[i];
+  __syncthreads();
+  const IxDag* dag = &sdag;
   const uint32_t lane = threadIdx.x & 31;
   const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
   const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;

@@ -255,86 +255,140 @@ __device__ __forceinline__ void ix_items(const DevGraph& g, const uint32_t* pool
 // for the changed directed entries keys[0, L) and, when it is not kNone, the
 // new or removed vertex `vert`.  The marks come first; then, step by step of
 // the order, the flags on the work lists of the step's query vertices, d1
-// before d2, each step followed by a grid barrier.  Query vertices that do not
-// draw on one another's flags share a step, and a step of empty lists costs a
-// load each and no barrier.  What bounds a round is the number of barriers and
-// the chain of loads between two: for one edge update of a 13-vertex query on
-// 2^19 vertices 52 barriers over whole bitsets took 153 us, one barrier per
-// step 33 us, and 28 us with the DAG in shared memory and a warp trying all
-// segments of a vertex at once (a batch of 100: 289, 95 and 77 us).  A list's length is read by every block between the
-// barrier after the last mark it can get and the one after its own work, so
-// all blocks take the same way.
+// before d2.  Query vertices that do not draw on one another's flags share a
+// step, and steps of empty lists are passed over.  What bounds a round is the
+// number of grid barriers and the chain of loads between two, so the marks of a
+// few entries and every run of steps of at most kAlone vertices are worked off by
+// block 0 alone, with barriers of the block, while the others wait at one grid
+// barrier; after it they go on with the step that block 0 left (b.count[2 nq]).
+// For one edge update of a 13-vertex query on 2^19 vertices 52 barriers over
+// whole bitsets took 153 us, a barrier per step with work 28 us, block 0 alone
+// 18.7 us (a batch of 100: 289, 78 and 71 us).
+//
+// All blocks take the same way: a list's length is final when the last step
+// that can mark it is done, and it is taken back only by block 0 after a barrier
+// from which on nobody asks for it.
+// Two vertices a warp.  Two batches of 100: 8 0.73 ms, 32 0.69, 128 0.72; single
+// updates do not tell them apart.
+constexpr uint32_t kAlone = 32;
+
 __global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __restrict__ gdag, IxBits b, IxOrder ord,
                                                   const uint64_t* __restrict__ keys, uint32_t L, uint32_t vert) {
   cg::grid_group grid = cg::this_grid();
   __shared__ __align__(16) IxDag sdag;  // every step's chain of loads starts in it
+  __shared__ uint32_t scount[2 * kMaxQ];
   for (uint32_t i = threadIdx.x; i < sizeof(IxDag) / 4; i += blockDim.x)
     reinterpret_cast<uint32_t*>(&sdag)[i] = reinterpret_cast<const uint32_t*>(gdag)[i];
   __syncthreads();
   const IxDag* dag = &sdag;
   const uint32_t lane = threadIdx.x & 31;
-  const uint32_t tid = blockIdx.x * blockDim.x + threadIdx.x, nthreads = gridDim.x * blockDim.x;
-  const uint32_t warp = tid >> 5, nwarps = nthreads >> 5;
   const uint32_t ne = dag->n_edges, nq = dag->nq;
   const uint32_t* pool = g.pools[g.ps->active];
-  if (L <= 64) {  // a thread per (entry, DAG edge)
-    for (uint32_t i = tid; i < L * ne; i += nthreads) {
-      const uint64_t k = keys[i / ne];
-      if (g.kb.real(k)) ix_seed(g, dag, b, k, g.vlabel[g.kb.x_of(k)], i % ne);
-    }
-  } else {
-    for (uint32_t i = tid; i < L; i += nthreads) {
-      const uint64_t k = keys[i];
-      if (!g.kb.real(k)) continue;
-      const uint32_t lx = g.vlabel[g.kb.x_of(k)];
-      for (uint32_t e = 0; e < ne; e++) ix_seed(g, dag, b, k, lx, e);
-    }
-  }
-  if (vert != kNone && tid < nq) {
-    ix_mark(b, nq, 1, tid, vert);
-    ix_mark(b, nq, 2, tid, vert);
-  }
-  grid.sync();
-  for (uint32_t phase = 1; phase <= 2; phase++) {
-    uint32_t beg = 0;
-    for (uint32_t step = 0; step < ord.steps[phase - 1]; step++) {
-      const uint32_t end = ord.end[phase - 1][step];
-      uint32_t used = 0;  // warps' shares given out in this step so far: the next list starts with the next warp
-      for (uint32_t i = beg; i < end; i++) {
-        const uint32_t u = ord.order[phase - 1][i];
-        const uint32_t row = (phase == 1 ? 0u : nq) + u;
-        const uint32_t n = *(volatile unsigned int*)&b.count[row];
-        if (n == 0) continue;
-        const uint32_t w0 = (warp + nwarps - used % nwarps) % nwarps;
-        if (n <= b.list_cap) {
-          // as many items per warp as it takes to share them out; with several,
-          // each lane first tries its own
-          const uint32_t* list = b.list + (size_t)row * b.list_cap;
-          const uint32_t per = min(32u, (n + nwarps - 1) / nwarps);
-          for (uint32_t base = w0 * per; base < n; base += nwarps * per) {
-            const bool has = lane < per && base + lane < n;
-            ix_items(g, pool, dag, b, u, phase, has, has ? __ldcg(list + base + lane) : 0u, per > 4, lane);
-          }
-          used += (n + per - 1) / per;
-        } else {
-          const uint64_t* mark = (phase == 1 ? b.m1 : b.m2) + (uint64_t)u * b.words;
-          for (uint64_t wi = w0; wi < b.words; wi += nwarps) {
-            const uint64_t word = __ldcg(mark + wi);
-            if (!word) continue;
-#pragma unroll 1
-            for (uint32_t half = 0; half < 2; half++)
-              ix_items(g, pool, dag, b, u, phase, (word >> (32u * half + lane)) & 1ULL,
-                       (uint32_t)(wi * 64 + 32u * half + lane), true, lane);
-          }
-          used += nwarps;
-        }
+  const uint32_t steps1 = ord.steps[0], steps = steps1 + ord.steps[1];
+  const bool first = blockIdx.x == 0;
+  bool alone = L * ne <= blockDim.x;  // block 0 works, the others wait
+  uint32_t from = 0;                  // block 0: first step whose lists' lengths are to be taken back
+  if (!alone || first) {
+    const uint32_t tid = (alone ? 0u : blockIdx.x * blockDim.x) + threadIdx.x;
+    const uint32_t nthreads = alone ? blockDim.x : gridDim.x * blockDim.x;
+    if (L <= 64) {  // a thread per (entry, DAG edge)
+      for (uint32_t i = tid; i < L * ne; i += nthreads) {
+        const uint64_t k = keys[i / ne];
+        if (g.kb.real(k)) ix_seed(g, dag, b, k, g.vlabel[g.kb.x_of(k)], i % ne);
       }
-      if (used) {
+    } else {
+      for (uint32_t i = tid; i < L; i += nthreads) {
+        const uint64_t k = keys[i];
+        if (!g.kb.real(k)) continue;
+        const uint32_t lx = g.vlabel[g.kb.x_of(k)];
+        for (uint32_t e = 0; e < ne; e++) ix_seed(g, dag, b, k, lx, e);
+      }
+    }
+    if (vert != kNone && tid < nq) {
+      ix_mark(b, nq, 1, tid, vert);
+      ix_mark(b, nq, 2, tid, vert);
+    }
+    if (alone) { __threadfence(); __syncthreads(); }
+  }
+  if (!alone) grid.sync();
+  for (uint32_t s = 0;;) {
+    if (alone && !first) {
+      grid.sync();
+      alone = false;
+      s = *(volatile unsigned int*)&b.count[2 * nq];
+      if (s == steps) break;
+    }
+    if (threadIdx.x < 2 * nq) scount[threadIdx.x] = *(volatile unsigned int*)&b.count[threadIdx.x];
+    __syncthreads();
+    uint32_t n_step = 0, phase = 1, beg = 0, end = 0;
+    for (; s < steps; s++) {
+      phase = s < steps1 ? 1u : 2u;
+      const uint32_t t = phase == 1 ? s : s - steps1;
+      beg = t ? ord.end[phase - 1][t - 1] : 0u;
+      end = ord.end[phase - 1][t];
+      for (uint32_t i = beg; i < end; i++) n_step += scount[(phase == 1 ? 0u : nq) + ord.order[phase - 1][i]];
+      if (n_step) break;
+    }
+    if (alone) {  // block 0
+      if (n_step == 0 || n_step > kAlone) {
+        if (threadIdx.x == 0) *(volatile unsigned int*)&b.count[2 * nq] = s;
         grid.sync();
-        if (tid >= beg && tid < end) b.count[(phase == 1 ? 0u : nq) + ord.order[phase - 1][tid]] = 0;
+        alone = false;
+        for (uint32_t r = from; r < s; r++) {
+          const uint32_t ph = r < steps1 ? 0u : 1u, t = ph ? r - steps1 : r;
+          const uint32_t i = (t ? ord.end[ph][t - 1] : 0u) + threadIdx.x;
+          if (i < ord.end[ph][t]) b.count[ph * nq + ord.order[ph][i]] = 0;
+        }
+        if (n_step == 0) break;
       }
-      beg = end;
+    } else if (n_step == 0) {
+      break;
+    } else if (n_step <= kAlone) {
+      alone = true;
+      from = s;
+      if (!first) continue;
     }
+    const uint32_t warp = (alone ? 0u : blockIdx.x * (blockDim.x >> 5)) + (threadIdx.x >> 5);
+    const uint32_t nwarps = (alone ? 1u : gridDim.x) * (blockDim.x >> 5);
+    uint32_t used = 0;  // warps' shares given out in this step so far: the next list starts with the next warp
+    for (uint32_t i = beg; i < end; i++) {
+      const uint32_t u = ord.order[phase - 1][i];
+      const uint32_t row = (phase == 1 ? 0u : nq) + u;
+      const uint32_t n = scount[row];
+      if (n == 0) continue;
+      const uint32_t w0 = (warp + nwarps - used % nwarps) % nwarps;
+      if (n <= b.list_cap) {
+        // as many items per warp as it takes to share them out; with several,
+        // each lane first tries its own
+        const uint32_t* list = b.list + (size_t)row * b.list_cap;
+        const uint32_t per = min(32u, (n + nwarps - 1) / nwarps);
+        for (uint32_t base = w0 * per; base < n; base += nwarps * per) {
+          const bool has = lane < per && base + lane < n;
+          ix_items(g, pool, dag, b, u, phase, has, has ? __ldcg(list + base + lane) : 0u, per > 4, lane);
+        }
+        used += (n + per - 1) / per;
+      } else {
+        const uint64_t* mark = (phase == 1 ? b.m1 : b.m2) + (uint64_t)u * b.words;
+        for (uint64_t wi = w0; wi < b.words; wi += nwarps) {
+          const uint64_t word = __ldcg(mark + wi);
+          if (!word) continue;
+#pragma unroll 1
+          for (uint32_t half = 0; half < 2; half++)
+            ix_items(g, pool, dag, b, u, phase, (word >> (32u * half + lane)) & 1ULL,
+                     (uint32_t)(wi * 64 + 32u * half + lane), true, lane);
+        }
+        used += nwarps;
+      }
+    }
+    if (alone) {
+      __threadfence();
+      __syncthreads();
+    } else {
+      grid.sync();
+      const uint32_t i = beg + threadIdx.x;
+      if (first && i < end) b.count[(phase == 1 ? 0u : nq) + ord.order[phase - 1][i]] = 0;
+    }
+    s++;
   }
 }
 
@@ -574,14 +628,14 @@ static int index_finish(IndexState& ix, DevMem& mem, const DevGraph& g, const In
   blk.add(ix.d_dag, sizeof(IxDag));
   blk.add(ix.d_pop, 16);
   blk.add(ix.bits.list, 4ull * 2 * nq * ix.bits.list_cap);
-  blk.add(ix.bits.count, 8ull * nq);
+  blk.add(ix.bits.count, 8ull * nq + 4);
   rc = blk.alloc(mem, &ix.block);
   if (rc) return rc;
   ix.block_bytes = blk.total;
   ix.bits.d2 = ix.bits.d1 + nq * ix.words;
   ix.bits.m1 = ix.bits.d2 + nq * ix.words;
   ix.bits.m2 = ix.bits.m1 + nq * ix.words;
-  IXCK(cudaMemsetAsync(ix.bits.count, 0, 8ull * nq, st));
+  IXCK(cudaMemsetAsync(ix.bits.count, 0, 8ull * nq + 4, st));
   IXCK(cudaMemsetAsync(ix.bits.d1, 0, 4 * fam, st));
   IXCK(cudaMemcpyAsync(ix.d_dag, &D, sizeof(IxDag), cudaMemcpyHostToDevice, st));
   ix.d2 = ix.bits.d2;

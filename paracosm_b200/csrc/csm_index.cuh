@@ -75,6 +75,7 @@ struct IxDag {
 // [n_q][words] each.  A marked vertex is also on its query vertex's work list
 // (list [2][n_q][list_cap], lengths count [2][n_q], the d1 lists first) while
 // that has room; a list that overflowed is worked off from its marks.
+// count[2 n_q] is the step a round goes on with after its first block's own.
 struct IxBits {
   uint64_t *d1, *d2, *m1, *m2;
   uint64_t words;

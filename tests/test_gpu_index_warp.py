@@ -47,3 +47,44 @@ def test_last_entry_supports(arms, n, algo):
                 want = fresh.index(len(vl))
             if (got["root"], got["order"]) == (want["root"], want["order"]):  # it follows the label frequencies
                 assert np.array_equal(got["d1"], want["d1"]) and np.array_equal(got["d2"], want["d2"])
+
+
+@pytest.mark.parametrize("algo", ["parallel_turboflux", "parallel_symbi", "parallel_calig"])
+@pytest.mark.parametrize("mode", ["batched", "plain"])
+@pytest.mark.parametrize("widths", [[1] * 6, [1, 32, 1, 33, 1, 40], [1, 1, 40, 1, 40, 1], [33, 1, 31, 1, 64, 1],
+                                    [104, 1, 33, 33, 1, 2]])
+def test_runs_of_short_and_long_steps(widths, mode, algo):
+    """Levels of vertices, each wholly joined to the next, under a path query: the edges between the first two levels
+    go and come back, so the round's work lists are as long as the levels are wide, short and long in turn."""
+    levels, n = [], 0
+    for w in widths:
+        levels.append(list(range(n, n + w)))
+        n += w
+    vl = np.repeat(np.arange(len(widths)), widths).astype(np.uint32)
+    pairs = [[(x, y, 0) for x in a for y in b] for a, b in zip(levels, levels[1:])]
+    base = np.array(sum(pairs, []), np.uint32)
+    rest = np.array(sum(pairs[1:], []), np.uint32)
+    embeddings = int(np.prod(widths, dtype=np.int64))
+
+    def engine(edges):
+        eng = Engine(algo, max_results=10**9, mode=mode)
+        eng.set_query(list(range(len(widths))), [(i, i + 1, 0) for i in range(len(widths) - 1)])
+        eng.load_graph(vl, edges)
+        eng.build_index()
+        return eng
+
+    compared = 0
+    with engine(base) as eng:
+        for add in (0, 1):
+            u = np.zeros(len(pairs[0]), UPDATE_DTYPE)
+            u["type"], u["is_add"] = ord("e"), add
+            u["id1"], u["id2"] = [p[0] for p in pairs[0]], [p[1] for p in pairs[0]]
+            res = eng.run(u)
+            assert int(res["pos" if add else "neg"].sum()) == embeddings
+            got = eng.index(n)
+            with engine(base if add else rest) as fresh:
+                want = fresh.index(n)
+            if (got["root"], got["order"]) == (want["root"], want["order"]):
+                compared += 1
+                assert np.array_equal(got["d1"], want["d1"]) and np.array_equal(got["d2"], want["d2"])
+    assert compared

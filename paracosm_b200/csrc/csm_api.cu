@@ -412,16 +412,28 @@ static int batch_mutate_insert(csm_ctx* ctx, const csm_update* ups, uint32_t B, 
   unsigned int* c = ctx->d_cnt;
   k_batch_init<<<blocks_for(B, 256), 256, 0, st>>>(ups, B, g, ctx->d_ukey, ctx->d_useq, ctx->d_info, c); CKL();
   size_t tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, ctx->d_ukey, ctx->d_ukey2, ctx->d_useq, ctx->d_useq2, (int)B, 0, (int)(2 * kb.yb), st));
+  if (B <= kSortMax && 2 * kb.yb <= kSortMaxBits) {  // useq is the place itself
+    CK(launch_sort_block({{{ctx->d_ukey, ctx->d_ukey2, ctx->d_useq2, nullptr, nullptr, B, 2 * kb.yb}}}, 1, st));
+    ctx->launches++;
+  } else {
+    CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, ctx->d_ukey, ctx->d_ukey2, ctx->d_useq, ctx->d_useq2, (int)B, 0, (int)(2 * kb.yb), st));
+  }
   ResolveOut ro{ins, c + 0, del, c + 1, tk, ctx->d_ts, c + 2, L};
   k_resolve<<<blocks_for(B, 128), 128, 0, st>>>(ctx->d_ukey2, ctx->d_useq2, B, g, ups, ctx->d_info, ro); CKL();
   const int end_bit = (int)kb.total();
-  tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, ins, ctx->d_ins2, (int)L, 0, end_bit, st));
-  tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, del, ctx->d_del2, (int)L, 0, end_bit, st));
-  tb = ctx->cub_bytes;
-  CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, tk, ctx->d_tk2, ctx->d_ts, ctx->d_ts2, (int)L, 0, end_bit, st));
+  if (L <= kSortMax && kb.total() <= kSortMaxBits) {
+    CK(launch_sort_block({{{ins, ctx->d_ins2, nullptr, nullptr, nullptr, L, kb.total()},
+                           {del, ctx->d_del2, nullptr, nullptr, nullptr, L, kb.total()},
+                           {tk, ctx->d_tk2, nullptr, ctx->d_ts, ctx->d_ts2, L, kb.total()}}}, 3, st));
+    ctx->launches++;
+  } else {
+    tb = ctx->cub_bytes;
+    CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, ins, ctx->d_ins2, (int)L, 0, end_bit, st));
+    tb = ctx->cub_bytes;
+    CK(cub::DeviceRadixSort::SortKeys(ctx->d_cub, tb, del, ctx->d_del2, (int)L, 0, end_bit, st));
+    tb = ctx->cub_bytes;
+    CK(cub::DeviceRadixSort::SortPairs(ctx->d_cub, tb, tk, ctx->d_tk2, ctx->d_ts, ctx->d_ts2, (int)L, 0, end_bit, st));
+  }
   k_ranges<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_ins2, L, kb, ctx->d_rins, c + 3, g.dir, g.nc); CKL();
   k_ranges<<<blocks_for(L, 256), 256, 0, st>>>(ctx->d_del2, L, kb, ctx->d_rdel, c + 4, g.dir, g.nc); CKL();
   g.t_key = ctx->d_tk2;

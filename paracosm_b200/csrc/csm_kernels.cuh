@@ -50,6 +50,23 @@ __host__ __device__ inline uint32_t temporal_slots(uint32_t B) {
   return s;
 }
 __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges, DevGraph g);
+// Lists that k_sort_block sorts, one block each: job.n keys of job.bits bits to
+// out (stable; unused slots, all ones, come out as job.bits ones); pos: where to
+// put each key's place in the list, or null; val: moved along to val_out, or
+// null.  A list fits when n <= kSortMax and bits <= kSortMaxBits.
+constexpr uint32_t kSortMax = 9 * 1024;  // the lists of a batch of 4,096
+constexpr uint32_t kSortPosBits = 14;    // > log2(kSortMax)
+constexpr uint32_t kSortMaxBits = 64 - kSortPosBits;
+struct SortJob {
+  const uint64_t* key;
+  uint64_t* out;
+  uint32_t* pos;
+  const uint64_t* val;
+  uint64_t* val_out;
+  uint32_t n, bits;
+};
+struct SortJobs { SortJob job[3]; };
+cudaError_t launch_sort_block(const SortJobs& jobs, uint32_t n_jobs, cudaStream_t st);
 __global__ void k_compact_copy(DevGraph g);
 void launch_mut_insert(const VRange* ranges, const unsigned int* n_ranges, const uint64_t* ins_key,
                        uint32_t* ins_dst, const DevGraph& g, uint32_t warp_blocks, uint32_t big_blocks,

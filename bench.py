@@ -732,7 +732,7 @@ def main():
             # between its completion stamp and the previous one's
             svc = np.diff(np.concatenate([[0], np.sort(pr["latency_ns"].astype(np.float64))]))
             # launches per update: the label-triple test decides the sequence (2-3 launches when no
-            # query edge matches, about 9 otherwise); reported as the mean and per class
+            # query edge matches, 5 or 6 otherwise); reported as the mean and per class
             lpu = np.array(peng.kernel_launches() - l0, dtype=np.float64) / P
             forms[graphs] = {"value": P / plain_s, "updates": P, "first_update": first, "device_ms": pst["total_device_ms"],
                              "p50_us": float(np.percentile(svc, 50)) / 1e3,

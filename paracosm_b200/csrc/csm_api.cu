@@ -1235,7 +1235,12 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
     if (rc) return rc;
     set_err(CSM_OK, "");
   }
-  auto release = [&]() { ctx->mem.release(mem, mem_bytes); };
+  struct Held {  // released on every way out
+    DevMem& m;
+    void* p;
+    size_t bytes;
+    ~Held() { m.release(p, bytes); }
+  } held{ctx->mem, mem, mem_bytes};
   unsigned long long* cnt = reinterpret_cast<unsigned long long*>(mem);
   unsigned long long* off = cnt + n_cap;
   unsigned long long* total = off + n_cap;
@@ -1263,27 +1268,32 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
   const uint32_t stride = ctx->cfg.shard_count > 1 ? ctx->cfg.shard_count : 1u;
   const uint32_t rank = stride > 1 ? ctx->cfg.shard_rank : 0u;
   const unsigned long long n_seeds = n_all > rank ? (n_all - rank + stride - 1) / stride : 0ull;
-  uint32_t warps, bps;
-  search_shape(ctx, warps, bps);
   unsigned int* c = ctx->d_cnt;
+  SearchParams sp{};
+  sp.g = g; sp.plan = ctx->d_plan; sp.tasks = s_tasks; sp.n_tasks = c + 6;
+  sp.task_next = c + 7; sp.info = s_info; sp.count = s_count; sp.hash = ctx->d_hash;
+  sp.bytes = s_bytes; sp.stop = s_stop;
+  sp.d2 = ctx->index.d2; sp.d2_words = ctx->index.words; sp.cap = 0;
+  sp.homo = ctx->cfg.homomorphism; sp.want_hash = 0; sp.error = &g.ps->error;
+  sp.q = ctx->d_q; sp.dq = ctx->d_dq; sp.qseq = ctx->d_qseq; sp.qcap = ctx->qcap;
+  sp.wait_limit_ns = 30ull * 1000000000ull;
+  sp.slot_limit_ns = 100ull * 1000000ull;
+  sp.task_limit_ns = 20ull * 1000000000ull;
+  sp.sstat = ctx->d_sstat;
+  sp.tail = ctx->cfg.tail_enumerate ? 0u : 1u;
+  set_search_shape(sp, *ctx->h_plan);
+  // fitted to the instantiation that is launched here: a context that asks for
+  // hashes or match sets searches its batches with another one, whose walks
+  // may take a level less of shared memory
+  const int mode = search_mode(sp);
+  uint32_t warps, bps;
+  search_fit(ctx, SearchShape{sp.levels, sp.warp_bytes}, mode, warps, bps);
   for (unsigned long long first = 0; first < n_seeds; first += chunk) {
     const uint32_t B = (uint32_t)std::min<unsigned long long>(chunk, n_seeds - first);
     k_init_fill<<<blocks_for(B, 256), 256, 0, st>>>(g, combo, A.el, off, first, B, stride, rank, s_info, s_tasks,
                                                     s_count, s_bytes, s_stop, c); CKL();
-    SearchParams sp{};
-    sp.g = g; sp.plan = ctx->d_plan; sp.tasks = s_tasks; sp.n_tasks = c + 6; sp.task_cap = B;
-    sp.task_next = c + 7; sp.info = s_info; sp.count = s_count; sp.hash = ctx->d_hash;
-    sp.bytes = s_bytes; sp.stop = s_stop;
-    sp.d2 = ctx->index.d2; sp.d2_words = ctx->index.words; sp.cap = 0;
-    sp.homo = ctx->cfg.homomorphism; sp.want_hash = 0; sp.error = &g.ps->error;
-    sp.q = ctx->d_q; sp.dq = ctx->d_dq; sp.qseq = ctx->d_qseq; sp.qcap = ctx->qcap;
-    sp.wait_limit_ns = 30ull * 1000000000ull;
-    sp.slot_limit_ns = 100ull * 1000000ull;
-    sp.task_limit_ns = 20ull * 1000000000ull;
+    sp.task_cap = B;
     sp.batch = B;
-    sp.sstat = ctx->d_sstat;
-    sp.tail = ctx->cfg.tail_enumerate ? 0u : 1u;
-    set_search_shape(sp, *ctx->h_plan);
     launch_search(sp, (uint32_t)ctx->sm_count * bps, warps, st); CKL();
     ctx->search_launches++;
     k_init_sum<<<std::min<uint32_t>(blocks_for(B, 256), 1024), 256, 0, st>>>(B, s_count, total); CKL();
@@ -1292,7 +1302,6 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
   unsigned long long h = 0;
   CK(cudaMemcpyAsync(&h, total, 8, cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  release();
   rc = check_device_error(ctx);
   if (rc) return rc;
   *out = h;

@@ -1207,33 +1207,27 @@ __global__ void __launch_bounds__(W * 32, min_blocks(W)) k_search_tail(const __g
 
 namespace {
 
+using SearchKernel = void (*)(SearchParams);
+
 // mode: 0 plain, 1 match sets, 2 tail counting
 template <int W>
-cudaError_t search_occupancy(int* nb, size_t smem, int mode) {
-  if (mode == 2) {
-    cudaFuncSetAttribute(k_search_tail<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_search_tail<W>, W * 32, smem);
-  }
-  if (mode == 1) {
-    cudaFuncSetAttribute(k_search<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    return cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_search<W, true>, W * 32, smem);
-  }
-  cudaFuncSetAttribute(k_search<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k_search<W, false>, W * 32, smem);
+SearchKernel search_kernel(int mode) {
+  return mode == 2 ? k_search_tail<W> : mode == 1 ? k_search<W, true> : k_search<W, false>;
 }
 
 template <int W>
+cudaError_t search_occupancy(int* nb, size_t smem, int mode) {
+  const SearchKernel k = search_kernel<W>(mode);
+  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k, W * 32, smem);
+}
+
+// A shape that does not fit is not launched; the caller's cudaGetLastError reports it.
+template <int W>
 void search_launch(const SearchParams& p, uint32_t blocks, size_t smem, cudaStream_t s, int mode) {
-  if (mode == 2) {
-    cudaFuncSetAttribute(k_search_tail<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_search_tail<W><<<blocks, W * 32, smem, s>>>(p);
-  } else if (mode == 1) {
-    cudaFuncSetAttribute(k_search<W, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_search<W, true><<<blocks, W * 32, smem, s>>>(p);
-  } else {
-    cudaFuncSetAttribute(k_search<W, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-    k_search<W, false><<<blocks, W * 32, smem, s>>>(p);
-  }
+  const SearchKernel k = search_kernel<W>(mode);
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
+    k<<<blocks, W * 32, smem, s>>>(p);
 }
 
 }  // namespace

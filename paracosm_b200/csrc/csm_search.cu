@@ -231,7 +231,12 @@ __device__ __noinline__ uint32_t seg_size_slow(const SearchParams& p, uint32_t v
                                                int32_t t) {
   return seg_size_at(p.g, v, c, lo, hi, t);
 }
-// Join without row tables: a binary search in v's segment.
+// Join without row tables: a binary search in v's segment.  The first join of a
+// candidate runs before the gather here as well (run_levels): left to
+// check_rest, behind the filter and one after another from the last position
+// on, the joins took the search of 65,536 updates on 2^22 vertices 310 ms
+// (166 ms now, with tables 117), of 4,097 on 2^19 29 (25, 19), of a
+// hash-enumerating 3,001 on 2^17 8.4 (5.5, 4.1).
 __device__ __noinline__ uint32_t join_search(const SearchParams& p, const uint32_t* pool, uint32_t v, uint32_t c,
                                              uint32_t x) {
   uint64_t lo, hi;
@@ -692,7 +697,7 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
   const uint32_t every = p.donate_every ? p.donate_every : 1u;  // steps between hand-over checks (a power of two)
   bool enter = true;
   uint32_t cur = 0, total = 0, my_incl = 0, qv = 0, held = 0;
-  bool joins = false;
+  bool joins = false;  // the next position has a join beside its driver
   const uint64_t* filter = nullptr;  // candidate filter of the level's next position
   // the pair of this lane at cur, loaded a step ahead: entry, candidate, and
   // the row of the entry's first join; `fresh` when they are cur's
@@ -708,7 +713,7 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
     if (at < total) {
       const LevelSM& L = lv[d];
       x = ld_stream(pool + (L.base[own] + at));
-      if (joins) jrow = g.row[L.jv[own]];
+      if (joins && g.htab) jrow = g.row[L.jv[own]];
     }
   };
   // a single update's own range is handed over at once, while every other warp
@@ -724,7 +729,7 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
       my_incl = lane < L.cnt ? L.incl[lane] : 0xffffffffu;
       qv = wp.qv((uint32_t)d + 1u);
       filter = p.d2 ? p.d2 + (uint64_t)qv * p.d2_words : nullptr;
-      joins = wp.nb((uint32_t)d + 1u) > 1 && g.htab != nullptr;
+      joins = wp.nb((uint32_t)d + 1u) > 1;
       enter = false;
       fresh = false;
     }
@@ -807,7 +812,9 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
     uint32_t meta = own;
     bool valid = cur + lane < total;
     if (valid && joins) {
-      const uint32_t hit = row_find(g, jrow, row_entry(cx, lv[d].jel[own], g.hlb));
+      const uint32_t hit = g.htab ? row_find(g, jrow, row_entry(cx, lv[d].jel[own], g.hlb))
+                                  : join_search(p, pool, lv[d].jv[own],
+                                                back_combo(wp.back(pos, lv[d].jsel[own])), cx);
       valid = hit != kSlotEmpty;
       meta |= (hit & kSlotTouched) >> 15;
     }

@@ -456,7 +456,7 @@ static int search_mode_of(const csm_ctx* q) {
 }
 
 static void set_search_shape(SearchParams& sp, const Plan& plan) {
-  const SearchShape s = search_shape_of(plan, search_mode(sp));
+  const SearchShape s = search_shape_of(plan, search_mode(sp), sp.g);
   sp.levels = s.levels;
   sp.warp_bytes = s.warp_bytes;
 }
@@ -479,7 +479,7 @@ static void search_fit(const csm_ctx* q, const SearchShape& shape, int mode, uin
 // warps per block and as many blocks per SM as can be resident.
 static void search_shape(const csm_ctx* q, uint32_t& warps, uint32_t& bps) {
   const int mode = search_mode_of(q);
-  search_fit(q, search_shape_of(*q->h_plan, mode), mode, warps, bps);
+  search_fit(q, search_shape_of(*q->h_plan, mode, q->g), mode, warps, bps);
 }
 
 static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out);
@@ -1110,7 +1110,7 @@ static int autotune(csm_ctx* ctx, uint32_t n, const csm_update* h_edges, uint32_
   // shape replaces the default only when it is at least 5 % faster, since
   // capped updates make single timings vary by a few percent
   const int kmode = search_mode_of(ctx);  // as the batches run
-  const SearchShape shape = search_shape_of(*ctx->h_plan, kmode);
+  const SearchShape shape = search_shape_of(*ctx->h_plan, kmode, ctx->g);
   uint32_t best_w = 8, best_b = std::max<uint32_t>(1, search_max_blocks(shape, 8, kmode));
   float best = 0;
   rc = tune_run(ctx, B, best_w, best_b, &best);
@@ -1287,7 +1287,7 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
   // may take a level less of shared memory
   const int mode = search_mode(sp);
   uint32_t warps, bps;
-  search_fit(ctx, SearchShape{sp.levels, sp.warp_bytes}, mode, warps, bps);
+  search_fit(ctx, search_shape_of(*ctx->h_plan, mode, g), mode, warps, bps);
   for (unsigned long long first = 0; first < n_seeds; first += chunk) {
     const uint32_t B = (uint32_t)std::min<unsigned long long>(chunk, n_seeds - first);
     k_init_fill<<<blocks_for(B, 256), 256, 0, st>>>(g, combo, A.el, off, first, B, stride, rank, s_info, s_tasks,
@@ -2015,7 +2015,7 @@ bool ctx_view(csm_ctx* ctx, CtxView* v) {
   v->want_hash = ctx->cfg.want_hash;
   // the launch shape of the submit path's enumerating search (the probe does
   // not count tails)
-  v->shape = search_shape_of(*ctx->h_plan, 0);
+  v->shape = search_shape_of(*ctx->h_plan, 0, v->g);
   search_fit(ctx, v->shape, 0, v->warps, v->bps);
   return true;
 }

@@ -223,8 +223,9 @@ __global__ void k_seed(uint32_t B, const UpdInfo* info, DevGraph g, const Plan* 
 struct SearchShape {
   uint32_t levels;      // levels of a warp's walk
   uint32_t warp_bytes;  // shared memory of a warp
+  bool general;         // instantiation (search_general)
 };
-SearchShape search_shape_of(const Plan& plan, int mode);
+SearchShape search_shape_of(const Plan& plan, int mode, const DevGraph& g);
 uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode);
 int search_mode(const SearchParams& p);
 // `prepared`: k_seed has prepared the queue.

@@ -46,6 +46,22 @@ struct LevelSM {
   uint32_t cnt, cur, total, pad;
 };
 
+// Elements of a level's or a tail member's range: 32-bit positions, and a step
+// looks up to 64 past the last one.  (Another limit than the default is for
+// testing: it has every walk reach what otherwise takes rows of 2^27 entries.)
+#ifndef CSM_RANGE_MAX
+#define CSM_RANGE_MAX 0xffffff00u
+#endif
+constexpr uint32_t kRangeMax = CSM_RANGE_MAX;
+// 32 segments below this size fit in a range.
+constexpr uint32_t kRangeWide = kRangeMax / 32 + 1;
+
+// Graphs without row tables, or with rows that long, take instantiations of
+// their own (GEN below): the few instructions that look for either cost the
+// counting search of 2,000 insertions on a graph in L2 10 % and of 4,097 updates
+// on 2^19 vertices 7 %.
+static bool search_general(const DevGraph& g) { return !g.htab || g.n_cap >= kRangeWide; }
+
 // Levels a walk of this plan may use: 1 .. n - 2, or, where every order's
 // independent tail is counted, up to the tail with the class counters of
 // tail_stage above it.
@@ -61,8 +77,9 @@ static uint32_t search_levels(const Plan& plan, int mode) {
 }
 
 // Shared memory of one warp: its levels, then its walk's plan (WalkPlan).
-SearchShape search_shape_of(const Plan& plan, int mode) {
+SearchShape search_shape_of(const Plan& plan, int mode, const DevGraph& g) {
   SearchShape s;
+  s.general = search_general(g);
   s.levels = search_levels(plan, mode);
   const uint32_t words = 3 * plan.n + (plan.n_anchor ? plan.n_anchor - 1 : 0);  // every query edge but the anchor is a back entry once
   s.warp_bytes = s.levels * (uint32_t)sizeof(LevelSM) + ((4 * words + 15) & ~15u);
@@ -235,8 +252,8 @@ __device__ __noinline__ uint32_t seg_size_slow(const SearchParams& p, uint32_t v
 // candidate runs before the gather here as well (run_levels): left to
 // check_rest, behind the filter and one after another from the last position
 // on, the joins took the search of 65,536 updates on 2^22 vertices 310 ms
-// (166 ms now, with tables 117), of 4,097 on 2^19 29 (25, 19), of a
-// hash-enumerating 3,001 on 2^17 8.4 (5.5, 4.1).
+// (168 ms now, with tables 117), of 4,097 on 2^19 29 (27, 18), of a
+// hash-enumerating 3,001 on 2^17 8.4 (5.5, 4.0).
 __device__ __noinline__ uint32_t join_search(const SearchParams& p, const uint32_t* pool, uint32_t v, uint32_t c,
                                              uint32_t x) {
   uint64_t lo, hi;
@@ -249,9 +266,10 @@ __device__ __noinline__ uint32_t join_search(const SearchParams& p, const uint32
 // a word whose touched bit says that the edge's presence intervals must be
 // asked.  One probe of v's row table, or a binary search in v's segment where
 // the graph has no tables.
+template <bool GEN>
 __device__ __forceinline__ uint32_t join_find(const SearchParams& p, const uint32_t* pool, uint32_t v, uint32_t bw,
                                               uint32_t x) {
-  if (p.g.htab) return row_find(p.g, p.g.row[v], row_entry(x, back_el(bw), p.g.hlb));
+  if (!GEN || p.g.htab) return row_find(p.g, p.g.row[v], row_entry(x, back_el(bw), p.g.hlb));
   return join_search(p, pool, v, back_combo(bw), x);
 }
 
@@ -265,6 +283,7 @@ constexpr uint32_t kSelMask = 0x1fu, kSelTouched = 0x80u, kSelNone = 0xffu;
 // segment produced x (kSelNone: none) and `joined` one that was found before,
 // with word jhit (0xff: none).  The joins run one at a time and stop at the
 // first that fails; where no test needs the prefix, it is not walked.
+template <bool GEN>
 __device__ __forceinline__ bool check_rest(const SearchParams& p, const uint32_t* pool, const LevelSM* lv,
                                            const WalkPlan& wp, int d, uint32_t e, uint32_t pos, uint32_t x,
                                            uint32_t dsel, uint32_t joined, uint32_t jhit, int32_t t) {
@@ -278,7 +297,7 @@ __device__ __forceinline__ bool check_rest(const SearchParams& p, const uint32_t
     if (((joins >> j) & 1u) && ok) {
       const uint32_t b = __popc(bm & ((1u << j) - 1u));
       const uint32_t bw = wp.back(pos, b);
-      const uint32_t hit = b == joined ? jhit : join_find(p, pool, v, bw, x);
+      const uint32_t hit = b == joined ? jhit : join_find<GEN>(p, pool, v, bw, x);
       ok = hit != kSlotEmpty && (!(hit & kSlotTouched) || present_slow(p, v, back_combo(bw), x, t));
     }
   });
@@ -349,6 +368,28 @@ __device__ __forceinline__ bool pick_driver(const SearchParams& p, const LevelSM
   dn = best;
   bytes = b4;
   return !empty;
+}
+
+// The survivors of level d (one a lane: candidate x of entry `own`, driver
+// segment of `size` elements for the next position, 0: none) do not fit in one
+// range together: the first ones that do stay, one at least.  Returns the first
+// lane left out (32: none), and, in the upper half, the cursor of level d there.
+// Cold: it takes rows of 2^27 entries.
+__device__ __noinline__ unsigned long long range_refit(const uint32_t* pool, const LevelSM& S, uint32_t lane,
+                                                       uint32_t size, uint32_t own, uint32_t x, uint32_t cur) {
+  unsigned long long sum = size;
+#pragma unroll
+  for (int o = 1; o < 32; o <<= 1) {
+    const unsigned long long v = __shfl_up_sync(0xffffffffu, sum, o);
+    if (lane >= (uint32_t)o) sum += v;
+  }
+  const uint32_t out = __ballot_sync(0xffffffffu, size && sum > kRangeMax && sum != size);
+  if (!out) return 32ull | ((unsigned long long)cur << 32);
+  const uint32_t first = (uint32_t)__ffs((int)out) - 1u;
+  const uint32_t fx = __shfl_sync(0xffffffffu, x, first), fo = __shfl_sync(0xffffffffu, own, first);
+  const uint32_t beg = S.base[fo] + (fo ? S.incl[fo - 1] : 0u), end = S.base[fo] + S.incl[fo];
+  // a segment is sorted
+  return first | ((unsigned long long)((uint32_t)lower_bound_u32(pool, beg, end, fx) - S.base[fo]) << 32);
 }
 
 // Per-task accumulators, flushed to the update's counters when the task ends;
@@ -533,6 +574,7 @@ struct TailOut {
   uint32_t iters;
   bool stopped;                   // the update was stopped (deadline or stop flag)
 };
+template <bool GEN>
 __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t* pool, LevelSM* lv,
                                            const uint32_t* plan_words, uint32_t n, int L, uint32_t lane, uint32_t t,
                                            uint32_t anchor) {
@@ -552,6 +594,7 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
     const uint32_t ncls = (1u << g) - 1u;
     for (uint32_t c = 0; c < ncls; c++) cntr[c * 32 + lane] = 0;
     __syncwarp();
+    uint32_t done = 0;  // entries of member j taken so far, where they are taken one by one
 #pragma unroll 1
     for (uint32_t j = 0; j < g && !out.stopped; j++) {
       const uint32_t ps = A->gpos[gp + j];
@@ -564,8 +607,13 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
         } else {
           unsigned long long b4 = 0;
           if (!pick_driver(p, lv, wp, L, e_mine, false, 0u, ps, (int32_t)t, dlo, dn, dsel, jsel, jv, b4)) dn = 0;
-          out.bytes += b4;
+          if (!GEN || !done) out.bytes += b4;
         }
+      }
+      if (GEN && __any_sync(0xffffffffu, dn >= kRangeWide)) {  // not all in one range: member j again for every entry
+        const uint32_t todo = __ballot_sync(0xffffffffu, dn != 0) & ~done, who = todo & (0u - todo);
+        if (!((who >> lane) & 1u)) dn = 0;
+        done = todo == who ? 0u : done | who;
       }
       const uint32_t incl = warp_incl_scan(dn, lane);
       const uint32_t total = __shfl_sync(0xffffffffu, incl, 31);
@@ -598,17 +646,17 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
           bool ok = filter_bit(p, wp.qv(ps), x);
           if (ok && wp.nb(ps) > 1) {
             joined = o_sel >> 8;
-            jhit = join_find(p, pool, o_jv, wp.back(ps, joined), x);
+            jhit = join_find<GEN>(p, pool, o_jv, wp.back(ps, joined), x);
             ok = jhit != kSlotEmpty;
           }
-          if (ok && check_rest(p, pool, lv, wp, L, owner, ps, x, o_dsel, joined, jhit, (int32_t)t)) {
+          if (ok && check_rest<GEN>(p, pool, lv, wp, L, owner, ps, x, o_dsel, joined, jhit, (int32_t)t)) {
             uint32_t M = 1u << j;
             bool seen = false;
 #pragma unroll 1
             for (uint32_t i = 0; i < g && !seen; i++) {
               const uint32_t pi = A->gpos[gp + i];
               if (i == j || !filter_bit(p, wp.qv(pi), x) ||
-                  !check_rest(p, pool, lv, wp, L, owner, pi, x, kSelNone, 0xffu, 0u, (int32_t)t))
+                  !check_rest<GEN>(p, pool, lv, wp, L, owner, pi, x, kSelNone, 0xffu, 0u, (int32_t)t))
                 continue;
               if (i < j) seen = true;
               else M |= 1u << i;
@@ -618,6 +666,7 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
         }
       }
       __syncwarp();
+      if (GEN && done) j--;
     }
     gp += g;
     if (out.stopped) break;
@@ -681,7 +730,7 @@ struct WarpStat {
 // steps), and what they need next is a long chain of loads: they are gathered
 // over the level's steps in `wait` (x; entry, touched bit of the first join)
 // and go through it 32 at a time.
-template <int MODE>
+template <int MODE, bool GEN>
 __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t* pool, LevelSM* lv,
                                            const WalkPlan& wp, uint2* wait, int d, uint32_t lane, const Task& T,
                                            WarpStat& ws, TaskAcc& acc) {
@@ -713,7 +762,7 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
     if (at < total) {
       const LevelSM& L = lv[d];
       x = ld_stream(pool + (L.base[own] + at));
-      if (joins && g.htab) jrow = g.row[L.jv[own]];
+      if (joins && (!GEN || g.htab)) jrow = g.row[L.jv[own]];
     }
   };
   // a single update's own range is handed over at once, while every other warp
@@ -778,7 +827,7 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
     }
     if constexpr (MODE == 2) {
       if (d == tail_level) {
-        const TailOut r = tail_stage(p, pool, lv, wp.w, n, d, lane, t, T.anchor);
+        const TailOut r = tail_stage<GEN>(p, pool, lv, wp.w, n, d, lane, t, T.anchor);
         acc.bytes += r.bytes;
         acc.iters += r.iters;
         acc.cnt += r.sum;
@@ -812,9 +861,9 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
     uint32_t meta = own;
     bool valid = cur + lane < total;
     if (valid && joins) {
-      const uint32_t hit = g.htab ? row_find(g, jrow, row_entry(cx, lv[d].jel[own], g.hlb))
-                                  : join_search(p, pool, lv[d].jv[own],
-                                                back_combo(wp.back(pos, lv[d].jsel[own])), cx);
+      const uint32_t hit = !GEN || g.htab
+                               ? row_find(g, jrow, row_entry(cx, lv[d].jel[own], g.hlb))
+                               : join_search(p, pool, lv[d].jv[own], back_combo(wp.back(pos, lv[d].jsel[own])), cx);
       valid = hit != kSlotEmpty;
       meta |= (hit & kSlotTouched) >> 15;
     }
@@ -843,21 +892,33 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
     // injectivity, remaining joins, presence, next driver
     uint32_t ndlo = 0, ndn = 0, ndsel = 0, njsel = 0, njv = 0;
     uint32_t wx = 0, wown = 0;
+    unsigned long long nb4 = 0;
     valid = lane < held;
     if (valid) {
       const uint2 w = wait[lane];
       wx = w.x;
       wown = w.y & 31u;
       const uint32_t wsel = lv[d].dsel[wown];
-      valid = check_rest(p, pool, lv, wp, d, wown, pos, wx, wsel, joins ? lv[d].jsel[wown] : 0xffu,
-                         (w.y << 15) & kSlotTouched, (int32_t)t);
+      valid = check_rest<GEN>(p, pool, lv, wp, d, wown, pos, wx, wsel, joins ? lv[d].jsel[wown] : 0xffu,
+                              (w.y << 15) & kSlotTouched, (int32_t)t);
       if (valid && pos + 1 < n) {
-        unsigned long long nb4 = 0;
         valid = pick_driver(p, lv, wp, d, wown, true, wx, pos + 1, (int32_t)t, ndlo, ndn, ndsel, njsel, njv, nb4);
-        acc.bytes += nb4;
+        if (!GEN) acc.bytes += nb4;
       }
     }
     held = 0;
+    if constexpr (GEN) {
+      if (__any_sync(0xffffffffu, ndn >= kRangeWide)) {  // a leaf has no segment
+        const unsigned long long r = range_refit(pool, lv[d], lane, valid ? ndn : 0u, wown, wx, cur);
+        if ((uint32_t)r < 32u) {  // the level goes on from the first one left out
+          cur = (uint32_t)(r >> 32);
+          fresh = false;
+          valid = valid && lane < (uint32_t)r;
+          if (lane >= (uint32_t)r) nb4 = 0;
+        }
+      }
+      acc.bytes += nb4;
+    }
     const uint32_t mask = __ballot_sync(0xffffffffu, valid);
     if (!mask) continue;
     if (pos == n - 1) {
@@ -1057,7 +1118,7 @@ __device__ __noinline__ DonatedOut setup_donated(const SearchParams& p, LevelSM*
 
 // Kernel body; MODE 0 counts (and hashes), 1 also appends match sets, 2
 // counts independent tails (tail_stage).
-template <int W, int MODE>
+template <int W, int MODE, bool GEN>
 __device__ __forceinline__ void search_body(const SearchParams& p) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
   __shared__ uint4 task_scratch[W * 10];  // one 160-byte record per warp
@@ -1154,7 +1215,7 @@ __device__ __forceinline__ void search_body(const SearchParams& p) {
       d = r.depth;
     }
     if (lane == 0) ws.began = tb;
-    if (d > 0) run_levels<MODE>(p, pool, lv, wp, waiting[warp], d, lane, T, ws, acc);
+    if (d > 0) run_levels<MODE, GEN>(p, pool, lv, wp, waiting[warp], d, lane, T, ws, acc);
     if (T.upd < p.batch) flush_acc(p, T.upd, lane, acc);
     if (lane == 0) {
       if (p.dq) atomicSub(&p.q->pending, 1u);
@@ -1204,37 +1265,38 @@ constexpr int min_blocks(int w) { return w == 16 ? 1 : 16 / w; }
 
 template <int W, bool EN>
 __global__ void __launch_bounds__(W * 32, min_blocks(W)) k_search(const __grid_constant__ SearchParams p) {
-  search_body<W, EN ? 1 : 0>(p);
+  search_body<W, EN ? 1 : 0, false>(p);
 }
 
 template <int W>
 __global__ void __launch_bounds__(W * 32, min_blocks(W)) k_search_tail(const __grid_constant__ SearchParams p) {
-  search_body<W, 2>(p);
+  search_body<W, 2, false>(p);
+}
+
+// Graphs without row tables or with very long rows (search_general): eight warps
+// a block whatever is configured.
+template <int MODE>
+__global__ void __launch_bounds__(256, 2) k_search_general(const __grid_constant__ SearchParams p) {
+  search_body<8, MODE, true>(p);
 }
 
 namespace {
 
 using SearchKernel = void (*)(SearchParams);
 
-// mode: 0 plain, 1 match sets, 2 tail counting
 template <int W>
 SearchKernel search_kernel(int mode) {
   return mode == 2 ? k_search_tail<W> : mode == 1 ? k_search<W, true> : k_search<W, false>;
 }
 
-template <int W>
-cudaError_t search_occupancy(int* nb, size_t smem, int mode) {
-  const SearchKernel k = search_kernel<W>(mode);
-  const cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
-  return e != cudaSuccess ? e : cudaOccupancyMaxActiveBlocksPerMultiprocessor(nb, k, W * 32, smem);
-}
-
-// A shape that does not fit is not launched; the caller's cudaGetLastError reports it.
-template <int W>
-void search_launch(const SearchParams& p, uint32_t blocks, size_t smem, cudaStream_t s, int mode) {
-  const SearchKernel k = search_kernel<W>(mode);
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
-    k<<<blocks, W * 32, smem, s>>>(p);
+// mode: 0 plain, 1 match sets, 2 tail counting; `warps` is set to what the kernel takes
+SearchKernel search_kernel(uint32_t& warps, int mode, bool general) {
+  if (warps != 4 && warps != 16) warps = 8;
+  if (general) {
+    warps = 8;
+    return mode == 2 ? k_search_general<2> : mode == 1 ? k_search_general<1> : k_search_general<0>;
+  }
+  return warps == 4 ? search_kernel<4>(mode) : warps == 16 ? search_kernel<16>(mode) : search_kernel<8>(mode);
 }
 
 }  // namespace
@@ -1244,29 +1306,24 @@ void search_launch(const SearchParams& p, uint32_t blocks, size_t smem, cudaStre
 // occupancy API.  `mode` selects the instantiation: 0 plain counting (and hashes), 1 match
 // sets, 2 tail counting.
 uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode) {
+  const SearchKernel k = search_kernel(warps, mode, shape.general);
   const size_t smem = (size_t)shape.warp_bytes * warps;
   int nb = 0;
-  cudaError_t e = cudaSuccess;
-  switch (warps) {
-    case 4: e = search_occupancy<4>(&nb, smem, mode); break;
-    case 16: e = search_occupancy<16>(&nb, smem, mode); break;
-    default: e = search_occupancy<8>(&nb, smem, mode); break;
-  }
+  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, (int)warps * 32, smem);
   if (e != cudaSuccess) { cudaGetLastError(); return 0; }
   return (uint32_t)nb;
 }
 
 int search_mode(const SearchParams& p) { return p.enum_buf ? 1 : (p.tail ? 2 : 0); }
 
+// A shape that does not fit is not launched; the caller's cudaGetLastError reports it.
 void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s, bool prepared) {
-  const size_t smem = (size_t)p.warp_bytes * warps;
   if (p.q && !prepared) k_search_prep<<<1, 1, 0, s>>>(p.q, p.n_tasks, p.task_cap, p.sstat, p.error);
-  const int mode = search_mode(p);
-  switch (warps) {
-    case 4: search_launch<4>(p, blocks, smem, s, mode); break;
-    case 16: search_launch<16>(p, blocks, smem, s, mode); break;
-    default: search_launch<8>(p, blocks, smem, s, mode); break;
-  }
+  const SearchKernel k = search_kernel(warps, search_mode(p), search_general(p.g));
+  const size_t smem = (size_t)p.warp_bytes * warps;
+  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
+    k<<<blocks, warps * 32, smem, s>>>(p);
 }
 
 __global__ void k_finalize(uint32_t B, ResultArgs a) {

@@ -846,6 +846,9 @@ static int run_edge_batch_graph(csm_ctx* ctx, const csm_update* ups, uint32_t B_
 static int submit_common(csm_ctx* ctx, uint64_t n, const csm_update* d_ups, const csm_update* h_ups) {
   if (ctx->owner) return set_err(CSM_ESTATE, "updates of an attached query are submitted to its owner");
   if (!ctx->has_graph || !ctx->has_plan) return set_err(CSM_ESTATE, "load the query, the graph and build the index first");
+  // the copied error word does not stand for this submit, also when it fails
+  // halfway: what is queued until then may set the device's
+  ctx->pin_ps = false;
   int rc = ensure_batch_buffers(ctx);
   if (rc) return rc;
   rc = ensure_results(ctx, n);

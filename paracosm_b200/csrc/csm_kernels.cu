@@ -721,7 +721,6 @@ __device__ __forceinline__ void mut_delete(const VRange* ranges, uint32_t nr, co
       const uint32_t q = (uint32_t)lower_bound_u32(pool + off, dirx[c], dirx[c + 1], y);
       del_pos[s + j] = q;
       if (q >= dirx[c + 1] || pool[off + q] != y) missing = true;
-      else if (g.htab) row_table_delete(g, x, row, row_entry(y, c % g.n_el, g.hlb));
     }
     // a deleted entry missing from its row: leave the row, report
     if (G == 32) { __syncwarp(); missing = __any_sync(0xffffffffu, missing); }
@@ -729,6 +728,13 @@ __device__ __forceinline__ void mut_delete(const VRange* ranges, uint32_t nr, co
     if (missing) {
       if (lane == 0) atomicExch(&g.ps->error, kErrRowState);
       continue;
+    }
+    if (g.htab) {  // only now: the table follows the row
+      for (uint32_t j = lane; j < k; j += G) {
+        const uint64_t key = del_key[s + j];
+        row_table_delete(g, x, row, row_entry(g.kb.y_of(key), g.kb.c_of(key) % g.n_el, g.hlb));
+      }
+      group_sync<G>();
     }
     const uint32_t tomb = g.htab ? g.htomb[x] : 0u;  // read by every thread well before a build clears it
     group_delete_move<G>(pool, off, deg, del_pos + s, k, lane);

@@ -22,7 +22,10 @@ struct DevMem {
     if (budget && bytes + sz > budget)
       return set_err(CSM_ENOMEM, "HBM budget of %llu bytes exceeded", (unsigned long long)budget);
     cudaError_t e = cudaMalloc(p, sz);
-    if (e != cudaSuccess) return set_err(CSM_ENOMEM, "cudaMalloc(%zu): %s", sz, cudaGetErrorString(e));
+    if (e != cudaSuccess) {
+      cudaGetLastError();  // a caller that does without must not find it after its next launch
+      return set_err(CSM_ENOMEM, "cudaMalloc(%zu): %s", sz, cudaGetErrorString(e));
+    }
     ptrs.push_back(*p);
     bytes += sz;
     return CSM_OK;

@@ -301,8 +301,8 @@ __global__ void k_ring_init(SearchQueue* q, unsigned long long* seq, uint32_t qc
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < qcap; i += gridDim.x * blockDim.x) seq[i] = i;
 }
 
-static int ensure_batch_buffers(csm_ctx* ctx) {
-  if (ctx->d_ukey) return CSM_OK;
+// The batch buffers' sizes and, once allocated, their places.
+static int batch_block(csm_ctx* ctx, DevBlock& blk) {
   const uint32_t B = ctx->bmax;
   const uint32_t L = list_slots(B);
   ctx->lcap = L;
@@ -319,7 +319,6 @@ static int ensure_batch_buffers(csm_ctx* ctx) {
   }
   ctx->cub_bytes = std::max(b1, std::max(b2, b3));
   ctx->qcap = 1u << 16;  // outstanding handed-over tasks never exceed the idle warps
-  DevBlock blk;
 #define AL(p, sz) blk.add(p, sz)
   AL(ctx->d_ukey, 8ull * B); AL(ctx->d_ukey2, 8ull * B);
   AL(ctx->d_useq, 4ull * B); AL(ctx->d_useq2, 4ull * B);
@@ -348,10 +347,20 @@ static int ensure_batch_buffers(csm_ctx* ctx) {
   AL(ctx->d_dq, sizeof(DTask) * (size_t)ctx->qcap);
   AL(ctx->d_qseq, 8ull * ctx->qcap);
   AL(ctx->d_cub, ctx->cub_bytes);
+  if (!ctx->g.t_tab) AL(ctx->g.t_tab, sizeof(ulonglong2) * (size_t)temporal_slots(B));  // an attached query has its owner's
 #undef AL
-  void* base = nullptr;
-  int rc = blk.alloc(ctx->mem, &base);
+  return CSM_OK;
+}
+
+static int ensure_batch_buffers(csm_ctx* ctx) {
+  if (ctx->d_ukey) return CSM_OK;
+  DevBlock blk;
+  int rc = batch_block(ctx, blk);
   if (rc) return rc;
+  void* base = nullptr;
+  rc = blk.alloc(ctx->mem, &base);
+  if (rc) return rc;
+  const uint32_t B = ctx->bmax;
   if (ctx->d_enum_n) CK(cudaMemsetAsync(ctx->d_enum_n, 0, 16, ctx->st));
   if (ctx->d_gpad) {
     std::vector<csm_update> pad(B, csm_update{'e', 1, 0, 0, 0, 0});
@@ -1556,7 +1565,6 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
     blk.add(g.vlabel, 4ull * n_cap);
     blk.add(g.row, 8ull * n_cap);
     blk.add(g.dir, 4ull * n_cap * (nc + 1));
-    blk.add(g.t_tab, sizeof(ulonglong2) * (size_t)temporal_slots(ctx->bmax));
     blk.add(g.t_count, 4ull * n_cap);
     blk.add(g.ps, sizeof(PoolState));
     blk.add(ctx->d_qlab, 4ull * (ctx->qlab_v.size() + ctx->qlab_e.size()));
@@ -1600,12 +1608,11 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
     uint64_t* k = nullptr;
     CK(cub::DeviceRadixSort::SortPairs(nullptr, tb, k, k, k, k, (int64_t)n_e, 0, 64, st));
     CK(cub::DeviceRadixSort::SortKeys(nullptr, tb2, k, k, (int64_t)M, 0, (int)kb.total(), st));
-    CK(cub::DeviceScan::ExclusiveSum(nullptr, tb3, k, k, (int64_t)n_cap, st));
+    CK(cub::DeviceScan::ExclusiveSum(nullptr, tb3, k, k, (int64_t)n_cap, st));  // in place
   }
   const size_t tbmax = std::max(tb, std::max(tb2, tb3));
-  uint32_t *d_e = nullptr, *cap32 = nullptr;
-  uint64_t *dkey = nullptr, *ukey2 = nullptr, *uidx2 = nullptr, *dkey2 = nullptr;
-  uint64_t *first = nullptr, *cap64 = nullptr, *off64 = nullptr;
+  uint32_t* d_e = nullptr;
+  uint64_t *dkey = nullptr, *ukey2 = nullptr, *uidx2 = nullptr, *dkey2 = nullptr, *first = nullptr;
   unsigned long long* d_small = nullptr;
   void *tmp = nullptr, *early = nullptr, *late = nullptr;
   DevBlock blk1, blk2;
@@ -1617,9 +1624,6 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   blk2.add(d_small, 64);
   blk2.add(dkey2, 8ull * M);
   blk2.add(first, 8ull * n_cap);
-  blk2.add(cap64, 8ull * n_cap);
-  blk2.add(off64, 8ull * n_cap);
-  blk2.add(cap32, 4ull * n_cap);
   rc = blk1.alloc(m, &early);
   if (!rc) rc = blk2.alloc(m, &late);
   if (rc) { m.release(early, blk1.total); return rc; }
@@ -1646,42 +1650,68 @@ int csm_gpu_load_graph(csm_ctx* ctx, uint32_t n_v, const uint32_t* vlabels, uint
   }
   if (M) { k_load_count<<<blocks_for(M, 256), 256, 0, st>>>(dkey2, M, kb, (uint32_t)nc, g.dir, first, d_small + 1); CKL(); }
   k_dir_scan<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc); CKL();
-  k_load_caps<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc, cap32, cap64); CKL();
-  tb = tbmax;
-  CK(cub::DeviceScan::ExclusiveSum(tmp, tb, cap64, off64, (int64_t)n_cap, st));
-  k_load_rows<<<blocks_for(n_cap, 256), 256, 0, st>>>(off64, cap32, n_cap, g.row); CKL();
-  unsigned long long last_off = 0, last_cap = 0, n_valid = 0;
-  CK(cudaMemcpyAsync(&last_off, off64 + (n_cap - 1), 8, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(&last_cap, cap64 + (n_cap - 1), 8, cudaMemcpyDeviceToHost, st));
-  CK(cudaMemcpyAsync(&n_valid, d_small + 1, 8, cudaMemcpyDeviceToHost, st));
+  // row offsets, in place of the rows until they are known; sums of the
+  // capacities (d_small + 2: with tables, + 3: without)
+  g.hlb = ceil_log2(n_el);
+  const bool entries_fit = ((uint64_t)n_cap << g.hlb) < (kSlotTomb & ~kSlotTouched);
+  uint64_t* off64 = reinterpret_cast<uint64_t*>(g.row);
+  auto lay_out = [&](bool tables) {
+    k_load_caps<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc, tables, off64, d_small + 2); CKL();
+    tb = tbmax;
+    CK(cub::DeviceScan::ExclusiveSum(tmp, tb, off64, off64, (int64_t)n_cap, st));
+    return CSM_OK;
+  };
+  rc = lay_out(entries_fit);
+  if (rc) return rc;
+  unsigned long long sums[3] = {0, 0, 0};  // n_valid, with, without
+  CK(cudaMemcpyAsync(sums, d_small + 1, sizeof(sums), cudaMemcpyDeviceToHost, st));
   CK(cudaStreamSynchronize(st));
-  const uint64_t used = last_off + last_cap;
-  const uint64_t pool_cap = 2 * used + 16ull * ctx->bmax + (1ull << 20);  // a multiple of four, as every row's capacity
+  const uint64_t n_valid = sums[0], with = sums[1], without = sums[2];
   m.release(early, blk1.total);  // before the pools: they are the peak
   auto fail = [&](int code) { m.release(late, blk2.total); return code; };
-  if (pool_cap >= (1ull << 32)) return fail(set_err(CSM_EUNSUPPORTED, "graph too large for 32-bit pool offsets"));
-  g.pool_cap = pool_cap;
-  rc = m.alloc((void**)&g.pools[0], 4ull * pool_cap);
-  if (!rc) rc = m.alloc((void**)&g.pools[1], 4ull * pool_cap);
-  if (rc) return fail(rc);
-  // row tables: two slots per row slot.  Without room for them, or when an id
-  // and a folded edge label do not fit in 31 bits, the search joins by binary
-  // search in the rows instead
+  PoolPlan plan = pool_plan(with, without, ctx->bmax, entries_fit);
+  if (!plan.ok) return fail(set_err(CSM_EUNSUPPORTED, "graph too large for 32-bit pool offsets"));
+  // the pools and, where the budget has room for them beside what the context
+  // allocates next, the row tables: two slots per row slot.  Without tables the
+  // search joins by binary search in the rows
   g.htab = nullptr;
   g.htomb = nullptr;
-  g.hlb = ceil_log2(n_el);
-  if (((uint64_t)n_cap << g.hlb) < (kSlotTomb & ~kSlotTouched)) {
-    uint32_t *tab = nullptr, *tomb = nullptr;
-    if (m.alloc((void**)&tab, 8ull * pool_cap) == CSM_OK && m.alloc((void**)&tomb, 4ull * n_cap) == CSM_OK) {
-      g.htab = tab;
-      g.htomb = tomb;
-      CK(cudaMemsetAsync(g.htab, 0xff, 8ull * used, st));
-      CK(cudaMemsetAsync(g.htomb, 0, 4ull * n_cap, st));
+  if (plan.tables) {
+    DevBlock later;
+    rc = batch_block(ctx, later);
+    if (rc) return fail(rc);
+    // batch buffers, plan, index; updates and results of a batch, InitialMatching
+    const uint64_t next = later.total + sizeof(Plan) + index_bytes(ctx->cfg.algorithm, ctx->nq, n_cap) +
+                          (sizeof(csm_update) + sizeof(csm_result)) * (uint64_t)std::max<uint32_t>(ctx->bmax, 1024) +
+                          16ull * n_cap + tb3 + 512;
+    const uint64_t want = 16ull * plan.cap + 4ull * n_cap, done = blk2.total;
+    void* mem[4] = {};
+    const size_t size[4] = {4ull * plan.cap, 4ull * plan.cap, 8ull * plan.cap, 4ull * n_cap};
+    bool got = !m.budget || m.bytes + want + (next > done ? next - done : 0) <= m.budget;
+    for (int i = 0; i < 4 && got; i++) got = m.alloc(&mem[i], size[i]) == CSM_OK;
+    if (got) {
+      g.pools[0] = static_cast<uint32_t*>(mem[0]);
+      g.pools[1] = static_cast<uint32_t*>(mem[1]);
+      g.htab = static_cast<uint32_t*>(mem[2]);
+      g.htomb = static_cast<uint32_t*>(mem[3]);
     } else {
-      m.release(tab, 8ull * pool_cap);
+      for (int i = 0; i < 4; i++) m.release(mem[i], size[i]);
       set_err(CSM_OK, "");  // the tables are optional
+      plan = pool_plan(with, without, ctx->bmax, false);
     }
   }
+  const uint64_t used = g.htab ? with : without;
+  g.pool_cap = plan.cap;
+  if (g.htab) {
+    CK(cudaMemsetAsync(g.htab, 0xff, 8ull * used, st));
+    CK(cudaMemsetAsync(g.htomb, 0, 4ull * n_cap, st));
+  } else {
+    rc = m.alloc((void**)&g.pools[0], 4ull * plan.cap);
+    if (!rc) rc = m.alloc((void**)&g.pools[1], 4ull * plan.cap);
+    if (!rc && entries_fit) rc = lay_out(false);
+    if (rc) return fail(rc);
+  }
+  k_load_rows<<<blocks_for(n_cap, 256), 256, 0, st>>>(g.dir, n_cap, (uint32_t)nc, g.htab != nullptr, g.row); CKL();
   PoolState ps{};
   ps.top[0] = used;
   CK(cudaMemcpyAsync(g.ps, &ps, sizeof(ps), cudaMemcpyHostToDevice, st));

@@ -62,4 +62,22 @@ struct DevBlock {
   }
 };
 
+// Slots of a row pool, and whether the rows have tables.  `with` and `without`:
+// slots of the loaded rows with capacities in multiples of four, as tables need
+// them, and as they come; `entries_fit`: an id and a label fit in a table entry.
+struct PoolPlan {
+  bool ok, tables;
+  uint64_t cap;
+};
+inline PoolPlan pool_plan(uint64_t with, uint64_t without, uint32_t max_batch, bool entries_fit) {
+  constexpr uint64_t kLimit = 1ull << 32;  // offsets have 32 bits
+  const uint64_t room = 16ull * max_batch + (1ull << 20), plain = 2 * without + room;
+  if (plain >= kLimit) return {false, false, 0};
+  // rounding may not take the room to grow: a pool cut off at the limit has to
+  // keep as many free slots as without tables
+  const uint64_t cap = std::min(2 * with + room, kLimit - 4);
+  if (entries_fit && cap >= with + (plain - without)) return {true, true, cap};
+  return {true, false, plain};
+}
+
 }  // namespace csm

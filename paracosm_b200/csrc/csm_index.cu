@@ -415,6 +415,21 @@ namespace {
 // marks fewer vertices (a list that overflows is worked off from its marks).
 constexpr uint32_t kListCap = 32768;
 
+constexpr uint32_t kListCapSmall = 64;
+
+// Words of a flag bitset: 32-byte aligned rows.
+uint64_t index_words(uint32_t n_cap) { return (((uint64_t)n_cap + 63) / 64 + 3) & ~3ull; }
+
+// An index's arrays.
+void index_block(IndexState& ix, DevBlock& blk, uint32_t nq, uint32_t n_cap, uint32_t list_cap) {
+  ix.bits.list_cap = std::min<uint32_t>(n_cap, list_cap);
+  blk.add(ix.bits.d1, 32ull * nq * index_words(n_cap));
+  blk.add(ix.d_dag, sizeof(IxDag));
+  blk.add(ix.d_pop, 16);
+  blk.add(ix.bits.list, 4ull * 2 * nq * ix.bits.list_cap);
+  blk.add(ix.bits.count, 8ull * nq + 4);
+}
+
 // Root choice (ParaCOSM/CSM/matching/SymBi/symbi.cpp:116-195, identical in
 // TurboFlux/turboflux.cpp:82-149): the first query edge (u < u', adjacency
 // order) of least frequency; of its endpoints the one whose label is rarer in
@@ -617,20 +632,17 @@ static int index_finish(IndexState& ix, DevMem& mem, const DevGraph& g, const In
     }
   }
 
-  // flag bitsets, 32-byte aligned rows
-  ix.words = ((uint64_t)g.n_cap + 63) / 64;
-  ix.words = (ix.words + 3) & ~3ull;
+  ix.words = index_words(g.n_cap);
   const uint64_t fam = 8ull * nq * ix.words;
-  ix.bits.list_cap = std::min<uint32_t>(g.n_cap, kListCap);
   ix.bits.words = ix.words;
   DevBlock blk;
-  blk.add(ix.bits.d1, 4 * fam);
-  blk.add(ix.d_dag, sizeof(IxDag));
-  blk.add(ix.d_pop, 16);
-  blk.add(ix.bits.list, 4ull * 2 * nq * ix.bits.list_cap);
-  blk.add(ix.bits.count, 8ull * nq + 4);
-  rc = blk.alloc(mem, &ix.block);
-  if (rc) return rc;
+  for (uint32_t cap = kListCap;; cap = kListCapSmall) {  // short lists where there is no room for long ones
+    blk = DevBlock{};
+    index_block(ix, blk, nq, g.n_cap, cap);
+    rc = blk.alloc(mem, &ix.block);
+    if (rc == CSM_OK) break;
+    if (cap == kListCapSmall) return rc;
+  }
   ix.block_bytes = blk.total;
   ix.bits.d2 = ix.bits.d1 + nq * ix.words;
   ix.bits.m1 = ix.bits.d2 + nq * ix.words;
@@ -644,6 +656,15 @@ static int index_finish(IndexState& ix, DevMem& mem, const DevGraph& g, const In
   if (rc) return rc;
   IXCK(cudaStreamSynchronize(st));
   return CSM_OK;
+}
+
+uint64_t index_bytes(int algo, uint32_t nq, uint32_t n_cap) {
+  if (algo != CSM_ALGO_TURBOFLUX && algo != CSM_ALGO_SYMBI && algo != CSM_ALGO_CALIG && algo != CSM_ALGO_NEWSP)
+    return 0;
+  IndexState ix;
+  DevBlock blk;
+  index_block(ix, blk, nq, n_cap, kListCap);
+  return blk.total;
 }
 
 int index_build(IndexState& ix, DevMem& mem, const DevGraph& g, const IndexQuery& q, int algo, int sm_count,

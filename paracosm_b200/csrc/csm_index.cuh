@@ -112,6 +112,8 @@ struct IndexState {
   uint64_t entries = 0, vertices = 0;
 };
 
+// Device memory of an index, at the most.
+uint64_t index_bytes(int algo, uint32_t nq, uint32_t n_cap);
 int index_build(IndexState& ix, DevMem& mem, const DevGraph& g, const IndexQuery& q, int algo, int sm_count,
                 cudaStream_t st, uint64_t* launches);
 // Brings the flags to the CSR as it is now, after the directed entries in

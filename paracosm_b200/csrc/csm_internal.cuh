@@ -113,7 +113,7 @@ struct DevGraph {
 // bit, mark empty and deleted slots.
 constexpr uint32_t kSlotEmpty = 0xffffffffu, kSlotTomb = 0xfffffffeu, kSlotTouched = 0x80000000u;
 __host__ __device__ __forceinline__ uint32_t row_entry(uint32_t y, uint32_t l, uint32_t hlb) { return (y << hlb) | l; }
-// A row's slots come in multiples of four, so that its table starts on a bucket.
+// With tables a row's slots come in multiples of four, so that its table starts on a bucket.
 __host__ __device__ __forceinline__ uint32_t row_round(uint32_t cap) { return (cap + 3u) & ~3u; }
 // Home bucket of an entry in a row table of `buckets` buckets.
 __device__ __forceinline__ uint32_t row_bucket(uint32_t entry, uint32_t buckets) {

@@ -128,20 +128,43 @@ __global__ void k_load_count(const uint64_t* dkey, uint64_t M, KeyBits kb, uint3
   if (!kb.real(after) || (after >> kb.yb) != (k >> kb.yb)) atomicAdd(run, (uint32_t)(j + 1));
 }
 
-__device__ __forceinline__ uint32_t slack_cap(uint32_t d) { return d == 0 ? 0u : row_round(d + max(2u, d >> 2)); }
-__device__ __forceinline__ uint32_t grow_cap(uint32_t d) { return row_round(d + max(8u, d >> 1)); }
-
-__global__ void k_load_caps(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t* cap, uint64_t* cap64) {
-  uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v >= n_cap) return;
-  const uint32_t c = slack_cap(dir[(size_t)v * (nc + 1) + nc]);
-  cap[v] = c;
-  cap64[v] = c;
+// Capacities of a row of d entries when it is laid out and when it has to grow.
+__device__ __forceinline__ uint32_t slack_cap(uint32_t d, bool tables) {
+  const uint32_t c = d == 0 ? 0u : d + max(2u, d >> 2);
+  return tables ? row_round(c) : c;
+}
+__device__ __forceinline__ uint32_t grow_cap(uint32_t d, bool tables) {
+  const uint32_t c = d + max(8u, d >> 1);
+  return tables ? row_round(c) : c;
 }
 
-__global__ void k_load_rows(const uint64_t* off, const uint32_t* cap, uint32_t n_cap, uint2* row) {
+__global__ void k_load_caps(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t tables, uint64_t* cap64,
+                            unsigned long long* sums) {
   const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
-  if (v < n_cap) row[v] = make_uint2((uint32_t)off[v], cap[v]);
+  const uint32_t d = v < n_cap ? dir[(size_t)v * (nc + 1) + nc] : 0u;
+  const uint32_t with = slack_cap(d, true), without = slack_cap(d, false);
+  if (v < n_cap) cap64[v] = tables ? with : without;
+  __shared__ unsigned long long s_sum[2];
+  if (threadIdx.x < 2) s_sum[threadIdx.x] = 0;
+  __syncthreads();
+  unsigned long long a = with, b = without;
+  for (int o = 16; o; o >>= 1) {
+    a += __shfl_down_sync(0xffffffffu, a, o);
+    b += __shfl_down_sync(0xffffffffu, b, o);
+  }
+  if ((threadIdx.x & 31) == 0) {
+    atomicAdd(&s_sum[0], a);
+    atomicAdd(&s_sum[1], b);
+  }
+  __syncthreads();
+  if (threadIdx.x < 2) atomicAdd(sums + threadIdx.x, s_sum[threadIdx.x]);
+}
+
+// In place: row[v] holds the row's offset as one word before.
+__global__ void k_load_rows(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t tables, uint2* row) {
+  const uint32_t v = blockIdx.x * blockDim.x + threadIdx.x;
+  if (v >= n_cap) return;
+  row[v] = make_uint2(row[v].x, slack_cap(dir[(size_t)v * (nc + 1) + nc], tables));
 }
 
 // One thread per directed entry: its place in the row and its slot in the row
@@ -430,7 +453,7 @@ __global__ void k_reloc_need(const VRange* ranges, const unsigned int* n_ranges,
   if (i < *n_ranges) {
     const VRange r = ranges[i];
     const uint32_t deg = g.dir[(size_t)r.x * (g.nc + 1) + g.nc];
-    if (deg + r.count > g.row[r.x].y) need = grow_cap(deg + r.count);
+    if (deg + r.count > g.row[r.x].y) need = grow_cap(deg + r.count, g.htab);
   }
   // warp-aggregated add
   for (int o = 16; o; o >>= 1) need += __shfl_down_sync(0xffffffffu, need, o);
@@ -490,7 +513,7 @@ __global__ void k_compact_copy(DevGraph g) {
   for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x; v0 < g.n_cap; v0 += (uint64_t)gridDim.x * blockDim.x) {
     const uint64_t v = v0 + threadIdx.x;
     uint32_t deg = 0, cap = 0;
-    if (v < g.n_cap) { deg = g.dir[v * (g.nc + 1) + g.nc]; cap = slack_cap(deg); }
+    if (v < g.n_cap) { deg = g.dir[v * (g.nc + 1) + g.nc]; cap = slack_cap(deg, g.htab); }
     scan[threadIdx.x] = cap;
     __syncthreads();
     for (uint32_t o = 1; o < blockDim.x; o <<= 1) {  // inclusive scan
@@ -649,7 +672,7 @@ __device__ __forceinline__ void mut_insert(const VRange* ranges, uint32_t nr, co
     uint64_t dst_off = off;
     uint32_t new_cap = 0;
     if (new_deg > old.y) {
-      new_cap = grow_cap(new_deg);
+      new_cap = grow_cap(new_deg, g.htab);
       if (lane == 0) {
         unsigned long long o = atomicAdd(&ps->top[ps->active], (unsigned long long)new_cap);
         if (o + new_cap > g.pool_cap) { atomicExch(&ps->error, kErrPoolFull); o = ~0ULL; }
@@ -846,7 +869,7 @@ __global__ void k_plain_resolve(const csm_update* up, DevGraph g, UpdInfo* info,
   if (lane < 2 && (inf.flags & UF_MUT) && u.is_add) {
     const uint32_t v = lane ? y : x;
     const uint32_t deg = g.dir[(size_t)v * (g.nc + 1) + g.nc];
-    if (deg + 1 > g.row[v].y) need = grow_cap(deg + 1);
+    if (deg + 1 > g.row[v].y) need = grow_cap(deg + 1, g.htab);
   }
   need += __shfl_xor_sync(0xffffffffu, need, 1);
   if (lane == 0) {
@@ -886,7 +909,7 @@ __global__ void __launch_bounds__(256) k_plain_mutate(DevGraph g, const UpdInfo*
       if (lane == 0) s_pos = !add && (p >= end || pool[off + p] != y) ? kNone : p;  // a deleted entry must be there
     }
     if (add && deg + 1 > old.y) {
-      new_cap = grow_cap(deg + 1);
+      new_cap = grow_cap(deg + 1, g.htab);
       if (lane == 0) {
         unsigned long long o = atomicAdd(&ps->top[ps->active], (unsigned long long)new_cap);
         if (o + new_cap > g.pool_cap) { atomicExch(&ps->error, kErrPoolFull); o = ~0ULL; }

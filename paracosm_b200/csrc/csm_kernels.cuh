@@ -18,8 +18,11 @@ __global__ void k_load_directed(const uint64_t* ukey, const uint64_t* uidx, uint
                                 DevGraph g, uint64_t* dkey);
 __global__ void k_load_count(const uint64_t* dkey, uint64_t M, KeyBits kb, uint32_t nc, uint32_t* dir,
                              uint64_t* first, unsigned long long* n_valid);
-__global__ void k_load_caps(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t* cap, uint64_t* cap64);
-__global__ void k_load_rows(const uint64_t* off, const uint32_t* cap, uint32_t n_cap, uint2* row);
+// Row capacities for a graph with row tables or without, and the sums of both
+// (sums[0]: with, sums[1]: without).
+__global__ void k_load_caps(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t tables, uint64_t* cap64,
+                            unsigned long long* sums);
+__global__ void k_load_rows(const uint32_t* dir, uint32_t n_cap, uint32_t nc, uint32_t tables, uint2* row);
 __global__ void k_load_scatter(const uint64_t* dkey, uint64_t M, const uint64_t* first, DevGraph g, uint32_t* pool);
 __global__ void k_dir_scan(uint32_t* dir, uint32_t n_cap, uint32_t nc);
 

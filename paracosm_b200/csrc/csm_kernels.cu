@@ -537,9 +537,13 @@ __global__ void k_compact_copy(DevGraph g) {
       if (rdeg && g.htab)
         row_table_build<32>(g, dp, (uint32_t)x, make_uint2(roff, rcap), g.dir + x * (g.nc + 1), rdeg, lane);
     }
-    if (v < g.n_cap && fits) {
-      g.row[v] = make_uint2((uint32_t)off, cap);
-      if (deg == 0 && g.htab) g.htomb[v] = 0;
+    if (v < g.n_cap) {
+      // a row that finds no room is lost, and the context in error; it must not
+      // point into the other pool's slots, which nobody has written
+      g.row[v] = fits ? make_uint2((uint32_t)off, cap) : make_uint2(0, 0);
+      if (!fits)
+        for (uint32_t c = 0; c <= g.nc; c++) g.dir[v * (g.nc + 1) + c] = 0;
+      if ((deg == 0 || !fits) && g.htab) g.htomb[v] = 0;
     }
     __syncthreads();
   }

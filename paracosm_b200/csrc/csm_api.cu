@@ -757,7 +757,6 @@ static int run_vertex_update(csm_ctx* ctx, const csm_update* ups, const csm_upda
     if (rc) return rc;
   }
   k_vertex_update<<<1, 32, 0, st>>>(ups, 1, ctx->g, ctx->d_info); CKL();
-  CK(cudaMemsetAsync(ctx->d_safe, 0xff, 4, st));
   ResultArgs ra{};
   ra.info = ctx->d_info;
   ra.out = out;
@@ -976,7 +975,7 @@ static int check_device_error(csm_ctx* ctx) {
   if (ps.error) {
     static const char* names[] = {"none", "row pool exhausted", "batch list overflow", "task list overflow",
                                   "search queue wait limit", "malformed donated task", "ring left undrained",
-                                  "task time guard", "row state", "edge table full"};
+                                  "task time guard", "row state", "row table full"};
     char extra[256] = "";
     if (ctx->d_sstat) {
       SearchStats ss;

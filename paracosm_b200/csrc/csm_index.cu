@@ -64,7 +64,7 @@ __device__ __forceinline__ bool warp_support(const uint32_t* pool, uint64_t lo, 
 // Per query edge (u < u' in adjacency order): directed entries v -> v' with
 // L(v) = L(u), L(v') = L(u') and the edge's label = sum over v of L(u) of the
 // segment size S(v, L(u'), l).  Also the number of vertices per folded label.
-__global__ void k_ix_freq(DevGraph g, uint32_t ne, const uint32_t* __restrict__ eu, const uint32_t* __restrict__ ecombo,
+__global__ void k_ix_freq(DevGraph g, uint32_t ne, const uint32_t* __restrict__ ecombo,
                           const uint32_t* __restrict__ elab_u, unsigned long long* freq, unsigned long long* lcount) {
   __shared__ unsigned long long s_freq[kMaxQE];
   __shared__ unsigned long long s_lc[kMaxQ + 1];
@@ -83,7 +83,6 @@ __global__ void k_ix_freq(DevGraph g, uint32_t ne, const uint32_t* __restrict__ 
       if (sz) atomicAdd(&s_freq[e], (unsigned long long)sz);
     }
   }
-  (void)eu;
   __syncthreads();
   for (uint32_t i = threadIdx.x; i < ne; i += blockDim.x)
     if (s_freq[i]) atomicAdd(&freq[i], s_freq[i]);
@@ -477,25 +476,23 @@ static int dag_for(const IndexQuery& q, const DevGraph& g, int algo,
   const auto& el = *q.elabel;
   const uint32_t ne = (uint32_t)edges.size();
   // frequencies on the device
-  std::vector<uint32_t> h_eu(ne), h_ec(ne), h_el(ne);
+  std::vector<uint32_t> h_ec(ne), h_el(ne);
   for (uint32_t i = 0; i < ne; i++) {
-    h_eu[i] = edges[i].first;
     h_ec[i] = ql[edges[i].second] * g.n_el + e_lab[i];
     h_el[i] = ql[edges[i].first];
   }
   uint32_t* d_e = nullptr;
   unsigned long long* d_f = nullptr;
   DevBlock blk;
-  blk.add(d_e, 12ull * ne);
+  blk.add(d_e, 8ull * ne);
   blk.add(d_f, 8ull * (ne + kMaxQ + 1));
   void* tmp = nullptr;
   const int rc = blk.alloc(mem, &tmp);
   if (rc) return rc;
-  IXCK(cudaMemcpyAsync(d_e, h_eu.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
-  IXCK(cudaMemcpyAsync(d_e + ne, h_ec.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
-  IXCK(cudaMemcpyAsync(d_e + 2 * ne, h_el.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
+  IXCK(cudaMemcpyAsync(d_e, h_ec.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
+  IXCK(cudaMemcpyAsync(d_e + ne, h_el.data(), 4ull * ne, cudaMemcpyHostToDevice, st));
   IXCK(cudaMemsetAsync(d_f, 0, 8ull * (ne + kMaxQ + 1), st));
-  k_ix_freq<<<sm_count * 4, 256, 0, st>>>(g, ne, d_e, d_e + ne, d_e + 2 * ne, d_f, d_f + ne);
+  k_ix_freq<<<sm_count * 4, 256, 0, st>>>(g, ne, d_e, d_e + ne, d_f, d_f + ne);
   (*launches)++;
   IXCK(cudaGetLastError());
   std::vector<unsigned long long> freq(ne + kMaxQ + 1);
@@ -588,13 +585,11 @@ static int index_finish(IndexState& ix, DevMem& mem, const DevGraph& g, const In
       const uint32_t p = par[u][i], l = par_l[u][i];
       D.par[u][i] = (uint8_t)p;
       D.par_vcombo[u][i] = (uint16_t)(ql[p] * g.n_el + l);
-      D.par_ucombo[u][i] = (uint16_t)(ql[u] * g.n_el + l);
     }
     for (size_t i = 0; i < chd[u].size(); i++) {
       const uint32_t c = chd[u][i], l = chd_l[u][i];
       D.chd[u][i] = (uint8_t)c;
       D.chd_vcombo[u][i] = (uint16_t)(ql[c] * g.n_el + l);
-      D.chd_ucombo[u][i] = (uint16_t)(ql[u] * g.n_el + l);
       D.ep[D.n_edges] = (uint8_t)u; D.ec[D.n_edges] = (uint8_t)c; D.eel[D.n_edges] = (uint16_t)l;
       D.n_edges++;
     }

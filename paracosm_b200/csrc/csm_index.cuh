@@ -58,9 +58,7 @@ struct IxDag {
   uint32_t npar[kMaxQ], nchd[kMaxQ];
   uint8_t par[kMaxQ][kMaxQ], chd[kMaxQ][kMaxQ];
   uint16_t par_vcombo[kMaxQ][kMaxQ];  // combo (L(p), l(u,p)): from a vertex of u to its parent-side neighbours
-  uint16_t par_ucombo[kMaxQ][kMaxQ];  // combo (L(u), l(u,p)): from a vertex of p to its u-side neighbours
   uint16_t chd_vcombo[kMaxQ][kMaxQ];  // combo (L(c), l(u,c))
-  uint16_t chd_ucombo[kMaxQ][kMaxQ];  // combo (L(u), l(u,c))
   uint8_t ep[kMaxQE], ec[kMaxQE];    // DAG edge list: parent, child
   uint16_t eel[kMaxQE];              // folded edge label
   // lighting mode: d2 draws its support from the children's d1, and d1

@@ -71,7 +71,7 @@ struct PoolState {
   uint32_t arrived;           // blocks of a kernel that have arrived (last_block)
 };
 enum : uint32_t { kErrNone = 0, kErrPoolFull = 1, kErrListOverflow = 2, kErrTaskOverflow = 3, kErrWaitTimeout = 4,
-                  kErrBadTask = 5, kErrRingState = 6, kErrTaskGuard = 7, kErrRowState = 8, kErrEdgeTable = 9 };
+                  kErrBadTask = 5, kErrRingState = 6, kErrTaskGuard = 7, kErrRowState = 8, kErrRowTable = 9 };
 
 // Device view of the dynamic CSR (pointers into device memory).
 struct DevGraph {
@@ -117,7 +117,9 @@ __host__ __device__ __forceinline__ uint32_t row_entry(uint32_t y, uint32_t l, u
 __host__ __device__ __forceinline__ uint32_t row_round(uint32_t cap) { return (cap + 3u) & ~3u; }
 // Home bucket of an entry in a row table of `buckets` buckets.
 __device__ __forceinline__ uint32_t row_bucket(uint32_t entry, uint32_t buckets) {
-  uint32_t h = entry * 0x9E3779B1u;  // multiplicative hashing, folded once so that the low bits count too
+  // multiplicative hashing, folded once so that the low bits count too; the
+  // multipliers are the first two primes of xxHash32
+  uint32_t h = entry * 0x9E3779B1u;
   h ^= h >> 15;
   h *= 0x85EBCA77u;
   return __umulhi(h, buckets);
@@ -135,9 +137,8 @@ __device__ __forceinline__ RowBucket ld_bucket(const uint32_t* a) {
   return RowBucket{{(uint32_t)w0, (uint32_t)(w0 >> 32), (uint32_t)w1, (uint32_t)(w1 >> 32), (uint32_t)w2,
                     (uint32_t)(w2 >> 32), (uint32_t)w3, (uint32_t)(w3 >> 32)}};
 }
-// Loads of driver segments, read once per use: they may fill L1 but go first when L1 needs room,
-// so they do not push out the lines that are reused -- the search's register
-// spills and the plan.
+// Loads of driver segments, read once per use: they may fill L1 (the next step
+// reads on in the line) but go first when L1 needs room.
 __device__ __forceinline__ uint32_t ld_stream(const uint32_t* a) {
   uint32_t v;
   asm("ld.global.L1::evict_first.u32 %0, [%1];" : "=r"(v) : "l"(a));
@@ -151,17 +152,6 @@ __device__ __forceinline__ uint64_t ld_gather(const uint64_t* a) {
   asm("ld.global.L1::no_allocate.u64 %0, [%1];" : "=l"(v) : "l"(a));
   return v;
 }
-__device__ __forceinline__ uint32_t ld_gather(const uint32_t* a) {
-  uint32_t v;
-  asm("ld.global.L1::no_allocate.u32 %0, [%1];" : "=r"(v) : "l"(a));
-  return v;
-}
-
-// The word of `entry` in the row table of row r (with its touched bit), or
-// kSlotEmpty when it is not there.  One load settles nearly every search: at
-// the tables' load of 0.4 a bucket of 8 overflows for one row entry in 200,
-// where linear probing over single slots made a warp wait for the longest of
-// its 32 chains (about 8 dependent loads).
 // The word of `entry` in the row table of row r (with its touched bit), or
 // kSlotEmpty when it is not there.  One load settles nearly every search: at
 // the tables' load of 0.4 a bucket of 8 overflows for one row entry in 200,
@@ -201,10 +191,6 @@ __device__ __forceinline__ uint32_t fold_vlabel(const DevGraph& g, uint32_t l) {
   return l == kNone ? kNone : fold_label(g.qlab_v, g.n_qv, l);
 }
 __device__ __forceinline__ uint32_t fold_elabel(const DevGraph& g, uint32_t l) { return fold_label(g.qlab_e, g.n_qe, l); }
-
-__device__ __forceinline__ uint32_t combo_of(const DevGraph& g, uint32_t vl, uint32_t el) {
-  return vl * g.n_el + el;
-}
 
 // Segment [lo, hi) of combo c in row v, as absolute pool offsets.
 __device__ __forceinline__ void segment(const DevGraph& g, uint32_t v, uint32_t c, uint64_t& lo, uint64_t& hi) {

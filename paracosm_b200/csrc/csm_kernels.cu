@@ -28,7 +28,7 @@ __device__ __forceinline__ void row_table_insert(const DevGraph& g, uint2 r, uin
       if (b.k[i] == kSlotEmpty && atomicCAS(tab + 8ull * s + i, kSlotEmpty, entry) == kSlotEmpty) return;
     if (++s == buckets) s = 0;
   }
-  atomicExch(&g.ps->error, kErrEdgeTable);  // no empty slot left
+  atomicExch(&g.ps->error, kErrRowTable);  // no empty slot left
 }
 
 // Slot of `entry` in a row table (offset from its start), or kSlotEmpty;
@@ -494,8 +494,10 @@ __device__ __forceinline__ void row_table_build(const DevGraph& g, const uint32_
 }
 
 // Deleted slots a row's table may hold before a deletion builds it afresh: a
-// quarter of the row's capacity keeps the table (twice the capacity) below
-// two thirds full, so that most buckets keep an empty slot.
+// quarter of the row's capacity keeps the table (twice the capacity) at most
+// five eighths full, so that most buckets keep an empty slot; rows of up to 16
+// slots may have four (with eight live entries of a table of 16, three quarters).
+// A batch's own deletions come on top until its check.
 __device__ __forceinline__ uint32_t tomb_limit(uint32_t cap) { return max(4u, cap >> 2); }
 
 // Copies every row into the other pool with fresh slack (runs only when the

@@ -144,7 +144,7 @@ struct SearchStats {
   // first task stopped by the task time guard: its depth, iterations, update and level cursors
   unsigned int guard_set, guard_d, guard_upd, guard_pad;
   unsigned long long guard_iters;
-  unsigned int guard_lv[4 * 16];  // per level 1..16: cnt, cur_e, cur_k, dn[cur_e]
+  unsigned int guard_lv[4 * 16];  // per level 1..16: cnt, cur, total, incl[0]
 };
 
 // What the results of a batch's updates are made of.

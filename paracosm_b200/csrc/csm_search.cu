@@ -720,7 +720,8 @@ struct WarpStat {
 // What bounds a step is how many cache lines the SM can have in flight: its
 // loads are scattered over the lanes, and with 24 warps of 80 registers the
 // spilled ones swept through L1 with them and came back from L2.  Sixteen
-// warps of 128 registers spill nothing (12,000 -> 4,200 cycles a step, and the
+// warps of 128 registers spill nothing but six words where tails are counted
+// (12,000 -> 4,200 cycles a step, and the
 // search of a 65,536-update batch on the 2^22-vertex stream 131 -> 68 ms).  So
 // the common step -- no candidate survives -- reads little: the level's cursor
 // and segment ends live in registers, the range layout of LevelSM needs no

@@ -271,6 +271,11 @@ __device__ __forceinline__ void ix_items(const DevGraph& g, const uint32_t* pool
 // updates do not tell them apart.
 constexpr uint32_t kAlone = 32;
 
+// Do the marks of L entries and ne DAG edges keep no more than these threads busy?
+__host__ __device__ constexpr bool ix_few(uint32_t L, uint32_t ne, uint32_t threads) { return (uint64_t)L * ne <= threads; }
+static_assert(ix_few(2, 256, 512) && !ix_few(3, 256, 512), "the limit itself");
+static_assert(!ix_few(1u << 24, 256, 512), "a vertex of 2^23 edges under a query of 256: the product passes 32 bits");
+
 __global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __restrict__ gdag, IxBits b, IxOrder ord,
                                                   const uint64_t* __restrict__ keys, uint32_t L, uint32_t vert) {
   cg::grid_group grid = cg::this_grid();
@@ -285,7 +290,7 @@ __global__ void __launch_bounds__(512) k_ix_round(DevGraph g, const IxDag* __res
   const uint32_t* pool = g.pools[g.ps->active];
   const uint32_t steps1 = ord.steps[0], steps = steps1 + ord.steps[1];
   const bool first = blockIdx.x == 0;
-  bool alone = L * ne <= blockDim.x;  // block 0 works, the others wait
+  bool alone = ix_few(L, ne, blockDim.x);  // block 0 works, the others wait
   uint32_t from = 0;                  // block 0: first step whose lists' lengths are to be taken back
   if (!alone || first) {
     const uint32_t tid = (alone ? 0u : blockIdx.x * blockDim.x) + threadIdx.x;
@@ -671,7 +676,6 @@ int index_build(IndexState& ix, DevMem& mem, const DevGraph& g, const IndexQuery
     return CSM_OK;
   const bool lighting = algo == CSM_ALGO_CALIG || algo == CSM_ALGO_NEWSP;
   const uint32_t nq = q.n;
-  const auto& ql = *q.vlabels;
   const auto& nbr = *q.nbr;
   const auto& el = *q.elabel;
   // query edges u < u' in adjacency order, as the frequency scan visits them

@@ -270,28 +270,34 @@ __device__ __forceinline__ bool touched_present(const DevGraph& g, uint32_t v, u
   return val == kTempEmpty || temporal_present(g, val, t);
 }
 
+// Entries of a segment's run [beg, end) of touched entries that are absent at
+// batch time t, as far as every step-th index from `at` on tells: an entry's
+// intervals do not overlap, so it is its first index less the one interval that
+// holds t.  Negative shares are made up for by others.  (Unrolled four times it
+// takes the registers of every search: counting ones 4 to 8 % slower.)
+__device__ __forceinline__ int32_t seg_absent(const DevGraph& g, uint32_t at, uint32_t beg, uint32_t end,
+                                              uint32_t step, int32_t t) {
+  int32_t absent = 0;
+#pragma unroll 1
+  for (uint32_t i = at; i < end; i += step) {
+    const bool first = i == beg || g.t_key[i - 1] != g.t_key[i];
+    const int2 sp = g.t_span[i];
+    absent += (int32_t)first - (int32_t)(sp.x <= t && t <= sp.y);
+  }
+  return absent;
+}
+
 // Number of entries of segment (v, c) present at batch time t, given its
 // union-graph bounds: entries touched in this batch and absent at t are
-// subtracted (an entry may carry several presence intervals).
+// subtracted.
 __device__ __forceinline__ uint32_t seg_size_at(const DevGraph& g, uint32_t v, uint32_t c, uint64_t lo, uint64_t hi,
                                                 int32_t t) {
-  uint32_t size = (uint32_t)(hi - lo);
+  const uint32_t size = (uint32_t)(hi - lo);
   if (size == 0 || g.t_count[v] == 0) return size;
   const uint64_t run = temporal_find(g, temporal_head(g, v, c));
   if (run == kTempEmpty) return size;
   const uint32_t beg = (uint32_t)run, end = beg + (uint32_t)(run >> 32);
-#pragma unroll 1
-  for (uint32_t i = beg; i < end;) {
-    const uint64_t key = g.t_key[i];
-    bool present = false;
-#pragma unroll 1
-    for (; i < end && g.t_key[i] == key; i++) {
-      const int2 sp = g.t_span[i];
-      if (sp.x <= t && t <= sp.y) present = true;
-    }
-    if (!present) size--;
-  }
-  return size;
+  return size - (uint32_t)seg_absent(g, beg, beg, end, 1, t);
 }
 
 // ---- query plan ------------------------------------------------------

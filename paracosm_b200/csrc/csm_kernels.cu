@@ -350,6 +350,20 @@ __global__ void k_resolve(const uint64_t* skey, const uint32_t* sseq, uint32_t B
   }
 }
 
+// First index after j, up to `end`, whose key is not below `limit` (key[j] is):
+// the end of a run in a sorted list.  Steps that double keep a run of one entry
+// at one load and a hub's at a few.
+__device__ __forceinline__ uint32_t run_end(const uint64_t* key, uint32_t j, uint32_t end, uint64_t limit) {
+  uint32_t lo = j, step = 1;
+  while (step < end - lo && key[lo + step] < limit) { lo += step; step <<= 1; }
+  uint32_t hi = step < end - lo ? lo + step : end;
+  while (hi - lo > 1) {
+    const uint32_t mid = (lo + hi) >> 1;
+    if (key[mid] < limit) lo = mid; else hi = mid;
+  }
+  return hi;
+}
+
 // Appends one VRange per vertex run of a sorted packed-key list.  pad = 1
 // marks a row longer than kBigRow entries before the batch: the mutation
 // kernels give such rows a whole block instead of a warp.
@@ -361,8 +375,7 @@ __global__ void k_ranges(const uint64_t* key, uint32_t cap, KeyBits kb, VRange* 
   if (!kb.real(k)) return;
   const uint32_t x = kb.x_of(k);
   if (j > 0 && kb.x_of(key[j - 1]) == x) return;
-  uint32_t t = j + 1;
-  while (t < cap && kb.real(key[t]) && kb.x_of(key[t]) == x) t++;
+  const uint32_t t = run_end(key, j, cap, kb.pack(x + 1, 0, 0));
   unsigned int i = atomicAdd(n_ranges, 1u);
   const uint32_t big = dir[(size_t)x * (nc + 1) + nc] > kBigRow ? 1u : 0u;
   ranges[i] = VRange{x, j, t - j, big};
@@ -400,15 +413,13 @@ __global__ void k_temporal_set(uint32_t L, DevGraph g) {
   }
   const uint64_t before = j > 0 ? g.t_key[j - 1] : ~0ULL;
   if (before != k) {  // the entry's intervals
-    uint32_t n = 1;
-    while (j + n < L && g.t_key[j + n] == k) n++;
+    const uint32_t n = run_end(g.t_key, j, L, k + 1) - j;
     const int2 s = g.t_span[j];
     temporal_put(g, k, n == 1 ? (uint64_t)(uint32_t)(s.x + 1) | ((uint64_t)(uint32_t)s.y << 32)
                               : kTempMany | (uint64_t)j | ((uint64_t)n << 32));
   }
   if (j > 0 && (before >> g.kb.yb) == (k >> g.kb.yb)) return;
-  uint32_t n = 1;  // the segment's entries
-  while (j + n < L && (g.t_key[j + n] >> g.kb.yb) == (k >> g.kb.yb)) n++;
+  const uint32_t n = run_end(g.t_key, j, L, ((k >> g.kb.yb) + 1) << g.kb.yb) - j;  // the segment's entries
   temporal_put(g, temporal_head(g, x, g.kb.c_of(k)), (uint64_t)j | ((uint64_t)n << 32));
   atomicAdd(&g.t_count[x], n);
 }

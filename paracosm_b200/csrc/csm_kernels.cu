@@ -513,50 +513,70 @@ __device__ __forceinline__ uint32_t tomb_limit(uint32_t cap) { return max(4u, ca
 
 // Copies every row into the other pool with fresh slack (runs only when the
 // active pool cannot absorb this batch's relocations) and builds its table at
-// its new place; each warp moves the 32 rows its threads sized.
-__global__ void k_compact_copy(DevGraph g) {
+// its new place.  The rows that a block's threads size lie side by side there: the
+// block empties their tables and takes their entries as one run, a thread an
+// entry, whatever the rows' lengths.  What bounds it is the chain of loads of an
+// entry's table insertion, so that no row may be one warp's: 3.5M rows and 11M
+// entries, the longest row of 52,000, took 18 ms row by row, a warp each, and
+// 2.5 ms so (4.1 ms for the copies alone, by a thread a row).
+__global__ void __launch_bounds__(1024) k_compact_copy(DevGraph g) {
   PoolState* ps = g.ps;
   if (!ps->compact) return;
   const uint32_t src = ps->active, dst = 1u - src;
   const uint32_t* sp = g.pools[src];
   uint32_t* dp = g.pools[dst];
   __shared__ unsigned long long base;
-  __shared__ uint32_t scan[1024];
-  const uint32_t lane = threadIdx.x & 31;
+  __shared__ uint32_t scan[1024], incl[1024];   // capacities and entries up to each row
+  __shared__ uint32_t s_from[1024];             // where each row comes from
+  const uint32_t me = threadIdx.x;
   for (uint64_t v0 = (uint64_t)blockIdx.x * blockDim.x; v0 < g.n_cap; v0 += (uint64_t)gridDim.x * blockDim.x) {
-    const uint64_t v = v0 + threadIdx.x;
+    const uint64_t v = v0 + me;
     uint32_t deg = 0, cap = 0;
     if (v < g.n_cap) { deg = g.dir[v * (g.nc + 1) + g.nc]; cap = slack_cap(deg, g.htab); }
-    scan[threadIdx.x] = cap;
+    scan[me] = cap;
+    incl[me] = deg;
+    s_from[me] = v < g.n_cap ? g.row[v].x : 0u;
     __syncthreads();
-    for (uint32_t o = 1; o < blockDim.x; o <<= 1) {  // inclusive scan
-      uint32_t t = threadIdx.x >= o ? scan[threadIdx.x - o] : 0;
+    for (uint32_t o = 1; o < blockDim.x; o <<= 1) {  // inclusive scans
+      const uint32_t t = me >= o ? scan[me - o] : 0, u = me >= o ? incl[me - o] : 0;
       __syncthreads();
-      scan[threadIdx.x] += t;
+      scan[me] += t;
+      incl[me] += u;
       __syncthreads();
     }
-    if (threadIdx.x == blockDim.x - 1) base = atomicAdd(&ps->top[dst], (unsigned long long)scan[threadIdx.x]);
+    if (me == blockDim.x - 1) base = atomicAdd(&ps->top[dst], (unsigned long long)scan[me]);
     __syncthreads();
-    const unsigned long long off = base + scan[threadIdx.x] - cap;
+    const unsigned long long off = base + scan[me] - cap;
     const bool fits = off + cap <= g.pool_cap;
     if (!fits) atomicExch(&ps->error, kErrPoolFull);
-    const uint64_t so = (fits && v < g.n_cap) ? g.row[v].x : 0;
-    for (uint32_t r = 0; r < 32; r++) {
-      const uint32_t rdeg = __shfl_sync(0xffffffffu, fits ? deg : 0u, r), rcap = __shfl_sync(0xffffffffu, cap, r);
-      const uint32_t roff = (uint32_t)__shfl_sync(0xffffffffu, off, r), rso = (uint32_t)__shfl_sync(0xffffffffu, so, r);
-      for (uint32_t i = lane; i < rdeg; i += 32) dp[(uint64_t)roff + i] = sp[(uint64_t)rso + i];
-      __syncwarp();
-      const uint64_t x = v - lane + r;
-      if (rdeg && g.htab)
-        row_table_build<32>(g, dp, (uint32_t)x, make_uint2(roff, rcap), g.dir + x * (g.nc + 1), rdeg, lane);
+    const uint32_t rows = (uint32_t)__syncthreads_count(fits);  // the first ones: offsets ascend
+    const uint32_t total = rows ? incl[rows - 1] : 0u;
+    if (g.htab) {
+      uint32_t* tab = g.htab + 2ull * base;
+      const unsigned long long words = rows ? 2ull * scan[rows - 1] : 0ull;
+      for (unsigned long long i = me; i < words; i += blockDim.x) tab[i] = kSlotEmpty;
+      __syncthreads();
     }
+    for (unsigned long long e = me; e < total; e += blockDim.x) {
+      uint32_t r = 0;  // rows that end before entry e
+#pragma unroll
+      for (uint32_t step = 512; step; step >>= 1)
+        if (incl[r + step - 1] <= e) r += step;
+      const uint32_t i = (uint32_t)e - (r ? incl[r - 1] : 0u), before = r ? scan[r - 1] : 0u;
+      const uint2 row = make_uint2((uint32_t)base + before, scan[r] - before);
+      const uint32_t y = sp[(uint64_t)s_from[r] + i];
+      dp[(uint64_t)row.x + i] = y;
+      if (g.htab)
+        row_table_insert(g, row, row_entry(y, combo_at(g.dir + (v0 + r) * (g.nc + 1), g.nc, i) % g.n_el, g.hlb));
+    }
+    __syncthreads();
     if (v < g.n_cap) {
       // a row that finds no room is lost, and the context in error; it must not
       // point into the other pool's slots, which nobody has written
       g.row[v] = fits ? make_uint2((uint32_t)off, cap) : make_uint2(0, 0);
       if (!fits)
         for (uint32_t c = 0; c <= g.nc; c++) g.dir[v * (g.nc + 1) + c] = 0;
-      if ((deg == 0 || !fits) && g.htab) g.htomb[v] = 0;
+      if (g.htab) g.htomb[v] = 0;
     }
     __syncthreads();
   }

@@ -536,7 +536,7 @@ static int query_seed_search(csm_ctx* q, csm_ctx* o, uint32_t B, csm_result* out
   sp.deadline_ns = q->cfg.deadline_ns;
   sp.donate_every = q->cfg.donate_every;
   sp.split_deep = q->cfg.split_deep;
-  sp.tail = (!q->cfg.want_hash && !q->d_enum && !q->cfg.tail_enumerate) ? 1u : 0u;
+  sp.tail = (!q->cfg.want_hash && !q->d_enum && !q->cfg.tail_enumerate) ? tail_first(sp.cap) : 0u;
   if (q->d_enum) {
     sp.enum_buf = q->d_enum; sp.enum_n = q->d_enum_n; sp.enum_cap = q->cfg.enum_capacity;
     sp.enum_base = (uint32_t)(out - q->d_results);  // this batch's first update within the submit
@@ -1097,7 +1097,7 @@ static int tune_run(csm_ctx* ctx, uint32_t B, uint32_t warps, uint32_t bps, floa
   sp.sstat = ctx->d_sstat;
   sp.donate_every = donate_every;
   sp.split_deep = split_deep;
-  sp.tail = (!ctx->cfg.want_hash && !ctx->d_enum && !ctx->cfg.tail_enumerate) ? 1u : 0u;  // as the batches run
+  sp.tail = (!ctx->cfg.want_hash && !ctx->d_enum && !ctx->cfg.tail_enumerate) ? tail_first(sp.cap) : 0u;  // as the batches run
   set_search_shape(sp, *ctx->h_plan);
   CK(cudaEventRecord(ctx->ev_start, st));
   launch_search(sp, (uint32_t)ctx->sm_count * bps, warps, st); CKL();
@@ -1291,7 +1291,7 @@ static int initial_match(csm_ctx* ctx, uint64_t* out) {
   sp.slot_limit_ns = 100ull * 1000000ull;
   sp.task_limit_ns = 20ull * 1000000000ull;
   sp.sstat = ctx->d_sstat;
-  sp.tail = ctx->cfg.tail_enumerate ? 0u : 1u;
+  sp.tail = ctx->cfg.tail_enumerate ? 0u : tail_first(sp.cap);
   set_search_shape(sp, *ctx->h_plan);
   // fitted to the instantiation that is launched here: a context that asks for
   // hashes or match sets searches its batches with another one, whose walks

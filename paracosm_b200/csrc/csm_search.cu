@@ -43,7 +43,8 @@ struct LevelSM {
   uint8_t dsel[32];   // back entry that is the driver (kSelTouched: its row has touched entries)
   uint8_t jsel[32];   // back entry of the first join: the smallest segment but the driver's
   uint8_t jel[32];    // its edge label
-  uint32_t cnt, cur, total, pad;
+  uint32_t cnt, cur, total;
+  uint32_t burst;     // tail's level: entries the next stage takes
 };
 
 // Elements of a level's or a tail member's range: 32-bit positions, and a step
@@ -559,8 +560,9 @@ __device__ __noinline__ unsigned long long group_assignments(uint32_t g, const u
   return f[full];
 }
 
-// Counts the completions of the entries of level L (= the anchor's tail_at:
-// complete matches of the positions before the independent tail).  For each
+// Counts the completions of the next LevelSM::burst entries of level L (= the
+// anchor's tail_at: complete matches of the positions before the independent
+// tail) and moves the level's cursor past them.  For each
 // label group of the tail, every member's candidates are listed from its
 // driver segment (32 (entry, element) pairs at a time, as in run_levels) and
 // classified by the other members they are candidates of; a candidate is
@@ -581,8 +583,11 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
   const PlanAnchor* A = &p.plan->anchors[anchor];
   const WalkPlan wp{plan_words, n};
   volatile unsigned int* stop = p.stop;
-  const LevelSM& S = lv[L];
-  const bool has = lane < S.cnt;
+  LevelSM& S = lv[L];
+  const uint32_t cnt = S.cnt, cur = S.cur;
+  const uint32_t first = __popc(__ballot_sync(0xffffffffu, lane < cnt && S.incl[lane] <= cur));
+  const uint32_t end = min(cnt, first + S.burst);
+  const bool has = lane >= first && lane < end;
   const uint32_t e_mine = has ? lane : 0u;
   uint32_t* cntr = reinterpret_cast<uint32_t*>(&lv[L + 1]);  // [class][entry], levels L+1.. are unused here
   TailOut out{0, 0, 0, false};
@@ -683,6 +688,12 @@ __device__ __noinline__ TailOut tail_stage(const SearchParams& p, const uint32_t
 #pragma unroll
   for (int o = 16; o; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
   out.sum = out.stopped ? 0ull : sum;
+  __syncwarp();
+  if (lane == 0) {
+    S.cur = S.incl[end - 1];
+    S.burst = min(32u, 2u * S.burst);
+  }
+  __syncwarp();
   return out;
 }
 
@@ -842,7 +853,8 @@ __device__ __forceinline__ void run_levels(const SearchParams& p, const uint32_t
           acc.cnt = 0;
           if (__shfl_sync(0xffffffffu, hit, 0)) break;
         }
-        cur = total;  // the stage took every entry
+        cur = lv[d].cur;
+        if (cur < total) continue;
       }
     }
     if (cur >= total) {  // level done (and none of its candidates waits)
@@ -1068,6 +1080,7 @@ __device__ __noinline__ RootOut setup_root(const SearchParams& p, LevelSM* lv, u
     lv[1].incl[0] = minsz; lv[1].base[0] = dlo0;
     lv[1].dsel[0] = (uint8_t)(sel | (touched ? kSelTouched : 0u));
     lv[1].v[0] = m1; lv[1].par[0] = 1; lv[1].v[1] = m0;
+    if (MODE == 2 && A->tail_at) lv[A->tail_at].burst = p.tail;
     lv[1].jsel[0] = (uint8_t)other;
     lv[1].jel[0] = P2.nb > 1 ? A->back_el[P2.boff + other] : 0;
     lv[1].jv[0] = P2.nb > 1 ? (A->back_pos[P2.boff + other] == 0 ? m0 : m1) : 0u;
@@ -1123,7 +1136,10 @@ __device__ __noinline__ DonatedOut setup_donated(const SearchParams& p, LevelSM*
     S.incl[0] = dn; S.base[0] = dlo; S.dsel[0] = (uint8_t)dsel;
     S.jsel[0] = (uint8_t)jsel; S.jel[0] = A->back_el[N.boff + min(jsel, N.nb - 1u)]; S.jv[0] = jv;
   }
-  if (lane == 0) lv[1].v[1] = mv;
+  if (lane == 0) {
+    lv[1].v[1] = mv;
+    if (p.tail && A->tail_at) lv[A->tail_at].burst = p.tail;
+  }
   load_walk_plan(plan_words, A, n, same_mask(p, A), lane);
   out.depth = (int)depth;
   return out;

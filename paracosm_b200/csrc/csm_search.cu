@@ -1328,6 +1328,16 @@ SearchKernel search_kernel(uint32_t& warps, int mode, bool general) {
   return warps == 4 ? search_kernel<4>(mode) : warps == 16 ? search_kernel<16>(mode) : search_kernel<8>(mode);
 }
 
+// Lets a kernel take all of a block's shared memory that its own arrays leave.
+// The limit is the kernel's, for every context of the device: set to a launch's
+// own size, another thread's smaller query would lower it between setting and
+// launch.
+cudaError_t allow_shared(SearchKernel k, uint32_t warps) {
+  constexpr uint32_t kBlock = 227 * 1024;
+  const uint32_t own = warps * (uint32_t)(10 * sizeof(uint4) + 32 * sizeof(uint2) + sizeof(WarpStat)) + 64u;
+  return cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)(kBlock - own));
+}
+
 }  // namespace
 
 // Blocks of the search kernel that can be resident on one SM for walks of
@@ -1338,7 +1348,7 @@ uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode) {
   const SearchKernel k = search_kernel(warps, mode, shape.general);
   const size_t smem = (size_t)shape.warp_bytes * warps;
   int nb = 0;
-  cudaError_t e = cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  cudaError_t e = allow_shared(k, warps);
   if (e == cudaSuccess) e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, k, (int)warps * 32, smem);
   if (e != cudaSuccess) { cudaGetLastError(); return 0; }
   return (uint32_t)nb;
@@ -1346,13 +1356,12 @@ uint32_t search_max_blocks(const SearchShape& shape, uint32_t warps, int mode) {
 
 int search_mode(const SearchParams& p) { return p.enum_buf ? 1 : (p.tail ? 2 : 0); }
 
-// A shape that does not fit is not launched; the caller's cudaGetLastError reports it.
+// A shape that does not fit fails to launch, which the caller's cudaGetLastError reports.
 void launch_search(const SearchParams& p, uint32_t blocks, uint32_t warps, cudaStream_t s, bool prepared) {
   if (p.q && !prepared) k_search_prep<<<1, 1, 0, s>>>(p.q, p.n_tasks, p.task_cap, p.sstat, p.error);
   const SearchKernel k = search_kernel(warps, search_mode(p), search_general(p.g));
   const size_t smem = (size_t)p.warp_bytes * warps;
-  if (cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem) == cudaSuccess)
-    k<<<blocks, warps * 32, smem, s>>>(p);
+  if (allow_shared(k, warps) == cudaSuccess) k<<<blocks, warps * 32, smem, s>>>(p);
 }
 
 __global__ void k_finalize(uint32_t B, ResultArgs a) {
